@@ -80,6 +80,26 @@ def load():
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host module (csrc/host.cpp), loaded once.  Raises RuntimeError when it has not been built."""
+    global _host
+    if _host is None:
+        load()   # the module links against the library
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("mlstm_kernels_b200/_host.so is missing or does not fit this PyTorch: build it with "
+                               f"`python -m mlstm_kernels_b200.build` ({e})") from e
+        from .chunkwise import select_chunk_size
+
+        module.setup(select_chunk_size)
+        _host = module
+    return _host
+
+
 def dtype_code(dt: torch.dtype) -> int:
     try:
         return _DTYPE_CODE[dt]

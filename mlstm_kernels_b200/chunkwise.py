@@ -6,20 +6,18 @@ mlstm_chunkwise__xl_chunk (mlstm_kernels/torch/chunkwise/triton_xl_chunk/fwbw.py
 mlstm_siging_chunkwise__xl_chunk (mlstm_kernels/torch/chunkwise/triton_xl_chunk_siging/fwbw.py:211-269),
 so they can be registered as chunkwise kernels of the reference's mLSTMBackend.
 The Triton tuning keyword arguments are accepted and ignored.
+
+An eager call is handed to the native host module (csrc/host.cpp): argument checks, allocations, the autograd node
+and the launches run without a Python frame in between.  MLSTM_B200_CHECK_STATUS=1 in the environment makes every
+backward synchronise and raise if a bounded wait of the tcgen05 kernels ran out (off by default: the check waits for the
+device).  The *_raw functions below go through the C ABI; the multi-GPU helpers and the traced operators use them.
 """
 
 from __future__ import annotations
 
-import os
-
 import torch
-from torch.amp import custom_bwd, custom_fwd
 
 from . import _lib, _ops
-
-# MLSTM_B200_CHECK_STATUS=1: after every backward, synchronise and raise if a bounded wait of the tcgen05 kernels
-# ran out (their results are then invalid).  Off by default because the check waits for the device.
-_CHECK_STATUS = os.environ.get("MLSTM_B200_CHECK_STATUS", "0") == "1"
 
 
 def _is_pow2(x: int) -> bool:
@@ -220,65 +218,6 @@ def chunkwise_bw_raw(q, k, v, i, f, m_initial, c_states, n_out, dh, dc_last=None
     return dq, dk, dv, di, df, dc0
 
 
-def _make_fwbw(autocast_kernel_dtype: torch.dtype, variant: int):
-    class _mlstm_chunkwise_fwbw(torch.autograd.Function):
-        @staticmethod
-        @custom_fwd(device_type="cuda", cast_inputs=autocast_kernel_dtype)
-        def forward(ctx, q, k, v, i, f, c_initial, n_initial, m_initial, return_last_states, eps, chunk_size, impl,
-                    recompute_states_in_bw):
-            B, NH, S, DHQK = q.shape
-            L = resolve_chunk_size(q, v, chunk_size, impl)
-            out = chunkwise_fw_raw(q, k, v, i, f, c_initial, n_initial, m_initial, chunk_size=L, eps=eps,
-                                   variant=variant, impl=impl, want_last=return_last_states)
-            # The forward's gate vectors (its scratch buffer and m_out) are kept for the backward: 24 B per token.
-            # The per-chunk C states (2 * DHQK * DHHV / L bytes per token on the tcgen05 path) are kept only when
-            # the caller asks for it; otherwise the backward runs the recurrence again, as the reference does
-            # (mlstm_kernels/torch/chunkwise/triton_xl_chunk/fwbw.py:88-115).
-            kept = None if recompute_states_in_bw else out["C_states"]
-            ctx.save_for_backward(q, k, v, i, f, c_initial if recompute_states_in_bw else None, m_initial, kept,
-                                  out["n_out"], out["m_out"], out["workspace"])
-            ctx.cfg = (L, eps, impl, c_initial is not None, n_initial is not None, m_initial is not None,
-                       None if c_initial is None else c_initial.dtype,
-                       None if n_initial is None else n_initial.dtype)
-            ctx.mark_non_differentiable(out["n_out"], out["m_out"])
-            if return_last_states:
-                return out["H"], out["C_last"], out["n_last"], out["m_last"]
-            return out["H"], None, None, None
-
-        @staticmethod
-        @custom_bwd(device_type="cuda")
-        def backward(ctx, dH, dC_last, dN_last, dM_last):
-            q, k, v, i, f, c_initial, m_initial, c_states, n_out, m_out, fw_ws = ctx.saved_tensors
-            L, eps, impl, has_c0, has_n0, has_m0, c0_dtype, n0_dtype = ctx.cfg
-            # c_states is None: the forward did not keep them; the call runs the recurrence again in front of its own
-            # chains of launches
-            dq, dk, dv, di, df, dc0 = chunkwise_bw_raw(
-                q, k, v, i, f, m_initial, c_states, n_out, dH, dC_last, chunk_size=L, eps=eps, variant=variant,
-                impl=impl, want_dc_initial=has_c0, m_out=m_out, fw_workspace=fw_ws, recompute_c_initial=c_initial)
-            B, NH, S, DHQK = q.shape
-            dn0 = torch.zeros((B, NH, DHQK), dtype=n0_dtype, device=q.device) if has_n0 else None
-            dm0 = torch.zeros_like(m_initial) if has_m0 else None
-            if dc0 is not None:
-                dc0 = dc0.to(c0_dtype)
-            if _CHECK_STATUS and _lib.device_status() != 0:
-                raise RuntimeError("mlstm_kernels_b200: a bounded wait of the tcgen05 kernels ran out; results invalid")
-            return (dq, dk, dv, di.to(i.dtype), df.to(f.dtype), dc0, dn0, dm0, None, None, None, None, None)
-
-    return _mlstm_chunkwise_fwbw
-
-
-_FWBW = {}
-
-
-def _get_fwbw(autocast_kernel_dtype: torch.dtype, variant: int):
-    if autocast_kernel_dtype not in (torch.float32, torch.float16, torch.bfloat16):
-        raise ValueError(f"Unsupported kernel dtype {autocast_kernel_dtype}.")
-    key = (autocast_kernel_dtype, variant)
-    if key not in _FWBW:
-        _FWBW[key] = _make_fwbw(autocast_kernel_dtype, variant)
-    return _FWBW[key]
-
-
 def mlstm_chunkwise__b200_xl_chunk(
     q: torch.Tensor,  # (B, NH, S, DHQK)
     k: torch.Tensor,  # (B, NH, S, DHQK)
@@ -316,9 +255,9 @@ def mlstm_chunkwise__b200_xl_chunk(
             q, k, v, i, f, c_initial, n_initial, m_initial, return_last_states, eps, chunk_size, impl,
             bool(recompute_states_in_bw), autocast_kernel_dtype, _lib.EXP)
     else:
-        fn = _get_fwbw(autocast_kernel_dtype, _lib.EXP)
-        h, c_last, n_last, m_last = fn.apply(q, k, v, i, f, c_initial, n_initial, m_initial, return_last_states,
-                                             eps, chunk_size, impl, bool(recompute_states_in_bw))
+        h, c_last, n_last, m_last = _lib.host().chunkwise(
+            q, k, v, i, f, c_initial, n_initial, m_initial, return_last_states, eps, chunk_size, impl,
+            recompute_states_in_bw, autocast_kernel_dtype, _lib.EXP)
     if return_last_states:
         return h, (c_last, n_last, m_last)
     return h
@@ -359,9 +298,9 @@ def mlstm_siging_chunkwise__b200_xl_chunk(
             q, k, v, i, f, c_initial, n_initial, None, return_last_states, eps, chunk_size, impl,
             bool(recompute_states_in_bw), autocast_kernel_dtype, variant)
     else:
-        fn = _get_fwbw(autocast_kernel_dtype, variant)
-        h, c_last, n_last, _ = fn.apply(q, k, v, i, f, c_initial, n_initial, None, return_last_states, eps,
-                                        chunk_size, impl, bool(recompute_states_in_bw))
+        h, c_last, n_last, _ = _lib.host().chunkwise(
+            q, k, v, i, f, c_initial, n_initial, None, return_last_states, eps, chunk_size, impl,
+            recompute_states_in_bw, autocast_kernel_dtype, variant)
     if return_last_states:
         return h, (c_last, n_last)
     return h

@@ -9,6 +9,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include "calls.h"
 #include "common.cuh"
 #include "launch.cuh"
 
@@ -347,114 +348,107 @@ int mlstm_b200_chunkwise_fw(const void* q, const void* k, const void* v, const v
                             float* c_last, float* n_last, float* m_last, void* workspace, size_t workspace_bytes,
                             int B, int NH, int S, int DHQK, int DHHV, int L, int dtype, int gate_dtype, int variant,
                             int impl, float eps, void* stream) {
-  return chunkwise_fw_body(q, k, v, i, f, c_initial, n_initial, m_initial, h, n_out, m_out, c_states, n_states, m_states,
-                           c_last, n_last, m_last, workspace, workspace_bytes, B, NH, S, DHQK, DHHV, L, dtype,
-                           gate_dtype, variant, impl, eps, stream, true);
+  if (!n_out || !m_out) return MLSTM_ERR_NULL;
+  return run_chunkwise_fw(FwCall{q, k, v, i, f, c_initial, n_initial, m_initial, h, n_out, m_out, c_states, n_states,
+                                 m_states, c_last, n_last, m_last, nullptr, workspace, workspace_bytes, true},
+                          CallDims{B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream});
 }
 
 }  // extern "C"
 
 namespace mlstm {
-int chunkwise_fw_body(const void* q, const void* k, const void* v, const void* i, const void* f,
-                      const float* c_initial, const float* n_initial, const float* m_initial, void* h,
-                      float* n_out, float* m_out, void* c_states, float* n_states, float* m_states,
-                      float* c_last, float* n_last, float* m_last, void* workspace, size_t workspace_bytes,
-                      int B, int NH, int S, int DHQK, int DHHV, int L, int dtype, int gate_dtype, int variant,
-                      int impl, float eps, void* stream, bool allow_split) {
-  int rc = check_dims(B, NH, S, DHQK, DHHV, L);
+
+static int check_call(const CallDims& c) {
+  if (int rc = check_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L)) return rc;
+  if (c.dtype != MLSTM_F32 && c.dtype != MLSTM_BF16 && c.dtype != MLSTM_F16) return MLSTM_ERR_DTYPE;
+  if (c.gate_dtype != MLSTM_F32 && c.gate_dtype != MLSTM_BF16 && c.gate_dtype != MLSTM_F16) return MLSTM_ERR_DTYPE;
+  if (c.variant < MLSTM_EXP || c.variant > MLSTM_SIG_NONORM) return MLSTM_ERR_UNSUPPORTED;
+  return MLSTM_OK;
+}
+
+int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
+  int rc = check_call(c);
   if (rc != MLSTM_OK) return rc;
-  if (dtype != MLSTM_F32 && dtype != MLSTM_BF16 && dtype != MLSTM_F16) return MLSTM_ERR_DTYPE;
-  if (gate_dtype != MLSTM_F32 && gate_dtype != MLSTM_BF16 && gate_dtype != MLSTM_F16) return MLSTM_ERR_DTYPE;
-  if (variant < MLSTM_EXP || variant > MLSTM_SIG_NONORM) return MLSTM_ERR_UNSUPPORTED;
-  if (!q || !k || !v || !i || !f || !h || !n_out || !m_out || !c_states || !n_states || !m_states || !workspace)
+  if (!a.q || !a.k || !a.v || !a.i || !a.f || !a.h || !a.c_states || !a.n_states || !a.m_states || !a.workspace)
     return MLSTM_ERR_NULL;
-  const void* ptrs[] = {q, k, v, i, f, c_initial, n_initial, m_initial, h, n_out, m_out, c_states, n_states, m_states,
-                        c_last, n_last, m_last, workspace};
+  const void* ptrs[] = {a.q, a.k, a.v, a.i, a.f, a.c_initial, a.n_initial, a.m_initial, a.h, a.n_out, a.m_out,
+                        a.c_states, a.n_states, a.m_states, a.c_last, a.n_last, a.m_last, a.inv_den, a.workspace};
   for (const void* p : ptrs) if (p && !aligned16(p)) return MLSTM_ERR_ALIGN;
   bool use_sm100 = false;
-  if ((rc = resolve_impl(impl, B, NH, S, DHQK, DHHV, L, dtype, &use_sm100)) != MLSTM_OK) return rc;
+  if ((rc = resolve_impl(c.impl, c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, &use_sm100)) != MLSTM_OK) return rc;
 
-  const ChunkwiseDims d = make_dims(B, NH, S, DHQK, DHHV, L, variant, eps, dtype);
-  FwLayout lay = carve_fw(workspace, B * NH, d.SP, d.NC);
-  if (workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const ChunkwiseDims d = make_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.variant, c.eps, c.dtype);
+  FwLayout lay = carve_fw(a.workspace, c.B * c.NH, d.SP, d.NC);
+  if (a.workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
+  cudaStream_t st = static_cast<cudaStream_t>(c.stream);
 
-  if ((rc = launch_gates(gate_dtype, i, f, variant == MLSTM_EXP ? m_initial : nullptr, nullptr, m_out, lay.gb, m_states, d, st)) != MLSTM_OK) return rc;
+  if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, nullptr, a.m_out, lay.gb, a.m_states, d, st)) != MLSTM_OK) return rc;
+  lay.gb.inv_den = a.inv_den;   // written by the intra-chunk kernel
   if (use_sm100) {
-    UnitChains ch(d, st, allow_split);
+    UnitChains ch(d, st, a.allow_split);
     if ((rc = ch.status()) != MLSTM_OK) return rc;
-    if ((rc = sm100_recurrent_fw(k, v, lay.gb, c_initial, n_initial, c_states, n_states, c_last, n_last, d, st, ch.first())) != MLSTM_OK) return rc;
-    if (ch.split() && (rc = sm100_recurrent_fw(k, v, lay.gb, c_initial, n_initial, c_states, n_states, c_last, n_last, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
-    if ((rc = sm100_parallel_fw(q, k, v, lay.gb, c_states, n_states, h, n_out, d, st, ch.first())) != MLSTM_OK) return rc;
-    if (ch.split() && (rc = sm100_parallel_fw(q, k, v, lay.gb, c_states, n_states, h, n_out, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
+    if ((rc = sm100_recurrent_fw(a.k, a.v, lay.gb, a.c_initial, a.n_initial, a.c_states, a.n_states, a.c_last, a.n_last, d, st, ch.first())) != MLSTM_OK) return rc;
+    if (ch.split() && (rc = sm100_recurrent_fw(a.k, a.v, lay.gb, a.c_initial, a.n_initial, a.c_states, a.n_states, a.c_last, a.n_last, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
+    if ((rc = sm100_parallel_fw(a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, d, st, ch.first())) != MLSTM_OK) return rc;
+    if (ch.split() && (rc = sm100_parallel_fw(a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
     if ((rc = ch.join()) != MLSTM_OK) return rc;
   } else {
-    if ((rc = simt_recurrent_fw(dtype, MLSTM_F32, k, v, lay.gb, c_initial, n_initial, c_states, n_states, c_last, n_last, d, st)) != MLSTM_OK) return rc;
-    if ((rc = simt_parallel_fw(dtype, MLSTM_F32, q, k, v, lay.gb, c_states, n_states, h, n_out, d, st)) != MLSTM_OK) return rc;
+    if ((rc = simt_recurrent_fw(c.dtype, MLSTM_F32, a.k, a.v, lay.gb, a.c_initial, a.n_initial, a.c_states, a.n_states, a.c_last, a.n_last, d, st)) != MLSTM_OK) return rc;
+    if ((rc = simt_parallel_fw(c.dtype, MLSTM_F32, a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, d, st)) != MLSTM_OK) return rc;
   }
-  if (m_last) {
-    MLSTM_CUDA_CHECK(cudaMemcpy2DAsync(m_last, sizeof(float), m_states + d.NC, sizeof(float) * (d.NC + 1),
-                                       sizeof(float), (size_t)B * NH, cudaMemcpyDeviceToDevice, st));
+  if (a.m_last) {
+    MLSTM_CUDA_CHECK(cudaMemcpy2DAsync(a.m_last, sizeof(float), a.m_states + d.NC, sizeof(float) * (d.NC + 1),
+                                       sizeof(float), (size_t)c.B * c.NH, cudaMemcpyDeviceToDevice, st));
   }
   return MLSTM_OK;
 }
-}  // namespace mlstm
 
-// Backward body.  With `fw_workspace` (the scratch buffer the forward call of the same problem left behind, still
-// intact) and `m_out` the gate pre-pass is not run again: its vectors are read from that buffer.
-static int bw_impl(const void* q, const void* k, const void* v, const void* i, const void* f,
-                   const float* m_initial, const void* c_states, const float* n_out, const void* dh,
-                   const float* dc_last, void* dq, void* dk, void* dv, float* di, float* df,
-                   float* dc_initial, void* workspace, size_t workspace_bytes, int B, int NH, int S, int DHQK,
-                   int DHHV, int L, int dtype, int gate_dtype, int variant, int impl, float eps, void* stream,
-                   const void* fw_workspace, size_t fw_workspace_bytes, const float* m_out,
-                   void* recompute_into = nullptr, const float* recompute_c_initial = nullptr) {
-  int rc = check_dims(B, NH, S, DHQK, DHHV, L);
+// Backward.  With `fw_workspace` (the scratch buffer the forward call of the same problem left behind, still intact)
+// the gate pre-pass is not run again: its vectors are read from that buffer.
+int run_chunkwise_bw(const BwCall& a, const CallDims& c) {
+  int rc = check_call(c);
   if (rc != MLSTM_OK) return rc;
-  if (dtype != MLSTM_F32 && dtype != MLSTM_BF16 && dtype != MLSTM_F16) return MLSTM_ERR_DTYPE;
-  if (gate_dtype != MLSTM_F32 && gate_dtype != MLSTM_BF16 && gate_dtype != MLSTM_F16) return MLSTM_ERR_DTYPE;
-  if (variant < MLSTM_EXP || variant > MLSTM_SIG_NONORM) return MLSTM_ERR_UNSUPPORTED;
-  if (!q || !k || !v || !i || !f || !c_states || !dh || !dq || !dk || !dv || !di || !df || !workspace)
+  // recompute_into: the per-chunk states are not there yet; the forward's recurrence is run again in front of each
+  // chain of backward launches.  Needs the forward's gate vectors (fw_workspace).
+  const void* c_states = a.recompute_into ? a.recompute_into : a.c_states;
+  if (!a.q || !a.k || !a.v || !a.i || !a.f || !c_states || !a.dh || !a.dq || !a.dk || !a.dv || !a.di || !a.df || !a.workspace)
     return MLSTM_ERR_NULL;
-  if (variant != MLSTM_SIG_NONORM && !n_out) return MLSTM_ERR_NULL;
-  const void* ptrs[] = {q, k, v, i, f, m_initial, c_states, n_out, dh, dc_last, dq, dk, dv, di, df, dc_initial, workspace,
-                        recompute_c_initial};
+  if (c.variant != MLSTM_SIG_NONORM && !a.n_out && !a.inv_den) return MLSTM_ERR_NULL;
+  if ((a.recompute_into || a.inv_den) && !a.fw_workspace) return MLSTM_ERR_NULL;
+  const void* ptrs[] = {a.q, a.k, a.v, a.i, a.f, a.m_initial, c_states, a.n_out, a.inv_den, a.dh, a.dc_last, a.dq, a.dk,
+                        a.dv, a.di, a.df, a.dc_initial, a.workspace, a.fw_workspace, a.recompute_c_initial};
   for (const void* p : ptrs) if (p && !aligned16(p)) return MLSTM_ERR_ALIGN;
-  // recompute_into (== c_states, writable): the per-chunk states are not there yet; the forward's recurrence is run
-  // again in front of each chain of backward launches.  Needs the forward's gate vectors (fw_workspace).
-  if (recompute_into != nullptr && fw_workspace == nullptr) return MLSTM_ERR_NULL;
   bool use_sm100 = false;
-  if ((rc = resolve_impl(impl, B, NH, S, DHQK, DHHV, L, dtype, &use_sm100)) != MLSTM_OK) return rc;
+  if ((rc = resolve_impl(c.impl, c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, &use_sm100)) != MLSTM_OK) return rc;
 
-  const ChunkwiseDims d = make_dims(B, NH, S, DHQK, DHHV, L, variant, eps, dtype);
-  const int sdt = use_sm100 ? dtype : MLSTM_F32;
-  BwLayout lay = carve_bw(workspace, B * NH, d.SP, d.NC, DHQK, DHHV, dtype_size(sdt));
-  if (workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const ChunkwiseDims d = make_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.variant, c.eps, c.dtype);
+  const int sdt = use_sm100 ? c.dtype : MLSTM_F32;
+  BwLayout lay = carve_bw(a.workspace, c.B * c.NH, d.SP, d.NC, c.DHQK, c.DHHV, dtype_size(sdt));
+  if (a.workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
+  cudaStream_t st = static_cast<cudaStream_t>(c.stream);
 
-  if (fw_workspace != nullptr) {
-    if (!aligned16(fw_workspace)) return MLSTM_ERR_ALIGN;
-    FwLayout fl = carve_fw(const_cast<void*>(fw_workspace), B * NH, d.SP, d.NC);
-    if (fw_workspace_bytes < fl.bytes) return MLSTM_ERR_WORKSPACE;
+  if (a.fw_workspace != nullptr) {
+    FwLayout fl = carve_fw(const_cast<void*>(a.fw_workspace), c.B * c.NH, d.SP, d.NC);
+    if (a.fw_workspace_bytes < fl.bytes) return MLSTM_ERR_WORKSPACE;
     float* inv_den = lay.gb.inv_den;
     lay.gb = fl.gb;
-    lay.gb.inv_den = inv_den;
-    if ((rc = launch_inv_den(n_out, inv_den, d, st)) != MLSTM_OK) return rc;
+    lay.gb.inv_den = a.inv_den ? const_cast<float*>(a.inv_den) : inv_den;
+    if (!a.inv_den && (rc = launch_inv_den(a.n_out, inv_den, d, st)) != MLSTM_OK) return rc;
   } else {
-    if ((rc = launch_gates(gate_dtype, i, f, variant == MLSTM_EXP ? m_initial : nullptr, n_out, nullptr, lay.gb, lay.m_states, d, st)) != MLSTM_OK) return rc;
+    if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, a.n_out, nullptr, lay.gb, lay.m_states, d, st)) != MLSTM_OK) return rc;
   }
   if (use_sm100) {
     {
       UnitChains ch(d, st, true);
       if ((rc = ch.status()) != MLSTM_OK) return rc;
-      if (recompute_into) {
-        if ((rc = sm100_recurrent_fw(k, v, lay.gb, recompute_c_initial, nullptr, recompute_into, nullptr, nullptr, nullptr, d, st, ch.first())) != MLSTM_OK) return rc;
-        if (ch.split() && (rc = sm100_recurrent_fw(k, v, lay.gb, recompute_c_initial, nullptr, recompute_into, nullptr, nullptr, nullptr, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
+      if (a.recompute_into) {
+        if ((rc = sm100_recurrent_fw(a.k, a.v, lay.gb, a.recompute_c_initial, nullptr, a.recompute_into, nullptr, nullptr, nullptr, d, st, ch.first())) != MLSTM_OK) return rc;
+        if (ch.split() && (rc = sm100_recurrent_fw(a.k, a.v, lay.gb, a.recompute_c_initial, nullptr, a.recompute_into, nullptr, nullptr, nullptr, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
       }
-      if ((rc = sm100_recurrent_bw(q, dh, lay.gb, dc_last, lay.dc_states, dc_initial, d, st, ch.first())) != MLSTM_OK) return rc;
-      if (ch.split() && (rc = sm100_recurrent_bw(q, dh, lay.gb, dc_last, lay.dc_states, dc_initial, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
-      if ((rc = sm100_parallel_bw(q, k, v, dh, lay.gb, c_states, lay.dc_states, dq, dk, dv, lay.acc, lay.kdk, d, st, ch.first())) != MLSTM_OK) return rc;
-      if (ch.split() && (rc = sm100_parallel_bw(q, k, v, dh, lay.gb, c_states, lay.dc_states, dq, dk, dv, lay.acc, lay.kdk, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
+      if ((rc = sm100_recurrent_bw(a.q, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, d, st, ch.first())) != MLSTM_OK) return rc;
+      if (ch.split() && (rc = sm100_recurrent_bw(a.q, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
+      if ((rc = sm100_parallel_bw(a.q, a.k, a.v, a.dh, lay.gb, c_states, lay.dc_states, a.dq, a.dk, a.dv, lay.acc, lay.kdk, d, st, ch.first())) != MLSTM_OK) return rc;
+      if (ch.split() && (rc = sm100_parallel_bw(a.q, a.k, a.v, a.dh, lay.gb, c_states, lay.dc_states, a.dq, a.dk, a.dv, lay.acc, lay.kdk, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
       if ((rc = ch.join()) != MLSTM_OK) return rc;
     }
     {
@@ -463,18 +457,20 @@ static int bw_impl(const void* q, const void* k, const void* v, const void* i, c
       // (sequences of up to kAnchorEvery chunks have no interior anchor: nothing to compute)
       if (n_anchors > 2 &&
           (rc = launch_state_dot(c_states, lay.dc_states, lay.anchors, kAnchorEvery, n_anchors, d, st)) != MLSTM_OK) return rc;
-      if ((rc = launch_gate_grad_scan(gate_dtype, i, f, lay.acc, lay.kdk, (DHQK + 127) / 128, di, df, d, st, lay.anchors,
-                                      n_anchors, kAnchorEvery * L)) != MLSTM_OK) return rc;
+      if ((rc = launch_gate_grad_scan(c.gate_dtype, a.i, a.f, lay.acc, lay.kdk, (c.DHQK + 127) / 128, a.di, a.df, a.grad_gate_dtype, d, st,
+                                      lay.anchors, n_anchors, kAnchorEvery * c.L)) != MLSTM_OK) return rc;
     }
   } else {
-    if (recompute_into &&
-        (rc = simt_recurrent_fw(dtype, MLSTM_F32, k, v, lay.gb, recompute_c_initial, nullptr, recompute_into, nullptr, nullptr, nullptr, d, st)) != MLSTM_OK) return rc;
-    if ((rc = simt_recurrent_bw(dtype, sdt, q, dh, lay.gb, dc_last, lay.dc_states, dc_initial, d, st)) != MLSTM_OK) return rc;
-    if ((rc = simt_parallel_bw(dtype, sdt, q, k, v, dh, lay.gb, c_states, lay.dc_states, dq, dk, dv, d, st)) != MLSTM_OK) return rc;
-    if ((rc = launch_gate_grads(dtype, gate_dtype, q, k, dq, dk, i, f, lay.acc, lay.kdk, di, df, d, st)) != MLSTM_OK) return rc;
+    if (a.recompute_into &&
+        (rc = simt_recurrent_fw(c.dtype, MLSTM_F32, a.k, a.v, lay.gb, a.recompute_c_initial, nullptr, a.recompute_into, nullptr, nullptr, nullptr, d, st)) != MLSTM_OK) return rc;
+    if ((rc = simt_recurrent_bw(c.dtype, sdt, a.q, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, d, st)) != MLSTM_OK) return rc;
+    if ((rc = simt_parallel_bw(c.dtype, sdt, a.q, a.k, a.v, a.dh, lay.gb, c_states, lay.dc_states, a.dq, a.dk, a.dv, d, st)) != MLSTM_OK) return rc;
+    if ((rc = launch_gate_grads(c.dtype, c.gate_dtype, a.q, a.k, a.dq, a.dk, a.i, a.f, lay.acc, lay.kdk, a.di, a.df, a.grad_gate_dtype, d, st)) != MLSTM_OK) return rc;
   }
   return MLSTM_OK;
 }
+
+}  // namespace mlstm
 
 extern "C" {
 
@@ -483,9 +479,9 @@ int mlstm_b200_chunkwise_bw(const void* q, const void* k, const void* v, const v
                             const float* dc_last, void* dq, void* dk, void* dv, float* di, float* df,
                             float* dc_initial, void* workspace, size_t workspace_bytes, int B, int NH, int S, int DHQK,
                             int DHHV, int L, int dtype, int gate_dtype, int variant, int impl, float eps, void* stream) {
-  return bw_impl(q, k, v, i, f, m_initial, c_states, n_out, dh, dc_last, dq, dk, dv, di, df, dc_initial, workspace,
-                 workspace_bytes, B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream, nullptr, 0,
-                 nullptr);
+  return run_chunkwise_bw(BwCall{q, k, v, i, f, m_initial, c_states, nullptr, nullptr, n_out, nullptr, nullptr, 0, dh,
+                                 dc_last, dq, dk, dv, di, df, MLSTM_F32, dc_initial, workspace, workspace_bytes},
+                          CallDims{B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream});
 }
 
 int mlstm_b200_chunkwise_bw_cached(const void* q, const void* k, const void* v, const void* i, const void* f,
@@ -495,10 +491,12 @@ int mlstm_b200_chunkwise_bw_cached(const void* q, const void* k, const void* v, 
                                    float* df, float* dc_initial, void* workspace, size_t workspace_bytes, int B,
                                    int NH, int S, int DHQK, int DHHV, int L, int dtype, int gate_dtype, int variant,
                                    int impl, float eps, void* stream) {
+  (void)m_out;
   if (!fw_workspace) return MLSTM_ERR_NULL;
-  return bw_impl(q, k, v, i, f, m_initial, c_states, n_out, dh, dc_last, dq, dk, dv, di, df, dc_initial, workspace,
-                 workspace_bytes, B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream, fw_workspace,
-                 fw_workspace_bytes, m_out);
+  return run_chunkwise_bw(BwCall{q, k, v, i, f, m_initial, c_states, nullptr, nullptr, n_out, nullptr, fw_workspace,
+                                 fw_workspace_bytes, dh, dc_last, dq, dk, dv, di, df, MLSTM_F32, dc_initial, workspace,
+                                 workspace_bytes},
+                          CallDims{B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream});
 }
 
 int mlstm_b200_chunkwise_bw_recompute(const void* q, const void* k, const void* v, const void* i, const void* f,
@@ -508,10 +506,12 @@ int mlstm_b200_chunkwise_bw_recompute(const void* q, const void* k, const void* 
                                       void* dk, void* dv, float* di, float* df, float* dc_initial, void* workspace,
                                       size_t workspace_bytes, int B, int NH, int S, int DHQK, int DHHV, int L,
                                       int dtype, int gate_dtype, int variant, int impl, float eps, void* stream) {
+  (void)m_out;
   if (!fw_workspace || !c_states_scratch) return MLSTM_ERR_NULL;
-  return bw_impl(q, k, v, i, f, m_initial, c_states_scratch, n_out, dh, dc_last, dq, dk, dv, di, df, dc_initial,
-                 workspace, workspace_bytes, B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream,
-                 fw_workspace, fw_workspace_bytes, m_out, c_states_scratch, c_initial);
+  return run_chunkwise_bw(BwCall{q, k, v, i, f, m_initial, nullptr, c_states_scratch, c_initial, n_out, nullptr,
+                                 fw_workspace, fw_workspace_bytes, dh, dc_last, dq, dk, dv, di, df, MLSTM_F32,
+                                 dc_initial, workspace, workspace_bytes},
+                          CallDims{B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream});
 }
 
 int mlstm_b200_chunkwise_states(const void* k, const void* v, const void* i, const void* f, const float* c_initial,

@@ -141,7 +141,8 @@ struct ParArgs {
   const TS* dc_states;  // slot k+1 used by DV and DK
   const float* n_states;
   void* out;     // T*
-  float* n_out;  // H only
+  float* n_out;       // H only, may be null
+  float* inv_den_out; // H only, may be null
   int S, L, NC, DHQK, DHHV, variant;
   float eps, qk_scale;
 };
@@ -328,7 +329,8 @@ __global__ void __launch_bounds__(NTHR) par_kernel(ParArgs<T, TS> p) {
       const float nn = rowsum + p.qk_scale * p.bbar[tok0 + r] * qn;
       if (p.variant == MLSTM_EXP) den = fmaxf(fabsf(nn), expf(-s_m[r]));
       else if (p.variant == MLSTM_SIG) den = fmaxf(fabsf(nn), 1.f);
-      if (ot == 0) p.n_out[tok0 + r] = den;
+      if (ot == 0 && p.n_out) p.n_out[tok0 + r] = den;
+      if (ot == 0 && p.inv_den_out) p.inv_den_out[tok0 + r] = p.variant == MLSTM_SIG_NONORM ? 1.f : 1.f / (den + p.eps);
     }
     s_row[tid] = den;
   }
@@ -400,7 +402,7 @@ ParArgs<T, TS> make_args(const void* q, const void* k, const void* v, const void
   a.q = (const T*)q; a.k = (const T*)k; a.v = (const T*)v; a.dh = (const T*)dh;
   a.vecB = gb.vecB; a.iota = gb.iota; a.m_tok = gb.m_tok; a.abar = gb.abar; a.bbar = gb.bbar; a.inv_den = gb.inv_den;
   a.c_states = (const TS*)c_states; a.dc_states = (const TS*)dc_states; a.n_states = n_states;
-  a.out = nullptr; a.n_out = nullptr;
+  a.out = nullptr; a.n_out = nullptr; a.inv_den_out = nullptr;
   a.S = d.S; a.L = d.L; a.NC = d.NC; a.DHQK = d.DHQK; a.DHHV = d.DHHV; a.variant = d.variant;
   a.eps = d.eps; a.qk_scale = d.qk_scale;
   return a;
@@ -410,7 +412,7 @@ template <typename T, typename TS>
 int par_fw_t(const void* q, const void* k, const void* v, const GateBuffers& gb, const void* c_states,
              const float* n_states, void* h, float* n_out, const ChunkwiseDims& d, cudaStream_t st) {
   auto a = make_args<T, TS>(q, k, v, nullptr, gb, c_states, nullptr, n_states, d);
-  a.out = h; a.n_out = n_out;
+  a.out = h; a.n_out = n_out; a.inv_den_out = gb.inv_den;
   PhaseScope ps(PH_PAR_FW, st);
   return par_launch<T, TS, PAR_H>(a, d, st);
 }

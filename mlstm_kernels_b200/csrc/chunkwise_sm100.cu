@@ -359,7 +359,8 @@ struct ParParams {
   const float *vecB, *iota, *m_tok, *abar, *bbar, *inv_den;  // per token, f32
   const float* n_states;                                     // H only
   uint16_t *out_h, *out_dv, *out_dk, *out_dq;   // 16-bit elements of the input type
-  float* n_out;               // H only
+  float* n_out;               // H only: denominator per token, or nullptr
+  float* inv_den_out;         // H only: 1 / (denominator + eps) per slot (0 past the sequence end), or nullptr
   float *rowdot_q, *rowdot_k; // sum_d q dq (from DQ), sum_d k dk (from DK); one partial per output tile: [DHQK/128][tokens]
   size_t nslots;              // B * NH * SP
   int S, SP, NC, DHQK, DHHV, variant;   // SP = NC * 128: slots per (batch, head) of the per-token gate vectors
@@ -739,7 +740,10 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         if (p.variant == MLSTM_EXP) den = fmaxf(fabsf(nn), __expf(-m_r));
         else if (p.variant == MLSTM_SIG) den = fmaxf(fabsf(nn), 1.f);
         if (p.variant != MLSTM_SIG_NONORM) inv = 1.f / (den + p.eps);
-        if (o_tile0 == 0 && half == 0 && r < valid) p.n_out[out_row0 + r] = den;
+        if (o_tile0 == 0 && half == 0) {
+          if (p.n_out != nullptr && r < valid) p.n_out[out_row0 + r] = den;
+          if (p.inv_den_out != nullptr) p.inv_den_out[tok] = r < valid ? inv : 0.f;
+        }
       }
       const int ldx = (sub == 0 ? 2 * ND : n0 + (sub - 1) * n1 + ND);    // ring index of this tile's X load; E follows it
       const uint8_t* erow = smem;
@@ -1027,7 +1031,7 @@ int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuf
       !state_map(&mC, c_states, d, 64))
     return MLSTM_ERR_CUDA;
   ParParams pp = base_params(gb, d);
-  pp.n_states = n_states; pp.out_h = (uint16_t*)h; pp.n_out = n_out;
+  pp.n_states = n_states; pp.out_h = (uint16_t*)h; pp.n_out = n_out; pp.inv_den_out = gb.inv_den;
   pp.bh0 = ur.first;
   const bool f16 = d.dtype == MLSTM_F16;
   static bool attr_done[2][64] = {};

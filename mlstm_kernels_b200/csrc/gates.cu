@@ -208,12 +208,19 @@ gate_grad_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
 // `anchor_tokens`-th token position (state_dot_kernel); the running sum of a token is then taken from the next anchor
 // instead of from the end of the sequence, which bounds the walk to one anchor interval (gate_grad_anchored_kernel).
 // gate_grad_scan_kernel is the plain form (portable path: f32 states, no anchors).
+// The gate gradients leave in the element type the caller asked for (f32, or that of the gate logits).
+__device__ __forceinline__ void store_gate_grad(void* p, size_t idx, float x, int dtype) {
+  if (dtype == MLSTM_F32) static_cast<float*>(p)[idx] = x;
+  else if (dtype == MLSTM_BF16) static_cast<__nv_bfloat16*>(p)[idx] = __float2bfloat16_rn(x);
+  else static_cast<__half*>(p)[idx] = __float2half_rn(x);
+}
+
 constexpr int kScanThreads = 1024;
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads)
 gate_grad_scan_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, const float* __restrict__ qdq,
-                      const float* __restrict__ kdk, float* __restrict__ dI, float* __restrict__ dF,
-                      int S, int SP, int variant, int nparts, size_t part_stride) {
+                      const float* __restrict__ kdk, void* __restrict__ dI, void* __restrict__ dF,
+                      int out_dtype, int S, int SP, int variant, int nparts, size_t part_stride) {
   __shared__ float s_part[kScanThreads];
   const int bh = blockIdx.x, t = threadIdx.x;
   const size_t base = (size_t)bh * S;      // gate logits and outputs: S tokens per (batch, head)
@@ -240,9 +247,9 @@ gate_grad_scan_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, co
   for (int s = s1 - 1; s >= s0; --s) {
     float di = parts(kdk, pbase + s);
     run += parts(qdq, pbase + s) - di;
-    dF[base + s] = run * sigmoid_f(-to_f32(vecF[base + s]));
+    store_gate_grad(dF, base + s, run * sigmoid_f(-to_f32(vecF[base + s])), out_dtype);
     if (variant != MLSTM_EXP) di *= sigmoid_f(-to_f32(vecI[base + s]));
-    dI[base + s] = di;
+    store_gate_grad(dI, base + s, di, out_dtype);
   }
 }
 
@@ -255,8 +262,8 @@ constexpr int kAnchorThreads = 512;
 template <typename T>
 __global__ void __launch_bounds__(kAnchorThreads)
 gate_grad_anchored_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, const float* __restrict__ qdq,
-                          const float* __restrict__ kdk, float* __restrict__ dI, float* __restrict__ dF, int S,
-                          int SP, int variant, int nparts, size_t part_stride,
+                          const float* __restrict__ kdk, void* __restrict__ dI, void* __restrict__ dF,
+                          int out_dtype, int S, int SP, int variant, int nparts, size_t part_stride,
                           const float* __restrict__ anchors, int n_anchors) {
   __shared__ float s_warp[kAnchorThreads / 32];
   const int nint = (S + kAnchorThreads - 1) / kAnchorThreads;   // 1-D grid: intervals of one (batch, head) adjacent
@@ -286,8 +293,8 @@ gate_grad_anchored_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF
   }
   if (live) {
     const size_t o = (size_t)bh * S + s;
-    dF[o] = total * sigmoid_f(-to_f32(vecF[o]));
-    dI[o] = (variant != MLSTM_EXP) ? kd * sigmoid_f(-to_f32(vecI[o])) : kd;
+    store_gate_grad(dF, o, total * sigmoid_f(-to_f32(vecF[o])), out_dtype);
+    store_gate_grad(dI, o, (variant != MLSTM_EXP) ? kd * sigmoid_f(-to_f32(vecI[o])) : kd, out_dtype);
   }
 }
 
@@ -375,7 +382,7 @@ int launch_gate_grad_rows_t(const void* q, const void* k, const void* dq, const 
 
 
 int launch_gate_grads(int dtype, int gate_dtype, const void* q, const void* k, const void* dq, const void* dk,
-                      const void* i, const void* f, float* acc, float* kdk, float* dI, float* dF,
+                      const void* i, const void* f, float* acc, float* kdk, void* dI, void* dF, int out_dtype,
                       const ChunkwiseDims& d, cudaStream_t st) {
   PhaseScope ps(PH_GATE_GRADS, st);
   int rc = MLSTM_ERR_DTYPE;
@@ -385,7 +392,7 @@ int launch_gate_grads(int dtype, int gate_dtype, const void* q, const void* k, c
     case MLSTM_F16: rc = launch_gate_grad_rows_t<__half>(q, k, dq, dk, acc, kdk, d, st); break;
   }
   if (rc != MLSTM_OK) return rc;
-  return launch_gate_grad_scan(gate_dtype, i, f, acc, kdk, 1, dI, dF, d, st, nullptr, 0, 1);
+  return launch_gate_grad_scan(gate_dtype, i, f, acc, kdk, 1, dI, dF, out_dtype, d, st, nullptr, 0, 1);
 }
 
 // Joins the state a sequence segment produced from the EMPTY state (C = 0, n = 0, m = -inf) onto the state that
@@ -457,16 +464,16 @@ int launch_inv_den(const float* n_out, float* inv_den, const ChunkwiseDims& d, c
 // With `anchors` (see above) the sum restarts from an exact value every `anchor_tokens` tokens and the intervals run
 // as independent CTAs; without, one CTA per (batch, head) scans the whole sequence.
 template <typename T>
-static int gate_grad_scan_t(const void* i, const void* f, const float* qdq, const float* kdk, int nparts, float* dI,
-                            float* dF, const ChunkwiseDims& d, cudaStream_t st, const float* anchors, int n_anchors,
+static int gate_grad_scan_t(const void* i, const void* f, const float* qdq, const float* kdk, int nparts, void* dI,
+                            void* dF, int out_dtype, const ChunkwiseDims& d, cudaStream_t st, const float* anchors, int n_anchors,
                             int anchor_tokens) {
   const size_t stride = (size_t)d.B * d.NH * d.SP;
   if (anchors != nullptr && anchor_tokens == kAnchorThreads) {
     const unsigned grid = (unsigned)ceil_div(d.S, kAnchorThreads) * (unsigned)(d.B * d.NH);
-    gate_grad_anchored_kernel<T><<<grid, kAnchorThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, d.S, d.SP,
+    gate_grad_anchored_kernel<T><<<grid, kAnchorThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, out_dtype, d.S, d.SP,
                                                                   d.variant, nparts, stride, anchors, n_anchors);
   } else {
-    gate_grad_scan_kernel<T><<<d.B * d.NH, kScanThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, d.S, d.SP,
+    gate_grad_scan_kernel<T><<<d.B * d.NH, kScanThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, out_dtype, d.S, d.SP,
                                                                   d.variant, nparts, stride);
   }
   MLSTM_LAUNCH_CHECK();
@@ -474,12 +481,12 @@ static int gate_grad_scan_t(const void* i, const void* f, const float* qdq, cons
 }
 
 int launch_gate_grad_scan(int dtype, const void* i, const void* f, const float* qdq, const float* kdk, int nparts,
-                          float* dI, float* dF, const ChunkwiseDims& d, cudaStream_t st, const float* anchors,
+                          void* dI, void* dF, int out_dtype, const ChunkwiseDims& d, cudaStream_t st, const float* anchors,
                           int n_anchors, int anchor_tokens) {
   switch (dtype) {
-    case MLSTM_F32: return gate_grad_scan_t<float>(i, f, qdq, kdk, nparts, dI, dF, d, st, anchors, n_anchors, anchor_tokens);
-    case MLSTM_BF16: return gate_grad_scan_t<__nv_bfloat16>(i, f, qdq, kdk, nparts, dI, dF, d, st, anchors, n_anchors, anchor_tokens);
-    case MLSTM_F16: return gate_grad_scan_t<__half>(i, f, qdq, kdk, nparts, dI, dF, d, st, anchors, n_anchors, anchor_tokens);
+    case MLSTM_F32: return gate_grad_scan_t<float>(i, f, qdq, kdk, nparts, dI, dF, out_dtype, d, st, anchors, n_anchors, anchor_tokens);
+    case MLSTM_BF16: return gate_grad_scan_t<__nv_bfloat16>(i, f, qdq, kdk, nparts, dI, dF, out_dtype, d, st, anchors, n_anchors, anchor_tokens);
+    case MLSTM_F16: return gate_grad_scan_t<__half>(i, f, qdq, kdk, nparts, dI, dF, out_dtype, d, st, anchors, n_anchors, anchor_tokens);
   }
   return MLSTM_ERR_DTYPE;
 }

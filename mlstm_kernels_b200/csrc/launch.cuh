@@ -14,10 +14,10 @@ int launch_state_combine(const float* c_in, const float* n_in, const float* m_in
                          const float* n_loc, const float* m_loc, const float* g_total, float* c_out, float* n_out,
                          float* m_out, int BNH, int DHQK, int DHHV, int variant, cudaStream_t st);
 int launch_gate_grads(int dtype, int gate_dtype, const void* q, const void* k, const void* dq, const void* dk, const void* i,
-                      const void* f, float* acc, float* kdk, float* dI, float* dF, const ChunkwiseDims& d,
+                      const void* f, float* acc, float* kdk, void* dI, void* dF, int out_dtype, const ChunkwiseDims& d,
                       cudaStream_t st);
 int launch_gate_grad_scan(int dtype, const void* i, const void* f, const float* qdq, const float* kdk, int nparts,
-                          float* dI, float* dF, const ChunkwiseDims& d, cudaStream_t st, const float* anchors,
+                          void* dI, void* dF, int out_dtype, const ChunkwiseDims& d, cudaStream_t st, const float* anchors,
                           int n_anchors, int anchor_tokens);
 int launch_state_dot(const void* c_states, const void* dc_states, float* anchors, int every, int n_anchors,
                      const ChunkwiseDims& d, cudaStream_t st);
@@ -56,15 +56,6 @@ int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* d
 // number of CTAs the recurrence launches for the whole problem with 128-column state tiles, and SMs of the device
 long sm100_recurrence_ctas(const ChunkwiseDims& d);
 int sm100_sm_count();
-
-// Forward of mlstm_b200_chunkwise_fw; `allow_split` = false keeps every launch on the caller's stream (no stream or
-// event of the library is created or used).
-int chunkwise_fw_body(const void* q, const void* k, const void* v, const void* i, const void* f,
-                      const float* c_initial, const float* n_initial, const float* m_initial, void* h,
-                      float* n_out, float* m_out, void* c_states, float* n_states, float* m_states,
-                      float* c_last, float* n_last, float* m_last, void* workspace, size_t workspace_bytes,
-                      int B, int NH, int S, int DHQK, int DHHV, int L, int dtype, int gate_dtype, int variant,
-                      int impl, float eps, void* stream, bool allow_split);
 
 int sm100_device_status(int reset, int* status);
 int sm100_wait_expiry_selftest(unsigned limit, int code, cudaStream_t st);

@@ -8,6 +8,7 @@
 // that exists as long as the library is loaded (every GPU that loads the library holds a copy).
 #include <mutex>
 
+#include "calls.h"
 #include "common.cuh"
 #include "launch.cuh"
 
@@ -78,9 +79,11 @@ int mlstm_b200_chunkwise_fw_static(const void* q, const void* k, const void* v, 
   // The forward writes every scratch word before it reads it, so nothing has to be cleared between calls.
   // Single-stream form of the forward: the two-stream split of the regular entry point would create a stream and two
   // events on its first use, which is driver memory this entry point promises not to take.
-  return mlstm::chunkwise_fw_body(q, k, v, i, f, c_initial, n_initial, m_initial, h, n_out, m_out, c_states, n_states,
-                                  m_states, c_last, n_last, m_last, scratch, kStaticScratchBytes, B, NH, S, DHQK, DHHV,
-                                  L, dtype, gate_dtype, variant, impl, eps, stream, false);
+  if (!n_out || !m_out) return MLSTM_ERR_NULL;
+  return mlstm::run_chunkwise_fw(
+      mlstm::FwCall{q, k, v, i, f, c_initial, n_initial, m_initial, h, n_out, m_out, c_states, n_states, m_states, c_last,
+                    n_last, m_last, nullptr, scratch, kStaticScratchBytes, false},
+      mlstm::CallDims{B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream});
 }
 
 }  // extern "C"
