@@ -382,7 +382,7 @@ int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   if (a.workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(c.stream);
 
-  if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, nullptr, a.m_out, lay.gb, a.m_states, d, st)) != MLSTM_OK) return rc;
+  if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, nullptr, a.m_out, lay.gb, a.m_states, a.m_last, d, st)) != MLSTM_OK) return rc;
   lay.gb.inv_den = a.inv_den;   // written by the intra-chunk kernel
   if (use_sm100) {
     UnitChains ch(d, st, a.allow_split);
@@ -395,10 +395,6 @@ int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   } else {
     if ((rc = simt_recurrent_fw(c.dtype, MLSTM_F32, a.k, a.v, lay.gb, a.c_initial, a.n_initial, a.c_states, a.n_states, a.c_last, a.n_last, d, st)) != MLSTM_OK) return rc;
     if ((rc = simt_parallel_fw(c.dtype, MLSTM_F32, a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, d, st)) != MLSTM_OK) return rc;
-  }
-  if (a.m_last) {
-    MLSTM_CUDA_CHECK(cudaMemcpy2DAsync(a.m_last, sizeof(float), a.m_states + d.NC, sizeof(float) * (d.NC + 1),
-                                       sizeof(float), (size_t)c.B * c.NH, cudaMemcpyDeviceToDevice, st));
   }
   return MLSTM_OK;
 }
@@ -435,7 +431,7 @@ int run_chunkwise_bw(const BwCall& a, const CallDims& c) {
     lay.gb.inv_den = a.inv_den ? const_cast<float*>(a.inv_den) : inv_den;
     if (!a.inv_den && (rc = launch_inv_den(a.n_out, inv_den, d, st)) != MLSTM_OK) return rc;
   } else {
-    if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, a.n_out, nullptr, lay.gb, lay.m_states, d, st)) != MLSTM_OK) return rc;
+    if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, a.n_out, nullptr, lay.gb, lay.m_states, nullptr, d, st)) != MLSTM_OK) return rc;
   }
   if (use_sm100) {
     {
@@ -541,7 +537,7 @@ int mlstm_b200_chunkwise_states(const void* k, const void* v, const void* i, con
     SumLayout lay = carve_summary(workspace, B * NH, d.SP, d.NC);
     if (workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
     gb = lay.gb;
-    if ((rc = launch_gates(gate_dtype, i, f, variant == MLSTM_EXP ? m_initial : nullptr, nullptr, nullptr, gb, lay.m_states, d, st)) != MLSTM_OK) return rc;
+    if ((rc = launch_gates(gate_dtype, i, f, variant == MLSTM_EXP ? m_initial : nullptr, nullptr, nullptr, gb, lay.m_states, nullptr, d, st)) != MLSTM_OK) return rc;
   }
   if (use_sm100) return sm100_recurrent_fw(k, v, gb, c_initial, nullptr, c_states, nullptr, nullptr, nullptr, d, st);
   return simt_recurrent_fw(dtype, MLSTM_F32, k, v, gb, c_initial, nullptr, c_states, nullptr, nullptr, nullptr, d, st);
@@ -594,14 +590,12 @@ int mlstm_b200_chunkwise_summary(const void* k, const void* v, const void* i, co
   if (workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // the segment starts from the empty state: C = 0, n = 0, m = -inf
-  if ((rc = launch_gates(gate_dtype, i, f, nullptr, nullptr, nullptr, lay.gb, lay.m_states, d, st, -INFINITY, g_total)) != MLSTM_OK) return rc;
+  if ((rc = launch_gates(gate_dtype, i, f, nullptr, nullptr, nullptr, lay.gb, lay.m_states, m_last, d, st, -INFINITY, g_total)) != MLSTM_OK) return rc;
   if (use_sm100) {
     if ((rc = sm100_recurrent_fw(k, v, lay.gb, nullptr, nullptr, nullptr, nullptr, c_last, n_last, d, st)) != MLSTM_OK) return rc;
   } else {
     if ((rc = simt_recurrent_fw(dtype, MLSTM_F32, k, v, lay.gb, nullptr, nullptr, nullptr, nullptr, c_last, n_last, d, st)) != MLSTM_OK) return rc;
   }
-  MLSTM_CUDA_CHECK(cudaMemcpy2DAsync(m_last, sizeof(float), lay.m_states + d.NC, sizeof(float) * (d.NC + 1),
-                                     sizeof(float), (size_t)B * NH, cudaMemcpyDeviceToDevice, st));
   return MLSTM_OK;
 }
 

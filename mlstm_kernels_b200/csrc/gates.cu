@@ -6,6 +6,8 @@
 // Follows mlstm_kernels/torch/chunkwise/triton_xl_chunk/chunkwise_gates.py:15-65 (vecB, vecA),
 // mlstm_kernels/triton/chunkwise/xl_chunk/fw_kernel_recurrent.py:150-176 (m recursion) and
 // mlstm_kernels/torch/chunkwise/native/fw.py:178-195 (per-token max state).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "common.cuh"
@@ -13,164 +15,187 @@
 
 namespace mlstm {
 
-constexpr int kGateThreads = 256;
+// One launch for the whole pre-pass: a cluster of up to eight CTAs per (batch, head), the chunks of a sequence split
+// contiguously over its CTAs, one warp per chunk at a time.
+//   1. per chunk:   b_j (inclusive sums of log f), a_j = sum_{t>j} log f_t + iota_j, g_k, max_j a_j
+//   2. per cluster: m_{k+1} = max(g_k + m_k, amax_k) as a scan over the maps x -> max(x + G, A): threads compose their
+//                   chunks, warps scan by shuffles, CTAs exchange their totals through distributed shared memory
+//   3. per chunk:   m_i, abar_j, bbar_i, 1/(den+eps)
+// The work is a few loads and transcendentals per token: launch and dependency latency are all there is to save.  As
+// three launches with a serial 256-step combine in the middle it took 15.2 us (8 heads x 4 chunks), 26 us
+// (128 heads x 64 chunks) and 27.6 us (8 heads x 1024 chunks).
+struct GateScan {
+  const float* m_initial;
+  float m_default;       // max state before the first chunk where m_initial is null
+  float* m_states;       // (BNH, NC+1)
+  float* m_last;         // (BNH) or null: copy of the last one
+  float* g_sum;          // (BNH) or null: total log forget gate of the sequence (for chaining segments)
+};
 
-// The pre-pass runs as three launches so that the per-chunk work (1 and 3) spreads over the whole GPU and only
-// the scan over chunks (2) is serial per (batch, head):
-//   gates_chunk_kernel  b_j, a_j, g_k, max_j a_j           one warp per chunk
-//   gates_scan_kernel   m_k, gbar_k, total G               one CTA per (batch, head)
-//   gates_token_kernel  m_i, abar_j, bbar_i, 1/(den+eps)   one warp per chunk
-template <typename T>
-__global__ void __launch_bounds__(kGateThreads)
-gates_chunk_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, GateBuffers gb, int S, int SP, int L,
-                   int NC, int variant) {
-  // 1-D grid (no 65535 limit on batch x heads): the chunk groups of one (batch, head) next to each other
-  const int ngrp = (NC + kGateThreads / 32 - 1) / (kGateThreads / 32);
-  const int bh = blockIdx.x / ngrp;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = (blockIdx.x % ngrp) * (kGateThreads / 32) + warp;
-  if (k >= NC) return;
+// NV: register-held token values per lane, NV * 32 >= L
+template <typename T, int NV>
+__global__ void __launch_bounds__(1024)
+gates_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, const float* __restrict__ n_out,
+             float* __restrict__ m_out, GateBuffers gb, GateScan sc, int S, int SP, int L, int NC, int variant, float eps) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ float s_wG[32], s_wA[32];    // totals of the warps
+  __shared__ float s_total[2];            // total of the CTA, read by the rest of the cluster
+  const int ncta = cluster.num_blocks(), rank = cluster.block_rank(), bh = blockIdx.x / ncta;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  const int per = (NC + ncta - 1) / ncta, c0 = min(NC, rank * per), c1 = min(NC, c0 + per);   // chunks of this CTA
   const bool siging = variant != MLSTM_EXP;
   float* g_arr = gb.scratch + (size_t)bh * 2 * NC;
   float* amax_arr = g_arr + NC;
   // inputs have S tokens per (batch, head), the gate vectors SP = NC * L slots; slots past the sequence end are
   // filled with neutral values: log forget gate 0 (nothing decays), input gate -inf (contributes nothing)
-  const size_t base_in = (size_t)bh * S + (size_t)k * L;
-  const size_t base = (size_t)bh * SP + (size_t)k * L;
-  const int valid = min(L, S - k * L);
-  float carry = 0.f;
-  for (int j0 = 0; j0 < L; j0 += 32) {
-    const int j = j0 + lane;
-    float x = (j < valid) ? logsigmoid_f(to_f32(vecF[base_in + j])) : 0.f;
+  for (int k = c0 + warp; k < c1; k += nwarp) {
+    const size_t base_in = (size_t)bh * S + (size_t)k * L;
+    const size_t base = (size_t)bh * SP + (size_t)k * L;
+    const int valid = min(L, S - k * L);
+    float lf[NV], iota[NV];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      float y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    x += carry;
-    if (j < L) gb.vecB[base + j] = x;
-    carry = __shfl_sync(0xffffffffu, x, 31);
-  }
-  const float g = carry;
-  // a_j = sum_{t>j} lf_t + iota_j as a reverse scan that never includes position j
-  float suffix = 0.f, amax = -INFINITY;
-  for (int j0 = ((L - 1) / 32) * 32; j0 >= 0; j0 -= 32) {
-    const int j = j0 + lane;
-    float x = (j < valid) ? logsigmoid_f(to_f32(vecF[base_in + j])) : 0.f;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      float y = __shfl_down_sync(0xffffffffu, x, o);
-      if (lane + o < 32) x += y;
-    }
-    float excl = __shfl_down_sync(0xffffffffu, x, 1);
-    if (lane == 31) excl = 0.f;
-    excl += suffix;
-    suffix += __shfl_sync(0xffffffffu, x, 0);
-    if (j < L) {
-      float iota = -INFINITY;
+    for (int u = 0; u < NV; ++u) {
+      const int j = u * 32 + lane;
+      lf[u] = 0.f; iota[u] = -INFINITY;
       if (j < valid) {
-        const float iv = to_f32(vecI[base_in + j]);
-        iota = siging ? logsigmoid_f(iv) : iv;
+        lf[u] = to_f32(vecF[base_in + j]);
+        iota[u] = to_f32(vecI[base_in + j]);
       }
-      const float a = excl + iota;
-      gb.iota[base + j] = iota;
-      gb.abar[base + j] = a;  // finalised by gates_token_kernel
-      amax = fmaxf(amax, a);
     }
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      if (u * 32 + lane < valid) {
+        lf[u] = logsigmoid_f(lf[u]);
+        if (siging) iota[u] = logsigmoid_f(iota[u]);
+      }
+    }
+    float carry = 0.f;
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      float x = lf[u];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      x += carry;
+      if (u * 32 + lane < L) gb.vecB[base + u * 32 + lane] = x;
+      carry = __shfl_sync(0xffffffffu, x, 31);
+    }
+    // a_j as a reverse scan that never includes position j
+    float suffix = 0.f, amax = -INFINITY;
+#pragma unroll
+    for (int u = NV - 1; u >= 0; --u) {
+      float x = lf[u];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float y = __shfl_down_sync(0xffffffffu, x, o);
+        if (lane + o < 32) x += y;
+      }
+      float excl = __shfl_down_sync(0xffffffffu, x, 1);
+      if (lane == 31) excl = 0.f;
+      excl += suffix;
+      suffix += __shfl_sync(0xffffffffu, x, 0);
+      if (u * 32 + lane < L) {
+        const float a = excl + iota[u];
+        gb.iota[base + u * 32 + lane] = iota[u];
+        gb.abar[base + u * 32 + lane] = a;  // finalised in step 3
+        amax = fmaxf(amax, a);
+      }
+    }
+    amax = warp_max(amax);
+    if (lane == 0) { g_arr[k] = carry; amax_arr[k] = amax; }
   }
-  amax = warp_max(amax);
-  if (lane == 0) { g_arr[k] = g; amax_arr[k] = amax; }
-}
+  __syncthreads();
 
-// m_{k+1} = max(g_k + m_k, amax_k) as a block scan over the maps x -> max(x + G, A)
-__global__ void __launch_bounds__(kGateThreads)
-gates_scan_kernel(const float* __restrict__ m_initial, GateBuffers gb, float* __restrict__ m_states, int NC,
-                  int variant, float m_default, float* __restrict__ g_sum) {
-  __shared__ float sG[kGateThreads], sA[kGateThreads], sMin[kGateThreads];
-  const int bh = blockIdx.x, t = threadIdx.x;
-  const bool siging = variant != MLSTM_EXP;
-  const float* g_arr = gb.scratch + (size_t)bh * 2 * NC;
-  const float* amax_arr = g_arr + NC;
-  const int seg = (NC + kGateThreads - 1) / kGateThreads;
-  const int k0 = min(NC, t * seg), k1 = min(NC, (t + 1) * seg);
-  float* ms = m_states + (size_t)bh * (NC + 1);
+  // composition of the maps of a thread's chunks, then exclusive scan over the threads of the CTA
+  const int seg = (c1 - c0 + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int k0 = min(c1, c0 + tid * seg), k1 = min(c1, k0 + seg);
   float G = 0.f, A = -INFINITY;
   for (int k = k0; k < k1; ++k) { A = fmaxf(A + g_arr[k], amax_arr[k]); G += g_arr[k]; }
-  sG[t] = G; sA[t] = A;
-  __syncthreads();
-  if (t == 0) {
-    float m = m_initial ? m_initial[bh] : m_default;
-    float Gt = 0.f;
-    for (int u = 0; u < kGateThreads; ++u) { sMin[u] = m; m = fmaxf(m + sG[u], sA[u]); Gt += sG[u]; }
-    if (g_sum != nullptr) g_sum[bh] = Gt;   // total log forget gate of the sequence (for chaining segments)
-  }
-  __syncthreads();
-  if (!siging) {
-    float m = sMin[t];
-    for (int k = k0; k < k1; ++k) {
-      ms[k] = m;
-      const float mn = fmaxf(g_arr[k] + m, amax_arr[k]);
-      gb.gbar[(size_t)bh * NC + k] = expf(g_arr[k] + m - mn);
-      m = mn;
-      if (k == NC - 1) ms[NC] = m;
-    }
-  } else {
-    for (int k = k0; k < k1; ++k) {
-      ms[k] = 0.f;
-      gb.gbar[(size_t)bh * NC + k] = expf(g_arr[k]);
-      if (k == NC - 1) ms[NC] = 0.f;
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kGateThreads)
-gates_token_kernel(const float* __restrict__ n_out, float* __restrict__ m_out, GateBuffers gb,
-                   const float* __restrict__ m_states, int S, int SP, int L, int NC, int variant, float eps) {
-  // 1-D grid (no 65535 limit on batch x heads): the chunk groups of one (batch, head) next to each other
-  const int ngrp = (NC + kGateThreads / 32 - 1) / (kGateThreads / 32);
-  const int bh = blockIdx.x / ngrp;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = (blockIdx.x % ngrp) * (kGateThreads / 32) + warp;
-  if (k >= NC) return;
-  const bool siging = variant != MLSTM_EXP;
-  const size_t base_in = (size_t)bh * S + (size_t)k * L;
-  const size_t base = (size_t)bh * SP + (size_t)k * L;
-  const int valid = min(L, S - k * L);
-  const float m_prev = m_states[(size_t)bh * (NC + 1) + k];
-  const float m_next = m_states[(size_t)bh * (NC + 1) + k + 1];
-  float carry = -INFINITY;
-  for (int j0 = 0; j0 < L; j0 += 32) {
-    const int j = j0 + lane;
-    float b = 0.f, x = -INFINITY;
-    if (j < L) { b = gb.vecB[base + j]; x = gb.iota[base + j] - b; }
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      float y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x = fmaxf(x, y);
+  for (int o = 1; o < 32; o <<= 1) {   // earlier map first: (G1, A1) then (G2, A2) = (G1 + G2, max(A1 + G2, A2))
+    const float g1 = __shfl_up_sync(0xffffffffu, G, o), a1 = __shfl_up_sync(0xffffffffu, A, o);
+    if (lane >= o) { A = fmaxf(a1 + G, A); G += g1; }
+  }
+  if (lane == 31) { s_wG[warp] = G; s_wA[warp] = A; }
+  float Gx = __shfl_up_sync(0xffffffffu, G, 1), Ax = __shfl_up_sync(0xffffffffu, A, 1);   // maps of the lanes before
+  if (lane == 0) { Gx = 0.f; Ax = -INFINITY; }
+  __syncthreads();
+  if (tid == 0) {
+    float g = 0.f, a = -INFINITY;
+    for (int w = 0; w < nwarp; ++w) { a = fmaxf(a + s_wG[w], s_wA[w]); g += s_wG[w]; }
+    s_total[0] = g; s_total[1] = a;
+  }
+  cluster.sync();
+  float m = sc.m_initial ? sc.m_initial[bh] : sc.m_default, g_before = 0.f;
+  for (int r = 0; r < rank; ++r) {     // the CTAs before this one
+    const float* t = cluster.map_shared_rank(s_total, r);
+    m = fmaxf(m + t[0], t[1]);
+    g_before += t[0];
+  }
+  float* ms = sc.m_states + (size_t)bh * (NC + 1);
+  if (tid == 0) {
+    // the max state after this CTA's chunks, by the same arithmetic as in the next CTA (which stores the same bits)
+    const float m_end = siging ? 0.f : fmaxf(m + s_total[0], s_total[1]);
+    ms[c1] = m_end;
+    if (rank == ncta - 1) {
+      if (sc.m_last != nullptr) sc.m_last[bh] = m_end;
+      if (sc.g_sum != nullptr) sc.g_sum[bh] = g_before + s_total[0];
     }
-    x = fmaxf(x, carry);
-    carry = __shfl_sync(0xffffffffu, x, 31);
-    if (j < L) {
-      float m_i, bbar, abar;
-      const float a = gb.abar[base + j];
-      if (siging) {
-        m_i = 0.f; bbar = expf(b); abar = expf(a);
-      } else {
-        m_i = fmaxf(b + m_prev, b + x);
-        bbar = expf(b + m_prev - m_i);
-        abar = expf(a - m_next);
+  }
+  for (int w = 0; w < warp; ++w) m = fmaxf(m + s_wG[w], s_wA[w]);
+  m = fmaxf(m + Gx, Ax);
+  for (int k = k0; k < k1; ++k) {
+    ms[k] = siging ? 0.f : m;
+    m = fmaxf(g_arr[k] + m, amax_arr[k]);
+  }
+  __syncthreads();
+  // the decay of a chunk from the stored max states at its two ends: every factor below uses the same values
+  for (int k = k0; k < k1; ++k) gb.gbar[(size_t)bh * NC + k] = siging ? expf(g_arr[k]) : expf(g_arr[k] + ms[k] - ms[k + 1]);
+
+  for (int k = c0 + warp; k < c1; k += nwarp) {
+    const size_t base_in = (size_t)bh * S + (size_t)k * L;
+    const size_t base = (size_t)bh * SP + (size_t)k * L;
+    const int valid = min(L, S - k * L);
+    const float m_prev = ms[k], m_next = ms[k + 1];
+    float carry = -INFINITY;
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      const int j = u * 32 + lane;
+      float b = 0.f, x = -INFINITY;
+      if (j < L) { b = gb.vecB[base + j]; x = gb.iota[base + j] - b; }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x = fmaxf(x, y);
       }
-      const bool pad = j >= valid;     // slot past the sequence end: finite max state, every factor zero
-      gb.m_tok[base + j] = m_i;
-      gb.bbar[base + j] = pad ? 0.f : bbar;
-      gb.abar[base + j] = pad ? 0.f : abar;
-      if (m_out != nullptr && !pad) m_out[base_in + j] = m_i;
-      if (gb.inv_den) {
-        gb.inv_den[base + j] = pad ? 0.f
-                               : ((variant == MLSTM_SIG_NONORM || n_out == nullptr) ? 1.f : 1.f / (n_out[base_in + j] + eps));
+      x = fmaxf(x, carry);
+      carry = __shfl_sync(0xffffffffu, x, 31);
+      if (j < L) {
+        float m_i, bbar, abar;
+        const float a = gb.abar[base + j];
+        if (siging) {
+          m_i = 0.f; bbar = expf(b); abar = expf(a);
+        } else {
+          m_i = fmaxf(b + m_prev, b + x);
+          bbar = expf(b + m_prev - m_i);
+          abar = expf(a - m_next);
+        }
+        const bool pad = j >= valid;     // slot past the sequence end: finite max state, every factor zero
+        gb.m_tok[base + j] = m_i;
+        gb.bbar[base + j] = pad ? 0.f : bbar;
+        gb.abar[base + j] = pad ? 0.f : abar;
+        if (m_out != nullptr && !pad) m_out[base_in + j] = m_i;
+        if (gb.inv_den) {
+          gb.inv_den[base + j] = pad ? 0.f
+                                 : ((variant == MLSTM_SIG_NONORM || n_out == nullptr) ? 1.f : 1.f / (n_out[base_in + j] + eps));
+        }
       }
     }
   }
+  cluster.sync();   // no CTA leaves while another may still read its total
 }
 
 // Per-token reductions for the gate gradients:
@@ -333,39 +358,54 @@ state_dot_kernel(const TS* __restrict__ c_states, const TS* __restrict__ dc_stat
 }
 
 // ---- launchers ----------------------------------------------------------------------------------
-template <typename T>
-int launch_gates_t(const void* i, const void* f, const float* m_initial, const float* n_out, float* m_out,
-                   const GateBuffers& gb, float* m_states, const ChunkwiseDims& d, cudaStream_t st, float m_default,
-                   float* g_sum) {
-  PhaseScope ps(PH_GATES, st);
-  const unsigned grid = (unsigned)ceil_div(d.NC, kGateThreads / 32) * (unsigned)(d.B * d.NH);
-  gates_chunk_kernel<T><<<grid, kGateThreads, 0, st>>>((const T*)i, (const T*)f, gb, d.S, d.SP, d.L, d.NC, d.variant);
-  MLSTM_LAUNCH_CHECK();
-  gates_scan_kernel<<<d.B * d.NH, kGateThreads, 0, st>>>(m_initial, gb, m_states, d.NC, d.variant, m_default, g_sum);
-  MLSTM_LAUNCH_CHECK();
-  gates_token_kernel<<<grid, kGateThreads, 0, st>>>(n_out, m_out, gb, m_states, d.S, d.SP, d.L, d.NC, d.variant, d.eps);
-  MLSTM_LAUNCH_CHECK();
+template <typename T, int NV>
+static int launch_gates_nv(const void* i, const void* f, const float* n_out, float* m_out, const GateBuffers& gb,
+                           const GateScan& sc, const ChunkwiseDims& d, cudaStream_t st) {
+  // enough CTAs per sequence that a warp has one chunk where possible (a cluster holds at most eight); larger CTAs once
+  // that leaves a warp more than two
+  int ncta = 1;
+  while (ncta < 8 && ncta * 8 < d.NC && (long)d.B * d.NH * ncta < 2048) ncta *= 2;
+  const int threads = ceil_div(d.NC, ncta) > 16 ? 1024 : 256;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(d.B * d.NH) * ncta);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ncta; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  note_launch();
+  MLSTM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gates_kernel<T, NV>, (const T*)i, (const T*)f, n_out, m_out, gb, sc, d.S, d.SP,
+                                      d.L, d.NC, d.variant, d.eps));
   return MLSTM_OK;
 }
 
 int launch_gates(int dtype, const void* i, const void* f, const float* m_initial, const float* n_out, float* m_out,
-                 const GateBuffers& gb, float* m_states, const ChunkwiseDims& d, cudaStream_t st, float m_default,
-                 float* g_sum) {
+                 const GateBuffers& gb, float* m_states, float* m_last, const ChunkwiseDims& d, cudaStream_t st,
+                 float m_default, float* g_sum) {
+  PhaseScope ps(PH_GATES, st);
+  const GateScan sc{m_initial, m_default, m_states, m_last, g_sum};
+#define GATES_CASE(DT, T) \
+  case DT: return d.L <= 128 ? launch_gates_nv<T, 4>(i, f, n_out, m_out, gb, sc, d, st) \
+                             : launch_gates_nv<T, 32>(i, f, n_out, m_out, gb, sc, d, st);
   switch (dtype) {
-    case MLSTM_F32: return launch_gates_t<float>(i, f, m_initial, n_out, m_out, gb, m_states, d, st, m_default, g_sum);
-    case MLSTM_BF16: return launch_gates_t<__nv_bfloat16>(i, f, m_initial, n_out, m_out, gb, m_states, d, st, m_default, g_sum);
-    case MLSTM_F16: return launch_gates_t<__half>(i, f, m_initial, n_out, m_out, gb, m_states, d, st, m_default, g_sum);
+    GATES_CASE(MLSTM_F32, float)
+    GATES_CASE(MLSTM_BF16, __nv_bfloat16)
+    GATES_CASE(MLSTM_F16, __half)
   }
+#undef GATES_CASE
   return MLSTM_ERR_DTYPE;
 }
 
 int gates_force_load() {
   cudaFuncAttributes a;
-  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, gates_chunk_kernel<float>));
-  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, gates_chunk_kernel<__nv_bfloat16>));
-  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, gates_chunk_kernel<__half>));
-  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, gates_scan_kernel));
-  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, gates_token_kernel));
+  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, (gates_kernel<float, 4>)));
+  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, (gates_kernel<__nv_bfloat16, 4>)));
+  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, (gates_kernel<__half, 4>)));
+  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, (gates_kernel<float, 32>)));
+  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, (gates_kernel<__nv_bfloat16, 32>)));
+  MLSTM_CUDA_CHECK(cudaFuncGetAttributes(&a, (gates_kernel<__half, 32>)));
   return MLSTM_OK;
 }
 

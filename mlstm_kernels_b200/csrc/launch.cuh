@@ -5,9 +5,10 @@
 namespace mlstm {
 
 // gates.cu
-// m_out (nullable): user-visible copy of the per-token max state, S entries per (batch, head)
+// m_out (nullable): user-visible copy of the per-token max state, S entries per (batch, head); m_last (nullable): copy of
+// the last entry of each m_states row
 int launch_gates(int dtype, const void* i, const void* f, const float* m_initial, const float* n_out, float* m_out,
-                 const GateBuffers& gb, float* m_states, const ChunkwiseDims& d, cudaStream_t st,
+                 const GateBuffers& gb, float* m_states, float* m_last, const ChunkwiseDims& d, cudaStream_t st,
                  float m_default = 0.f, float* g_sum = nullptr);
 int launch_inv_den(const float* n_out, float* inv_den, const ChunkwiseDims& d, cudaStream_t st);
 int launch_state_combine(const float* c_in, const float* n_in, const float* m_in, const float* c_loc,
