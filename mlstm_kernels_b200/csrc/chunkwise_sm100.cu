@@ -15,6 +15,8 @@
 //                    fw_kernel_parallel.py:14-289, bw_kernel_parallel_dV.py, bw_kernel_parallel_dK.py, bw_kernel_parallel_dQ.py
 // Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
 // one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded.
+#include <algorithm>
+
 #include "common.cuh"
 #include "launch.cuh"
 #include "sm100.cuh"
@@ -366,6 +368,7 @@ struct ParParams {
   int S, SP, NC, DHQK, DHHV, variant;   // SP = NC * 128: slots per (batch, head) of the per-token gate vectors
   float eps, qk_scale;
   int bh0;                    // first (batch, head) unit of this launch
+  int maxsub;                 // most output tiles a CTA of this launch produces (par_maxsub)
 };
 
 constexpr int PAR_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 element-wise
@@ -839,12 +842,12 @@ par_fw_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUt
              const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mC,
              const __grid_constant__ ParParams p) {
   __shared__ ParShared sh;
-  const int T = (p.DHHV + 127) / 128;                 // output tiles per chunk; a CTA takes up to PAR_MAXSUB of them
+  const int T = (p.DHHV + 127) / 128;                 // output tiles per chunk; a CTA takes up to maxsub of them
   // 1-D grid in the order (tile group, chunk, batch x head): no 65535 limit on chunks or batch x heads
-  const int gx = (T + PAR_MAXSUB - 1) / PAR_MAXSUB;
+  const int gx = (T + p.maxsub - 1) / p.maxsub;
   const int x = blockIdx.x % gx, ck = (blockIdx.x / gx) % p.NC, bh = p.bh0 + blockIdx.x / (gx * p.NC);
-  const int t0 = PAR_MAXSUB * x;
-  par_body<F16>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(PAR_MAXSUB, T - t0), ck, bh);
+  const int t0 = p.maxsub * x;
+  par_body<F16>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(p.maxsub, T - t0), ck, bh);
 }
 
 // deltaV, deltaK and deltaQ of one chunk in ONE launch: blockIdx.x enumerates the 128-wide output tiles of the three
@@ -859,7 +862,7 @@ par_bw_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUt
              const __grid_constant__ ParParams p) {
   __shared__ ParShared sh;
   const int T_dv = (p.DHHV + 127) / 128, T_dk = (p.DHQK + 127) / 128;   // output tiles per chunk of dV, and of dK / dQ
-  const int c_dv = (T_dv + PAR_MAXSUB - 1) / PAR_MAXSUB, c_dk = (T_dk + PAR_MAXSUB - 1) / PAR_MAXSUB;   // CTAs per mode
+  const int c_dv = (T_dv + p.maxsub - 1) / p.maxsub, c_dk = (T_dk + p.maxsub - 1) / p.maxsub;   // CTAs per mode
   const int gx = c_dv + 2 * c_dk;   // 1-D grid in the order (mode and tile group, chunk, batch x head)
   const int x = blockIdx.x % gx, ck = (blockIdx.x / gx) % p.NC, bh = p.bh0 + blockIdx.x / (gx * p.NC);
   int mode, pair, T;
@@ -867,7 +870,7 @@ par_bw_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUt
   if (x < c_dv) { mode = PM_DV; pair = x; T = T_dv; a = &mK; b = &mQ; xm = &mDH; stm = &mdC_mn; e = &mDH; }
   else if (x < c_dv + c_dk) { mode = PM_DK; pair = x - c_dv; T = T_dk; a = &mV; b = &mDH; xm = &mQ; stm = &mdC_k; e = &mK; }
   else { mode = PM_DQ; pair = x - c_dv - c_dk; T = T_dk; a = &mDH; b = &mV; xm = &mK; stm = &mC_k; e = &mQ; }
-  par_body<F16>(mode, a, b, xm, stm, e, p, sh, PAR_MAXSUB * pair, min(PAR_MAXSUB, T - PAR_MAXSUB * pair), ck, bh);
+  par_body<F16>(mode, a, b, xm, stm, e, p, sh, p.maxsub * pair, min(p.maxsub, T - p.maxsub * pair), ck, bh);
 }
 
 // =====================================================================================================
@@ -1020,6 +1023,17 @@ static ParParams base_params(const GateBuffers& gb, const ChunkwiseDims& d) {
   return pp;
 }
 
+// Output tiles per CTA.  Tiles of one chunk share the score tile and its gating, so a full launch gives a CTA up to
+// PAR_MAXSUB of them; a launch whose CTAs would not fill the GPU (two fit on an SM) splits them over more CTAs instead,
+// each computing the score for itself: one tile takes about 9 us, every further one 5.5 us, and the SMs are idle anyway
+// (500 tokens, 8 heads 256/512: 32 CTAs of four tiles 18.5 us).
+template <typename F>
+static int par_maxsub(F ctas, int tiles) {
+  int m = std::min(PAR_MAXSUB, tiles);
+  while (m > 1 && ctas(m) < 2L * sm_count() && ctas((m + 1) / 2) <= 2L * sm_count()) m = (m + 1) / 2;
+  return m;
+}
+
 int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuffers& gb, const void* c_states,
                       const float* n_states, void* h, float* n_out, const ChunkwiseDims& d, cudaStream_t st,
                       UnitRange ur) {
@@ -1037,8 +1051,9 @@ int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuf
   static bool attr_done[2][64] = {};
   if (int rc = f16 ? set_smem_once(par_fw_sm100<true>, PAR_SMEM, attr_done[1])
                    : set_smem_once(par_fw_sm100<false>, PAR_SMEM, attr_done[0])) return rc;
-  // up to PAR_MAXSUB output tiles per CTA
-  const unsigned grid = (unsigned)(((d.DHHV + 127) / 128 + PAR_MAXSUB - 1) / PAR_MAXSUB) * (unsigned)d.NC * (unsigned)units;
+  const int T = (d.DHHV + 127) / 128;
+  pp.maxsub = par_maxsub([&](int m) { return (long)ceil_div(T, m) * d.NC * units; }, T);
+  const unsigned grid = (unsigned)ceil_div(T, pp.maxsub) * (unsigned)d.NC * (unsigned)units;
   if (f16) par_fw_sm100<true><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mC, pp);
   else par_fw_sm100<false><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mC, pp);
   MLSTM_LAUNCH_CHECK();
@@ -1064,10 +1079,10 @@ int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* d
   static bool attr_done[2][64] = {};
   if (int rc = f16 ? set_smem_once(par_bw_sm100<true>, PAR_SMEM, attr_done[1])
                    : set_smem_once(par_bw_sm100<false>, PAR_SMEM, attr_done[0])) return rc;
-  // up to PAR_MAXSUB output tiles per CTA
-  const unsigned grid = (unsigned)(((d.DHHV + 127) / 128 + PAR_MAXSUB - 1) / PAR_MAXSUB +
-                                   2 * (((d.DHQK + 127) / 128 + PAR_MAXSUB - 1) / PAR_MAXSUB)) *
-                        (unsigned)d.NC * (unsigned)units;
+  const int T_dv = (d.DHHV + 127) / 128, T_dk = (d.DHQK + 127) / 128;
+  auto ctas = [&](int m) { return ((long)ceil_div(T_dv, m) + 2 * ceil_div(T_dk, m)) * d.NC * units; };
+  pp.maxsub = par_maxsub(ctas, std::max(T_dv, T_dk));
+  const unsigned grid = (unsigned)ctas(pp.maxsub);
   if (f16) par_bw_sm100<true><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k, pp);
   else par_bw_sm100<false><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k, pp);
   MLSTM_LAUNCH_CHECK();
