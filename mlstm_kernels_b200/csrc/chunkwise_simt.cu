@@ -2,10 +2,10 @@
 // dimension, f32 / bf16 / f16 inputs, exact f32 arithmetic).  It covers the shapes the tcgen05 path
 // does not (small chunks, odd head dims, f32 inputs) and is the on-device cross-check for it.
 //
-//   rec_kernel  : inter-chunk recurrence, forward (C_k, n_k) and backward (deltaC_k)
+//   rec_part_kernel, rec_scan_kernel, rec_final_kernel : inter-chunk recurrence, forward (C_k, n_k) and backward (deltaC_k)
 //                 mlstm_kernels/triton/chunkwise/xl_chunk/fw_kernel_recurrent.py:14-230,
 //                 bw_kernel_recurrent.py:15-181
-//   par_kernel  : intra-chunk gated products + inter-chunk contribution for H, deltaV, deltaK, deltaQ
+//   par_fw_kernel, par_bw_kernel  : intra-chunk gated products + inter-chunk contribution for H; deltaV, deltaK, deltaQ
 //                 fw_kernel_parallel.py:14-289, bw_kernel_parallel_dV.py, _dK.py, _dQ.py
 #include "common.cuh"
 #include "launch.cuh"
@@ -16,449 +16,639 @@ constexpr int TILE = 64;   // output tile edge per CTA
 constexpr int KSL = 32;    // contraction slice staged in shared memory
 constexpr int NTHR = 256;  // 16 x 16 threads, 4 x 4 outputs each
 
-// =====================================================================================================
-// Inter-chunk recurrence.  state <- gbar * state + (left * lscale * lmul)^T (right * rscale)
-//   forward : left = K, lscale = abar, right = V;  also n <- gbar n + sum_j abar_j k_j
-//   backward: left = Q, lscale = bbar, lmul = qk_scale, right = deltaH, rscale = 1/(den+eps); chunks reversed
-// grid (ceil(DHHV/64) * B*NH, ceil(DHQK/64))
-// =====================================================================================================
-template <typename T, typename TS, bool BWD>
-__global__ void __launch_bounds__(NTHR)
-rec_kernel(const T* __restrict__ left, const T* __restrict__ right, const float* __restrict__ lscale, float lmul,
-           const float* __restrict__ rscale, const float* __restrict__ gbar, const float* __restrict__ c_init,
-           const float* __restrict__ n_init, TS* __restrict__ c_states, float* __restrict__ n_states,
-           float* __restrict__ c_final, float* __restrict__ n_final, int S, int L, int NC, int DHQK, int DHHV) {
-  __shared__ float Ls[KSL][TILE + 1];
-  __shared__ float Rs[KSL][TILE + 1];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // grid (column tiles x batch x heads, row tiles): batch x heads sits in x, which has no 65535 limit
-  const int n_et = (DHHV + TILE - 1) / TILE, et = blockIdx.x % n_et;
-  const int e0 = et * TILE, d0 = blockIdx.y * TILE, bh = blockIdx.x / n_et;
-  const bool do_n = (!BWD) && (et == 0) && (n_states != nullptr || n_final != nullptr);
+// ---- 64 x 64 tile product: 256 threads, double-buffered slices of 32 along the contraction --------------------
+// Slices lie in shared memory contraction-major ([k][64]), so that a thread reads its 4 rows and 4 columns of one k as
+// two 16-byte words for 16 multiply-adds, issued as 8 packed fma.rn.f32x2 (same rounding as two fmaf).  16-byte
+// groups are XOR-swizzled by bits 2..4 of k: rows written transposed (contraction contiguous in memory) and rows
+// written straight both land without bank conflicts.  The next slice is fetched into registers while the current one
+// is multiplied.  Bound by the shared-memory port in large launches (84 % of its wavefronts: a warp's two reads return
+// 1 KB for 8 packed multiply-adds) and by load and barrier latency in small ones, where two warps per scheduler and CTA
+// measured faster than one with 8 x 4 outputs per thread.  Measured 30-34 TFLOP/s at B=4 NH=4 S=2048 128/256; unbuffered
+// slices, scalar reads and a serial recurrence ran at 4.
+__device__ __forceinline__ int swz(int k, int x) { return k * TILE + (((x >> 2) ^ ((k >> 2) & 7)) << 2) + (x & 3); }
 
-  float C[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int d = d0 + ty * 4 + a, e = e0 + tx * 4 + b;
-      C[a][b] = (c_init && d < DHQK && e < DHHV) ? c_init[((size_t)bh * DHQK + d) * DHHV + e] : 0.f;
-    }
-  float nval = 0.f;
-  if (do_n && tid < TILE && d0 + tid < DHQK && n_init) nval = n_init[(size_t)bh * DHQK + d0 + tid];
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
 
-  auto store_state = [&](int slot) {
-    if (c_states != nullptr) {
-      TS* cs = c_states + ((size_t)bh * (NC + 1) + slot) * DHQK * DHHV;
+__device__ __forceinline__ int row_group(int tid) { return tid >> 4; }
+__device__ __forceinline__ int col_group(int tid) { return tid & 15; }
+// sum over the 16 column groups of a row group
+__device__ __forceinline__ float sum_columns(float x) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int d = d0 + ty * 4 + a, e = e0 + tx * 4 + b;
-          if (d < DHQK && e < DHHV) cs[(size_t)d * DHHV + e] = from_f32<TS>(C[a][b]);
-        }
-    }
-    if (do_n && n_states != nullptr && tid < TILE && d0 + tid < DHQK) n_states[((size_t)bh * (NC + 1) + slot) * DHQK + d0 + tid] = nval;
-  };
+  for (int o = 1; o < 16; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
 
-  for (int s = 0; s < NC; ++s) {
-    const int slot = BWD ? NC - s : s;
-    const int ck = BWD ? NC - 1 - s : s;
-    store_state(slot);
-    const size_t tok0 = (size_t)bh * S + (size_t)ck * L;
-    float acc[4][4] = {};
-    float nacc = 0.f;
-    for (int r0 = 0; r0 < L; r0 += KSL) {
-      for (int idx = tid; idx < KSL * TILE; idx += NTHR) {
-        const int r = idx / TILE, c = idx % TILE;
-        const int row = r0 + r;
-        float lv = 0.f, rv = 0.f;
-        if (row < L) {
-          const size_t tok = tok0 + row;
-          if (d0 + c < DHQK) lv = to_f32(left[tok * DHQK + d0 + c]) * (lscale[tok] * lmul);
-          if (e0 + c < DHHV) rv = to_f32(right[tok * DHHV + e0 + c]) * (rscale ? rscale[tok] : 1.f);
-        }
-        Ls[r][c] = lv;
-        Rs[r][c] = rv;
-      }
-      __syncthreads();
-#pragma unroll 8
-      for (int r = 0; r < KSL; ++r) {
-        float a4[4], b4[4];
+struct Acc {   // rows 4 ty + {0..3} in pairs, columns 4 tx + {0..3}
+  uint64_t v[2][4];
+  __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int a = 0; a < 4; ++a) a4[a] = Ls[r][ty * 4 + a];
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) b4[b] = Rs[r][tx * 4 + b];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(a4[a], b4[b], acc[a][b]);
-      }
-      if (do_n && tid < TILE) {
-#pragma unroll 8
-        for (int r = 0; r < KSL; ++r) nacc += Ls[r][tid];
-      }
-      __syncthreads();
-    }
-    const float g = gbar[(size_t)bh * NC + ck];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) C[a][b] = fmaf(g, C[a][b], acc[a][b]);
-    nval = fmaf(g, nval, nacc);
+      for (int b = 0; b < 4; ++b) v[a][b] = 0ull;
   }
-  store_state(BWD ? 0 : NC);
-  if (c_final) {
+  __device__ __forceinline__ void get(float (&x)[4][4]) const {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int d = d0 + ty * 4 + a, e = e0 + tx * 4 + b;
-        if (d < DHQK && e < DHHV) c_final[((size_t)bh * DHQK + d) * DHHV + e] = C[a][b];
+        const float2 f = unpack2(v[a][b]);
+        x[2 * a][b] = f.x; x[2 * a + 1][b] = f.y;
       }
   }
-  if (do_n && n_final && tid < TILE && d0 + tid < DHQK) n_final[(size_t)bh * DHQK + d0 + tid] = nval;
+};
+
+// acc += A B over the 32 contraction steps of one staged slice pair.  Rolled over groups of four steps that share a
+// swizzle: unrolled further, the kernels' several copies of this loop outgrew the instruction cache.
+__device__ __forceinline__ void mma_slice(Acc& acc, const float* A, const float* B, int ty, int tx) {
+#pragma unroll 2
+  for (int kq = 0; kq < KSL / 4; ++kq) {
+    const float* pa = A + kq * 4 * TILE + ((ty ^ kq) << 2);
+    const float* pb = B + kq * 4 * TILE + ((tx ^ kq) << 2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(pa + k * TILE);
+      const float4 b = *reinterpret_cast<const float4*>(pb + k * TILE);
+      const uint64_t av[2] = {a.x, a.y};
+      const uint64_t bv[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) fma2(acc.v[m][n], av[m], bv[n]);
+    }
+  }
+}
+
+// four consecutive elements of a row, zero outside [0, cols); `vec`: rows start on 4-element boundaries
+__device__ __forceinline__ float4 load4(const float* p, int c, int cols, bool vec) {
+  if (vec) return c < cols ? *reinterpret_cast<const float4*>(p + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(c < cols ? p[c] : 0.f, c + 1 < cols ? p[c + 1] : 0.f, c + 2 < cols ? p[c + 2] : 0.f,
+                     c + 3 < cols ? p[c + 3] : 0.f);
+}
+template <typename T>
+__device__ __forceinline__ void store4(T* p, int c, int cols, bool vec, float4 v) {
+  if (vec && sizeof(T) == 4) {
+    if (c < cols) *reinterpret_cast<float4*>(p + c) = v;
+    return;
+  }
+  if (c < cols) p[c] = from_f32<T>(v.x);
+  if (c + 1 < cols) p[c + 1] = from_f32<T>(v.y);
+  if (c + 2 < cols) p[c + 2] = from_f32<T>(v.z);
+  if (c + 3 < cols) p[c + 3] = from_f32<T>(v.w);
+}
+
+// A matrix operand in global memory: rows x cols, `scale` (or null) multiplies whole rows.
+template <typename T>
+struct Mat {
+  const T* p;
+  const float* scale;
+  int rows, cols, ld;
+};
+
+// One slice of an operand in flight: 2048 elements, two groups of four per thread.  The loads' results are not touched
+// before put() (no conversion, no scaling: either would wait for the load), so they travel under the current slice's
+// multiply-adds.  VEC: rows start on four-element boundaries.
+//   TR = true   tile rows x0.. are matrix rows, the contraction k0.. runs along the columns (transposed into shared memory)
+//   TR = false  the contraction k0.. runs over matrix rows, the tile columns x0.. along the columns
+template <typename T, bool TR, bool VEC>
+struct Slice {
+  struct __align__(4 * sizeof(T)) Raw { T e[4]; };
+  Raw v[2];
+  float sc[2];
+  __device__ __forceinline__ void fetch(const Mat<T>& m, int x0, int k0, int tid) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int r = TR ? x0 + (tid >> 3) + 32 * u : k0 + (tid >> 4) + 16 * u;
+      const int c = TR ? k0 + 4 * (tid & 7) : x0 + 4 * (tid & 15);
+      const T* p = m.p + (size_t)r * m.ld + c;
+      if (VEC) {
+        v[u] = Raw{};
+        if (r < m.rows && c < m.cols) v[u] = *reinterpret_cast<const Raw*>(p);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          v[u].e[e] = from_f32<T>(0.f);
+          if (r < m.rows && c + e < m.cols) v[u].e[e] = p[e];
+        }
+      }
+      sc[u] = 1.f;
+      if (m.scale && r < m.rows) sc[u] = m.scale[r];
+    }
+  }
+  __device__ __forceinline__ void put(float* s, int tid) const {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float x[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = to_f32(v[u].e[e]) * sc[u];
+      if (TR) {
+        const int r = (tid >> 3) + 32 * u, k = 4 * (tid & 7);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[swz(k + e, r)] = x[e];
+      } else {
+        *reinterpret_cast<float4*>(s + swz((tid >> 4) + 16 * u, 4 * (tid & 15))) = make_float4(x[0], x[1], x[2], x[3]);
+      }
+    }
+  }
+};
+
+constexpr int SLICE = KSL * TILE;   // floats of one staged slice
+
+// acc += A B over the contraction [0, K); buf: 4 slices (two of A, two of B).  After the last slice every thread has
+// passed a barrier that follows its last read of the older buffer pair only: callers synchronise before reusing buf.
+// each(slice of A, k0) runs once per slice while it lies in shared memory.
+template <bool VEC, bool TRA, bool TRB, typename TA, typename TB, typename F>
+__device__ __forceinline__ void tile_product(Acc& acc, const Mat<TA>& A, int a0, const Mat<TB>& B, int b0, int K, float* buf,
+                                             int tid, F each) {
+  const int ty = row_group(tid), tx = col_group(tid);
+  Slice<TA, TRA, VEC> sa;
+  Slice<TB, TRB, VEC> sb;
+  sa.fetch(A, a0, 0, tid);
+  sb.fetch(B, b0, 0, tid);
+  int cur = 0;
+  for (int k0 = 0; k0 < K; k0 += KSL) {
+    float* As = buf + cur * SLICE;
+    float* Bs = buf + (2 + cur) * SLICE;
+    sa.put(As, tid);
+    sb.put(Bs, tid);
+    __syncthreads();
+    if (k0 + KSL < K) {
+      sa.fetch(A, a0, k0 + KSL, tid);
+      sb.fetch(B, b0, k0 + KSL, tid);
+    }
+    each(As, k0);
+    mma_slice(acc, As, Bs, ty, tx);
+    cur ^= 1;
+  }
+}
+struct NoEach { __device__ __forceinline__ void operator()(const float*, int) const {} };
+
+// =====================================================================================================
+// Inter-chunk recurrence.  state <- gbar * state + lmul * (left * lscale)^T (right * rscale)
+//   forward : left = K, lscale = abar, right = V;  also n <- gbar n + sum_j abar_j k_j
+//   backward: left = Q, lscale = bbar, lmul = qk_scale, right = deltaH, rscale = 1/(den+eps); chunks reversed
+// Where the per-chunk states are wanted, the chunks' contributions are independent CTAs that leave them in the state
+// buffer itself (rec_part_kernel), and an element-wise scan over the chunks turns them into states in place
+// (rec_scan_kernel, one thread per four elements): a CTA that walks a whole sequence took 9.6 us per chunk of 64 tokens
+// while most SMs idled.  Without a state buffer (segment summaries) rec_final_kernel walks the chunks of its tile.
+// =====================================================================================================
+template <typename T>
+struct RecArgs {
+  const T *left, *right;
+  const float *lscale, *rscale, *gbar;
+  float lmul;
+  const float *c_init, *n_init;
+  float *c_states, *n_states, *c_final, *n_final;
+  int S, L, NC, DHQK, DHHV;
+};
+
+// P = (left * lscale)^T (right * rscale) of chunk ck for the tile (d0, e0); ns: column sums of the scaled left rows
+template <typename T, bool VEC>
+__device__ __forceinline__ void chunk_part(const RecArgs<T>& p, int bh, int ck, int d0, int e0, bool do_n, float* buf, Acc& acc,
+                                           float (&ns)[4]) {
+  const int tid = threadIdx.x, ty = row_group(tid), tx = col_group(tid);
+  const size_t tok0 = (size_t)bh * p.S + (size_t)ck * p.L;
+  const Mat<T> A{p.left + tok0 * p.DHQK, p.lscale + tok0, p.L, p.DHQK, p.DHQK};
+  const Mat<T> B{p.right + tok0 * p.DHHV, p.rscale ? p.rscale + tok0 : nullptr, p.L, p.DHHV, p.DHHV};
+  acc.zero();
+#pragma unroll
+  for (int a = 0; a < 4; ++a) ns[a] = 0.f;
+  tile_product<VEC, false, false>(acc, A, d0, B, e0, p.L, buf, tid, [&](const float* As, int) {
+    if (!do_n) return;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int a = 0; a < 4; ++a) ns[a] += As[swz(2 * tx + u, 4 * ty + a)];
+  });
+  if (do_n) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) ns[a] = sum_columns(ns[a]);
+  }
+}
+
+template <typename T, bool BWD, bool VEC>
+__global__ void __launch_bounds__(NTHR) rec_part_kernel(RecArgs<T> p) {
+  __shared__ __align__(16) float buf[4 * SLICE];
+  // 1-D grid: the tiles of one chunk next to each other (they share its operands through L2)
+  const int n_et = (p.DHHV + TILE - 1) / TILE, n_dt = (p.DHQK + TILE - 1) / TILE;
+  const int et = blockIdx.x % n_et, dt = (blockIdx.x / n_et) % n_dt, bc = blockIdx.x / (n_et * n_dt);
+  const int bh = bc / p.NC, ck = bc % p.NC, e0 = et * TILE, d0 = dt * TILE;
+  const bool do_n = !BWD && et == 0 && p.n_states != nullptr;
+  const int ty = row_group(threadIdx.x), tx = col_group(threadIdx.x);
+  Acc acc;
+  float ns[4], x[4][4];
+  chunk_part<T, VEC>(p, bh, ck, d0, e0, do_n, buf, acc, ns);
+  acc.get(x);
+  const size_t slot = (size_t)bh * (p.NC + 1) + (BWD ? ck : ck + 1);
+  float* out = p.c_states + slot * p.DHQK * p.DHHV;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int d = d0 + 4 * ty + a;
+    if (d < p.DHQK)
+      store4(out + (size_t)d * p.DHHV, e0 + 4 * tx, p.DHHV, VEC,
+             make_float4(x[a][0] * p.lmul, x[a][1] * p.lmul, x[a][2] * p.lmul, x[a][3] * p.lmul));
+    if (do_n && tx == 0 && d < p.DHQK) p.n_states[slot * p.DHQK + d] = ns[a];
+  }
+}
+
+template <int V> struct Vec;
+template <> struct Vec<1> { float v[1]; __device__ void load(const float* p) { v[0] = *p; } __device__ void store(float* p) const { *p = v[0]; } };
+template <> struct Vec<4> {
+  float v[4];
+  __device__ void load(const float* p) { const float4 f = *reinterpret_cast<const float4*>(p); v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; }
+  __device__ void store(float* p) const { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+};
+
+// Element-wise: states[k+1] = gbar_k states[k] + states[k+1] in place (BWD: right to left).  Bound by memory (each
+// element read and written once); four loads in flight ahead of the dependent multiply-adds.
+template <int V, bool BWD>
+__device__ __forceinline__ void scan_elements(float* states, const float* init, float* fin, const float* gbar, size_t E, size_t e, int NC) {
+  Vec<V> c;
+#pragma unroll
+  for (int i = 0; i < V; ++i) c.v[i] = 0.f;
+  if (init) c.load(init + e);
+  c.store(states + (size_t)(BWD ? NC : 0) * E + e);
+  constexpr int AHEAD = 4;
+  for (int s0 = 0; s0 < NC; s0 += AHEAD) {
+    Vec<V> part[AHEAD];
+    float g[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      if (s0 + u < NC) {
+        const int ck = BWD ? NC - 1 - (s0 + u) : s0 + u;
+        part[u].load(states + (size_t)(BWD ? ck : ck + 1) * E + e);
+        g[u] = gbar[ck];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      if (s0 + u < NC) {
+        const int ck = BWD ? NC - 1 - (s0 + u) : s0 + u;
+#pragma unroll
+        for (int i = 0; i < V; ++i) c.v[i] = fmaf(g[u], c.v[i], part[u].v[i]);
+        c.store(states + (size_t)(BWD ? ck : ck + 1) * E + e);
+      }
+    }
+  }
+  if (fin) c.store(fin + e);
+}
+
+template <int V, bool BWD>
+__global__ void __launch_bounds__(128)
+rec_scan_kernel(float* c_states, const float* c_init, float* c_final, float* n_states, const float* n_init, float* n_final,
+                const float* gbar, int NC, int DHQK, int DHHV, int nblk) {
+  const int bh = blockIdx.x / nblk;
+  const size_t E = (size_t)DHQK * DHHV, t = (size_t)(blockIdx.x % nblk) * 128 + threadIdx.x;
+  const float* g = gbar + (size_t)bh * NC;
+  if (t * V < E) {
+    scan_elements<V, BWD>(c_states + (size_t)bh * (NC + 1) * E, c_init ? c_init + bh * E : nullptr,
+                          c_final ? c_final + bh * E : nullptr, g, E, t * V, NC);
+  } else if (!BWD && n_states != nullptr && t - (E + V - 1) / V < (size_t)DHQK) {   // threads past the tiles: n
+    scan_elements<1, BWD>(n_states + (size_t)bh * (NC + 1) * DHQK, n_init ? n_init + (size_t)bh * DHQK : nullptr,
+                          n_final ? n_final + (size_t)bh * DHQK : nullptr, g, DHQK, t - (E + V - 1) / V, NC);
+  }
+}
+
+// Final state only, one CTA per tile walking the chunks.
+template <typename T, bool BWD, bool VEC>
+__global__ void __launch_bounds__(NTHR) rec_final_kernel(RecArgs<T> p) {
+  __shared__ __align__(16) float buf[4 * SLICE];
+  const int n_et = (p.DHHV + TILE - 1) / TILE, n_dt = (p.DHQK + TILE - 1) / TILE;
+  const int et = blockIdx.x % n_et, dt = (blockIdx.x / n_et) % n_dt, bh = blockIdx.x / (n_et * n_dt);
+  const int e0 = et * TILE, d0 = dt * TILE, ty = row_group(threadIdx.x), tx = col_group(threadIdx.x);
+  const bool do_n = !BWD && et == 0 && p.n_final != nullptr;
+  float C[4][4], n[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int d = d0 + 4 * ty + a;
+    const float4 c = (p.c_init && d < p.DHQK) ? load4(p.c_init + ((size_t)bh * p.DHQK + d) * p.DHHV, e0 + 4 * tx, p.DHHV, VEC)
+                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+    C[a][0] = c.x; C[a][1] = c.y; C[a][2] = c.z; C[a][3] = c.w;
+    n[a] = (do_n && p.n_init && d < p.DHQK) ? p.n_init[(size_t)bh * p.DHQK + d] : 0.f;
+  }
+  for (int s = 0; s < p.NC; ++s) {
+    const int ck = BWD ? p.NC - 1 - s : s;
+    Acc acc;
+    float ns[4], x[4][4];
+    chunk_part<T, VEC>(p, bh, ck, d0, e0, do_n, buf, acc, ns);
+    acc.get(x);
+    const float g = p.gbar[(size_t)bh * p.NC + ck];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      n[a] = fmaf(g, n[a], ns[a]);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) C[a][b] = fmaf(g, C[a][b], x[a][b] * p.lmul);
+    }
+    __syncthreads();   // the slices are free for the next chunk
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int d = d0 + 4 * ty + a;
+    if (d >= p.DHQK) continue;
+    if (p.c_final) store4(p.c_final + ((size_t)bh * p.DHQK + d) * p.DHHV, e0 + 4 * tx, p.DHHV, VEC, make_float4(C[a][0], C[a][1], C[a][2], C[a][3]));
+    if (do_n && tx == 0) p.n_final[(size_t)bh * p.DHQK + d] = n[a];
+  }
 }
 
 // =====================================================================================================
 // Intra-chunk kernel, four modes.  For the output tile rows r (tokens of one chunk) and columns o:
-//   out[r,o] = sum_c P[r,c] X[c,o] + rowscale_r * sum_a A[r,a] Bm[a,o]
+//   out[r,o] = sum_c P[r,c] X[c,o] + rowscale_r * sum_a U[r,a] Bm[a,o]
 //   P[r,c]   = qk_scale * (U[r] . W[c]) * D(i,j),  D(i,j) = exp((b_i - b_j) + iota_j - m_i) for j <= i
-//   mode  U        W        (i,j)   X        A        rowscale        Bm
-//   H     Q        K        (r,c)   V        Q        qk_scale*bbar   C_k[a][o]
-//   DV    K        Q        (c,r)   dHbar    K        abar            dC_{k+1}[a][o]
-//   DK    V        dHbar    (c,r)   Q        V        abar            dC_{k+1}[o][a]
-//   DQ    dHbar    V        (r,c)   K        dHbar    qk_scale*bbar   C_k[o][a]
-// dHbar = deltaH / (den + eps).  grid (ceil(DO/64), ceil(L/64), B*NH*NC)
+//   mode  U        W        (i,j)   X        rowscale        Bm
+//   H     Q        K        (r,c)   V        qk_scale*bbar   C_k[a][o]
+//   DV    K        Q        (c,r)   dHbar    abar            dC_{k+1}[a][o]
+//   DK    V        dHbar    (c,r)   Q        abar            dC_{k+1}[o][a]
+//   DQ    dHbar    V        (r,c)   K        qk_scale*bbar   C_k[o][a]
+// dHbar = deltaH / (den + eps).  grid (output tiles x B*NH*NC, ceil(L/64)); the backward's three modes share a launch
+// (their CTAs fill each other's last wave and find a chunk's operands in L2).
+// The contraction runs on CUDA cores in exact f32: 64 x 64 tiles of the product above, at B=2 NH=4 S=512 128/256 a few
+// hundred CTAs of a few million multiply-adds each.
 // =====================================================================================================
 enum { PAR_H = 0, PAR_DV = 1, PAR_DK = 2, PAR_DQ = 3 };
 
-template <typename T, typename TS>
+template <typename T>
 struct ParArgs {
   const T *q, *k, *v, *dh;
   const float *vecB, *iota, *m_tok, *abar, *bbar, *inv_den;
-  const TS* c_states;   // slot k used by H and DQ
-  const TS* dc_states;  // slot k+1 used by DV and DK
+  const float* c_states;   // slot k used by H and DQ
+  const float* dc_states;  // slot k+1 used by DV and DK
   const float* n_states;
-  void* out;     // T*
-  float* n_out;       // H only, may be null
-  float* inv_den_out; // H only, may be null
+  T *out_h, *out_dv, *out_dk, *out_dq;
+  float* n_out;            // H only, may be null
+  float* inv_den_out;      // H only, may be null
   int S, L, NC, DHQK, DHHV, variant;
   float eps, qk_scale;
 };
 
-template <typename T, typename TS, int MODE>
-__global__ void __launch_bounds__(NTHR) par_kernel(ParArgs<T, TS> p) {
-  extern __shared__ float smem[];
+// FW: mode PAR_H only; otherwise `mode` is one of the gradients, uniform over the CTA - one body for the three (three
+// inlined copies stalled on instruction fetch as often as they issued).
+template <typename T, bool FW, bool VEC>
+__device__ __forceinline__ void par_tile(const ParArgs<T>& p, const int mode, int ot, int bc, int rb, float* smem) {
+  const bool LOWER = FW || mode == PAR_DQ;
+  const bool QK = FW || mode == PAR_DV;   // score over DHQK, output over DHHV (else the other way)
   const int L = p.L;
-  float* s_b = smem;              // [L]
-  float* s_iota = s_b + L;        // [L]
-  float* s_m = s_iota + L;        // [L]
-  float* Us = s_m + L;            // [64][33]   (also As)
-  float* Ws = Us + TILE * (KSL + 1);  // [64][33]
-  float* Ps = Ws + TILE * (KSL + 1);  // [64][65]
-  float* Xs = Ps + TILE * (TILE + 1);  // [64][65]  (also Bs [32][65])
-  float* s_row = Xs + TILE * (TILE + 1);  // [64] row sums / denominators
-  float* s_qn = s_row + TILE;             // [64]
-  float* s_n = s_qn + TILE;               // [32]
+  float* buf = smem;                  // [4][32][64] slices
+  float* Ps = buf + 4 * SLICE;        // [64 c][64 r] gated score block
+  float* s_b = Ps + TILE * TILE;      // [L] each
+  float* s_iota = s_b + L;
+  float* s_m = s_iota + L;
+  float* s_n = s_m + L;               // PAR_H: [DHQK, rounded up to whole slices] n_k
 
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // grid (output tiles x chunks x batch x heads, row blocks): the large factor sits in x, which has no 65535 limit
-  const int n_ot = (((MODE == PAR_H || MODE == PAR_DV) ? p.DHHV : p.DHQK) + TILE - 1) / TILE;
-  const int ot = blockIdx.x % n_ot, bc = blockIdx.x / n_ot;
-  const int o0 = ot * TILE, rb = blockIdx.y, r0 = rb * TILE;
-  const int bh = bc / p.NC, ck = bc % p.NC;
+  const int tid = threadIdx.x, ty = row_group(tid), tx = col_group(tid);
+  const int o0 = ot * TILE, r0 = rb * TILE, bh = bc / p.NC, ck = bc % p.NC;
   const size_t tok0 = (size_t)bh * p.S + (size_t)ck * L;
-  constexpr bool LOWER = (MODE == PAR_H || MODE == PAR_DQ);
-  const int DI = (MODE == PAR_H || MODE == PAR_DV) ? p.DHQK : p.DHHV;   // contraction dim of P
-  const int DO = (MODE == PAR_H || MODE == PAR_DV) ? p.DHHV : p.DHQK;   // output width
-  const int DA = (MODE == PAR_H || MODE == PAR_DV) ? p.DHQK : p.DHHV;   // contraction dim of the inter term
-
-  // element accessors (value of matrix `which` at chunk row r, column c; zero outside)
-  auto ldU = [&](int r, int c) -> float {
-    if (r >= L || c >= DI) return 0.f;
-    const size_t t = tok0 + r;
-    if (MODE == PAR_H) return to_f32(p.q[t * p.DHQK + c]);
-    if (MODE == PAR_DV) return to_f32(p.k[t * p.DHQK + c]);
-    if (MODE == PAR_DK) return to_f32(p.v[t * p.DHHV + c]);
-    return to_f32(p.dh[t * p.DHHV + c]) * p.inv_den[t];
-  };
-  auto ldW = [&](int r, int c) -> float {
-    if (r >= L || c >= DI) return 0.f;
-    const size_t t = tok0 + r;
-    if (MODE == PAR_H) return to_f32(p.k[t * p.DHQK + c]);
-    if (MODE == PAR_DV) return to_f32(p.q[t * p.DHQK + c]);
-    if (MODE == PAR_DK) return to_f32(p.dh[t * p.DHHV + c]) * p.inv_den[t];
-    return to_f32(p.v[t * p.DHHV + c]);
-  };
-  auto ldX = [&](int r, int c) -> float {
-    if (r >= L || c >= DO) return 0.f;
-    const size_t t = tok0 + r;
-    if (MODE == PAR_H) return to_f32(p.v[t * p.DHHV + c]);
-    if (MODE == PAR_DV) return to_f32(p.dh[t * p.DHHV + c]) * p.inv_den[t];
-    if (MODE == PAR_DK) return to_f32(p.q[t * p.DHQK + c]);
-    return to_f32(p.k[t * p.DHQK + c]);
-  };
+  const int DI = QK ? p.DHQK : p.DHHV;   // contraction of the score and of the inter-chunk term
+  const int DO = QK ? p.DHHV : p.DHQK;   // output width
+  const Mat<T> mq{p.q + tok0 * p.DHQK, nullptr, L, p.DHQK, p.DHQK}, mk{p.k + tok0 * p.DHQK, nullptr, L, p.DHQK, p.DHQK};
+  const Mat<T> mv{p.v + tok0 * p.DHHV, nullptr, L, p.DHHV, p.DHHV};
+  const Mat<T> mh{p.dh + tok0 * p.DHHV, p.inv_den + tok0, L, p.DHHV, p.DHHV};
+  const Mat<T> U = FW ? mq : mode == PAR_DV ? mk : mode == PAR_DK ? mv : mh;
+  const Mat<T> W = FW ? mk : mode == PAR_DV ? mq : mode == PAR_DK ? mh : mv;
+  const Mat<T> X = FW ? mv : mode == PAR_DV ? mh : mode == PAR_DK ? mq : mk;
+  const size_t state_elems = (size_t)p.DHQK * p.DHHV, slab = (size_t)bh * (p.NC + 1) + ck;
+  const Mat<float> St{LOWER ? p.c_states + slab * state_elems : p.dc_states + (slab + 1) * state_elems, nullptr, p.DHQK,
+                      p.DHHV, p.DHHV};
 
   for (int j = tid; j < L; j += NTHR) {
     s_b[j] = p.vecB[tok0 + j];
     s_iota[j] = p.iota[tok0 + j];
     s_m[j] = p.m_tok[tok0 + j];
   }
-  if (tid < TILE) { s_row[tid] = 0.f; s_qn[tid] = 0.f; }
-  __syncthreads();
+  // inter-chunk term first: scaled by row, it is what the intra-chunk products are added onto
+  Acc acc;
+  acc.zero();
+  float qn[4], rowsum[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) { qn[a] = 0.f; rowsum[a] = 0.f; }
+  const float* nsrc = (FW && p.n_states) ? p.n_states + slab * p.DHQK : nullptr;
+  if (FW && nsrc != nullptr)
+    for (int k = tid; k < (DI + KSL - 1) / KSL * KSL; k += NTHR) s_n[k] = k < DI ? nsrc[k] : 0.f;   // (a barrier follows in the product)
+  auto dot_n = [&](const float* As, int k0) {
+    if (!FW || nsrc == nullptr) return;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = 2 * tx + u;
+      const float n = s_n[k0 + k];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) qn[a] = fmaf(As[swz(k, 4 * ty + a)], n, qn[a]);
+    }
+  };
+  if (QK) tile_product<VEC, true, false>(acc, U, r0, St, o0, DI, buf, tid, dot_n);
+  else tile_product<VEC, true, true>(acc, U, r0, St, o0, DI, buf, tid, NoEach());
+  float rs[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int r = r0 + 4 * ty + a;
+    rs[a] = r < L ? (LOWER ? p.qk_scale * p.bbar[tok0 + r] : p.abar[tok0 + r]) : 0.f;
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float2 f = unpack2(acc.v[a][b]);
+      acc.v[a][b] = pack2(f.x * rs[2 * a], f.y * rs[2 * a + 1]);
+    }
 
-  float acc[4][4] = {};
-  float rowsum = 0.f;
   const int nblk = (L + TILE - 1) / TILE;
   const int cb_lo = LOWER ? 0 : rb, cb_hi = LOWER ? rb : nblk - 1;
   for (int cb = cb_lo; cb <= cb_hi; ++cb) {
     const int c0 = cb * TILE;
-    float pr[4][4] = {};
-    for (int di0 = 0; di0 < DI; di0 += KSL) {
-      for (int idx = tid; idx < TILE * KSL; idx += NTHR) {
-        const int r = idx / KSL, c = idx % KSL;
-        Us[r * (KSL + 1) + c] = ldU(r0 + r, di0 + c);
-        Ws[r * (KSL + 1) + c] = ldW(c0 + r, di0 + c);
-      }
-      __syncthreads();
-#pragma unroll 8
-      for (int d = 0; d < KSL; ++d) {
-        float a4[4], b4[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) a4[a] = Us[(ty * 4 + a) * (KSL + 1) + d];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) b4[b] = Ws[(tx * 4 + b) * (KSL + 1) + d];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) pr[a][b] = fmaf(a4[a], b4[b], pr[a][b]);
-      }
-      __syncthreads();
-    }
+    __syncthreads();   // the slices and the gated block of the previous round have been read
+    Acc pr;
+    pr.zero();
+    tile_product<VEC, true, true>(pr, U, r0, W, c0, DI, buf, tid, NoEach());
+    float s[4][4];
+    pr.get(s);
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int r = r0 + ty * 4 + a, c = c0 + tx * 4 + b;
+        const int r = r0 + 4 * ty + a, c = c0 + 4 * tx + b;
         const bool valid = (r < L) && (c < L) && (LOWER ? (c <= r) : (c >= r));
         float val = 0.f;
         if (valid) {
           const int ii = LOWER ? r : c, jj = LOWER ? c : r;
-          val = p.qk_scale * pr[a][b] * expf((s_b[ii] - s_b[jj]) + s_iota[jj] - s_m[ii]);
+          val = p.qk_scale * s[a][b] * expf((s_b[ii] - s_b[jj]) + s_iota[jj] - s_m[ii]);
         }
-        Ps[(ty * 4 + a) * (TILE + 1) + tx * 4 + b] = val;
+        s[a][b] = val;
+        if (FW) rowsum[a] += val;
       }
-    for (int idx = tid; idx < TILE * TILE; idx += NTHR) {
-      const int r = idx / TILE, c = idx % TILE;
-      Xs[r * (TILE + 1) + c] = ldX(c0 + r, o0 + c);
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int c = 0; c < TILE; ++c) {
-      float a4[4], b4[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) a4[a] = Ps[(ty * 4 + a) * (TILE + 1) + c];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) b4[b] = Xs[c * (TILE + 1) + tx * 4 + b];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(a4[a], b4[b], acc[a][b]);
-    }
-    if (MODE == PAR_H && tid < TILE) {
-      for (int c = 0; c < TILE; ++c) rowsum += Ps[tid * (TILE + 1) + c];
-    }
-    __syncthreads();
-  }
-
-  // ---- inter-chunk contribution ----
-  float acc2[4][4] = {};
-  float qn = 0.f;
-  const TS* Bsrc = (MODE == PAR_H || MODE == PAR_DQ)
-                       ? p.c_states + ((size_t)bh * (p.NC + 1) + ck) * p.DHQK * p.DHHV
-                       : p.dc_states + ((size_t)bh * (p.NC + 1) + ck + 1) * p.DHQK * p.DHHV;
-  const float* nsrc = (MODE == PAR_H && p.n_states) ? p.n_states + ((size_t)bh * (p.NC + 1) + ck) * p.DHQK : nullptr;
-  float* As = Us;
-  float* Bs = Xs;
-  for (int da0 = 0; da0 < DA; da0 += KSL) {
-    for (int idx = tid; idx < TILE * KSL; idx += NTHR) {
-      const int r = idx / KSL, c = idx % KSL;
-      As[r * (KSL + 1) + c] = ldU(r0 + r, da0 + c);  // A is the same matrix as U in every mode
-    }
-    if (MODE == PAR_H || MODE == PAR_DV) {
-      for (int idx = tid; idx < KSL * TILE; idx += NTHR) {
-        const int a = idx / TILE, o = idx % TILE;
-        float val = 0.f;
-        if (da0 + a < DA && o0 + o < DO) val = to_f32(Bsrc[(size_t)(da0 + a) * p.DHHV + o0 + o]);
-        Bs[a * (TILE + 1) + o] = val;
-      }
-    } else {
-      for (int idx = tid; idx < KSL * TILE; idx += NTHR) {
-        const int a = idx % KSL, o = idx / KSL;
-        float val = 0.f;
-        if (da0 + a < DA && o0 + o < DO) val = to_f32(Bsrc[(size_t)(o0 + o) * p.DHHV + da0 + a]);
-        Bs[a * (TILE + 1) + o] = val;
-      }
-    }
-    if (MODE == PAR_H && tid < KSL) s_n[tid] = (nsrc && da0 + tid < DA) ? nsrc[da0 + tid] : 0.f;
-    __syncthreads();
-#pragma unroll 8
-    for (int d = 0; d < KSL; ++d) {
-      float a4[4], b4[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) a4[a] = As[(ty * 4 + a) * (KSL + 1) + d];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) b4[b] = Bs[d * (TILE + 1) + tx * 4 + b];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc2[a][b] = fmaf(a4[a], b4[b], acc2[a][b]);
-    }
-    if (MODE == PAR_H && tid < TILE) {
-      for (int d = 0; d < KSL; ++d) qn = fmaf(As[tid * (KSL + 1) + d], s_n[d], qn);
-    }
-    __syncthreads();
-  }
-
-  // ---- epilogue ----
-  if (MODE == PAR_H && tid < TILE) {
-    const int r = r0 + tid;
-    float den = 1.f;
-    if (r < L) {
-      const float nn = rowsum + p.qk_scale * p.bbar[tok0 + r] * qn;
-      if (p.variant == MLSTM_EXP) den = fmaxf(fabsf(nn), expf(-s_m[r]));
-      else if (p.variant == MLSTM_SIG) den = fmaxf(fabsf(nn), 1.f);
-      if (ot == 0 && p.n_out) p.n_out[tok0 + r] = den;
-      if (ot == 0 && p.inv_den_out) p.inv_den_out[tok0 + r] = p.variant == MLSTM_SIG_NONORM ? 1.f : 1.f / (den + p.eps);
-    }
-    s_row[tid] = den;
-  }
-  __syncthreads();
-  T* out = (T*)p.out;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int r = r0 + ty * 4 + a;
-    if (r >= L) continue;
-    const size_t t = tok0 + r;
-    float rs;
-    if (MODE == PAR_H || MODE == PAR_DQ) rs = p.qk_scale * p.bbar[t];
-    else rs = p.abar[t];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const int o = o0 + tx * 4 + b;
-      if (o >= DO) continue;
-      float val = acc[a][b] + rs * acc2[a][b];
-      if (MODE == PAR_H && p.variant != MLSTM_SIG_NONORM) val = val / (s_row[ty * 4 + a] + p.eps);
-      out[t * DO + o] = from_f32<T>(val);
+      *reinterpret_cast<float4*>(Ps + swz(4 * tx + b, 4 * ty)) = make_float4(s[0][b], s[1][b], s[2][b], s[3][b]);
     }
+    Slice<T, false, VEC> x0, x1;
+    x0.fetch(X, o0, c0, tid);
+    x1.fetch(X, o0, c0 + KSL, tid);
+    __syncthreads();   // every thread has left the score product: its slices are free
+    x0.put(buf, tid);
+    x1.put(buf + SLICE, tid);
+    __syncthreads();
+#pragma unroll 1
+    for (int u = 0; u < 2; ++u) mma_slice(acc, Ps + u * SLICE, buf + u * SLICE, ty, tx);
+  }
+
+  float out[4][4];
+  acc.get(out);
+  T* dst = FW ? p.out_h : mode == PAR_DV ? p.out_dv : mode == PAR_DK ? p.out_dk : p.out_dq;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int r = r0 + 4 * ty + a;
+    if (FW) {
+      rowsum[a] = sum_columns(rowsum[a]);
+      qn[a] = sum_columns(qn[a]);
+    }
+    if (r >= L) continue;
+    const size_t t = tok0 + r;
+    if (FW) {
+      const float nn = rowsum[a] + rs[a] * qn[a];
+      float den = 1.f;
+      if (p.variant == MLSTM_EXP) den = fmaxf(fabsf(nn), expf(-s_m[r]));
+      else if (p.variant == MLSTM_SIG) den = fmaxf(fabsf(nn), 1.f);
+      const bool norm = p.variant != MLSTM_SIG_NONORM;
+      if (ot == 0 && tx == 0) {
+        if (p.n_out) p.n_out[t] = den;
+        if (p.inv_den_out) p.inv_den_out[t] = norm ? 1.f / (den + p.eps) : 1.f;
+      }
+      if (norm) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) out[a][b] = out[a][b] / (den + p.eps);
+      }
+    }
+    store4(dst + t * DO, o0 + 4 * tx, DO, VEC, make_float4(out[a][0], out[a][1], out[a][2], out[a][3]));
   }
 }
 
-static size_t par_smem_bytes(int L) {
-  return sizeof(float) * ((size_t)3 * L + 2 * TILE * (KSL + 1) + 2 * TILE * (TILE + 1) + 2 * TILE + KSL);
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(NTHR, 3) par_fw_kernel(ParArgs<T> p) {
+  extern __shared__ __align__(16) float smem[];
+  const int n_ot = (p.DHHV + TILE - 1) / TILE;
+  par_tile<T, true, VEC>(p, PAR_H, blockIdx.x % n_ot, blockIdx.x / n_ot, blockIdx.y, smem);
+}
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(NTHR, 3) par_bw_kernel(ParArgs<T> p) {
+  extern __shared__ __align__(16) float smem[];
+  const int n_v = (p.DHHV + TILE - 1) / TILE, n_k = (p.DHQK + TILE - 1) / TILE;
+  const int n = n_v + 2 * n_k, x = blockIdx.x % n, bc = blockIdx.x / n;
+  // the modes with the longer contraction first
+  const int mode = x < n_k ? PAR_DK : x < 2 * n_k ? PAR_DQ : PAR_DV;
+  par_tile<T, false, VEC>(p, mode, x < n_k ? x : x < 2 * n_k ? x - n_k : x - 2 * n_k, bc, blockIdx.y, smem);
+}
+
+static size_t par_smem_bytes(int L, int DHQK) {
+  return sizeof(float) * ((size_t)4 * SLICE + TILE * TILE + 3 * L + ceil_div(DHQK, KSL) * KSL);
 }
 
 // ---- launchers ----------------------------------------------------------------------------------------
-template <typename T, typename TS>
-int rec_fw_t(const void* k, const void* v, const GateBuffers& gb, const float* c_initial, const float* n_initial,
-             void* c_states, float* n_states, float* c_last, float* n_last, const ChunkwiseDims& d, cudaStream_t st) {
-  PhaseScope ps(PH_REC_FW, st);
-  dim3 grid(ceil_div(d.DHHV, TILE) * d.B * d.NH, ceil_div(d.DHQK, TILE));
-  rec_kernel<T, TS, false><<<grid, NTHR, 0, st>>>((const T*)k, (const T*)v, gb.abar, 1.f, nullptr, gb.gbar, c_initial,
-                                                  n_initial, (TS*)c_states, n_states, c_last, n_last, d.S, d.L, d.NC,
-                                                  d.DHQK, d.DHHV);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
-}
-template <typename T, typename TS>
-int rec_bw_t(const void* q, const void* dh, const GateBuffers& gb, const float* dc_last, void* dc_states,
-             float* dc_initial, const ChunkwiseDims& d, cudaStream_t st) {
-  PhaseScope ps(PH_REC_BW, st);
-  dim3 grid(ceil_div(d.DHHV, TILE) * d.B * d.NH, ceil_div(d.DHQK, TILE));
-  rec_kernel<T, TS, true><<<grid, NTHR, 0, st>>>((const T*)q, (const T*)dh, gb.bbar, d.qk_scale, gb.inv_den, gb.gbar,
-                                                 dc_last, nullptr, (TS*)dc_states, nullptr, dc_initial, nullptr, d.S,
-                                                 d.L, d.NC, d.DHQK, d.DHHV);
+static bool vec_dims(const ChunkwiseDims& d) { return d.DHQK % 4 == 0 && d.DHHV % 4 == 0; }
+
+template <bool BWD>
+static int launch_rec_scan(float* c_states, const float* c_init, float* c_final, float* n_states, const float* n_init,
+                           float* n_final, const float* gbar, const ChunkwiseDims& d, cudaStream_t st) {
+  const size_t E = (size_t)d.DHQK * d.DHHV;
+  const int V = E % 4 == 0 ? 4 : 1;
+  const int nblk = (int)((E / V + (n_states ? d.DHQK : 0) + 127) / 128);
+  const unsigned grid = (unsigned)nblk * (unsigned)(d.B * d.NH);
+  if (V == 4) rec_scan_kernel<4, BWD><<<grid, 128, 0, st>>>(c_states, c_init, c_final, n_states, n_init, n_final, gbar, d.NC, d.DHQK, d.DHHV, nblk);
+  else rec_scan_kernel<1, BWD><<<grid, 128, 0, st>>>(c_states, c_init, c_final, n_states, n_init, n_final, gbar, d.NC, d.DHQK, d.DHHV, nblk);
   MLSTM_LAUNCH_CHECK();
   return MLSTM_OK;
 }
 
-template <typename T, typename TS, int MODE>
-int par_launch(ParArgs<T, TS>& a, const ChunkwiseDims& d, cudaStream_t st) {
-  const int DO = (MODE == PAR_H || MODE == PAR_DV) ? d.DHHV : d.DHQK;
-  const size_t smem = par_smem_bytes(d.L);
-  auto kern = par_kernel<T, TS, MODE>;
+template <typename T, bool BWD>
+static int rec_t(const RecArgs<T>& a, const ChunkwiseDims& d, cudaStream_t st) {
+  PhaseScope ps(BWD ? PH_REC_BW : PH_REC_FW, st);
+  const unsigned tiles = (unsigned)ceil_div(d.DHHV, TILE) * ceil_div(d.DHQK, TILE) * (unsigned)(d.B * d.NH);
+  if (a.c_states == nullptr) {
+    if (vec_dims(d)) rec_final_kernel<T, BWD, true><<<tiles, NTHR, 0, st>>>(a);
+    else rec_final_kernel<T, BWD, false><<<tiles, NTHR, 0, st>>>(a);
+    MLSTM_LAUNCH_CHECK();
+    return MLSTM_OK;
+  }
+  if (vec_dims(d)) rec_part_kernel<T, BWD, true><<<tiles * (unsigned)d.NC, NTHR, 0, st>>>(a);
+  else rec_part_kernel<T, BWD, false><<<tiles * (unsigned)d.NC, NTHR, 0, st>>>(a);
+  MLSTM_LAUNCH_CHECK();
+  return launch_rec_scan<BWD>(a.c_states, a.c_init, a.c_final, a.n_states, a.n_init, a.n_final, a.gbar, d, st);
+}
+
+template <typename T>
+static int par_t(ParArgs<T>& a, bool backward, const ChunkwiseDims& d, cudaStream_t st) {
+  PhaseScope ps(backward ? PH_PAR_BW : PH_PAR_FW, st);
+  const size_t smem = par_smem_bytes(d.L, d.DHQK);
+  const int n_v = ceil_div(d.DHHV, TILE), n_k = ceil_div(d.DHQK, TILE);
+  const dim3 grid((unsigned)(backward ? n_v + 2 * n_k : n_v) * (unsigned)(d.B * d.NH * d.NC), ceil_div(d.L, TILE));
+  auto kern = vec_dims(d) ? (backward ? par_bw_kernel<T, true> : par_fw_kernel<T, true>)
+                          : (backward ? par_bw_kernel<T, false> : par_fw_kernel<T, false>);
   MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid(ceil_div(DO, TILE) * d.B * d.NH * d.NC, ceil_div(d.L, TILE));
   kern<<<grid, NTHR, smem, st>>>(a);
   MLSTM_LAUNCH_CHECK();
   return MLSTM_OK;
 }
 
-template <typename T, typename TS>
-ParArgs<T, TS> make_args(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
-                         const void* c_states, const void* dc_states, const float* n_states, const ChunkwiseDims& d) {
-  ParArgs<T, TS> a;
-  a.q = (const T*)q; a.k = (const T*)k; a.v = (const T*)v; a.dh = (const T*)dh;
+template <typename T>
+static ParArgs<T> par_args(const void* q, const void* k, const void* v, const GateBuffers& gb, const void* c_states,
+                           const ChunkwiseDims& d) {
+  ParArgs<T> a{};
+  a.q = (const T*)q; a.k = (const T*)k; a.v = (const T*)v; a.dh = (const T*)v;
   a.vecB = gb.vecB; a.iota = gb.iota; a.m_tok = gb.m_tok; a.abar = gb.abar; a.bbar = gb.bbar; a.inv_den = gb.inv_den;
-  a.c_states = (const TS*)c_states; a.dc_states = (const TS*)dc_states; a.n_states = n_states;
-  a.out = nullptr; a.n_out = nullptr; a.inv_den_out = nullptr;
+  a.c_states = (const float*)c_states;
   a.S = d.S; a.L = d.L; a.NC = d.NC; a.DHQK = d.DHQK; a.DHHV = d.DHHV; a.variant = d.variant;
   a.eps = d.eps; a.qk_scale = d.qk_scale;
   return a;
 }
 
-template <typename T, typename TS>
-int par_fw_t(const void* q, const void* k, const void* v, const GateBuffers& gb, const void* c_states,
-             const float* n_states, void* h, float* n_out, const ChunkwiseDims& d, cudaStream_t st) {
-  auto a = make_args<T, TS>(q, k, v, nullptr, gb, c_states, nullptr, n_states, d);
-  a.out = h; a.n_out = n_out; a.inv_den_out = gb.inv_den;
-  PhaseScope ps(PH_PAR_FW, st);
-  return par_launch<T, TS, PAR_H>(a, d, st);
-}
-template <typename T, typename TS>
-int par_bw_t(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb, const void* c_states,
-             const void* dc_states, void* dq, void* dk, void* dv, const ChunkwiseDims& d, cudaStream_t st) {
-  auto a = make_args<T, TS>(q, k, v, dh, gb, c_states, dc_states, nullptr, d);
-  int rc;
-  PhaseScope ps(PH_PAR_BW, st);
-  a.out = dv; if ((rc = par_launch<T, TS, PAR_DV>(a, d, st)) != MLSTM_OK) return rc;
-  a.out = dk; if ((rc = par_launch<T, TS, PAR_DK>(a, d, st)) != MLSTM_OK) return rc;
-  a.out = dq; if ((rc = par_launch<T, TS, PAR_DQ>(a, d, st)) != MLSTM_OK) return rc;
-  return MLSTM_OK;
-}
+#define MLSTM_DISPATCH(dtype, ...)                                          \
+  switch (dtype) {                                                          \
+    case MLSTM_F32: { using T = float; __VA_ARGS__ }                        \
+    case MLSTM_BF16: { using T = __nv_bfloat16; __VA_ARGS__ }               \
+    case MLSTM_F16: { using T = __half; __VA_ARGS__ }                       \
+  }                                                                         \
+  return MLSTM_ERR_DTYPE;
 
-#define MLSTM_DISPATCH(dtype, state_dtype, FN, ...)                                                      \
-  do {                                                                                                   \
-    if (state_dtype == MLSTM_F32) {                                                                      \
-      if (dtype == MLSTM_F32) return FN<float, float>(__VA_ARGS__);                                      \
-      if (dtype == MLSTM_BF16) return FN<__nv_bfloat16, float>(__VA_ARGS__);                             \
-      if (dtype == MLSTM_F16) return FN<__half, float>(__VA_ARGS__);                                     \
-    } else if (state_dtype == MLSTM_BF16) {                                                              \
-      if (dtype == MLSTM_BF16) return FN<__nv_bfloat16, __nv_bfloat16>(__VA_ARGS__);                     \
-    }                                                                                                    \
-    return MLSTM_ERR_DTYPE;                                                                              \
-  } while (0)
-
-int simt_recurrent_fw(int dtype, int state_dtype, const void* k, const void* v, const GateBuffers& gb,
-                      const float* c_initial, const float* n_initial, void* c_states, float* n_states,
-                      float* c_last, float* n_last, const ChunkwiseDims& d, cudaStream_t st) {
-  MLSTM_DISPATCH(dtype, state_dtype, rec_fw_t, k, v, gb, c_initial, n_initial, c_states, n_states, c_last, n_last, d, st);
+int simt_recurrent_fw(int dtype, const void* k, const void* v, const GateBuffers& gb, const float* c_initial,
+                      const float* n_initial, void* c_states, float* n_states, float* c_last, float* n_last,
+                      const ChunkwiseDims& d, cudaStream_t st) {
+  MLSTM_DISPATCH(dtype, {
+    return rec_t<T, false>(RecArgs<T>{(const T*)k, (const T*)v, gb.abar, nullptr, gb.gbar, 1.f, c_initial, n_initial,
+                                      (float*)c_states, n_states, c_last, n_last, d.S, d.L, d.NC, d.DHQK, d.DHHV}, d, st);
+  })
 }
-int simt_parallel_fw(int dtype, int state_dtype, const void* q, const void* k, const void* v, const GateBuffers& gb,
-                     const void* c_states, const float* n_states, void* h, float* n_out, const ChunkwiseDims& d,
+int simt_parallel_fw(int dtype, const void* q, const void* k, const void* v, const GateBuffers& gb, const void* c_states,
+                     const float* n_states, void* h, float* n_out, const ChunkwiseDims& d, cudaStream_t st) {
+  MLSTM_DISPATCH(dtype, {
+    auto a = par_args<T>(q, k, v, gb, c_states, d);
+    a.n_states = n_states; a.out_h = (T*)h; a.n_out = n_out; a.inv_den_out = gb.inv_den;
+    return par_t<T>(a, false, d, st);
+  })
+}
+int simt_recurrent_bw(int dtype, const void* q, const void* dh, const GateBuffers& gb, const float* dc_last, void* dc_states,
+                      float* dc_initial, const ChunkwiseDims& d, cudaStream_t st) {
+  MLSTM_DISPATCH(dtype, {
+    return rec_t<T, true>(RecArgs<T>{(const T*)q, (const T*)dh, gb.bbar, gb.inv_den, gb.gbar, d.qk_scale, dc_last, nullptr,
+                                     (float*)dc_states, nullptr, dc_initial, nullptr, d.S, d.L, d.NC, d.DHQK, d.DHHV}, d, st);
+  })
+}
+int simt_parallel_bw(int dtype, const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
+                     const void* c_states, const void* dc_states, void* dq, void* dk, void* dv, const ChunkwiseDims& d,
                      cudaStream_t st) {
-  MLSTM_DISPATCH(dtype, state_dtype, par_fw_t, q, k, v, gb, c_states, n_states, h, n_out, d, st);
-}
-int simt_recurrent_bw(int dtype, int state_dtype, const void* q, const void* dh, const GateBuffers& gb,
-                      const float* dc_last, void* dc_states, float* dc_initial, const ChunkwiseDims& d,
-                      cudaStream_t st) {
-  MLSTM_DISPATCH(dtype, state_dtype, rec_bw_t, q, dh, gb, dc_last, dc_states, dc_initial, d, st);
-}
-int simt_parallel_bw(int dtype, int state_dtype, const void* q, const void* k, const void* v, const void* dh,
-                     const GateBuffers& gb, const void* c_states, const void* dc_states, void* dq, void* dk, void* dv,
-                     const ChunkwiseDims& d, cudaStream_t st) {
-  MLSTM_DISPATCH(dtype, state_dtype, par_bw_t, q, k, v, dh, gb, c_states, dc_states, dq, dk, dv, d, st);
+  MLSTM_DISPATCH(dtype, {
+    auto a = par_args<T>(q, k, v, gb, c_states, d);
+    a.dh = (const T*)dh; a.dc_states = (const float*)dc_states;
+    a.out_dq = (T*)dq; a.out_dk = (T*)dk; a.out_dv = (T*)dv;
+    return par_t<T>(a, true, d, st);
+  })
 }
 
 }  // namespace mlstm

@@ -24,16 +24,16 @@ int launch_state_dot(const void* c_states, const void* dc_states, float* anchors
                      const ChunkwiseDims& d, cudaStream_t st);
 
 // chunkwise_simt.cu : portable CUDA-core kernels, any shape, any element type
-int simt_recurrent_fw(int dtype, int state_dtype, const void* k, const void* v, const GateBuffers& gb,
+int simt_recurrent_fw(int dtype, const void* k, const void* v, const GateBuffers& gb,
                       const float* c_initial, const float* n_initial, void* c_states, float* n_states,
                       float* c_last, float* n_last, const ChunkwiseDims& d, cudaStream_t st);
-int simt_parallel_fw(int dtype, int state_dtype, const void* q, const void* k, const void* v, const GateBuffers& gb,
+int simt_parallel_fw(int dtype, const void* q, const void* k, const void* v, const GateBuffers& gb,
                      const void* c_states, const float* n_states, void* h, float* n_out, const ChunkwiseDims& d,
                      cudaStream_t st);
-int simt_recurrent_bw(int dtype, int state_dtype, const void* q, const void* dh, const GateBuffers& gb,
+int simt_recurrent_bw(int dtype, const void* q, const void* dh, const GateBuffers& gb,
                       const float* dc_last, void* dc_states, float* dc_initial, const ChunkwiseDims& d,
                       cudaStream_t st);
-int simt_parallel_bw(int dtype, int state_dtype, const void* q, const void* k, const void* v, const void* dh,
+int simt_parallel_bw(int dtype, const void* q, const void* k, const void* v, const void* dh,
                      const GateBuffers& gb, const void* c_states, const void* dc_states, void* dq, void* dk, void* dv,
                      const ChunkwiseDims& d, cudaStream_t st);
 
