@@ -150,74 +150,128 @@ step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restric
   }
 }
 
-// T tokens in one launch, C slice resident in registers.  ROWS = rows of C per thread.
-template <typename T, int ROWS>
+// T tokens in one launch, the state resident in registers: a CTA owns all DHQK rows of a TV-wide column slice, a thread
+// ROWS rows of four columns.  Tokens go through in blocks of SEQ_TB.  What a block needs besides C - gates and their
+// max-state recursion, scaled q and k, v, q.n' - is prepared for the whole block at once (one exposed load latency and
+// three barriers per block), the token loop itself runs on registers and broadcast shared-memory reads without a
+// barrier, and the partial h of the block's tokens are summed over the warps together.  Token by token with five
+// barriers and a load latency each it took 4.3 us per token (4 sequences x 13 tokens, 8 heads 256/512: 56.5 us, of which
+// the state traffic is 5.3); now bound by the multiply-adds, 12 per row, thread and token.
+constexpr int SEQ_TB = 8;
+
+template <typename T, int ROWS, int TV>
 __global__ void __launch_bounds__(STEP_THREADS)
 step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                      const void* __restrict__ gi, const void* __restrict__ gf, int gate_dtype, const float* __restrict__ c,
                      const float* __restrict__ n, const float* __restrict__ m, T* __restrict__ h,
                      float* __restrict__ c_new, float* __restrict__ n_new, float* __restrict__ m_new, int Tn, int DHQK,
                      int DHHV, float eps) {
-  extern __shared__ float sm[];
-  float* s_q = sm;
-  float* s_k = s_q + DHQK;
-  float* s_n = s_k + DHQK;
-  float* s_red = s_n + DHQK;
-  __shared__ float s_warp[STEP_THREADS / 32];
-  __shared__ float s_den;
+  constexpr int CG = TV / 4, RG = STEP_THREADS / CG, NW = STEP_THREADS / 32;
+  constexpr int ND = ROWS * RG > STEP_THREADS ? 2 : 1;         // rows per thread of the q, k, n work
+  extern __shared__ __align__(16) float sm[];
+  float* s_v = sm;                                             // [SEQ_TB][TV]
+  float* s_red = s_v + SEQ_TB * TV;                            // [SEQ_TB][NW][TV] partial h
+  float2* s_kq = reinterpret_cast<float2*>(s_red + SEQ_TB * NW * TV);   // [SEQ_TB][DHQK] (ibar k, scaled q)
+  __shared__ float s_qn[SEQ_TB][NW], s_floor[SEQ_TB];
 
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // 1-D grid (no 65535 limit on batch x heads): the column tiles of one (batch, head) next to each other
-  const int ntile = (DHHV + STEP_TV - 1) / STEP_TV;
-  const int bh = blockIdx.x / ntile, tile = blockIdx.x % ntile, e0 = tile * STEP_TV;
-  const int cgi = tid % STEP_CG, rg = tid / STEP_CG;
+  const int ntile = (DHHV + TV - 1) / TV;
+  const int bh = blockIdx.x / ntile, tile = blockIdx.x % ntile, e0 = tile * TV;
+  const int cgi = tid % CG, rg = tid / CG;
   const int e = e0 + cgi * 4;
   const float scale = rsqrtf((float)DHQK);
 
   float4 C[ROWS];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    const int d = rg + r * STEP_RG;
-    C[r] = (c && d < DHQK && e < DHHV) ? *reinterpret_cast<const float4*>(c + ((size_t)bh * DHQK + d) * DHHV + e)
+    const int d = rg + r * RG;
+    C[r] = (c && d < DHQK && e < DHHV) ? __ldcs(reinterpret_cast<const float4*>(c + ((size_t)bh * DHQK + d) * DHHV + e))
                                       : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  for (int d = tid; d < DHQK; d += STEP_THREADS) s_n[d] = n ? n[(size_t)bh * DHQK + d] : 0.f;
+  float nv[ND];
+#pragma unroll
+  for (int u = 0; u < ND; ++u) {
+    const int d = tid + u * STEP_THREADS;
+    nv[u] = (n && d < DHQK) ? n[(size_t)bh * DHQK + d] : 0.f;
+  }
   float m_run = m ? m[bh] : 0.f;
-  __syncthreads();
 
-  for (int t = 0; t < Tn; ++t) {
-    const size_t tok = (size_t)bh * Tn + t;
-    const float lf = logsigmoid_f(load_gate(gf, tok, gate_dtype));
-    const float iv = load_gate(gi, tok, gate_dtype);
-    const float m_n = fmaxf(lf + m_run, iv);
-    const float fbar = expf(lf + m_run - m_n);
-    const float ibar = expf(iv - m_n);
-    m_run = m_n;
-    float qn = 0.f;
-    for (int d = tid; d < DHQK; d += STEP_THREADS) {
-      const float qs = to_f32(q[tok * DHQK + d]) * scale;
-      const float ik = ibar * to_f32(k[tok * DHQK + d]);
-      const float nn = fmaf(fbar, s_n[d], ik);
-      s_q[d] = qs; s_k[d] = ik; s_n[d] = nn;
-      qn = fmaf(qs, nn, qn);
+  for (int t0 = 0; t0 < Tn; t0 += SEQ_TB) {
+    const int nt = min(SEQ_TB, Tn - t0);
+    const size_t tok0 = (size_t)bh * Tn + t0;
+    // raw operands of the block first: all loads of a thread in flight together
+    T qr[ND][SEQ_TB], kr[ND][SEQ_TB];
+#pragma unroll
+    for (int u = 0; u < ND; ++u)
+#pragma unroll
+      for (int t = 0; t < SEQ_TB; ++t) {
+        const int d = tid + u * STEP_THREADS;
+        if (d < DHQK && t < nt) {
+          qr[u][t] = q[(tok0 + t) * DHQK + d];
+          kr[u][t] = k[(tok0 + t) * DHQK + d];
+        }
+      }
+    for (int idx = tid; idx < nt * TV; idx += STEP_THREADS) {
+      const int t = idx / TV, col = e0 + idx % TV;
+      s_v[idx] = col < DHHV ? to_f32(v[(tok0 + t) * DHHV + col]) : 0.f;
     }
-    qn = warp_sum(qn);
-    if ((tid & 31) == 0) s_warp[tid >> 5] = qn;
+    // gates: lane t holds token t of the block (every warp for itself); the recursion hands m from lane to lane
+    float lf = 0.f, iv = 0.f;
+    if (lane < nt) {
+      lf = logsigmoid_f(load_gate(gf, tok0 + lane, gate_dtype));
+      iv = load_gate(gi, tok0 + lane, gate_dtype);
+    }
+    float m_prev = 0.f, m_tok = 0.f;
+    for (int t = 0; t < nt; ++t) {
+      const float m_n = fmaxf(__shfl_sync(0xffffffffu, lf, t) + m_run, __shfl_sync(0xffffffffu, iv, t));
+      if (lane == t) { m_prev = m_run; m_tok = m_n; }
+      m_run = m_n;
+    }
+    const float fbar_l = expf(lf + m_prev - m_tok), ibar_l = expf(iv - m_tok);
+    if (warp == 0 && lane < nt) s_floor[lane] = expf(-m_tok);
+    float qn[SEQ_TB];
+#pragma unroll
+    for (int t = 0; t < SEQ_TB; ++t) {
+      const float fbar = __shfl_sync(0xffffffffu, fbar_l, t), ibar = __shfl_sync(0xffffffffu, ibar_l, t);
+      qn[t] = 0.f;
+#pragma unroll
+      for (int u = 0; u < ND; ++u) {
+        const int d = tid + u * STEP_THREADS;
+        if (d < DHQK && t < nt) {
+          const float qs = to_f32(qr[u][t]) * scale;
+          const float ik = ibar * to_f32(kr[u][t]);
+          nv[u] = fmaf(fbar, nv[u], ik);
+          s_kq[t * DHQK + d] = make_float2(ik, qs);
+          qn[t] = fmaf(qs, nv[u], qn[t]);
+        }
+      }
+    }
+    // the eight sums over the warp together: each step halves the tokens a lane still carries (9 shuffles, not 40)
+    static_assert(SEQ_TB == 8, "three halving steps");
+#pragma unroll
+    for (int half = 4; half >= 1; half >>= 1) {
+      const bool up = (lane & (half * 4)) != 0;
+#pragma unroll
+      for (int t = 0; t < half; ++t) {
+        const float mine = up ? qn[t + half] : qn[t], theirs = up ? qn[t] : qn[t + half];
+        qn[t] = mine + __shfl_xor_sync(0xffffffffu, theirs, half * 4);
+      }
+    }
+    qn[0] += __shfl_xor_sync(0xffffffffu, qn[0], 2);
+    qn[0] += __shfl_xor_sync(0xffffffffu, qn[0], 1);
+    if ((lane & 3) == 0) s_qn[lane >> 2][warp] = qn[0];   // bits 4, 3, 2 of the lane spell the token
     __syncthreads();
-    if (tid == 0) {
-      float a = 0.f;
-      for (int w = 0; w < STEP_THREADS / 32; ++w) a += s_warp[w];
-      s_den = fmaxf(fabsf(a), expf(-m_n)) + eps;
-    }
-    float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (e < DHHV) {
-      const float4 vv = make_float4(to_f32(v[tok * DHHV + e]), to_f32(v[tok * DHHV + e + 1]),
-                                    to_f32(v[tok * DHHV + e + 2]), to_f32(v[tok * DHHV + e + 3]));
+#pragma unroll 1
+    for (int t = 0; t < nt; ++t) {
+      const float fbar = __shfl_sync(0xffffffffu, fbar_l, t);
+      const float4 vv = *reinterpret_cast<const float4*>(s_v + t * TV + cgi * 4);
+      float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float2* kq = s_kq + t * DHQK + rg;
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
-        const int d = rg + r * STEP_RG;
-        if (d < DHQK) {
-          const float kk = s_k[d], qq = s_q[d];
+        if (rg + r * RG < DHQK) {
+          const float kk = kq[r * RG].x, qq = kq[r * RG].y;
           C[r].x = fmaf(fbar, C[r].x, kk * vv.x);
           C[r].y = fmaf(fbar, C[r].y, kk * vv.y);
           C[r].z = fmaf(fbar, C[r].z, kk * vv.z);
@@ -226,31 +280,39 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
           hv.z = fmaf(qq, C[r].z, hv.z); hv.w = fmaf(qq, C[r].w, hv.w);
         }
       }
-    }
-    hv.x += __shfl_xor_sync(0xffffffffu, hv.x, 16);
-    hv.y += __shfl_xor_sync(0xffffffffu, hv.y, 16);
-    hv.z += __shfl_xor_sync(0xffffffffu, hv.z, 16);
-    hv.w += __shfl_xor_sync(0xffffffffu, hv.w, 16);
-    if ((tid & 31) < 16) {
-      float* dst = s_red + (tid >> 5) * STEP_TV + cgi * 4;
-      dst[0] = hv.x; dst[1] = hv.y; dst[2] = hv.z; dst[3] = hv.w;
-    }
-    __syncthreads();
-    if (tid < STEP_TV && e0 + tid < DHHV) {
-      float a = 0.f;
+      // over the row groups of the warp (lanes CG apart)
 #pragma unroll
-      for (int w = 0; w < STEP_THREADS / 32; ++w) a += s_red[w * STEP_TV + tid];
-      h[tok * DHHV + e0 + tid] = from_f32<T>(a / s_den);
+      for (int o = CG; o < 32; o <<= 1) {
+        hv.x += __shfl_xor_sync(0xffffffffu, hv.x, o);
+        hv.y += __shfl_xor_sync(0xffffffffu, hv.y, o);
+        hv.z += __shfl_xor_sync(0xffffffffu, hv.z, o);
+        hv.w += __shfl_xor_sync(0xffffffffu, hv.w, o);
+      }
+      if (lane < CG) *reinterpret_cast<float4*>(s_red + (t * NW + warp) * TV + cgi * 4) = hv;
     }
     __syncthreads();
+    for (int idx = tid; idx < nt * TV; idx += STEP_THREADS) {
+      const int t = idx / TV, col = idx % TV;
+      if (e0 + col < DHHV) {
+        float a = 0.f, qn = 0.f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) { a += s_red[(t * NW + w) * TV + col]; qn += s_qn[t][w]; }
+        h[(tok0 + t) * DHHV + e0 + col] = from_f32<T>(a / (fmaxf(fabsf(qn), s_floor[t]) + eps));
+      }
+    }
+    __syncthreads();   // the block's buffers are free
   }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    const int d = rg + r * STEP_RG;
-    if (d < DHQK && e < DHHV) *reinterpret_cast<float4*>(c_new + ((size_t)bh * DHQK + d) * DHHV + e) = C[r];
+    const int d = rg + r * RG;
+    if (d < DHQK && e < DHHV) __stcs(reinterpret_cast<float4*>(c_new + ((size_t)bh * DHQK + d) * DHHV + e), C[r]);
   }
   if (tile == 0) {
-    for (int d = tid; d < DHQK; d += STEP_THREADS) n_new[(size_t)bh * DHQK + d] = s_n[d];
+#pragma unroll
+    for (int u = 0; u < ND; ++u) {
+      const int d = tid + u * STEP_THREADS;
+      if (d < DHQK) n_new[(size_t)bh * DHQK + d] = nv[u];
+    }
     if (tid == 0) m_new[bh] = m_run;
   }
 }
@@ -287,13 +349,13 @@ int launch_step(const void* q, const void* k, const void* v, const void* i, cons
   return MLSTM_ERR_DTYPE;
 }
 
-template <typename T, int ROWS>
+template <typename T, int ROWS, int TV>
 int step_seq_t(const void* q, const void* k, const void* v, const void* i, const void* f, int gate_dtype, const float* c,
                const float* n, const float* m, void* h, float* c_new, float* n_new, float* m_new, int B, int NH, int Tn,
                int DHQK, int DHHV, float eps, cudaStream_t st) {
-  const unsigned grid = (unsigned)ceil_div(DHHV, STEP_TV) * (unsigned)(B * NH);
-  const size_t smem = sizeof(float) * (3 * (size_t)DHQK + (STEP_THREADS / 32) * STEP_TV);
-  auto kern = step_sequence_kernel<T, ROWS>;
+  const unsigned grid = (unsigned)ceil_div(DHHV, TV) * (unsigned)(B * NH);
+  const size_t smem = sizeof(float) * SEQ_TB * (TV + (STEP_THREADS / 32) * TV + 2 * (size_t)DHQK);
+  auto kern = step_sequence_kernel<T, ROWS, TV>;
   if (smem > 48 * 1024) MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<grid, STEP_THREADS, smem, st>>>((const T*)q, (const T*)k, (const T*)v, i, f, gate_dtype, c, n, m,
                                          (T*)h, c_new, n_new, m_new, Tn, DHQK, DHHV, eps);
@@ -305,10 +367,14 @@ template <typename T>
 int step_seq_rows(const void* q, const void* k, const void* v, const void* i, const void* f, int gate_dtype,
                   const float* c, const float* n, const float* m, void* h, float* c_new, float* n_new, float* m_new,
                   int B, int NH, int Tn, int DHQK, int DHHV, float eps, cudaStream_t st) {
-  const int rows = ceil_div(DHQK, STEP_RG);
-#define SEQ_CASE(R) \
-  if (rows <= R) return step_seq_t<T, R>(q, k, v, i, f, gate_dtype, c, n, m, h, c_new, n_new, m_new, B, NH, Tn, DHQK, DHHV, eps, st);
-  SEQ_CASE(4) SEQ_CASE(8) SEQ_CASE(16) SEQ_CASE(32)
+  // 32-column slices while 64-column ones would leave SMs without a CTA: half the multiply-adds per thread and token,
+  // for q, k and n prepared once more
+  const bool narrow = (long)ceil_div(DHHV, 64) * B * NH < 148;
+#define SEQ_CASE(R, TV) \
+  if (ceil_div(DHQK, STEP_THREADS / (TV / 4)) <= R) \
+    return step_seq_t<T, R, TV>(q, k, v, i, f, gate_dtype, c, n, m, h, c_new, n_new, m_new, B, NH, Tn, DHQK, DHHV, eps, st);
+  if (narrow) { SEQ_CASE(4, 32) SEQ_CASE(8, 32) SEQ_CASE(16, 32) }
+  SEQ_CASE(4, 64) SEQ_CASE(8, 64) SEQ_CASE(16, 64) SEQ_CASE(32, 64)
 #undef SEQ_CASE
   return MLSTM_ERR_SHAPE;
 }

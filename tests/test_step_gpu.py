@@ -133,6 +133,25 @@ def test_sequence_kernel_equals_step_loop_and_chunkwise(dtype):
     assert max_rel_err(npy(h_seq), npy(h_cw)) < (1e-4 if dtype == torch.float32 else 2e-2)
 
 
+@pytest.mark.parametrize("B,S,DHQK,DHHV", [(1, 1, 40, 36), (1, 7, 256, 512), (1, 8, 512, 64), (1, 9, 72, 100),
+                                           (40, 17, 256, 64), (20, 8, 512, 128), (40, 16, 24, 68)])
+def test_sequence_kernel_token_blocks(B, S, DHQK, DHHV):
+    """Token counts around the kernel's blocks of eight, narrow and wide column slices (few / many sequences), row
+    counts of every register variant, head dims off the tiles: against the oracle's step by step recursion."""
+    NH = 4
+    inp = make_step_inputs(dict(seed=31 + S, B=B, NH=NH, DHQK=DHQK, DHHV=DHHV, steps=S))
+    q, k, v = (to_dev(np.moveaxis(inp[x], 0, 2), torch.float32) for x in "qkv")
+    i, f = (to_dev(np.moveaxis(inp[x][..., 0], 0, 2), torch.float32) for x in "if")
+    c, n, m = (to_dev(inp[x], torch.float32) for x in "cnm")
+    h, last = mk.mlstm_recurrent_sequence__b200(q, k, v, i, f, c, n, m, return_last_states=True)
+    state = tuple(inp[x].astype(np.float64) for x in "cnm")
+    for t in range(S):
+        ho, state = O.recurrent_step(*(inp[x][t].astype(np.float64) for x in "qkvif"), *state)
+        assert max_rel_err(npy(h[:, :, t]), ho) < 2e-5, t
+    for a, b in zip(last, state):
+        assert max_rel_err(npy(a), b) < 2e-5
+
+
 def test_step_full_size_decay_property():
     """Size-independent check at the full decode geometry (B=64, NH=8, 256/512): with k = 0 the step
     must scale C by exp(logsigmoid(f) + m - m') exactly and leave it otherwise unchanged."""
