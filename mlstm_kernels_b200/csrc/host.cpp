@@ -66,6 +66,7 @@ void check(int rc, const char* what) {
 }
 
 size_t up256(size_t n) { return (n + 255) / 256 * 256; }
+Tensor bytes(size_t n, const at::Device& dev) { return empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, dev); }
 
 // ---- chunkwise ------------------------------------------------------------------------------------------
 PyObject* g_select_chunk_size = nullptr;   // chunkwise.select_chunk_size: the rule of the portable kernels, and its errors
@@ -95,7 +96,6 @@ Problem resolve(const Tensor& q, const Tensor& v, const Tensor& i, int L, int va
   return p;
 }
 
-Tensor bytes(size_t n, const at::Device& dev) { return empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, dev); }
 
 // What a forward leaves behind for its backward: the gate vectors and 1 / (denominator + eps) in one block, and the
 // per-chunk states where they are kept.

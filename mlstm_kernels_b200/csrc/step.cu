@@ -13,9 +13,6 @@
 namespace mlstm {
 
 constexpr int STEP_THREADS = 256;
-constexpr int STEP_TV = 64;              // columns per CTA
-constexpr int STEP_CG = STEP_TV / 4;     // threads across the columns (float4 each)
-constexpr int STEP_RG = STEP_THREADS / STEP_CG;  // row groups
 
 template <typename TS> struct Vec4;
 template <> struct Vec4<float> {
@@ -45,25 +42,45 @@ __device__ __forceinline__ float load_gate(const void* p, size_t idx, int gate_d
   return __half2float(static_cast<const __half*>(p)[idx]);
 }
 
-template <typename T, typename TS>
+// Bound by HBM where the state does not fit L2 (B = 256: 329 us, the copy bandwidth): four CTAs per SM, rows in batches of
+// eight loads then eight stores.  Bound by latency at small batch: while 64-wide column slices would leave SMs without a
+// CTA the slices are 32 wide (TV), twice the CTAs with half the rows per thread, and the first eight rows are requested
+// before anything waits for the gates, q, k or n (one sequence of 8 heads 256/512: 4.5 -> 3.6 us).  In the wide form the
+// early request costs registers, an SM then holds three CTAs, and B = 256 takes 5 % longer (forcing four CTAs by a
+// register bound: 1.5 %).
+template <typename T, typename TS, int TV, bool PDL>
 __global__ void __launch_bounds__(STEP_THREADS)
 step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const void* __restrict__ gi,
             const void* __restrict__ gf, int gate_dtype, const TS* __restrict__ c, const TS* __restrict__ n,
             const TS* __restrict__ m, T* __restrict__ h, TS* __restrict__ c_new, TS* __restrict__ n_new,
             TS* __restrict__ m_new, int DHQK, int DHHV, float eps) {
+  constexpr int CG = TV / 4, RG = STEP_THREADS / CG, NW = STEP_THREADS / 32, UNR = 8;
+  constexpr bool EARLY = TV == 32;
   extern __shared__ float sm[];
-  float* s_q = sm;             // [DHQK] scaled q
-  float* s_k = s_q + DHQK;     // [DHQK] ibar * k
-  float* s_red = s_k + DHQK;   // [STEP_RG][STEP_TV] partial h, then reused
-  __shared__ float s_warp[STEP_THREADS / 32];
+  float* s_q = sm;                 // [DHQK] scaled q
+  float* s_k = s_q + DHQK;         // [DHQK] ibar k
+  float* s_red = s_k + DHQK;       // [NW][TV] partial h
+  __shared__ float s_warp[NW];
   __shared__ float s_den;
 
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // 1-D grid (no 65535 limit on batch x heads): the column tiles of one (batch, head) next to each other
-  const int ntile = (DHHV + STEP_TV - 1) / STEP_TV;
-  const int bh = blockIdx.x / ntile, tile = blockIdx.x % ntile, e0 = tile * STEP_TV;
-  const int cgi = tid % STEP_CG, rg = tid / STEP_CG;
+  const int ntile = (DHHV + TV - 1) / TV;
+  const int bh = blockIdx.x / ntile, tile = blockIdx.x % ntile, e0 = tile * TV;
+  const int cgi = tid % CG, rg = tid / CG;
   const int e = e0 + cgi * 4;
+  const bool live = e < DHHV;
+
+  if (PDL) {
+    pdl_launch_dependents();
+    pdl_wait();
+  }
+  float4 first[EARLY ? UNR : 1];
+  if (EARLY && live) {
+#pragma unroll
+    for (int u = 0; u < UNR; ++u)
+      if (rg + u * RG < DHQK) first[EARLY ? u : 0] = Vec4<TS>::load(c + ((size_t)bh * DHQK + rg + u * RG) * DHHV + e);
+  }
 
   const float lf = logsigmoid_f(load_gate(gf, bh, gate_dtype));
   const float iv = load_gate(gi, bh, gate_dtype);
@@ -85,67 +102,66 @@ step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restric
     if (tile == 0) n_new[(size_t)bh * DHQK + d] = from_f32<TS>(nn);
   }
   qn = warp_sum(qn);
-  if ((tid & 31) == 0) s_warp[tid >> 5] = qn;
+  if (lane == 0) s_warp[warp] = qn;
   __syncthreads();
   if (tid == 0) {
     float t = 0.f;
-    for (int w = 0; w < STEP_THREADS / 32; ++w) t += s_warp[w];
+    for (int w = 0; w < NW; ++w) t += s_warp[w];
     s_den = fmaxf(fabsf(t), expf(-m_n)) + eps;
     if (tile == 0) m_new[bh] = from_f32<TS>(m_n);
   }
 
-  float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (e < DHHV) {
-    const float4 vv = make_float4(to_f32(v[(size_t)bh * DHHV + e]), to_f32(v[(size_t)bh * DHHV + e + 1]),
-                                  to_f32(v[(size_t)bh * DHHV + e + 2]), to_f32(v[(size_t)bh * DHHV + e + 3]));
+  float4 hv = make_float4(0.f, 0.f, 0.f, 0.f), vv = hv;
+  auto step_row = [&](int d, const float4& x, TS* cn) {
+    const float kk = s_k[d], qq = s_q[d];
+    float4 o;
+    o.x = fmaf(fbar, x.x, kk * vv.x);
+    o.y = fmaf(fbar, x.y, kk * vv.y);
+    o.z = fmaf(fbar, x.z, kk * vv.z);
+    o.w = fmaf(fbar, x.w, kk * vv.w);
+    Vec4<TS>::store(cn + (size_t)d * DHHV, o);
+    hv.x = fmaf(qq, o.x, hv.x); hv.y = fmaf(qq, o.y, hv.y);
+    hv.z = fmaf(qq, o.z, hv.z); hv.w = fmaf(qq, o.w, hv.w);
+  };
+  if (live)
+    vv = make_float4(to_f32(v[(size_t)bh * DHHV + e]), to_f32(v[(size_t)bh * DHHV + e + 1]),
+                     to_f32(v[(size_t)bh * DHHV + e + 2]), to_f32(v[(size_t)bh * DHHV + e + 3]));
+  if (live) {
     const TS* cp = c + (size_t)bh * DHQK * DHHV + e;
     TS* cn = c_new + (size_t)bh * DHQK * DHHV + e;
-    constexpr int UNR = 8;
     int d = rg;
-    for (; d + (UNR - 1) * STEP_RG < DHQK; d += UNR * STEP_RG) {
+    if (EARLY) {
+#pragma unroll
+      for (int u = 0; u < UNR; ++u, d += RG)
+        if (d < DHQK) step_row(d, first[EARLY ? u : 0], cn);
+    }
+    for (; d + (UNR - 1) * RG < DHQK; d += UNR * RG) {
       float4 cv[UNR];
 #pragma unroll
-      for (int u = 0; u < UNR; ++u) cv[u] = Vec4<TS>::load(cp + (size_t)(d + u * STEP_RG) * DHHV);
+      for (int u = 0; u < UNR; ++u)
+        cv[u] = Vec4<TS>::load(cp + (size_t)(d + u * RG) * DHHV);
 #pragma unroll
-      for (int u = 0; u < UNR; ++u) {
-        const float kk = s_k[d + u * STEP_RG], qq = s_q[d + u * STEP_RG];
-        float4 o;
-        o.x = fmaf(fbar, cv[u].x, kk * vv.x);
-        o.y = fmaf(fbar, cv[u].y, kk * vv.y);
-        o.z = fmaf(fbar, cv[u].z, kk * vv.z);
-        o.w = fmaf(fbar, cv[u].w, kk * vv.w);
-        Vec4<TS>::store(cn + (size_t)(d + u * STEP_RG) * DHHV, o);
-        hv.x = fmaf(qq, o.x, hv.x); hv.y = fmaf(qq, o.y, hv.y);
-        hv.z = fmaf(qq, o.z, hv.z); hv.w = fmaf(qq, o.w, hv.w);
-      }
+      for (int u = 0; u < UNR; ++u) step_row(d + u * RG, cv[u], cn);
     }
-    for (; d < DHQK; d += STEP_RG) {
-      const float4 cv = Vec4<TS>::load(cp + (size_t)d * DHHV);
-      const float kk = s_k[d], qq = s_q[d];
-      float4 o;
-      o.x = fmaf(fbar, cv.x, kk * vv.x);
-      o.y = fmaf(fbar, cv.y, kk * vv.y);
-      o.z = fmaf(fbar, cv.z, kk * vv.z);
-      o.w = fmaf(fbar, cv.w, kk * vv.w);
-      Vec4<TS>::store(cn + (size_t)d * DHHV, o);
-      hv.x = fmaf(qq, o.x, hv.x); hv.y = fmaf(qq, o.y, hv.y);
-      hv.z = fmaf(qq, o.z, hv.z); hv.w = fmaf(qq, o.w, hv.w);
-    }
+    for (; d < DHQK; d += RG) step_row(d, Vec4<TS>::load(cp + (size_t)d * DHHV), cn);
   }
-  // reduce the column partials over the row groups: first inside the warp (a warp spans 2 row groups)
-  hv.x += __shfl_xor_sync(0xffffffffu, hv.x, 16);
-  hv.y += __shfl_xor_sync(0xffffffffu, hv.y, 16);
-  hv.z += __shfl_xor_sync(0xffffffffu, hv.z, 16);
-  hv.w += __shfl_xor_sync(0xffffffffu, hv.w, 16);
-  if ((tid & 31) < 16) {
-    float* dst = s_red + (tid >> 5) * STEP_TV + cgi * 4;
+  // reduce the column partials over the row groups: first inside the warp (lanes CG apart), then over the warps
+#pragma unroll
+  for (int o = CG; o < 32; o <<= 1) {
+    hv.x += __shfl_xor_sync(0xffffffffu, hv.x, o);
+    hv.y += __shfl_xor_sync(0xffffffffu, hv.y, o);
+    hv.z += __shfl_xor_sync(0xffffffffu, hv.z, o);
+    hv.w += __shfl_xor_sync(0xffffffffu, hv.w, o);
+  }
+  if (lane < CG) {
+    float* dst = s_red + warp * TV + cgi * 4;
     dst[0] = hv.x; dst[1] = hv.y; dst[2] = hv.z; dst[3] = hv.w;
   }
   __syncthreads();
-  if (tid < STEP_TV && e0 + tid < DHHV) {
+  if (tid < TV && e0 + tid < DHHV) {
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < STEP_THREADS / 32; ++w) t += s_red[w * STEP_TV + tid];
+    for (int w = 0; w < NW; ++w) t += s_red[w * TV + tid];
     h[(size_t)bh * DHHV + e0 + tid] = from_f32<T>(t / s_den);
   }
 }
@@ -318,20 +334,31 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
 }
 
 // ---- launchers ----------------------------------------------------------------------------------------
+template <typename T, typename TS, int TV, bool PDL>
+static int step_tv(const void* q, const void* k, const void* v, const void* i, const void* f, int gate_dtype, const void* c,
+                   const void* n, const void* m, void* h, void* c_new, void* n_new, void* m_new, int B, int NH, int DHQK,
+                   int DHHV, float eps, cudaStream_t st) {
+  const unsigned grid = (unsigned)ceil_div(DHHV, TV) * (unsigned)(B * NH);
+  const size_t smem = sizeof(float) * (2 * (size_t)DHQK + (STEP_THREADS / 32) * TV);
+  auto kern = step_kernel<T, TS, TV, PDL>;
+  if (smem > 48 * 1024) MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  return launch_pdl(PDL, kern, grid, STEP_THREADS, smem, st, (const T*)q, (const T*)k, (const T*)v, i, f, gate_dtype,
+                    (const TS*)c, (const TS*)n, (const TS*)m, (T*)h, (TS*)c_new, (TS*)n_new, (TS*)m_new, DHQK, DHHV, eps);
+}
+
 template <typename T, typename TS>
 int step_t(const void* q, const void* k, const void* v, const void* i, const void* f, int gate_dtype, const void* c,
            const void* n, const void* m, void* h, void* c_new, void* n_new, void* m_new, int B, int NH, int DHQK,
            int DHHV, float eps, cudaStream_t st) {
   PhaseScope ps(PH_STEP, st);
-  const unsigned grid = (unsigned)ceil_div(DHHV, STEP_TV) * (unsigned)(B * NH);
-  const size_t smem = sizeof(float) * (2 * (size_t)DHQK + (STEP_THREADS / 32) * STEP_TV);
-  auto kern = step_kernel<T, TS>;
-  if (smem > 48 * 1024) MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<grid, STEP_THREADS, smem, st>>>((const T*)q, (const T*)k, (const T*)v, i, f, gate_dtype,
-                                         (const TS*)c, (const TS*)n, (const TS*)m, (T*)h, (TS*)c_new, (TS*)n_new,
-                                         (TS*)m_new, DHQK, DHHV, eps);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+#define STEP_RUN(TV, PDL) step_tv<T, TS, TV, PDL>(q, k, v, i, f, gate_dtype, c, n, m, h, c_new, n_new, m_new, B, NH, DHQK, DHHV, eps, st)
+  // launches of more than one wave (four CTAs per SM) start plainly: they gain nothing from overlapping their start with
+  // the last step's end
+  const long ctas = (long)ceil_div(DHHV, 64) * B * NH;
+  if (ctas < 148) return STEP_RUN(32, true);
+  if (ctas <= 4 * 148) return STEP_RUN(64, true);
+  return STEP_RUN(64, false);
+#undef STEP_RUN
 }
 
 int launch_step(const void* q, const void* k, const void* v, const void* i, const void* f, const void* c,
