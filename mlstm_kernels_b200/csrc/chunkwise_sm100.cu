@@ -127,11 +127,8 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
         const float g = __shfl_sync(0xffffffffu, g_blk, s & 31);
         if (lane == 0) s_g[s & 7] = g;   // read two or more barrier hand-overs later (MMA commit -> state warps)
       }
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(&bar_empty[st], ((h / REC_STAGES) & 1) ^ 1, &s_abort, &g_sm100_status, 101) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      if (lane == 0) {
+      if (!mbar_wait(&bar_empty[st], ((h / REC_STAGES) & 1) ^ 1, &s_abort, &g_sm100_status, 101)) break;
+      if (elect_one()) {
         const int ck = BWD ? NC - 1 - s : s;
         // token rows past the end of the sequence (ragged last chunk) arrive as zeros; their scale slots hold zeros
         const int y = ck * CL + (h & 1) * REC_HALF;          // first token of this half chunk inside the sequence
@@ -153,7 +150,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_16(F16, 128, TN, 1, 1);
       for (int h = 0; h < NH2; ++h) {
         const int st = h % REC_STAGES, s = h >> 1, buf = s & 1;
@@ -221,7 +218,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
     }
   } else if (warp == 18) {
     // ---------------- store warp: one TMA store per 64-column box of each staged state tile ----------------
-    if (lane == 0 && p.c_states != nullptr) {
+    if (p.c_states != nullptr && elect_one()) {
       uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (BWD ? 0 : REC_NPART_BYTES);
       for (int n = 0; n <= NC; ++n) {
         const int ob = n & 1;
@@ -464,7 +461,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const int slot = LOWER ? ck : ck + 1;
       const int sz = bh * (NC + 1) + slot;   // slab of the state tensor (one DHQK x DHHV matrix per chunk boundary)
       int issued = 0;
@@ -527,7 +524,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_16(F16, 128, 128, 0, 0);
       const uint32_t idesc_st = ST_MN ? umma_idesc_16(F16, 128, 128, 0, 1) : umma_idesc_16(F16, 128, 128, 0, 0);
       constexpr uint32_t idesc_x = umma_idesc_16(F16, 128, 128, 0, 1);

@@ -56,6 +56,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* a
   return false;
 }
 
+// True in one lane of a fully active warp.  Preferred to `lane == 0` for the threads that issue copies and MMAs: the compiler
+// then knows that one thread runs and keeps descriptors and coordinates in uniform registers (a TMA issue takes 15 cycles
+// instead of 45).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---- proxies and fences -------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
