@@ -94,11 +94,11 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
   if (tid == 0) {
     s_abort = 0;
     for (int s = 0; s < REC_STAGES; ++s) {
-      mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); mbar_init(&bar_scaled[s], 256);
+      mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); mbar_init(&bar_scaled[s], 4);   // (arrivals once per warp)
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&bar_acc_full[s], 1); mbar_init(&bar_acc_free[s], 256); mbar_init(&bar_nsum[s], 256); mbar_init(&bar_nread[s], 1);
-      mbar_init(&bar_out_full[s], 256); mbar_init(&bar_out_free[s], 1);
+      mbar_init(&bar_acc_full[s], 1); mbar_init(&bar_acc_free[s], 8); mbar_init(&bar_nsum[s], 8); mbar_init(&bar_nread[s], 1);
+      mbar_init(&bar_out_full[s], 8); mbar_init(&bar_out_free[s], 1);
     }
     fence_barrier_init();
     tma_prefetch_desc(&mapL); tma_prefetch_desc(&mapR); tma_prefetch_desc(&mapS);
@@ -168,54 +168,60 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
     }
   } else if (warp < 10) {
     // ---------------- gating warps: scale the rows of the left tile in place; column sums give n ----------------
-    const int ct = tid - 64;                       // 0..255
+    // Two groups of four warps take the half chunks in turn: a stage costs 750 cycles of dependent work and 500 of waits and
+    // hand-over, which one group of eight paid for every stage (2700 cycles per chunk, the limit of the whole kernel).
+    const int grp = (warp - 2) >> 2, ct = (tid - 64) & 127;
+    const int row0 = ct >> 3;                      // rows row0 + 16 u of the stage, 16-byte piece ct & 7 of either box
     bool ok = true;
-    float ns[2][8];
-    for (int h = 0; h < NH2; ++h) {
+    for (int h = grp; h < NH2; h += 2) {
       const int st = h % REC_STAGES, s = h >> 1, nb = s & 1;
       if (!mbar_wait(&bar_full[st], (h / REC_STAGES) & 1, &s_abort, &g_sm100_status, 105)) { ok = false; break; }
       // two 64-column boxes of 64 rows x 128 B, 128-byte swizzle: the scale depends on the row only
-      uint8_t* sl = smem + st * REC_STAGE_BYTES;
-      if ((h & 1) == 0) {
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) ns[b][e] = 0.f;
-      }
+      uint8_t* sl = smem + st * REC_STAGE_BYTES + row0 * 128 + (ct & 7) * 16;
+      float sc[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int r = (ct >> 3) + 32 * (u & 1);
-        float sc = s_scale[st][r] * p.lmul;
-        if (BWD) sc *= s_scale2[st][r];
-        uint4* ptr = reinterpret_cast<uint4*>(sl + (u >> 1) * 8192 + r * 128 + (ct & 7) * 16);
-        uint4 v = *ptr;
-        uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float lo, hi;
-          Pair16<F16>::unpack(w[e], lo, hi);
-          lo *= sc; hi *= sc;
-          ns[u >> 1][2 * e] += lo; ns[u >> 1][2 * e + 1] += hi;
-          w[e] = Pair16<F16>::pack(lo, hi);
-        }
-        *ptr = make_uint4(w[0], w[1], w[2], w[3]);
+        sc[u] = s_scale[st][row0 + 16 * u] * p.lmul;
+        if (BWD) sc[u] *= s_scale2[st][row0 + 16 * u];
       }
-      float* npart = reinterpret_cast<float*>(smem + REC_STAGES * REC_STAGE_BYTES) + nb * (32 * 128);
-      if (do_n && (h & 1)) {
-        // the n warp has read the partial sums of chunk s - 2 out of this buffer
-        if (s >= 2 && !mbar_wait(&bar_nread[nb], ((s >> 1) - 1) & 1, &s_abort, &g_sm100_status, 109)) { ok = false; break; }
-        const int lc = (ct & 7) ^ ((ct >> 3) & 7);   // logical 16-byte column chunk behind the swizzle
+      uint64_t ns[2][4];
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          float4* dst = reinterpret_cast<float4*>(npart + (ct >> 3) * 128 + b * 64 + lc * 8);
-          dst[0] = make_float4(ns[b][0], ns[b][1], ns[b][2], ns[b][3]);
-          dst[1] = make_float4(ns[b][4], ns[b][5], ns[b][6], ns[b][7]);
+      for (int b = 0; b < 2; ++b) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint4*>(sl + b * 8192 + u * 2048);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ns[b][e] = 0ull;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint64_t ss = f2(sc[u], sc[u]);
+          uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint64_t x = mul2(unpack2<F16>(w[e]), ss);
+            ns[b][e] = add2(ns[b][e], x);
+            w[e] = pack2<F16>(x);
+          }
+          *reinterpret_cast<uint4*>(sl + b * 8192 + u * 2048) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
       fence_proxy_async_smem();
-      mbar_arrive(&bar_scaled[st]);
-      if (do_n && (h & 1)) mbar_arrive(&bar_nsum[nb]);   // partial column sums of chunk s are complete (n warp)
+      warp_arrive(&bar_scaled[st]);
+      if (do_n) {   // partial column sums of this half: 16 rows of the chunk's 32
+        // the n warp has read the partial sums of chunk s - 2 out of this buffer
+        if (s >= 2 && !mbar_wait(&bar_nread[nb], ((s >> 1) - 1) & 1, &s_abort, &g_sm100_status, 109)) { ok = false; break; }
+        float* npart = reinterpret_cast<float*>(smem + REC_STAGES * REC_STAGE_BYTES) + nb * (32 * 128) + (grp * 16 + row0) * 128;
+        const int lc = (ct & 7) ^ (row0 & 7);   // logical 16-byte column chunk behind the swizzle
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          ulonglong2* dst = reinterpret_cast<ulonglong2*>(npart + b * 64 + lc * 8);
+          dst[0] = make_ulonglong2(ns[b][0], ns[b][1]);
+          dst[1] = make_ulonglong2(ns[b][2], ns[b][3]);
+        }
+        warp_arrive(&bar_nsum[nb]);   // (complete when both halves of chunk s are in)
+      }
     }
+    (void)ok;
   } else if (warp == 18) {
     // ---------------- store warp: one TMA store per 64-column box of each staged state tile ----------------
     if (p.c_states != nullptr && elect_one()) {
@@ -297,7 +303,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
         *reinterpret_cast<uint4*>(rowp + (((piece0 + c) ^ (row & 7)) << 4)) = v;
       }
       fence_proxy_async_smem();
-      mbar_arrive(&bar_out_full[ob]);   // the store warp ships the tile
+      warp_arrive(&bar_out_full[ob]);   // the store warp ships the tile
       ++n_out;
       return true;
     };
@@ -317,7 +323,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
         for (int c = 0; c < 16; ++c) C[q4 * 16 + c] = fmaf(g, C[q4 * 16 + c], __uint_as_float(rr[c]));
       }
       tc_fence_before_sync();
-      mbar_arrive(&bar_acc_free[buf]);
+      warp_arrive(&bar_acc_free[buf]);
       ok = store_c();
     }
     if (ok && p.c_final) {

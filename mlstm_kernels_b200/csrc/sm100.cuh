@@ -65,6 +65,12 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// one arrival per warp, after what its lanes did before
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+  __syncwarp();
+  if (elect_one()) mbar_arrive(bar);
+}
+
 // ---- proxies and fences -------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -243,6 +249,40 @@ template <bool F16> struct Pair16 {
     }
   }
 };
+
+// Two floats in one register pair: packed instructions halve the issue slots of the element-wise work.
+__device__ __forceinline__ uint64_t f2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unf2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// two 16-bit elements as a pair of floats, and back
+template <bool F16> __device__ __forceinline__ uint64_t unpack2(uint32_t w) {
+  float lo, hi;
+  Pair16<F16>::unpack(w, lo, hi);
+  return f2(lo, hi);
+}
+template <bool F16> __device__ __forceinline__ uint32_t pack2(uint64_t v) {
+  float lo, hi;
+  unf2(v, lo, hi);
+  return Pair16<F16>::pack(lo, hi);
+}
 
 }  // namespace sm100
 
