@@ -49,13 +49,14 @@ struct RecParams {
 
 constexpr int REC_THREADS = 640;                 // warp 0 TMA, 1 MMA, 2..9 gate the left tile, 10..17 own the state, 18 stores it, 19 keeps n
 constexpr int REC_HALF = 64;                     // tokens per ring stage: half a chunk
-constexpr int REC_STAGE_BYTES = 32768;           // 64 tokens: left tile 16 KB + right tile 16 KB
 constexpr int REC_NPART_BYTES = 2 * 32 * 128 * 4;   // double-buffered partial column sums of the gated left tile
-constexpr int REC_OUT_BYTES = 2 * 32768;         // double-buffered bf16 state tile staged for the TMA store
-// operand ring depth (two chunks in flight)
-constexpr int rec_stages(bool) { return 4; }
-constexpr int rec_smem_bytes(bool bwd) {
-  return rec_stages(bwd) * REC_STAGE_BYTES + (bwd ? 0 : REC_NPART_BYTES) + REC_OUT_BYTES + 1024;
+constexpr int rec_stage_bytes(int TN) { return 16384 + TN * 128; }    // 64 tokens: left tile 16 KB + right tile
+constexpr int rec_out_bytes(int TN) { return TN * 256; }              // 16-bit state tile staged for the TMA store (two of them)
+// Operand ring depth, as deep as shared memory allows.  A stage comes round in about 4600 cycles (load 2500, gating and
+// hand-over 1300, MMA and hand-back 800), so the 64-column form with its smaller stages runs three chunks ahead.
+constexpr int rec_stages(bool bwd, int TN) { return TN == 128 ? 4 : (bwd ? 7 : 6); }
+constexpr int rec_smem_bytes(bool bwd, int TN) {
+  return rec_stages(bwd, TN) * rec_stage_bytes(TN) + (bwd ? 0 : REC_NPART_BYTES) + 2 * rec_out_bytes(TN) + 1024;
 }
 
 // One ring stage holds 64 tokens of the left and of the right operand (boxes of 64 rows x 64 columns, 8 KB each:
@@ -71,7 +72,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
           const __grid_constant__ CUtensorMap mapS, RecParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int REC_STAGES = rec_stages(BWD);
+  constexpr int REC_STAGES = rec_stages(BWD, TN), REC_STAGE_BYTES = rec_stage_bytes(TN), REC_OUT = rec_out_bytes(TN);
   __shared__ uint64_t bar_full[REC_STAGES], bar_empty[REC_STAGES], bar_scaled[REC_STAGES], bar_acc_full[2], bar_acc_free[2], bar_nsum[2], bar_nread[2], bar_out_full[2], bar_out_free[2];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;   // set by the first wait of this CTA that runs out; every other wait polls it
@@ -231,8 +232,8 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
         if (!mbar_wait(&bar_out_full[ob], (n >> 1) & 1, &s_abort, &g_sm100_status, 108)) break;
         const int slot = BWD ? NC - n : n;
         const int z = bh * (NC + 1) + slot;
-        tma_store_3d(&mapS, stage_base + ob * 32768, e0, d0, z);
-        if (TN == 128 && e0 + 64 < p.DHHV) tma_store_3d(&mapS, stage_base + ob * 32768 + 16384, e0 + 64, d0, z);
+        tma_store_3d(&mapS, stage_base + ob * REC_OUT, e0, d0, z);
+        if (TN == 128 && e0 + 64 < p.DHHV) tma_store_3d(&mapS, stage_base + ob * REC_OUT + 16384, e0 + 64, d0, z);
         tma_store_commit();
         asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the previous tile has left its buffer
         if (n >= 1) mbar_arrive(&bar_out_free[ob ^ 1]);
@@ -293,7 +294,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
       const int ob = n_out & 1;
       if (n_out >= 2 && !mbar_wait(&bar_out_free[ob], ((n_out >> 1) - 1) & 1, &s_abort, &g_sm100_status, 107)) return false;
       // TN = 128: each group fills its own 64-column box; TN = 64: the groups share one box (four 16-byte pieces each)
-      uint8_t* rowp = stage_base + ob * 32768 + (TN == 128 ? half * 16384 : 0) + row * 128;
+      uint8_t* rowp = stage_base + ob * REC_OUT + (TN == 128 ? half * 16384 : 0) + row * 128;
       const int piece0 = (TN == 128) ? 0 : half * 4;
 #pragma unroll
       for (int c = 0; c < HC / 8; ++c) {
@@ -954,9 +955,9 @@ static int launch_rec_tn(const CUtensorMap& mL, const CUtensorMap& mR, const CUt
                          const ChunkwiseDims& d, int units, cudaStream_t st) {
   auto kern = rec_sm100<BWD, TN, F16>;
   static bool attr_done[64] = {};
-  if (int rc = set_smem_once(kern, rec_smem_bytes(BWD), attr_done)) return rc;
+  if (int rc = set_smem_once(kern, rec_smem_bytes(BWD, TN), attr_done)) return rc;
   const unsigned grid = (unsigned)((d.DHHV + TN - 1) / TN) * (unsigned)((d.DHQK + 127) / 128) * (unsigned)units;
-  kern<<<grid, REC_THREADS, rec_smem_bytes(BWD), st>>>(mL, mR, mS, rp);
+  kern<<<grid, REC_THREADS, rec_smem_bytes(BWD, TN), st>>>(mL, mR, mS, rp);
   MLSTM_LAUNCH_CHECK();
   return MLSTM_OK;
 }
