@@ -122,8 +122,8 @@ class UnitChains {
       return;
     }
     side_ = s;
-    first_ = UnitRange{0, (units + 1) / 2};
-    second_ = UnitRange{first_.count, -1};
+    first_ = UnitRange{0, (units + 1) / 2, false};
+    second_ = UnitRange{first_.count, -1, false};
   }
   ~UnitChains() { (void)join(); }
   UnitChains(const UnitChains&) = delete;

@@ -109,6 +109,8 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = s_tmem;
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -446,6 +448,8 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
   tc_fence_after_sync();
   const uint32_t tmem = sh.tmem;
   const uint32_t tS = tmem, tAcc = tmem + 128;
+  pdl_launch_dependents();
+  pdl_wait();
   // Ring loads, in order: ND (A, B) slice pairs for the score product, ND (A, state) slice pairs for the inter-chunk
   // product (A comes from L2 the second time), the X tile, the E tile.  The score is complete - and the element-wise
   // warps start gating - while the second group is still arriving.
@@ -952,14 +956,12 @@ static bool state_map(CUtensorMap* m, const void* base, const ChunkwiseDims& d, 
 
 template <bool BWD, int TN, bool F16>
 static int launch_rec_tn(const CUtensorMap& mL, const CUtensorMap& mR, const CUtensorMap& mS, const RecParams& rp,
-                         const ChunkwiseDims& d, int units, cudaStream_t st) {
+                         const ChunkwiseDims& d, int units, bool overlap, cudaStream_t st) {
   auto kern = rec_sm100<BWD, TN, F16>;
   static bool attr_done[64] = {};
   if (int rc = set_smem_once(kern, rec_smem_bytes(BWD, TN), attr_done)) return rc;
   const unsigned grid = (unsigned)((d.DHHV + TN - 1) / TN) * (unsigned)((d.DHQK + 127) / 128) * (unsigned)units;
-  kern<<<grid, REC_THREADS, rec_smem_bytes(BWD, TN), st>>>(mL, mR, mS, rp);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  return launch_pdl(overlap && grid <= kPdlMaxCtas, kern, grid, REC_THREADS, rec_smem_bytes(BWD, TN), st, mL, mR, mS, rp);
 }
 
 // number of SMs of the current device (queried once per device)
@@ -996,8 +998,8 @@ static int launch_rec(const void* left, const void* right, RecParams rp, const C
   const long ctas128 = sm100_recurrence_ctas(d);
   const bool f16 = d.dtype == MLSTM_F16;
   if (2 * ctas128 <= sm_count())
-    return f16 ? launch_rec_tn<BWD, 64, true>(mL, mR, mS, rp, d, units, st) : launch_rec_tn<BWD, 64, false>(mL, mR, mS, rp, d, units, st);
-  return f16 ? launch_rec_tn<BWD, 128, true>(mL, mR, mS, rp, d, units, st) : launch_rec_tn<BWD, 128, false>(mL, mR, mS, rp, d, units, st);
+    return f16 ? launch_rec_tn<BWD, 64, true>(mL, mR, mS, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 64, false>(mL, mR, mS, rp, d, units, ur.overlap, st);
+  return f16 ? launch_rec_tn<BWD, 128, true>(mL, mR, mS, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 128, false>(mL, mR, mS, rp, d, units, ur.overlap, st);
 }
 
 int sm100_recurrent_fw(const void* k, const void* v, const GateBuffers& gb, const float* c_initial,
@@ -1058,10 +1060,8 @@ int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuf
   const int T = (d.DHHV + 127) / 128;
   pp.maxsub = par_maxsub([&](int m) { return (long)ceil_div(T, m) * d.NC * units; }, T);
   const unsigned grid = (unsigned)ceil_div(T, pp.maxsub) * (unsigned)d.NC * (unsigned)units;
-  if (f16) par_fw_sm100<true><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mC, pp);
-  else par_fw_sm100<false><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mC, pp);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  return launch_pdl(ur.overlap && grid <= kPdlMaxCtas, f16 ? par_fw_sm100<true> : par_fw_sm100<false>, grid, PAR_THREADS, PAR_SMEM, st,
+                    mQ, mK, mV, mC, pp);
 }
 
 int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
@@ -1087,10 +1087,8 @@ int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* d
   auto ctas = [&](int m) { return ((long)ceil_div(T_dv, m) + 2 * ceil_div(T_dk, m)) * d.NC * units; };
   pp.maxsub = par_maxsub(ctas, std::max(T_dv, T_dk));
   const unsigned grid = (unsigned)ctas(pp.maxsub);
-  if (f16) par_bw_sm100<true><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k, pp);
-  else par_bw_sm100<false><<<grid, PAR_THREADS, PAR_SMEM, st>>>(mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k, pp);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  return launch_pdl(ur.overlap && grid <= kPdlMaxCtas, f16 ? par_bw_sm100<true> : par_bw_sm100<false>, grid, PAR_THREADS, PAR_SMEM, st,
+                    mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k, pp);
 }
 
 // Self-test of the bounded wait: one thread waits, for at most `limit` polls, on an mbarrier that nothing arrives

@@ -45,6 +45,8 @@ gates_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, const float
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
   const int per = (NC + ncta - 1) / ncta, c0 = min(NC, rank * per), c1 = min(NC, c0 + per);   // chunks of this CTA
   const bool siging = variant != MLSTM_EXP;
+  pdl_launch_dependents();
+  pdl_wait();
   float* g_arr = gb.scratch + (size_t)bh * 2 * NC;
   float* amax_arr = g_arr + NC;
   // inputs have S tokens per (batch, head), the gate vectors SP = NC * L slots; slots past the sequence end are
@@ -293,6 +295,8 @@ gate_grad_anchored_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF
   __shared__ float s_warp[kAnchorThreads / 32];
   const int nint = (S + kAnchorThreads - 1) / kAnchorThreads;   // 1-D grid: intervals of one (batch, head) adjacent
   const int a = blockIdx.x % nint, bh = blockIdx.x / nint, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = a * kAnchorThreads + t;
   const bool live = s < S;
   float qd = 0.f, kd = 0.f;
@@ -332,6 +336,8 @@ state_dot_kernel(const TS* __restrict__ c_states, const TS* __restrict__ dc_stat
   __shared__ float s_w[8];
   const int bh = blockIdx.x / (n_anchors - 1), a = blockIdx.x % (n_anchors - 1) + 1;   // 1-D grid
   const int k = min(a * every, NC);
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t off = ((size_t)bh * (NC + 1) + k) * state_elems;
   const uint4* pc = reinterpret_cast<const uint4*>(c_states + off);
   const uint4* pd = reinterpret_cast<const uint4*>(dc_states + off);
@@ -370,11 +376,13 @@ static int launch_gates_nv(const void* i, const void* f, const float* n_out, flo
   cfg.gridDim = dim3((unsigned)(d.B * d.NH) * ncta);
   cfg.blockDim = dim3(threads);
   cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = ncta; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ncta; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cfg.gridDim.x <= kPdlMaxCtas ? 2 : 1;
   note_launch();
   MLSTM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gates_kernel<T, NV>, (const T*)i, (const T*)f, n_out, m_out, gb, sc, d.S, d.SP,
                                       d.L, d.NC, d.variant, d.eps));
@@ -510,8 +518,8 @@ static int gate_grad_scan_t(const void* i, const void* f, const float* qdq, cons
   const size_t stride = (size_t)d.B * d.NH * d.SP;
   if (anchors != nullptr && anchor_tokens == kAnchorThreads) {
     const unsigned grid = (unsigned)ceil_div(d.S, kAnchorThreads) * (unsigned)(d.B * d.NH);
-    gate_grad_anchored_kernel<T><<<grid, kAnchorThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, out_dtype, d.S, d.SP,
-                                                                  d.variant, nparts, stride, anchors, n_anchors);
+    return launch_pdl(grid <= kPdlMaxCtas, gate_grad_anchored_kernel<T>, grid, kAnchorThreads, 0, st, (const T*)i, (const T*)f, qdq,
+                      kdk, dI, dF, out_dtype, d.S, d.SP, d.variant, nparts, stride, anchors, n_anchors);
   } else {
     gate_grad_scan_kernel<T><<<d.B * d.NH, kScanThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, out_dtype, d.S, d.SP,
                                                                   d.variant, nparts, stride);
@@ -536,14 +544,12 @@ int launch_state_dot(const void* c_states, const void* dc_states, float* anchors
                      const ChunkwiseDims& d, cudaStream_t st) {
   if (n_anchors < 2) return MLSTM_OK;
   const unsigned grid = (unsigned)(n_anchors - 1) * (unsigned)(d.B * d.NH);
+  const size_t elems = (size_t)d.DHQK * d.DHHV;
   if (d.dtype == MLSTM_F16)
-    state_dot_kernel<__half><<<grid, 256, 0, st>>>((const __half*)c_states, (const __half*)dc_states, anchors, d.NC,
-                                                   every, n_anchors, (size_t)d.DHQK * d.DHHV);
-  else
-    state_dot_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)c_states, (const __nv_bfloat16*)dc_states,
-                                                          anchors, d.NC, every, n_anchors, (size_t)d.DHQK * d.DHHV);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+    return launch_pdl(grid <= kPdlMaxCtas, state_dot_kernel<__half>, grid, 256, 0, st, (const __half*)c_states,
+                      (const __half*)dc_states, anchors, d.NC, every, n_anchors, elems);
+  return launch_pdl(grid <= kPdlMaxCtas, state_dot_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)c_states,
+                    (const __nv_bfloat16*)dc_states, anchors, d.NC, every, n_anchors, elems);
 }
 
 }  // namespace mlstm

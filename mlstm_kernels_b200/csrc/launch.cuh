@@ -42,7 +42,8 @@ bool sm100_supported(int S, int DHQK, int DHHV, int L, int dtype);
 bool sm100_sizes_ok(int B, int NH, int S, int DHQK, int DHHV);
 // A launch may cover a sub-range of the B * NH independent (batch, head) units; all pointers stay those of the whole
 // problem.  count < 0: every unit from `first` on.
-struct UnitRange { int first = 0; int count = -1; };
+// overlap: the launch may begin while the one before it in the stream drains (launch_pdl).
+struct UnitRange { int first = 0; int count = -1; bool overlap = true; };
 int sm100_recurrent_fw(const void* k, const void* v, const GateBuffers& gb, const float* c_initial,
                        const float* n_initial, void* c_states, float* n_states, float* c_last, float* n_last,
                        const ChunkwiseDims& d, cudaStream_t st, UnitRange ur = UnitRange());
