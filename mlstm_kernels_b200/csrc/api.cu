@@ -97,9 +97,9 @@ static SideStream* side_stream_for_current_device() {
 
 // worth it only when the recurrence needs more than one wave of CTAs and the last one is far from full (and never
 // while phases are being timed)
-static bool want_unit_split(const ChunkwiseDims& d, bool allow) {
+static bool want_unit_split(const ChunkwiseDims& d, bool allow, int recurrences) {
   if (!allow || g_split_on.load(std::memory_order_relaxed) == 0 || g_prof_on || d.B * d.NH < 2) return false;
-  const long ctas = sm100_recurrence_ctas(d), sms = sm100_sm_count();
+  const long ctas = recurrences * sm100_recurrence_ctas(d), sms = sm100_sm_count();
   const long waves = (ctas + sms - 1) / sms;
   return waves > 1 && ctas * 100 < waves * sms * 95;   // the last wave leaves more than 5 % of the SM time idle
 }
@@ -108,10 +108,10 @@ static bool want_unit_split(const ChunkwiseDims& d, bool allow) {
 // leaves the scope early, in the destructor - a stream that is being captured must never be left forked.
 class UnitChains {
  public:
-  UnitChains(const ChunkwiseDims& d, cudaStream_t st, bool allow) : st_(st), lk_(g_side_mu, std::defer_lock) {
+  UnitChains(const ChunkwiseDims& d, cudaStream_t st, bool allow, int recurrences = 1) : st_(st), lk_(g_side_mu, std::defer_lock) {
     const int units = d.B * d.NH;
     first_ = UnitRange{0, units};
-    if (!want_unit_split(d, allow)) return;
+    if (!want_unit_split(d, allow, recurrences)) return;
     lk_.lock();
     SideStream* s = side_stream_for_current_device();
     if (s == nullptr) { lk_.unlock(); return; }
@@ -435,14 +435,14 @@ int run_chunkwise_bw(const BwCall& a, const CallDims& c) {
   }
   if (use_sm100) {
     {
-      UnitChains ch(d, st, true);
+      UnitChains ch(d, st, true, a.recompute_into ? 2 : 1);
       if ((rc = ch.status()) != MLSTM_OK) return rc;
-      if (a.recompute_into) {
-        if ((rc = sm100_recurrent_fw(a.k, a.v, lay.gb, a.recompute_c_initial, nullptr, a.recompute_into, nullptr, nullptr, nullptr, d, st, ch.first())) != MLSTM_OK) return rc;
-        if (ch.split() && (rc = sm100_recurrent_fw(a.k, a.v, lay.gb, a.recompute_c_initial, nullptr, a.recompute_into, nullptr, nullptr, nullptr, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
-      }
-      if ((rc = sm100_recurrent_bw(a.q, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, d, st, ch.first())) != MLSTM_OK) return rc;
-      if (ch.split() && (rc = sm100_recurrent_bw(a.q, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
+      auto recurrences = [&](cudaStream_t s, UnitRange ur) {
+        return a.recompute_into ? sm100_recurrent_pair(a.k, a.v, a.recompute_c_initial, a.recompute_into, a.q, a.dh, a.dc_last, lay.dc_states, a.dc_initial, lay.gb, d, s, ur)
+                                : sm100_recurrent_bw(a.q, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, d, s, ur);
+      };
+      if ((rc = recurrences(st, ch.first())) != MLSTM_OK) return rc;
+      if (ch.split() && (rc = recurrences(ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
       if ((rc = sm100_parallel_bw(a.q, a.k, a.v, a.dh, lay.gb, c_states, lay.dc_states, a.dq, a.dk, a.dv, lay.acc, lay.kdk, d, st, ch.first())) != MLSTM_OK) return rc;
       if (ch.split() && (rc = sm100_parallel_bw(a.q, a.k, a.v, a.dh, lay.gb, c_states, lay.dc_states, a.dq, a.dk, a.dv, lay.acc, lay.kdk, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
       if ((rc = ch.join()) != MLSTM_OK) return rc;

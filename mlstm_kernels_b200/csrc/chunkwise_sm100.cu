@@ -54,10 +54,20 @@ constexpr int rec_stage_bytes(int TN) { return 16384 + TN * 128; }    // 64 toke
 constexpr int rec_out_bytes(int TN) { return TN * 256; }              // 16-bit state tile staged for the TMA store (two of them)
 // Operand ring depth, as deep as shared memory allows.  A stage comes round in about 4600 cycles (load 2500, gating and
 // hand-over 1300, MMA and hand-back 800), so the 64-column form with its smaller stages runs three chunks ahead.
-constexpr int rec_stages(bool bwd, int TN) { return TN == 128 ? 4 : (bwd ? 7 : 6); }
-constexpr int rec_smem_bytes(bool bwd, int TN) {
-  return rec_stages(bwd, TN) * rec_stage_bytes(TN) + (bwd ? 0 : REC_NPART_BYTES) + 2 * rec_out_bytes(TN) + 1024;
+constexpr int rec_stages(bool has_n, int TN) { return TN == 128 ? 4 : (has_n ? 6 : 7); }
+constexpr int rec_smem_bytes(bool has_n, int TN) {
+  return rec_stages(has_n, TN) * rec_stage_bytes(TN) + (has_n ? REC_NPART_BYTES : 0) + 2 * rec_out_bytes(TN) + 1024;
 }
+
+template <int STAGES, bool TWO_SCALES>
+struct RecShared {
+  uint64_t bar_full[STAGES], bar_empty[STAGES], bar_scaled[STAGES], bar_acc_full[2], bar_acc_free[2], bar_nsum[2], bar_nread[2], bar_out_full[2], bar_out_free[2];
+  uint32_t s_tmem;
+  int s_abort;   // set by the first wait of this CTA that runs out; every other wait polls it
+  // per-row scale factors of the left tile, copied with the stage (backward: two factors per row)
+  __align__(16) float s_scale[STAGES][REC_HALF], s_scale2[TWO_SCALES ? STAGES : 1][REC_HALF];
+  float s_g[8];  // decay of the chunk, ring of eight (outlives the operand ring)
+};
 
 // One ring stage holds 64 tokens of the left and of the right operand (boxes of 64 rows x 64 columns, 8 KB each:
 // left columns d0.., d0+64.., right columns e0.., e0+64..).  A chunk is two stages; the product of a chunk is
@@ -66,19 +76,22 @@ constexpr int rec_smem_bytes(bool bwd, int TN) {
 // TN = columns of the state tile (128, or 64 for small problems: twice as many CTAs, so that a launch with few
 // (batch, head) units still covers the GPU).
 // F16: the 16-bit element type is IEEE half instead of bf16 (operands, gated tiles, stored states, outputs).
-template <bool BWD, int TN, bool F16>
-__global__ void __launch_bounds__(REC_THREADS, 1)
-rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUtensorMap mapR,
-          const __grid_constant__ CUtensorMap mapS, RecParams p) {
+// HAS_N: the vector n is kept as well (forward, unless only the states are wanted again).
+template <bool BWD, int TN, bool F16, bool HAS_N, typename Shared>
+__device__ __forceinline__ void
+rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& mapS, const RecParams& p, Shared& sh,
+         const unsigned block) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int REC_STAGES = rec_stages(BWD, TN), REC_STAGE_BYTES = rec_stage_bytes(TN), REC_OUT = rec_out_bytes(TN);
-  __shared__ uint64_t bar_full[REC_STAGES], bar_empty[REC_STAGES], bar_scaled[REC_STAGES], bar_acc_full[2], bar_acc_free[2], bar_nsum[2], bar_nread[2], bar_out_full[2], bar_out_free[2];
-  __shared__ uint32_t s_tmem;
-  __shared__ int s_abort;   // set by the first wait of this CTA that runs out; every other wait polls it
-  // per-row scale factors of the left tile, copied with the stage (backward: two factors per row)
-  __shared__ __align__(16) float s_scale[REC_STAGES][REC_HALF], s_scale2[BWD ? REC_STAGES : 1][REC_HALF];
-  __shared__ float s_g[8];          // decay of the chunk, ring of eight (outlives the operand ring)
+  constexpr int REC_STAGES = rec_stages(HAS_N, TN), REC_STAGE_BYTES = rec_stage_bytes(TN), REC_OUT = rec_out_bytes(TN);
+  auto &bar_full = sh.bar_full, &bar_empty = sh.bar_empty, &bar_scaled = sh.bar_scaled;
+  auto &bar_acc_full = sh.bar_acc_full, &bar_acc_free = sh.bar_acc_free, &bar_nsum = sh.bar_nsum, &bar_nread = sh.bar_nread;
+  auto &bar_out_full = sh.bar_out_full, &bar_out_free = sh.bar_out_free;
+  auto &s_tmem = sh.s_tmem;
+  auto &s_abort = sh.s_abort;
+  auto &s_scale = sh.s_scale;
+  auto &s_scale2 = sh.s_scale2;
+  auto &s_g = sh.s_g;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 1-D grid (no 65535 limit on batch x heads), state tiles of one (batch, head) next to each other
@@ -87,10 +100,10 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
   // head dims need not be multiples of the tile: the last tile hangs over the edge, where loads read zeros (the
   // tensor maps know the true extents), plain accesses are masked and the state store is clipped
   const int n_et = (p.DHHV + TN - 1) / TN, n_dt = (p.DHQK + 127) / 128;
-  const int et = blockIdx.x % n_et, dt = (blockIdx.x / n_et) % n_dt, bh = p.bh0 + blockIdx.x / (n_et * n_dt);
+  const int et = block % n_et, dt = (block / n_et) % n_dt, bh = p.bh0 + block / (n_et * n_dt);
   const int e0 = et * TN, d0 = dt * 128;
   const int NC = p.NC, NH2 = 2 * p.NC;   // ring steps: two per chunk
-  const bool do_n = (!BWD) && et == 0 && (p.n_states != nullptr || p.n_final != nullptr);
+  const bool do_n = HAS_N && et == 0 && (p.n_states != nullptr || p.n_final != nullptr);
 
   if (tid == 0) {
     s_abort = 0;
@@ -228,7 +241,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
   } else if (warp == 18) {
     // ---------------- store warp: one TMA store per 64-column box of each staged state tile ----------------
     if (p.c_states != nullptr && elect_one()) {
-      uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (BWD ? 0 : REC_NPART_BYTES);
+      uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (HAS_N ? REC_NPART_BYTES : 0);
       for (int n = 0; n <= NC; ++n) {
         const int ob = n & 1;
         if (!mbar_wait(&bar_out_full[ob], (n >> 1) & 1, &s_abort, &g_sm100_status, 108)) break;
@@ -289,7 +302,7 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
     }
     // The bf16 state tile goes to shared memory in the 128-byte-swizzled box layout and leaves with one TMA store
     // per 64-column box (coalesced, asynchronous); two staging buffers, one store group in flight.
-    uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (BWD ? 0 : REC_NPART_BYTES);
+    uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (HAS_N ? REC_NPART_BYTES : 0);
     int n_out = 0;   // tiles written so far
     auto store_c = [&]() -> bool {
       if (p.c_states == nullptr) return true;
@@ -339,6 +352,28 @@ rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUte
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 256);
+}
+
+template <bool BWD, int TN, bool F16>
+__global__ void __launch_bounds__(REC_THREADS, 1)
+rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUtensorMap mapR,
+          const __grid_constant__ CUtensorMap mapS, const __grid_constant__ RecParams p) {
+  __shared__ RecShared<rec_stages(!BWD, TN), BWD> sh;
+  rec_body<BWD, TN, F16, !BWD>(mapL, mapR, mapS, p, sh, blockIdx.x);
+}
+
+// Both recurrences of a backward that finds no per-chunk states in one launch: the first n_fw CTAs run the forward's
+// again (states only), the others the state gradient's.  They are independent, and a launch of few CTAs takes as long as one
+// of them takes for its sequence: side by side they take half.
+template <int TN, bool F16>
+__global__ void __launch_bounds__(REC_THREADS, 1)
+rec_pair_sm100(const __grid_constant__ CUtensorMap mL, const __grid_constant__ CUtensorMap mR,
+               const __grid_constant__ CUtensorMap mS, const __grid_constant__ RecParams p,
+               const __grid_constant__ CUtensorMap mLb, const __grid_constant__ CUtensorMap mRb,
+               const __grid_constant__ CUtensorMap mSb, const __grid_constant__ RecParams pb, const unsigned n_fw) {
+  __shared__ RecShared<rec_stages(false, TN), true> sh;
+  if (blockIdx.x < n_fw) rec_body<false, TN, F16, false>(mL, mR, mS, p, sh, blockIdx.x);
+  else rec_body<true, TN, F16, false>(mLb, mRb, mSb, pb, sh, blockIdx.x - n_fw);
 }
 
 // =====================================================================================================
@@ -959,9 +994,9 @@ static int launch_rec_tn(const CUtensorMap& mL, const CUtensorMap& mR, const CUt
                          const ChunkwiseDims& d, int units, bool overlap, cudaStream_t st) {
   auto kern = rec_sm100<BWD, TN, F16>;
   static bool attr_done[64] = {};
-  if (int rc = set_smem_once(kern, rec_smem_bytes(BWD, TN), attr_done)) return rc;
+  if (int rc = set_smem_once(kern, rec_smem_bytes(!BWD, TN), attr_done)) return rc;
   const unsigned grid = (unsigned)((d.DHHV + TN - 1) / TN) * (unsigned)((d.DHQK + 127) / 128) * (unsigned)units;
-  return launch_pdl(overlap && grid <= kPdlMaxCtas, kern, grid, REC_THREADS, rec_smem_bytes(BWD, TN), st, mL, mR, mS, rp);
+  return launch_pdl(overlap && grid <= kPdlMaxCtas, kern, grid, REC_THREADS, rec_smem_bytes(!BWD, TN), st, mL, mR, mS, rp);
 }
 
 // number of SMs of the current device (queried once per device)
@@ -982,24 +1017,39 @@ long sm100_recurrence_ctas(const ChunkwiseDims& d) {
 }
 int sm100_sm_count() { return sm_count(); }
 
+struct RecMaps { CUtensorMap l, r, s; };
+static bool rec_maps(RecMaps* m, const void* left, const void* right, const void* states, const ChunkwiseDims& d) {
+  // recurrence operands arrive in half-chunk boxes (64 tokens x 64 columns)
+  return tok_map(&m->l, left, d, d.DHQK, REC_HALF) && tok_map(&m->r, right, d, d.DHHV, REC_HALF) &&
+         // store map over the per-chunk states; when no states are wanted (segment summary) the map is never used
+         state_map(&m->s, states ? states : left, d, 128);
+}
+
 template <bool BWD>
 static int launch_rec(const void* left, const void* right, RecParams rp, const ChunkwiseDims& d, UnitRange ur,
                       cudaStream_t st) {
   rp.bh0 = ur.first;
   const int units = ur.count < 0 ? d.B * d.NH - ur.first : ur.count;
   if (units <= 0) return MLSTM_OK;
-  CUtensorMap mL, mR, mS;
-  // recurrence operands arrive in half-chunk boxes (64 tokens x 64 columns)
-  if (!tok_map(&mL, left, d, d.DHQK, REC_HALF) || !tok_map(&mR, right, d, d.DHHV, REC_HALF)) return MLSTM_ERR_CUDA;
-  // store map over the per-chunk states; when no states are wanted (segment summary) the map is never used
-  if (!state_map(&mS, rp.c_states ? (const void*)rp.c_states : left, d, 128)) return MLSTM_ERR_CUDA;
+  RecMaps m;
+  if (!rec_maps(&m, left, right, rp.c_states, d)) return MLSTM_ERR_CUDA;
   // One CTA per SM walks all chunks of its state tile.  With 128-column tiles a launch of few (batch, head) units
   // leaves SMs idle; 64-column tiles double the CTAs as long as they still fit one wave.
-  const long ctas128 = sm100_recurrence_ctas(d);
   const bool f16 = d.dtype == MLSTM_F16;
-  if (2 * ctas128 <= sm_count())
-    return f16 ? launch_rec_tn<BWD, 64, true>(mL, mR, mS, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 64, false>(mL, mR, mS, rp, d, units, ur.overlap, st);
-  return f16 ? launch_rec_tn<BWD, 128, true>(mL, mR, mS, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 128, false>(mL, mR, mS, rp, d, units, ur.overlap, st);
+  if (2 * sm100_recurrence_ctas(d) <= sm_count())
+    return f16 ? launch_rec_tn<BWD, 64, true>(m.l, m.r, m.s, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 64, false>(m.l, m.r, m.s, rp, d, units, ur.overlap, st);
+  return f16 ? launch_rec_tn<BWD, 128, true>(m.l, m.r, m.s, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 128, false>(m.l, m.r, m.s, rp, d, units, ur.overlap, st);
+}
+
+template <int TN, bool F16>
+static int launch_rec_pair(const RecMaps& m, const RecParams& rp, const RecMaps& mb, const RecParams& rpb, const ChunkwiseDims& d,
+                           int units, bool overlap, cudaStream_t st) {
+  auto kern = rec_pair_sm100<TN, F16>;
+  static bool attr_done[64] = {};
+  if (int rc = set_smem_once(kern, rec_smem_bytes(false, TN), attr_done)) return rc;
+  const unsigned n = (unsigned)((d.DHHV + TN - 1) / TN) * (unsigned)((d.DHQK + 127) / 128) * (unsigned)units;
+  return launch_pdl(overlap && 2 * n <= kPdlMaxCtas, kern, 2 * n, REC_THREADS, rec_smem_bytes(false, TN), st, m.l, m.r, m.s, rp, mb.l, mb.r,
+                    mb.s, rpb, n);
 }
 
 int sm100_recurrent_fw(const void* k, const void* v, const GateBuffers& gb, const float* c_initial,
@@ -1017,6 +1067,24 @@ int sm100_recurrent_bw(const void* q, const void* dh, const GateBuffers& gb, con
   RecParams rp{gb.bbar, gb.inv_den, d.qk_scale, gb.gbar, dc_last, nullptr, dc_states, nullptr,
                dc_initial, nullptr, d.S, d.SP, d.NC, d.DHQK, d.DHHV, 0};
   return launch_rec<true>(q, dh, rp, d, ur, st);
+}
+
+int sm100_recurrent_pair(const void* k, const void* v, const float* c_initial, void* c_states, const void* q, const void* dh,
+                         const float* dc_last, void* dc_states, float* dc_initial, const GateBuffers& gb,
+                         const ChunkwiseDims& d, cudaStream_t st, UnitRange ur) {
+  const int units = ur.count < 0 ? d.B * d.NH - ur.first : ur.count;
+  if (units <= 0) return MLSTM_OK;
+  PhaseScope ps(PH_REC_BW, st);
+  const RecParams rp{gb.abar, nullptr, 1.f, gb.gbar, c_initial, nullptr, c_states, nullptr, nullptr, nullptr,
+                     d.S, d.SP, d.NC, d.DHQK, d.DHHV, ur.first};
+  const RecParams rpb{gb.bbar, gb.inv_den, d.qk_scale, gb.gbar, dc_last, nullptr, dc_states, nullptr, dc_initial, nullptr,
+                      d.S, d.SP, d.NC, d.DHQK, d.DHHV, ur.first};
+  RecMaps m, mb;
+  if (!rec_maps(&m, k, v, c_states, d) || !rec_maps(&mb, q, dh, dc_states, d)) return MLSTM_ERR_CUDA;
+  const bool f16 = d.dtype == MLSTM_F16;
+  if (4 * sm100_recurrence_ctas(d) <= sm_count())   // (the rule of launch_rec, for twice the CTAs)
+    return f16 ? launch_rec_pair<64, true>(m, rp, mb, rpb, d, units, ur.overlap, st) : launch_rec_pair<64, false>(m, rp, mb, rpb, d, units, ur.overlap, st);
+  return f16 ? launch_rec_pair<128, true>(m, rp, mb, rpb, d, units, ur.overlap, st) : launch_rec_pair<128, false>(m, rp, mb, rpb, d, units, ur.overlap, st);
 }
 
 static ParParams base_params(const GateBuffers& gb, const ChunkwiseDims& d) {

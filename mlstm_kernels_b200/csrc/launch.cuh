@@ -52,6 +52,10 @@ int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuf
                       UnitRange ur = UnitRange());
 int sm100_recurrent_bw(const void* q, const void* dh, const GateBuffers& gb, const float* dc_last, void* dc_states,
                        float* dc_initial, const ChunkwiseDims& d, cudaStream_t st, UnitRange ur = UnitRange());
+// the forward's recurrence again (states only) and the state gradient's, in one launch
+int sm100_recurrent_pair(const void* k, const void* v, const float* c_initial, void* c_states, const void* q, const void* dh,
+                         const float* dc_last, void* dc_states, float* dc_initial, const GateBuffers& gb,
+                         const ChunkwiseDims& d, cudaStream_t st, UnitRange ur = UnitRange());
 int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
                       const void* c_states, const void* dc_states, void* dq, void* dk, void* dv, float* qdq_parts,
                       float* kdk_parts, const ChunkwiseDims& d, cudaStream_t st, UnitRange ur = UnitRange());
