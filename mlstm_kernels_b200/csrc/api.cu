@@ -67,7 +67,7 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // first half runs on the caller's stream and the second half on a stream of the library, forked and joined with
 // events (the pattern stream capture allows), and the block scheduler fills the idle SMs of one chain's last wave
 // with the other chain's CTAs.  No kernel waits for another one: the order is the streams' and events' only.
-struct SideStream { cudaStream_t st = nullptr; cudaEvent_t fork = nullptr, join = nullptr; };
+struct SideStream { cudaStream_t st = nullptr, first = nullptr; cudaEvent_t fork = nullptr, join = nullptr, started = nullptr; };   // first: placed before default-priority work
 static std::mutex g_side_mu;          // held while a split call enqueues: one stream and one event pair per device
 static SideStream g_side[64];
 static std::atomic<int> g_split_on{1};
@@ -77,20 +77,26 @@ static SideStream* side_stream_for_current_device() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   SideStream& s = g_side[dev];
   if (s.st == nullptr) {
-    cudaStream_t st = nullptr;
-    cudaEvent_t a = nullptr, b = nullptr;
+    cudaStream_t st = nullptr, first = nullptr;
+    int least = 0, greatest = 0;
+    cudaEvent_t a = nullptr, b = nullptr, c = nullptr;
     // default priority: giving this stream a higher one (so that the second half's recurrence CTAs are placed before
     // the first half's intra-chunk CTAs) measured slower
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
+    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&first, cudaStreamNonBlocking, greatest) != cudaSuccess ||
         cudaEventCreateWithFlags(&a, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&b, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c, cudaEventDisableTiming) != cudaSuccess) {
       (void)cudaGetLastError();
       if (st) cudaStreamDestroy(st);
+      if (first) cudaStreamDestroy(first);
       if (a) cudaEventDestroy(a);
       if (b) cudaEventDestroy(b);
+      if (c) cudaEventDestroy(c);
       return nullptr;
     }
-    s.st = st; s.fork = a; s.join = b;
+    s.st = st; s.first = first; s.fork = a; s.join = b; s.started = c;
   }
   return &s;
 }
@@ -188,9 +194,9 @@ struct Carver {
   }
 };
 
-struct FwLayout { GateBuffers gb; size_t bytes; };
+struct FwLayout { GateBuffers gb; float *c_carry, *n_carry; size_t bytes; };   // carry: state between two segments
 // per-token arrays have SP = NC * L slots per (batch, head)
-static FwLayout carve_fw(void* ws, int BNH, int SP, int NC) {
+static FwLayout carve_fw(void* ws, int BNH, int SP, int NC, size_t carry_dhqk = 0, size_t carry_dhhv = 0) {
   Carver c(ws);
   FwLayout l{};
   const size_t tok = (size_t)BNH * SP;
@@ -201,6 +207,8 @@ static FwLayout carve_fw(void* ws, int BNH, int SP, int NC) {
   l.gb.m_tok = c.take<float>(tok);
   l.gb.gbar = c.take<float>((size_t)BNH * NC);
   l.gb.scratch = c.take<float>((size_t)BNH * NC * 2);
+  l.c_carry = c.take<float>(BNH * carry_dhqk * carry_dhhv);
+  l.n_carry = c.take<float>(BNH * carry_dhqk);
   l.gb.inv_den = nullptr;
   l.bytes = align_up(c.off, 256);
   return l;
@@ -330,13 +338,15 @@ int mlstm_b200_chunkwise_state_dtype(int S, int DHQK, int DHHV, int L, int dtype
 
 size_t mlstm_b200_chunkwise_workspace_bytes(int B, int NH, int S, int DHQK, int DHHV, int L, int dtype, int variant,
                                             int impl, int backward) {
-  (void)variant;
   if (check_dims(B, NH, S, DHQK, DHHV, L) != MLSTM_OK) return 0;
   bool use_sm100 = false;
   if (resolve_impl(impl, B, NH, S, DHQK, DHHV, L, dtype, &use_sm100) != MLSTM_OK) return 0;
   const int NC = (S + L - 1) / L, SP = NC * L;
   if (backward == 2) return carve_summary(nullptr, B * NH, SP, NC).bytes;
-  if (!backward) return carve_fw(nullptr, B * NH, SP, NC).bytes;
+  if (!backward) {
+    const bool seg = use_sm100 && sm100_forward_segments(make_dims(B, NH, S, DHQK, DHHV, L, variant, 0.f, dtype)) > 1;
+    return carve_fw(nullptr, B * NH, SP, NC, seg ? DHQK : 0, seg ? DHHV : 0).bytes;
+  }
   return carve_bw(nullptr, B * NH, SP, NC, DHQK, DHHV, dtype_size(use_sm100 ? dtype : MLSTM_F32)).bytes;
 }
 
@@ -366,6 +376,52 @@ static int check_call(const CallDims& c) {
   return MLSTM_OK;
 }
 
+// ---- a long sequence of few units in segments -----------------------------------------------------------
+// With few (batch, head) units the recurrence is a serial chain on part of the SMs, and all of the intra-chunk work
+// used to follow it.  Here the recurrence goes through the sequence in segments on a stream of the library, handing its
+// f32 state from one to the next, and the intra-chunk kernel of each finished segment runs on the caller's stream
+// beside it.  Same arithmetic in the same order, so the results are the same bits.
+// 8 heads 256/512, 131072 tokens: 2180 -> 1880 us; 65536 tokens: 1085 -> 970; 4 heads, 131072 tokens: 1573 -> 1341.
+static int forward_in_segments(const FwCall& a, const FwLayout& lay, const ChunkwiseDims& d, int n_seg, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_side_mu);
+  SideStream* s = side_stream_for_current_device();
+  if (s == nullptr) return MLSTM_ERR_CUDA;
+  auto ok = [](cudaError_t e) {
+    if (e == cudaSuccess) return (int)MLSTM_OK;
+    set_last_cuda_error(cudaGetLastError(), "hand-over between the segments' streams");
+    return (int)MLSTM_ERR_CUDA;
+  };
+  auto record = [&](cudaEvent_t ev, cudaStream_t on) { return ok(cudaEventRecord(ev, on)); };
+  auto wait = [&](cudaStream_t on, cudaEvent_t ev) { return ok(cudaStreamWaitEvent(on, ev, 0)); };
+  int rc = record(s->fork, st);
+  if (rc == MLSTM_OK) rc = wait(s->first, s->fork);
+  if (rc != MLSTM_OK) return rc;
+  // The intra-chunk kernel of a segment starts when the next segment's recurrence has all its CTAs running: were it first, it
+  // would spread over every SM, and a recurrence CTA needs one for itself.  (A stream being captured takes the order of the
+  // launches alone: same results, and mostly the same placement.)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if ((rc = ok(cudaStreamIsCapturing(st, &cap))) != MLSTM_OK) return rc;
+  cudaEvent_t started = cap == cudaStreamCaptureStatusNone ? s->started : nullptr;
+  const int step = (d.NC + n_seg - 1) / n_seg;
+  cudaEvent_t done[2] = {s->join, s->fork};
+  UnitRange before;
+  for (int c0 = 0, j = 0; rc == MLSTM_OK; c0 += step, ++j) {
+    const bool first = c0 == 0, last = c0 + step >= d.NC, end = c0 >= d.NC;
+    const UnitRange ur{0, -1, false, c0, std::min(step, d.NC - c0), started};
+    if (!end) rc = sm100_recurrent_fw(a.k, a.v, lay.gb, first ? a.c_initial : lay.c_carry, first ? a.n_initial : lay.n_carry, a.c_states, a.n_states,
+                                      last ? a.c_last : lay.c_carry, last ? a.n_last : lay.n_carry, d, s->first, ur);
+    if (rc == MLSTM_OK && !end) rc = record(done[j & 1], s->first);
+    if (j > 0 && rc == MLSTM_OK) rc = wait(st, done[(j - 1) & 1]);
+    if (j > 0 && !end && started != nullptr && rc == MLSTM_OK) rc = wait(st, started);
+    if (j > 0 && rc == MLSTM_OK) rc = sm100_parallel_fw(a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, d, st, before);
+    if (end) break;
+    before = ur;
+  }
+  // after a failed launch too: a stream that is being captured must never be left forked
+  if (rc != MLSTM_OK && record(s->join, s->first) == MLSTM_OK) (void)wait(st, s->join);
+  return rc;
+}
+
 int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   int rc = check_call(c);
   if (rc != MLSTM_OK) return rc;
@@ -378,12 +434,16 @@ int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   if ((rc = resolve_impl(c.impl, c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, &use_sm100)) != MLSTM_OK) return rc;
 
   const ChunkwiseDims d = make_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.variant, c.eps, c.dtype);
-  FwLayout lay = carve_fw(a.workspace, c.B * c.NH, d.SP, d.NC);
+  const int n_seg = use_sm100 ? sm100_forward_segments(d) : 1;
+  FwLayout lay = carve_fw(a.workspace, c.B * c.NH, d.SP, d.NC, n_seg > 1 ? c.DHQK : 0, n_seg > 1 ? c.DHHV : 0);
   if (a.workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(c.stream);
 
   if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, nullptr, a.m_out, lay.gb, a.m_states, a.m_last, d, st)) != MLSTM_OK) return rc;
   lay.gb.inv_den = a.inv_den;   // written by the intra-chunk kernel
+  // (off together with the unit split, and while phases are being timed)
+  if (n_seg > 1 && a.allow_split && g_split_on.load(std::memory_order_relaxed) != 0 && !g_prof_on)
+    return forward_in_segments(a, lay, d, n_seg, st);
   if (use_sm100) {
     UnitChains ch(d, st, a.allow_split);
     if ((rc = ch.status()) != MLSTM_OK) return rc;

@@ -16,6 +16,7 @@
 // Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
 // one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded.
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "launch.cuh"
@@ -45,6 +46,7 @@ struct RecParams {
   float* n_final;
   int S, SP, NC, DHQK, DHHV;   // SP = NC * 128: slots per (batch, head) of the per-token scale vectors
   int bh0;                     // first (batch, head) unit of this launch (a launch may cover a sub-range of the units)
+  int ck0, n_ck;               // forward: first chunk and number of chunks of this launch (backward: all of them)
 };
 
 constexpr int REC_THREADS = 640;                 // warp 0 TMA, 1 MMA, 2..9 gate the left tile, 10..17 own the state, 18 stores it, 19 keeps n
@@ -102,7 +104,8 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
   const int n_et = (p.DHHV + TN - 1) / TN, n_dt = (p.DHQK + 127) / 128;
   const int et = block % n_et, dt = (block / n_et) % n_dt, bh = p.bh0 + block / (n_et * n_dt);
   const int e0 = et * TN, d0 = dt * 128;
-  const int NC = p.NC, NH2 = 2 * p.NC;   // ring steps: two per chunk
+  const int NC = p.NC, NS = p.n_ck, NH2 = 2 * NS;   // ring steps: two per chunk
+  const int ck0 = BWD ? 0 : p.ck0;
   const bool do_n = HAS_N && et == 0 && (p.n_states != nullptr || p.n_final != nullptr);
 
   if (tid == 0) {
@@ -132,7 +135,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
     // block ahead, so no global-memory latency sits between a stage becoming free and the next issue.
     auto load_g = [&](int blk) -> float {
       const int s = blk * 32 + lane;
-      return s < NC ? p.gbar[(size_t)bh * NC + (BWD ? NC - 1 - s : s)] : 0.f;
+      return s < NS ? p.gbar[(size_t)bh * NC + (BWD ? NC - 1 - s : ck0 + s)] : 0.f;
     };
     float g_blk = load_g(0), g_nxt = load_g(1);
     int issued = 0;
@@ -145,7 +148,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       }
       if (!mbar_wait(&bar_empty[st], ((h / REC_STAGES) & 1) ^ 1, &s_abort, &g_sm100_status, 101)) break;
       if (elect_one()) {
-        const int ck = BWD ? NC - 1 - s : s;
+        const int ck = BWD ? NC - 1 - s : ck0 + s;
         // token rows past the end of the sequence (ragged last chunk) arrive as zeros; their scale slots hold zeros
         const int y = ck * CL + (h & 1) * REC_HALF;          // first token of this half chunk inside the sequence
         const size_t slot0 = (size_t)bh * p.SP + y;
@@ -242,10 +245,10 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
     // ---------------- store warp: one TMA store per 64-column box of each staged state tile ----------------
     if (p.c_states != nullptr && elect_one()) {
       uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (HAS_N ? REC_NPART_BYTES : 0);
-      for (int n = 0; n <= NC; ++n) {
+      for (int n = 0; n <= NS; ++n) {
         const int ob = n & 1;
         if (!mbar_wait(&bar_out_full[ob], (n >> 1) & 1, &s_abort, &g_sm100_status, 108)) break;
-        const int slot = BWD ? NC - n : n;
+        const int slot = BWD ? NC - n : ck0 + n;
         const int z = bh * (NC + 1) + slot;
         tma_store_3d(&mapS, stage_base + ob * REC_OUT, e0, d0, z);
         if (TN == 128 && e0 + 64 < p.DHHV) tma_store_3d(&mapS, stage_base + ob * REC_OUT + 16384, e0 + 64, d0, z);
@@ -264,9 +267,9 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       const bool d_in = d0 + 4 * lane < p.DHQK;   // the lane's four rows exist (DHQK is a multiple of 8)
       if (p.n_init && d_in) nv = *reinterpret_cast<const float4*>(p.n_init + (size_t)bh * p.DHQK + d0 + 4 * lane);
       if (p.n_states != nullptr && d_in)
-        *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1)) * p.DHQK + d0 + 4 * lane) = nv;
+        *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1) + ck0) * p.DHQK + d0 + 4 * lane) = nv;
       bool ok = true;
-      for (int s = 0; s < NC; ++s) {
+      for (int s = 0; s < NS; ++s) {
         const int nb = s & 1;
         if (!mbar_wait(&bar_nsum[nb], (s >> 1) & 1, &s_abort, &g_sm100_status, 106)) { ok = false; break; }
         const float4* np4 = reinterpret_cast<const float4*>(smem + REC_STAGES * REC_STAGE_BYTES) + nb * (32 * 32) + lane;
@@ -278,7 +281,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
         const float g = s_g[s & 7];
         nv.x = fmaf(g, nv.x, cs.x); nv.y = fmaf(g, nv.y, cs.y); nv.z = fmaf(g, nv.z, cs.z); nv.w = fmaf(g, nv.w, cs.w);
         if (p.n_states != nullptr && d_in)
-          *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1) + s + 1) * p.DHQK + d0 + 4 * lane) = nv;
+          *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1) + ck0 + s + 1) * p.DHQK + d0 + 4 * lane) = nv;
       }
       if (ok && p.n_final && d_in) *reinterpret_cast<float4*>(p.n_final + (size_t)bh * p.DHQK + d0 + 4 * lane) = nv;
     }
@@ -324,7 +327,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       return true;
     };
     bool ok = store_c();   // the state before the first step (slot 0 forward, slot NC backward)
-    for (int s = 0; s < NC && ok; ++s) {
+    for (int s = 0; s < NS && ok; ++s) {
       const int buf = s & 1;
       if (!mbar_wait(&bar_acc_full[buf], (s >> 1) & 1, &s_abort, &g_sm100_status, 104)) { ok = false; break; }
       tc_fence_after_sync();
@@ -409,6 +412,7 @@ struct ParParams {
   int S, SP, NC, DHQK, DHHV, variant;   // SP = NC * 128: slots per (batch, head) of the per-token gate vectors
   float eps, qk_scale;
   int bh0;                    // first (batch, head) unit of this launch
+  int ck0, n_ck;              // first chunk and number of chunks of this launch
   int maxsub;                 // most output tiles a CTA of this launch produces (par_maxsub)
 };
 
@@ -444,11 +448,14 @@ struct ParShared {
 // underflows the exact value is below 2^-100 as well.  The diagonal block keeps the exact per-element form (its
 // masked columns may carry arbitrarily large colE).  The special-function unit (16 results per clock and SM) was
 // the limit of the gating phase before: the warps of the busiest row quarter share one SM sub-partition.
-template <bool F16>
+// LOOP: the CTA runs the body again for another chunk afterwards (H only): it keeps its tensor memory from the first run
+// to the last, and leaves each run with no arrival on any barrier outstanding, so that the next one can set them up anew.
+template <bool F16, bool LOOP = false>
 __device__ __forceinline__ void
 par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* mapX,
          const CUtensorMap* mapSt, const CUtensorMap* mapE, const ParParams& p,
-         ParShared& sh, const int o_tile0, const int nsub, const int ck, const int bh) {
+         ParShared& sh, const int o_tile0, const int nsub, const int ck, const int bh, const bool first_run = true,
+         const bool last_run = true) {
   const bool LOWER = (mode == PM_H || mode == PM_DQ);
   const bool ST_MN = (mode == PM_H || mode == PM_DV);  // state operand N-contiguous in shared memory
   const bool HAS_E = (mode == PM_DQ || mode == PM_DK);  // extra tile for the gate-gradient row sums
@@ -466,6 +473,12 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
   const bool use_n = (mode == PM_H) && p.variant != MLSTM_SIG_NONORM && p.n_states != nullptr;
 
   if (tid == 0) {
+    if (LOOP && !first_run) {
+      for (int s = 0; s < PAR_NST; ++s) { mbar_inval(&sh.bar_full[s]); mbar_inval(&sh.bar_empty[s]); mbar_inval(&sh.bar_qdone[s]); }
+      for (int s = 0; s < 4; ++s) mbar_inval(&sh.bar_pair[s]);
+      mbar_inval(&sh.bar_sfull); mbar_inval(&sh.bar_afull); mbar_inval(&sh.bar_gated); mbar_inval(&sh.bar_hfull); mbar_inval(&sh.bar_dot);
+      mbar_inval(&sh.bar_out); mbar_inval(&sh.bar_accfree); mbar_inval(&sh.bar_done);
+    }
     sh.abort = 0;
     for (int s = 0; s < PAR_NST; ++s) {
       mbar_init(&sh.bar_full[s], 1); mbar_init(&sh.bar_empty[s], 1); mbar_init(&sh.bar_qdone[s], 8);
@@ -477,7 +490,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     tma_prefetch_desc(mapA); tma_prefetch_desc(mapB); tma_prefetch_desc(mapX); tma_prefetch_desc(mapSt);
     if (HAS_E) tma_prefetch_desc(mapE);
   }
-  if (warp == 1) { tmem_alloc(&sh.tmem, 256); tmem_relinquish(); }
+  if (warp == 1 && (!LOOP || first_run)) { tmem_alloc(&sh.tmem, 256); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -566,6 +579,11 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       if (issued < n_loads && issued > 0) {  // error path: let the copies in flight land before the CTA retires
         for (int ld = max(0, issued - PAR_NST); ld < issued; ++ld)
           mbar_wait(&sh.bar_full[ld % PAR_NST], (ld / PAR_NST) & 1, nullptr, nullptr, 0);
+      }
+      if (LOOP && issued == n_loads) {   // the hand-backs of the last uses, which nobody else waits for
+        if (rm0 > 0) mbar_wait(&sh.bar_empty[0], (rm0 - 1) & 1, &sh.abort, &g_sm100_status, 217);
+        if (rm1 > 0) mbar_wait(&sh.bar_empty[1], (rm1 - 1) & 1, &sh.abort, &g_sm100_status, 217);
+        if (rm2 > 0) mbar_wait(&sh.bar_empty[2], (rm2 - 1) & 1, &sh.abort, &g_sm100_status, 217);
       }
     }
   } else if (warp == 1) {
@@ -874,9 +892,10 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       }
     }
   }
+  if (LOOP) fence_proxy_async_smem();   // staging writes above, the next run's copies after the barrier
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, 256);
+  if (warp == 1 && (!LOOP || last_run)) tmem_dealloc(tmem, 256);
 }
 
 template <bool F16>
@@ -888,9 +907,26 @@ par_fw_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUt
   const int T = (p.DHHV + 127) / 128;                 // output tiles per chunk; a CTA takes up to maxsub of them
   // 1-D grid in the order (tile group, chunk, batch x head): no 65535 limit on chunks or batch x heads
   const int gx = (T + p.maxsub - 1) / p.maxsub;
-  const int x = blockIdx.x % gx, ck = (blockIdx.x / gx) % p.NC, bh = p.bh0 + blockIdx.x / (gx * p.NC);
+  const int x = blockIdx.x % gx, ck = p.ck0 + (blockIdx.x / gx) % p.n_ck, bh = p.bh0 + blockIdx.x / (gx * p.n_ck);
   const int t0 = p.maxsub * x;
   par_body<F16>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(p.maxsub, T - t0), ck, bh);
+}
+
+// The same for a range of chunks, beside the recurrence of the following chunks: one CTA per resident place on the SMs that
+// the recurrence leaves, each going through the work items with a stride.  A launch of one CTA per item would fill every SM
+// between two segments, and the next recurrence, whose CTAs need a whole SM each, would wait for 25 us until they drain.
+template <bool F16>
+__global__ void __launch_bounds__(PAR_THREADS, 2)
+par_fw_range_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
+                   const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mC,
+                   const __grid_constant__ ParParams p, const unsigned n_items) {
+  __shared__ ParShared sh;
+  const int T = (p.DHHV + 127) / 128, gx = (T + p.maxsub - 1) / p.maxsub;
+  for (unsigned w = blockIdx.x; w < n_items; w += gridDim.x) {
+    const int x = w % gx, ck = p.ck0 + (w / gx) % p.n_ck, bh = p.bh0 + w / (gx * p.n_ck), t0 = p.maxsub * x;
+    const bool last = w + gridDim.x >= n_items;
+    par_body<F16, true>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(p.maxsub, T - t0), ck, bh, w == blockIdx.x, last);
+  }
 }
 
 // deltaV, deltaK and deltaQ of one chunk in ONE launch: blockIdx.x enumerates the 128-wide output tiles of the three
@@ -907,7 +943,7 @@ par_bw_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUt
   const int T_dv = (p.DHHV + 127) / 128, T_dk = (p.DHQK + 127) / 128;   // output tiles per chunk of dV, and of dK / dQ
   const int c_dv = (T_dv + p.maxsub - 1) / p.maxsub, c_dk = (T_dk + p.maxsub - 1) / p.maxsub;   // CTAs per mode
   const int gx = c_dv + 2 * c_dk;   // 1-D grid in the order (mode and tile group, chunk, batch x head)
-  const int x = blockIdx.x % gx, ck = (blockIdx.x / gx) % p.NC, bh = p.bh0 + blockIdx.x / (gx * p.NC);
+  const int x = blockIdx.x % gx, ck = p.ck0 + (blockIdx.x / gx) % p.n_ck, bh = p.bh0 + blockIdx.x / (gx * p.n_ck);
   int mode, pair, T;
   const CUtensorMap *a, *b, *xm, *stm, *e;
   if (x < c_dv) { mode = PM_DV; pair = x; T = T_dv; a = &mK; b = &mQ; xm = &mDH; stm = &mdC_mn; e = &mDH; }
@@ -991,12 +1027,12 @@ static bool state_map(CUtensorMap* m, const void* base, const ChunkwiseDims& d, 
 
 template <bool BWD, int TN, bool F16>
 static int launch_rec_tn(const CUtensorMap& mL, const CUtensorMap& mR, const CUtensorMap& mS, const RecParams& rp,
-                         const ChunkwiseDims& d, int units, bool overlap, cudaStream_t st) {
+                         const ChunkwiseDims& d, int units, const UnitRange& ur, cudaStream_t st) {
   auto kern = rec_sm100<BWD, TN, F16>;
   static bool attr_done[64] = {};
   if (int rc = set_smem_once(kern, rec_smem_bytes(!BWD, TN), attr_done)) return rc;
   const unsigned grid = (unsigned)((d.DHHV + TN - 1) / TN) * (unsigned)((d.DHQK + 127) / 128) * (unsigned)units;
-  return launch_pdl(overlap && grid <= kPdlMaxCtas, kern, grid, REC_THREADS, rec_smem_bytes(!BWD, TN), st, mL, mR, mS, rp);
+  return launch_ex(ur.overlap && grid <= kPdlMaxCtas, ur.started, kern, grid, REC_THREADS, rec_smem_bytes(!BWD, TN), st, mL, mR, mS, rp);
 }
 
 // number of SMs of the current device (queried once per device)
@@ -1012,6 +1048,22 @@ static int sm_count() {
   return cached[dev];
 }
 
+// Segments of the sequence for a forward whose recurrence covers at most half of the SMs: the intra-chunk kernel of a
+// finished segment runs beside the recurrence of the next.  Estimate in microseconds, from measurements at 8 heads 256/512
+// (64 CTAs): the intra-chunk kernel alone takes 0.013 per chunk and 128 x 128 state tile; a chunk of the recurrence 1.15 with
+// 64-column tiles, 1.5 with the 128-column tiles that leave half of the SMs free; one more segment costs 15 (drain, launch,
+// refill).  What stays exposed is the last segment's intra-chunk work, which gives n = sqrt(P / 15).  Below a gain of 8 % the
+// extra launches are not worth their host time (8 heads, 32768 tokens: 522 us in one piece, 517 in four).
+int sm100_forward_segments(const ChunkwiseDims& d) {
+  const long c = sm100_recurrence_ctas(d);
+  if (2 * c > sm_count()) return 1;
+  const double P = 0.013 * (double)c * d.NC, slower = 4 * c <= sm_count() ? 0.0 : 0.35 * d.NC;
+  const int n = std::min(16, (int)std::lround(std::sqrt(P / 15.0)));
+  if (n < 2) return 1;
+  const double gain = P - P / n - 15.0 * (n - 1) - slower;
+  return gain > 0.08 * (P + 1.15 * d.NC) ? n : 1;
+}
+
 long sm100_recurrence_ctas(const ChunkwiseDims& d) {
   return (long)((d.DHHV + 127) / 128) * ((d.DHQK + 127) / 128) * d.B * d.NH;
 }
@@ -1025,10 +1077,17 @@ static bool rec_maps(RecMaps* m, const void* left, const void* right, const void
          state_map(&m->s, states ? states : left, d, 128);
 }
 
+// CTAs of the recurrence of one segment: at most half of the SMs, the others run the intra-chunk kernel
+static long segment_ctas(const ChunkwiseDims& d) {
+  const long c = sm100_recurrence_ctas(d);
+  return 4 * c <= sm_count() ? 2 * c : c;
+}
+
 template <bool BWD>
 static int launch_rec(const void* left, const void* right, RecParams rp, const ChunkwiseDims& d, UnitRange ur,
                       cudaStream_t st) {
   rp.bh0 = ur.first;
+  rp.ck0 = ur.chunk0; rp.n_ck = ur.chunks < 0 ? d.NC - ur.chunk0 : ur.chunks;
   const int units = ur.count < 0 ? d.B * d.NH - ur.first : ur.count;
   if (units <= 0) return MLSTM_OK;
   RecMaps m;
@@ -1036,9 +1095,10 @@ static int launch_rec(const void* left, const void* right, RecParams rp, const C
   // One CTA per SM walks all chunks of its state tile.  With 128-column tiles a launch of few (batch, head) units
   // leaves SMs idle; 64-column tiles double the CTAs as long as they still fit one wave.
   const bool f16 = d.dtype == MLSTM_F16;
-  if (2 * sm100_recurrence_ctas(d) <= sm_count())
-    return f16 ? launch_rec_tn<BWD, 64, true>(m.l, m.r, m.s, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 64, false>(m.l, m.r, m.s, rp, d, units, ur.overlap, st);
-  return f16 ? launch_rec_tn<BWD, 128, true>(m.l, m.r, m.s, rp, d, units, ur.overlap, st) : launch_rec_tn<BWD, 128, false>(m.l, m.r, m.s, rp, d, units, ur.overlap, st);
+  const long ctas64 = 2 * sm100_recurrence_ctas(d);
+  if (ur.chunks < 0 ? ctas64 <= sm_count() : segment_ctas(d) == ctas64)
+    return f16 ? launch_rec_tn<BWD, 64, true>(m.l, m.r, m.s, rp, d, units, ur, st) : launch_rec_tn<BWD, 64, false>(m.l, m.r, m.s, rp, d, units, ur, st);
+  return f16 ? launch_rec_tn<BWD, 128, true>(m.l, m.r, m.s, rp, d, units, ur, st) : launch_rec_tn<BWD, 128, false>(m.l, m.r, m.s, rp, d, units, ur, st);
 }
 
 template <int TN, bool F16>
@@ -1057,7 +1117,7 @@ int sm100_recurrent_fw(const void* k, const void* v, const GateBuffers& gb, cons
                        const ChunkwiseDims& d, cudaStream_t st, UnitRange ur) {
   PhaseScope ps(PH_REC_FW, st);
   RecParams rp{gb.abar, nullptr, 1.f, gb.gbar, c_initial, n_initial, c_states,
-               d.variant == MLSTM_SIG_NONORM ? nullptr : n_states, c_last, d.variant == MLSTM_SIG_NONORM ? nullptr : n_last, d.S, d.SP, d.NC, d.DHQK, d.DHHV, 0};
+               d.variant == MLSTM_SIG_NONORM ? nullptr : n_states, c_last, d.variant == MLSTM_SIG_NONORM ? nullptr : n_last, d.S, d.SP, d.NC, d.DHQK, d.DHHV, 0, 0, d.NC};
   return launch_rec<false>(k, v, rp, d, ur, st);
 }
 
@@ -1065,7 +1125,7 @@ int sm100_recurrent_bw(const void* q, const void* dh, const GateBuffers& gb, con
                        float* dc_initial, const ChunkwiseDims& d, cudaStream_t st, UnitRange ur) {
   PhaseScope ps(PH_REC_BW, st);
   RecParams rp{gb.bbar, gb.inv_den, d.qk_scale, gb.gbar, dc_last, nullptr, dc_states, nullptr,
-               dc_initial, nullptr, d.S, d.SP, d.NC, d.DHQK, d.DHHV, 0};
+               dc_initial, nullptr, d.S, d.SP, d.NC, d.DHQK, d.DHHV, 0, 0, d.NC};
   return launch_rec<true>(q, dh, rp, d, ur, st);
 }
 
@@ -1076,9 +1136,9 @@ int sm100_recurrent_pair(const void* k, const void* v, const float* c_initial, v
   if (units <= 0) return MLSTM_OK;
   PhaseScope ps(PH_REC_BW, st);
   const RecParams rp{gb.abar, nullptr, 1.f, gb.gbar, c_initial, nullptr, c_states, nullptr, nullptr, nullptr,
-                     d.S, d.SP, d.NC, d.DHQK, d.DHHV, ur.first};
+                     d.S, d.SP, d.NC, d.DHQK, d.DHHV, ur.first, 0, d.NC};
   const RecParams rpb{gb.bbar, gb.inv_den, d.qk_scale, gb.gbar, dc_last, nullptr, dc_states, nullptr, dc_initial, nullptr,
-                      d.S, d.SP, d.NC, d.DHQK, d.DHHV, ur.first};
+                      d.S, d.SP, d.NC, d.DHQK, d.DHHV, ur.first, 0, d.NC};
   RecMaps m, mb;
   if (!rec_maps(&m, k, v, c_states, d) || !rec_maps(&mb, q, dh, dc_states, d)) return MLSTM_ERR_CUDA;
   const bool f16 = d.dtype == MLSTM_F16;
@@ -1120,16 +1180,22 @@ int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuf
     return MLSTM_ERR_CUDA;
   ParParams pp = base_params(gb, d);
   pp.n_states = n_states; pp.out_h = (uint16_t*)h; pp.n_out = n_out; pp.inv_den_out = gb.inv_den;
-  pp.bh0 = ur.first;
+  pp.bh0 = ur.first; pp.ck0 = ur.chunk0; pp.n_ck = ur.chunks < 0 ? d.NC - ur.chunk0 : ur.chunks;
   const bool f16 = d.dtype == MLSTM_F16;
-  static bool attr_done[2][64] = {};
-  if (int rc = f16 ? set_smem_once(par_fw_sm100<true>, PAR_SMEM, attr_done[1])
-                   : set_smem_once(par_fw_sm100<false>, PAR_SMEM, attr_done[0])) return rc;
   const int T = (d.DHHV + 127) / 128;
-  pp.maxsub = par_maxsub([&](int m) { return (long)ceil_div(T, m) * d.NC * units; }, T);
-  const unsigned grid = (unsigned)ceil_div(T, pp.maxsub) * (unsigned)d.NC * (unsigned)units;
-  return launch_pdl(ur.overlap && grid <= kPdlMaxCtas, f16 ? par_fw_sm100<true> : par_fw_sm100<false>, grid, PAR_THREADS, PAR_SMEM, st,
-                    mQ, mK, mV, mC, pp);
+  pp.maxsub = par_maxsub([&](int m) { return (long)ceil_div(T, m) * pp.n_ck * units; }, T);
+  const unsigned grid = (unsigned)ceil_div(T, pp.maxsub) * (unsigned)pp.n_ck * (unsigned)units;
+  if (ur.chunks >= 0 && ur.chunk0 + ur.chunks < d.NC) {   // another segment's recurrence runs beside this launch
+    const unsigned places = 2u * (unsigned)(sm_count() - (int)segment_ctas(d));
+    auto kern = f16 ? par_fw_range_sm100<true> : par_fw_range_sm100<false>;
+    static bool range_attr[2][64] = {};
+    if (int rc = set_smem_once(kern, PAR_SMEM, range_attr[f16])) return rc;
+    return launch_pdl(false, kern, std::min(grid, places), PAR_THREADS, PAR_SMEM, st, mQ, mK, mV, mC, pp, grid);
+  }
+  auto kern = f16 ? par_fw_sm100<true> : par_fw_sm100<false>;
+  static bool attr_done[2][64] = {};
+  if (int rc = set_smem_once(kern, PAR_SMEM, attr_done[f16])) return rc;
+  return launch_pdl(ur.overlap && grid <= kPdlMaxCtas, kern, grid, PAR_THREADS, PAR_SMEM, st, mQ, mK, mV, mC, pp);
 }
 
 int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
@@ -1146,7 +1212,7 @@ int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* d
   ParParams pp = base_params(gb, d);
   pp.out_dv = (uint16_t*)dv; pp.out_dk = (uint16_t*)dk; pp.out_dq = (uint16_t*)dq;
   pp.rowdot_q = qdq_parts; pp.rowdot_k = kdk_parts;
-  pp.bh0 = ur.first;
+  pp.bh0 = ur.first; pp.n_ck = d.NC;
   const bool f16 = d.dtype == MLSTM_F16;
   static bool attr_done[2][64] = {};
   if (int rc = f16 ? set_smem_once(par_bw_sm100<true>, PAR_SMEM, attr_done[1])

@@ -69,21 +69,32 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // room on an SM from those of a second chain of launches.
 constexpr unsigned kPdlMaxCtas = 4 * 148;
 
+// started (nullable): recorded once every CTA of the launch is running.
 template <typename... KArgs, typename... Args>
-int launch_pdl(bool overlap, void (*kern)(KArgs...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, Args... args) {
+int launch_ex(bool overlap, cudaEvent_t started, void (*kern)(KArgs...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = overlap ? 1 : 0;
+  cudaLaunchAttribute at[2] = {};
+  if (overlap) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (started != nullptr) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeLaunchCompletionEvent;
+    at[cfg.numAttrs++].val.launchCompletionEvent.event = started;
+  }
+  cfg.attrs = at;
   note_launch();
   MLSTM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, KArgs(args)...));
   return MLSTM_OK;
+}
+
+template <typename... KArgs, typename... Args>
+int launch_pdl(bool overlap, void (*kern)(KArgs...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, Args... args) {
+  return launch_ex(overlap, nullptr, kern, grid, threads, smem, st, args...);
 }
 
 // Optional per-phase device timing (mlstm_b200_profile_*): when enabled, a pair of CUDA events

@@ -43,7 +43,9 @@ bool sm100_sizes_ok(int B, int NH, int S, int DHQK, int DHHV);
 // A launch may cover a sub-range of the B * NH independent (batch, head) units; all pointers stay those of the whole
 // problem.  count < 0: every unit from `first` on.
 // overlap: the launch may begin while the one before it in the stream drains (launch_pdl).
-struct UnitRange { int first = 0; int count = -1; bool overlap = true; };
+// The forward's launches may cover a range of chunks too (chunks < 0: every chunk from chunk0 on).
+// started (forward recurrence, nullable): recorded once all of its CTAs are running.
+struct UnitRange { int first = 0; int count = -1; bool overlap = true; int chunk0 = 0; int chunks = -1; cudaEvent_t started = nullptr; };
 int sm100_recurrent_fw(const void* k, const void* v, const GateBuffers& gb, const float* c_initial,
                        const float* n_initial, void* c_states, float* n_states, float* c_last, float* n_last,
                        const ChunkwiseDims& d, cudaStream_t st, UnitRange ur = UnitRange());
@@ -61,6 +63,8 @@ int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* d
                       float* kdk_parts, const ChunkwiseDims& d, cudaStream_t st, UnitRange ur = UnitRange());
 // number of CTAs the recurrence launches for the whole problem with 128-column state tiles, and SMs of the device
 long sm100_recurrence_ctas(const ChunkwiseDims& d);
+// segments the forward cuts the sequence into (1: none); a function of the sizes alone
+int sm100_forward_segments(const ChunkwiseDims& d);
 int sm100_sm_count();
 
 int sm100_device_status(int reset, int* status);
