@@ -1003,9 +1003,16 @@ static bool cached_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t
       return true;
     }
   }
-  const bool ok = slabs == 0 ? sm100_host::make_map_bf16(m, base, rows, cols, box_rows, box_cols, f16)
-                             : sm100_host::make_map_bf16_3d(m, base, slabs, rows, cols, box_rows, box_cols, f16);
-  if (!ok) return false;
+  auto encode = [&]() {
+    return slabs == 0 ? sm100_host::make_map_bf16(m, base, rows, cols, box_rows, box_cols, f16)
+                      : sm100_host::make_map_bf16_3d(m, base, slabs, rows, cols, box_rows, box_cols, f16);
+  };
+  if (!encode()) {
+    // A thread whose first CUDA work this is (an autograd worker that found all its memory in the allocator's cache) has
+    // no context bound yet, and the driver's encoder asks for one: cudaSetDevice binds the device's own.
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || !encode()) return false;
+  }
   keys[next] = MapKey{base, rows, cols, slabs, box_rows, box_cols, f16};
   maps[next] = *m;
   next = (next + 1) % N;
