@@ -126,7 +126,8 @@ size_t mlstm_b200_chunkwise_workspace_bytes(int B, int NH, int S, int DHQK, int 
  */
 /* Large problems (more recurrence CTAs than SMs) are run as two halves of the (batch, head) units on two streams: the
  * caller's and one the library creates per device on first use, forked and joined with events, so that one half's
- * last, partly filled wave of CTAs overlaps the other half's work.  Legal under stream capture.  on = 0 keeps every
+ * last, partly filled wave of CTAs overlaps the other half's work.  Forwards of a long sequence with few units run in
+ * segments the same way, the intra-chunk work of one beside the recurrence of the next.  Legal under stream capture.  on = 0 keeps every
  * launch on the caller's stream; returns the previous setting.  mlstm_b200_chunkwise_fw_static never splits. */
 int mlstm_b200_set_unit_split(int on);
 

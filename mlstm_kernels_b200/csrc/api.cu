@@ -422,6 +422,14 @@ static int forward_in_segments(const FwCall& a, const FwLayout& lay, const Chunk
   return rc;
 }
 
+size_t fw_bytes_one_stream(const CallDims& c) {
+  bool use_sm100 = false;
+  if (check_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L) != MLSTM_OK ||
+      resolve_impl(c.impl, c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, &use_sm100) != MLSTM_OK) return 0;
+  const int NC = (c.S + c.L - 1) / c.L;
+  return carve_fw(nullptr, c.B * c.NH, NC * c.L, NC).bytes;
+}
+
 int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   int rc = check_call(c);
   if (rc != MLSTM_OK) return rc;
@@ -434,7 +442,7 @@ int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   if ((rc = resolve_impl(c.impl, c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, &use_sm100)) != MLSTM_OK) return rc;
 
   const ChunkwiseDims d = make_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.variant, c.eps, c.dtype);
-  const int n_seg = use_sm100 ? sm100_forward_segments(d) : 1;
+  const int n_seg = use_sm100 && a.allow_split ? sm100_forward_segments(d) : 1;
   FwLayout lay = carve_fw(a.workspace, c.B * c.NH, d.SP, d.NC, n_seg > 1 ? c.DHQK : 0, n_seg > 1 ? c.DHHV : 0);
   if (a.workspace_bytes < lay.bytes) return MLSTM_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(c.stream);
@@ -442,7 +450,7 @@ int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   if ((rc = launch_gates(c.gate_dtype, a.i, a.f, c.variant == MLSTM_EXP ? a.m_initial : nullptr, nullptr, a.m_out, lay.gb, a.m_states, a.m_last, d, st)) != MLSTM_OK) return rc;
   lay.gb.inv_den = a.inv_den;   // written by the intra-chunk kernel
   // (off together with the unit split, and while phases are being timed)
-  if (n_seg > 1 && a.allow_split && g_split_on.load(std::memory_order_relaxed) != 0 && !g_prof_on)
+  if (n_seg > 1 && g_split_on.load(std::memory_order_relaxed) != 0 && !g_prof_on)
     return forward_in_segments(a, lay, d, n_seg, st);
   if (use_sm100) {
     UnitChains ch(d, st, a.allow_split);

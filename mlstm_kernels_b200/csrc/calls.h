@@ -50,6 +50,8 @@ struct BwCall {
 #if defined(__GNUC__)
 #pragma GCC visibility push(default)
 #endif
+// scratch of a forward with allow_split = false (0: sizes it does not take)
+size_t fw_bytes_one_stream(const CallDims& c);
 int run_chunkwise_fw(const FwCall& a, const CallDims& c);
 int run_chunkwise_bw(const BwCall& a, const CallDims& c);
 #if defined(__GNUC__)

@@ -13,7 +13,7 @@
 //                    into the same TMEM tile first and row-scaled in place.  The L x L gate matrix never
 //                    leaves the SM.
 //                    fw_kernel_parallel.py:14-289, bw_kernel_parallel_dV.py, bw_kernel_parallel_dK.py, bw_kernel_parallel_dQ.py
-// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
+// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four to seven half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
 // one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded.
 #include <algorithm>
 #include <cmath>

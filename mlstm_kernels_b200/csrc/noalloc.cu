@@ -69,7 +69,7 @@ int mlstm_b200_chunkwise_fw_static(const void* q, const void* k, const void* v, 
                                    float* c_last, float* n_last, float* m_last, int B, int NH, int S, int DHQK,
                                    int DHHV, int L, int dtype, int gate_dtype, int variant, int impl, float eps,
                                    void* stream) {
-  const size_t need = mlstm_b200_chunkwise_workspace_bytes(B, NH, S, DHQK, DHHV, L, dtype, variant, impl, 0);
+  const size_t need = mlstm::fw_bytes_one_stream(mlstm::CallDims{B, NH, S, DHQK, DHHV, L, dtype, gate_dtype, variant, impl, eps, stream});
   if (need == 0) return MLSTM_ERR_SHAPE;
   if (need > kStaticScratchBytes) return MLSTM_ERR_WORKSPACE;  // problem too large for the built-in scratch
   void* scratch = nullptr;

@@ -52,3 +52,22 @@ def test_segments_under_capture():
         g.replay()
     torch.cuda.synchronize()
     assert torch.equal(h0, h1) and all(torch.equal(a, b) for a, b in zip(last0, last1))
+
+
+def test_allocation_free_forward_keeps_one_stream():
+    """Sizes that the regular entry point cuts into segments: the static one still takes them, with its fixed scratch."""
+    B, NH, S, DHQK, DHHV = 1, 4, 88000, 256, 512
+    q, k, v = (torch.randn(B, NH, S, d, device="cuda").bfloat16() for d in (DHQK, DHQK, DHHV))
+    i, f = torch.randn(B, NH, S, device="cuda"), torch.randn(B, NH, S, device="cuda") + 4.0
+    NC = -(-S // 128)
+    h = torch.empty_like(v)
+    n_out, m_out = torch.empty(B, NH, S, device="cuda"), torch.empty(B, NH, S, device="cuda")
+    cs = torch.empty(B, NH, NC + 1, DHQK, DHHV, device="cuda", dtype=torch.bfloat16)
+    ns, ms = torch.empty(B, NH, NC + 1, DHQK, device="cuda"), torch.empty(B, NH, NC + 1, device="cuda")
+    p = lambda t: t.data_ptr()
+    rc = _lib.load().mlstm_b200_chunkwise_fw_static(p(q), p(k), p(v), p(i), p(f), None, None, None, p(h), p(n_out), p(m_out),
+                                                    p(cs), p(ns), p(ms), None, None, None, B, NH, S, DHQK, DHHV, 128,
+                                                    _lib.BF16, _lib.F32, _lib.EXP, 0, 1e-6,
+                                                    torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    assert torch.equal(h, mlstm_chunkwise__b200_xl_chunk(q, k, v, i, f, chunk_size=128))
