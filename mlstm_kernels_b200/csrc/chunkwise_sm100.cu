@@ -61,16 +61,6 @@ constexpr int rec_smem_bytes(bool has_n, int TN) {
   return rec_stages(has_n, TN) * rec_stage_bytes(TN) + (has_n ? REC_NPART_BYTES : 0) + 2 * rec_out_bytes(TN) + 1024;
 }
 
-template <int STAGES, bool TWO_SCALES>
-struct RecShared {
-  uint64_t bar_full[STAGES], bar_empty[STAGES], bar_scaled[STAGES], bar_acc_full[2], bar_acc_free[2], bar_nsum[2], bar_nread[2], bar_out_full[2], bar_out_free[2];
-  uint32_t s_tmem;
-  int s_abort;   // set by the first wait of this CTA that runs out; every other wait polls it
-  // per-row scale factors of the left tile, copied with the stage (backward: two factors per row)
-  __align__(16) float s_scale[STAGES][REC_HALF], s_scale2[TWO_SCALES ? STAGES : 1][REC_HALF];
-  float s_g[8];  // decay of the chunk, ring of eight (outlives the operand ring)
-};
-
 // One ring stage holds 64 tokens of the left and of the right operand (boxes of 64 rows x 64 columns, 8 KB each:
 // left columns d0.., d0+64.., right columns e0.., e0+64..).  A chunk is two stages; the product of a chunk is
 // accumulated over both before the state warps fold it in.  The ring is deeper than one chunk so that the load of
@@ -79,21 +69,20 @@ struct RecShared {
 // (batch, head) units still covers the GPU).
 // F16: the 16-bit element type is IEEE half instead of bf16 (operands, gated tiles, stored states, outputs).
 // HAS_N: the vector n is kept as well (forward, unless only the states are wanted again).
-template <bool BWD, int TN, bool F16, bool HAS_N, typename Shared>
+template <bool BWD, int TN, bool F16, bool HAS_N>
 __device__ __forceinline__ void
-rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& mapS, const RecParams& p, Shared& sh,
-         const unsigned block) {
+rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& mapS, const RecParams& p, const unsigned block) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr int REC_STAGES = rec_stages(HAS_N, TN), REC_STAGE_BYTES = rec_stage_bytes(TN), REC_OUT = rec_out_bytes(TN);
-  auto &bar_full = sh.bar_full, &bar_empty = sh.bar_empty, &bar_scaled = sh.bar_scaled;
-  auto &bar_acc_full = sh.bar_acc_full, &bar_acc_free = sh.bar_acc_free, &bar_nsum = sh.bar_nsum, &bar_nread = sh.bar_nread;
-  auto &bar_out_full = sh.bar_out_full, &bar_out_free = sh.bar_out_free;
-  auto &s_tmem = sh.s_tmem;
-  auto &s_abort = sh.s_abort;
-  auto &s_scale = sh.s_scale;
-  auto &s_scale2 = sh.s_scale2;
-  auto &s_g = sh.s_g;
+  // (separate arrays: members of one shared struct cost 68 bytes of register spills in the 128-column forward)
+  __shared__ uint64_t bar_full[REC_STAGES], bar_empty[REC_STAGES], bar_scaled[REC_STAGES], bar_acc_full[2], bar_acc_free[2], bar_nsum[2],
+      bar_nread[2], bar_out_full[2], bar_out_free[2];
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_abort;   // set by the first wait of this CTA that runs out; every other wait polls it
+  // per-row scale factors of the left tile, copied with the stage (backward: two factors per row)
+  __shared__ __align__(16) float s_scale[REC_STAGES][REC_HALF], s_scale2[BWD ? REC_STAGES : 1][REC_HALF];
+  __shared__ float s_g[8];  // decay of the chunk, ring of eight (outlives the operand ring)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 1-D grid (no 65535 limit on batch x heads), state tiles of one (batch, head) next to each other
@@ -361,8 +350,7 @@ template <bool BWD, int TN, bool F16>
 __global__ void __launch_bounds__(REC_THREADS, 1)
 rec_sm100(const __grid_constant__ CUtensorMap mapL, const __grid_constant__ CUtensorMap mapR,
           const __grid_constant__ CUtensorMap mapS, const __grid_constant__ RecParams p) {
-  __shared__ RecShared<rec_stages(!BWD, TN), BWD> sh;
-  rec_body<BWD, TN, F16, !BWD>(mapL, mapR, mapS, p, sh, blockIdx.x);
+  rec_body<BWD, TN, F16, !BWD>(mapL, mapR, mapS, p, blockIdx.x);
 }
 
 // Both recurrences of a backward that finds no per-chunk states in one launch: the first n_fw CTAs run the forward's
@@ -374,9 +362,8 @@ rec_pair_sm100(const __grid_constant__ CUtensorMap mL, const __grid_constant__ C
                const __grid_constant__ CUtensorMap mS, const __grid_constant__ RecParams p,
                const __grid_constant__ CUtensorMap mLb, const __grid_constant__ CUtensorMap mRb,
                const __grid_constant__ CUtensorMap mSb, const __grid_constant__ RecParams pb, const unsigned n_fw) {
-  __shared__ RecShared<rec_stages(false, TN), true> sh;
-  if (blockIdx.x < n_fw) rec_body<false, TN, F16, false>(mL, mR, mS, p, sh, blockIdx.x);
-  else rec_body<true, TN, F16, false>(mLb, mRb, mSb, pb, sh, blockIdx.x - n_fw);
+  if (blockIdx.x < n_fw) rec_body<false, TN, F16, false>(mL, mR, mS, p, blockIdx.x);
+  else rec_body<true, TN, F16, false>(mLb, mRb, mSb, pb, blockIdx.x - n_fw);
 }
 
 // =====================================================================================================
