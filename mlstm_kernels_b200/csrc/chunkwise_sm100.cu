@@ -13,7 +13,7 @@
 //                    into the same TMEM tile first and row-scaled in place.  The L x L gate matrix never
 //                    leaves the SM.
 //                    fw_kernel_parallel.py:14-289, bw_kernel_parallel_dV.py, bw_kernel_parallel_dK.py, bw_kernel_parallel_dQ.py
-// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four to seven half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
+// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four or six half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
 // one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded.
 #include <algorithm>
 #include <cmath>
@@ -54,11 +54,14 @@ constexpr int REC_HALF = 64;                     // tokens per ring stage: half 
 constexpr int REC_NPART_BYTES = 2 * 32 * 128 * 4;   // double-buffered partial column sums of the gated left tile
 constexpr int rec_stage_bytes(int TN) { return 16384 + TN * 128; }    // 64 tokens: left tile 16 KB + right tile
 constexpr int rec_out_bytes(int TN) { return TN * 256; }              // 16-bit state tile staged for the TMA store (two of them)
-// Operand ring depth, as deep as shared memory allows.  A stage comes round in about 4600 cycles (load 2500, gating and
-// hand-over 1300, MMA and hand-back 800), so the 64-column form with its smaller stages runs three chunks ahead.
-constexpr int rec_stages(bool has_n, int TN) { return TN == 128 ? 4 : (has_n ? 6 : 7); }
+// Operand ring depth.  A stage comes round in about 4600 cycles (load 2500, gating and hand-over 1300, MMA and hand-back
+// 800), so the 64-column form with its smaller stages runs three chunks ahead.  The depth is even, so that a stage always
+// goes to the same group of gating warps: a wait sees the parity of a phase only, and in an odd ring a group would come back
+// to a stage two phases later, where the load before the other group's last one passes for its own.  (The 64-column form
+// without n has room for a seventh stage, which measured the same: 4 x 4 x 1024, 96/192, the call 88.4 and 88.8 us.)
+constexpr int rec_stages(int TN) { return TN == 128 ? 4 : 6; }
 constexpr int rec_smem_bytes(bool has_n, int TN) {
-  return rec_stages(has_n, TN) * rec_stage_bytes(TN) + (has_n ? REC_NPART_BYTES : 0) + 2 * rec_out_bytes(TN) + 1024;
+  return rec_stages(TN) * rec_stage_bytes(TN) + (has_n ? REC_NPART_BYTES : 0) + 2 * rec_out_bytes(TN) + 1024;
 }
 
 // One ring stage holds 64 tokens of the left and of the right operand (boxes of 64 rows x 64 columns, 8 KB each:
@@ -74,7 +77,7 @@ __device__ __forceinline__ void
 rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& mapS, const RecParams& p, const unsigned block) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int REC_STAGES = rec_stages(HAS_N, TN), REC_STAGE_BYTES = rec_stage_bytes(TN), REC_OUT = rec_out_bytes(TN);
+  constexpr int REC_STAGES = rec_stages(TN), REC_STAGE_BYTES = rec_stage_bytes(TN), REC_OUT = rec_out_bytes(TN);
   // (separate arrays: members of one shared struct cost 68 bytes of register spills in the 128-column forward)
   __shared__ uint64_t bar_full[REC_STAGES], bar_empty[REC_STAGES], bar_scaled[REC_STAGES], bar_acc_full[2], bar_acc_free[2], bar_nsum[2],
       bar_nread[2], bar_out_full[2], bar_out_free[2];
@@ -87,6 +90,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 1-D grid (no 65535 limit on batch x heads), state tiles of one (batch, head) next to each other
   static_assert(TN == 128 || TN == 64, "state tile width");
+  static_assert(REC_STAGES % 2 == 0, "the gating groups take the half chunks in turn: a stage must always meet the same group");
   constexpr int HC = TN / 2;   // columns each of the two state-warp groups owns
   // head dims need not be multiples of the tile: the last tile hangs over the edge, where loads read zeros (the
   // tensor maps know the true extents), plain accesses are masked and the state store is clipped

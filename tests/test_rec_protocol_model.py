@@ -1,17 +1,29 @@
-"""Model of the barrier protocol of the recurrence kernel (csrc/chunkwise_sm100.cu, rec_sm100), run on the CPU.
+"""Model of the barrier protocol of the recurrence kernel (csrc/chunkwise_sm100.cu, rec_body), run on the CPU.
 
 Six roles hand work around two rings whose barriers run on over the whole sequence (thousands of phases), every wait
-seeing only the phase PARITY: the TMA producer (ring of four half-chunk stages), the gating warps, the MMA thread (two
-accumulator buffers), the state warps, the store warp (two staging buffers) and the n warp (two buffers of partial
-sums).  The order of waits, arrivals, copy issues and MMA commits of each role is restated here and run under random
-interleavings - copies land in any order, commits fire in order - with every wait checked against the true phase
-count (a waiter two phases away from its barrier, early or late, is a hang or a corruption), every barrier against
-over-arrival, the run against deadlock, and the eight-entry ring of chunk decays against being overwritten before
-its readers are done.  A model, kept next to the kernel by hand."""
+seeing only the phase PARITY: the TMA producer (operand ring of half-chunk stages), two groups of four gating warps, the
+MMA thread (two accumulator buffers), the state warps, the store warp (two staging buffers) and the n warp (two buffers
+of partial sums, each filled by both halves of a chunk).  The order of waits, arrivals, copy issues and MMA commits of
+each role is restated here and run under random interleavings - copies land in any order, commits fire in order - with
+every wait checked against the true phase count (a waiter two phases away from its barrier, early or late, is a hang or
+a corruption), every barrier against over-arrival, the run against deadlock, and the eight-entry ring of chunk decays
+against being overwritten before its readers are done.  The ring depths are read from the kernel's source; the order of
+operations is a model, kept next to the kernel by hand."""
 
+import os
 import random
+import re
 
 import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlstm_kernels_b200", "csrc")
+
+
+def ring_depths():
+    """Stages of the operand ring with 128-column and with 64-column tiles."""
+    with open(os.path.join(CSRC, "chunkwise_sm100.cu")) as f:
+        m = re.search(r"int rec_stages\(int TN\) \{ return TN == 128 \? (\d+) : (\d+); \}", f.read())
+    return tuple(int(x) for x in m.groups())
 
 
 class Bar:
@@ -35,12 +47,12 @@ class Bar:
         return passes
 
 
-def run(NC, do_n, store_states, seed, stages=4):
+def run(NC, do_n, store_states, seed, stages):
     rnd = random.Random(seed)
     NH2 = 2 * NC
     B = {}
     for s in range(stages):
-        B[f"full{s}"], B[f"empty{s}"], B[f"scaled{s}"] = Bar(f"full{s}", 1), Bar(f"empty{s}", 1), Bar(f"scaled{s}", 8)
+        B[f"full{s}"], B[f"empty{s}"], B[f"scaled{s}"] = Bar(f"full{s}", 1), Bar(f"empty{s}", 1), Bar(f"scaled{s}", 4)
     for s in range(2):
         B[f"acc_full{s}"], B[f"acc_free{s}"] = Bar(f"acc_full{s}", 1), Bar(f"acc_free{s}", 8)
         B[f"nsum{s}"], B[f"nread{s}"] = Bar(f"nsum{s}", 8), Bar(f"nread{s}", 1)
@@ -72,15 +84,16 @@ def run(NC, do_n, store_states, seed, stages=4):
             if h % 2 == 1:
                 commits.append(f"acc_full{buf}")
 
-    def gating():
-        for h in range(NH2):
+    def gating(group):
+        for h in range(group, NH2, 2):
             st, s = h % stages, h >> 1
             nb = s & 1
             yield ("wait", f"full{st}", h // stages)
-            if do_n and h % 2 == 1 and s >= 2:
-                yield ("wait", f"nread{nb}", (s >> 1) - 1)
             B[f"scaled{st}"].arrive()
-            if do_n and h % 2 == 1:
+            if do_n:
+                yield ("step",)
+                if s >= 2:
+                    yield ("wait", f"nread{nb}", (s >> 1) - 1)
                 B[f"nsum{nb}"].arrive()
 
     def store_warp():
@@ -95,7 +108,8 @@ def run(NC, do_n, store_states, seed, stages=4):
             nb = s & 1
             yield ("wait", f"nsum{nb}", s >> 1)
             B[f"nread{nb}"].arrive()
-            n_done[0] = s
+            yield ("step",)
+            n_done[0] = s      # (reads the chunk's decay after that)
 
     def state_warp(w):
         n_out = 0
@@ -118,7 +132,7 @@ def run(NC, do_n, store_states, seed, stages=4):
 
     agents = {"prod": producer(), "mma": mma()}
     for w in range(8):
-        agents[f"gate{w}"] = gating()
+        agents[f"gate{w}"] = gating(w >> 2)
         agents[f"state{w}"] = state_warp(w)
     if store_states:
         agents["store"] = store_warp()
@@ -161,8 +175,25 @@ def run(NC, do_n, store_states, seed, stages=4):
             raise AssertionError(f"DEADLOCK: {blocked}")
 
 
+DEPTHS = ring_depths()
+
+
 @pytest.mark.parametrize("NC", [1, 2, 3, 5, 8, 17, 40])
 @pytest.mark.parametrize("do_n,store_states", [(True, True), (False, True), (False, False), (True, False)])
-def test_recurrence_protocol_has_no_aliasing_deadlock_or_over_arrival(NC, do_n, store_states):
+@pytest.mark.parametrize("stages", DEPTHS)
+def test_recurrence_protocol_has_no_aliasing_deadlock_or_over_arrival(NC, do_n, store_states, stages):
     for seed in range(25):
-        run(NC, do_n, store_states, seed)
+        run(NC, do_n, store_states, seed, stages)
+
+
+@pytest.mark.parametrize("stages", [5, 7])
+def test_odd_ring_would_alias(stages):
+    """With an odd number of stages a gating group returns to a stage two phases later, and its wait passes on the load
+    before the one it wants."""
+    for seed in range(400):
+        try:
+            run(16, False, True, seed, stages)
+        except AssertionError as e:
+            assert "ALIAS early pass on full" in str(e)
+            return
+    raise AssertionError("no interleaving out of 400 showed the hazard")
