@@ -130,17 +130,18 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       const int s = blk * 32 + lane;
       return s < NS ? p.gbar[(size_t)bh * NC + (BWD ? NC - 1 - s : ck0 + s)] : 0.f;
     };
-    float g_blk = load_g(0), g_nxt = load_g(1);
+    float g_blk = load_g(0), g_nxt = load_g(1), g = 0.f;
     int issued = 0;
     for (int h = 0; h < NH2; ++h) {
       const int st = h % REC_STAGES, s = h >> 1;
       if ((h & 1) == 0) {
         if (s > 0 && (s & 31) == 0) { g_blk = g_nxt; g_nxt = load_g((s >> 5) + 1); }
-        const float g = __shfl_sync(0xffffffffu, g_blk, s & 31);
-        if (lane == 0) s_g[s & 7] = g;   // read two or more barrier hand-overs later (MMA commit -> state warps)
+        g = __shfl_sync(0xffffffffu, g_blk, s & 31);
       }
       if (!mbar_wait(&bar_empty[st], ((h / REC_STAGES) & 1) ^ 1, &s_abort, &g_sm100_status, 101)) break;
       if (elect_one()) {
+        // by the lane whose arrival below releases it (to the gating warps and the MMA thread, and by theirs to the readers)
+        if ((h & 1) == 0) s_g[s & 7] = g;
         const int ck = BWD ? NC - 1 - s : ck0 + s;
         // token rows past the end of the sequence (ragged last chunk) arrive as zeros; their scale slots hold zeros
         const int y = ck * CL + (h & 1) * REC_HALF;          // first token of this half chunk inside the sequence

@@ -7,7 +7,8 @@ of partial sums, each filled by both halves of a chunk).  The order of waits, ar
 each role is restated here and run under random interleavings - copies land in any order, commits fire in order - with
 every wait checked against the true phase count (a waiter two phases away from its barrier, early or late, is a hang or
 a corruption), every barrier against over-arrival, the run against deadlock, and the eight-entry ring of chunk decays
-against being overwritten before its readers are done.  The ring depths are read from the kernel's source; the order of
+against races: every thread carries a vector clock, handed on by arrivals and taken up by waits, and a read of a decay
+must be ordered after its write, the write that overwrites it after all its reads.  The ring depths are read from the kernel's source; the order of
 operations is a model, kept next to the kernel by hand."""
 
 import os
@@ -26,16 +27,26 @@ def ring_depths():
     return tuple(int(x) for x in m.groups())
 
 
+def join(into, other):
+    for a, t in other.items():
+        if into.get(a, 0) < t:
+            into[a] = t
+
+
 class Bar:
     def __init__(self, name, count):
         self.name, self.count, self.pending, self.phase = name, count, count, 0
+        self.clock, self.released = {}, {}    # of the arrivals of the current phase; per completed phase
 
-    def arrive(self):
+    def arrive(self, clock):
         self.pending -= 1
         assert self.pending >= 0, f"over-arrival on {self.name}"
+        join(self.clock, clock)
         if self.pending == 0:
+            self.released = {self.phase: self.clock, self.phase - 1: self.released.get(self.phase - 1, {})}
             self.phase += 1
             self.pending = self.count
+            self.clock = {}
 
     def test(self, want):
         passes = (self.phase & 1) != (want & 1)      # what the hardware sees
@@ -47,7 +58,7 @@ class Bar:
         return passes
 
 
-def run(NC, do_n, store_states, seed, stages):
+def run(NC, do_n, store_states, seed, stages, decay_writer="issuing lane"):
     rnd = random.Random(seed)
     NH2 = 2 * NC
     B = {}
@@ -58,19 +69,40 @@ def run(NC, do_n, store_states, seed, stages):
         B[f"nsum{s}"], B[f"nread{s}"] = Bar(f"nsum{s}", 8), Bar(f"nread{s}", 1)
         B[f"out_full{s}"], B[f"out_free{s}"] = Bar(f"out_full{s}", 8), Bar(f"out_free{s}", 1)
     loads, commits = [], []          # copies in flight (land in any order), MMA commits (fire in order)
-    decay_written = [-1] * 8         # chunk whose decay sits in each slot of the ring of eight
-    state_done = [-1] * 8            # last chunk each state warp has folded (it reads the chunk's decay while folding)
-    n_done = [-1 if do_n else 10 ** 9]
+    clocks = {}                      # per agent: what it knows of every agent's operations
+    written = [None] * 8             # slot of the decay ring: (writer, its time, chunk)
+    reads = [[] for _ in range(8)]   # (reader, its time) since the last write
+
+    def tick(a):
+        clocks[a][a] = clocks[a].get(a, 0) + 1
+        return clocks[a][a]
+
+    def arrive(a, name):
+        tick(a)
+        B[name].arrive(clocks[a])
+
+    def write_decay(a, s):
+        for r, t in reads[s & 7]:
+            assert clocks[a].get(r, 0) >= t, f"decay of chunk {s - 8} overwritten before {r} is known to have read it"
+        reads[s & 7].clear()
+        written[s & 7] = (a, tick(a), s)
+
+    def read_decay(a, s):
+        w, t, chunk = written[s & 7]
+        assert chunk == s, f"{a} reads the decay of chunk {chunk} for that of {s}"
+        assert clocks[a].get(w, 0) >= t, f"{a} reads the decay of chunk {s}, whose write by {w} nothing orders before it"
+        reads[s & 7].append((a, tick(a)))
 
     def producer():
         for h in range(NH2):
             st, s = h % stages, h >> 1
-            if h % 2 == 0:
-                if decay_written[s & 7] >= 0:   # about to overwrite the decay of chunk s - 8
-                    assert min(state_done + n_done) >= decay_written[s & 7], "decay ring overwritten too early"
-                decay_written[s & 7] = s
+            if h % 2 == 0 and decay_writer != "issuing lane":
+                write_decay("prod other lane", s)
             yield ("wait", f"empty{st}", h // stages - 1)
-            loads.append(st)
+            if h % 2 == 0 and decay_writer == "issuing lane":
+                write_decay("prod", s)
+            tick("prod")
+            loads.append((st, dict(clocks["prod"])))   # (the copy's completion; the arrival that expects it)
             yield ("step",)
 
     def mma():
@@ -80,36 +112,37 @@ def run(NC, do_n, store_states, seed, stages):
             yield ("wait", f"scaled{st}", h // stages)
             if h % 2 == 0:
                 yield ("wait", f"acc_free{buf}", (s >> 1) - 1)
-            commits.append(f"empty{st}")
+            tick("mma")
+            commits.append((f"empty{st}", dict(clocks["mma"])))
             if h % 2 == 1:
-                commits.append(f"acc_full{buf}")
+                commits.append((f"acc_full{buf}", dict(clocks["mma"])))
 
-    def gating(group):
+    def gating(w, group):
         for h in range(group, NH2, 2):
             st, s = h % stages, h >> 1
             nb = s & 1
             yield ("wait", f"full{st}", h // stages)
-            B[f"scaled{st}"].arrive()
+            arrive(w, f"scaled{st}")
             if do_n:
                 yield ("step",)
                 if s >= 2:
                     yield ("wait", f"nread{nb}", (s >> 1) - 1)
-                B[f"nsum{nb}"].arrive()
+                arrive(w, f"nsum{nb}")
 
     def store_warp():
         for n in range(NC + 1):
             ob = n & 1
             yield ("wait", f"out_full{ob}", n >> 1)
             if n >= 1:
-                B[f"out_free{ob ^ 1}"].arrive()
+                arrive("store", f"out_free{ob ^ 1}")
 
     def n_warp():
         for s in range(NC):
             nb = s & 1
             yield ("wait", f"nsum{nb}", s >> 1)
-            B[f"nread{nb}"].arrive()
+            arrive("n", f"nread{nb}")
             yield ("step",)
-            n_done[0] = s      # (reads the chunk's decay after that)
+            read_decay("n", s)
 
     def state_warp(w):
         n_out = 0
@@ -120,25 +153,33 @@ def run(NC, do_n, store_states, seed, stages):
                 ob = n_out & 1
                 if n_out >= 2:
                     yield ("wait", f"out_free{ob}", (n_out >> 1) - 1)
-                B[f"out_full{ob}"].arrive()
+                arrive(w, f"out_full{ob}")
             n_out += 1
         yield from store_c()
         for s in range(NC):
             buf = s & 1
             yield ("wait", f"acc_full{buf}", s >> 1)
-            B[f"acc_free{buf}"].arrive()
-            state_done[w] = s
+            read_decay(w, s)
+            arrive(w, f"acc_free{buf}")
             yield from store_c()
 
     agents = {"prod": producer(), "mma": mma()}
     for w in range(8):
-        agents[f"gate{w}"] = gating(w >> 2)
-        agents[f"state{w}"] = state_warp(w)
+        agents[f"gate{w}"] = gating(f"gate{w}", w >> 2)
+        agents[f"state{w}"] = state_warp(f"state{w}")
     if store_states:
         agents["store"] = store_warp()
     if do_n:
         agents["n"] = n_warp()
+    clocks.update({a: {} for a in [*agents, "prod other lane"]})
     blocked, alive = {}, set(agents)
+
+    def acquire(a, bar, phase):
+        if phase < 0:
+            return
+        for lane in (a, "prod other lane") if a == "prod" else (a,):
+            join(clocks[lane], B[bar].released.get(phase, {}))
+
     while alive:
         choices = [("agent", a) for a in alive]
         if loads:
@@ -149,11 +190,13 @@ def run(NC, do_n, store_states, seed, stages):
         progressed = False
         for kind, a in choices:
             if kind == "load":
-                B[f"full{loads.pop(rnd.randrange(len(loads)))}"].arrive()
+                st, clock = loads.pop(rnd.randrange(len(loads)))
+                B[f"full{st}"].arrive(clock)
                 progressed = True
                 break
             if kind == "commit":
-                B[commits.pop(0)].arrive()
+                bar, clock = commits.pop(0)
+                B[bar].arrive(clock)
                 progressed = True
                 break
             if a in blocked:
@@ -161,14 +204,18 @@ def run(NC, do_n, store_states, seed, stages):
                 if not B[bn].test(ph):
                     continue
                 del blocked[a]
+                acquire(a, bn, ph)
             try:
                 op = next(agents[a])
             except StopIteration:
                 alive.discard(a)
                 progressed = True
                 break
-            if op[0] == "wait" and not B[op[1]].test(op[2]):
-                blocked[a] = op
+            if op[0] == "wait":
+                if B[op[1]].test(op[2]):
+                    acquire(a, op[1], op[2])
+                else:
+                    blocked[a] = op
             progressed = True
             break
         if not progressed:
@@ -197,3 +244,10 @@ def test_odd_ring_would_alias(stages):
             assert "ALIAS early pass on full" in str(e)
             return
     raise AssertionError("no interleaving out of 400 showed the hazard")
+
+
+def test_decay_written_by_another_lane_than_the_arriving_one_would_race():
+    """The decay has to be written by the lane that arrives on the stage's barrier: nothing orders another lane's write
+    before the readers."""
+    with pytest.raises(AssertionError, match="nothing orders"):
+        run(4, True, True, 0, DEPTHS[0], decay_writer="another lane")
