@@ -14,7 +14,8 @@
 //                    leaves the SM.
 //                    fw_kernel_parallel.py:14-289, bw_kernel_parallel_dV.py, bw_kernel_parallel_dK.py, bw_kernel_parallel_dQ.py
 // Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four or six half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
-// one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded.
+// one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded
+// and a lane whose wait has run out keeps its warp company to the end of the role, without arriving anywhere: see warp_arrive.
 #include <algorithm>
 #include <cmath>
 
@@ -131,15 +132,16 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       return s < NS ? p.gbar[(size_t)bh * NC + (BWD ? NC - 1 - s : ck0 + s)] : 0.f;
     };
     float g_blk = load_g(0), g_nxt = load_g(1), g = 0.f;
-    int issued = 0;
+    int issued = 0;   // by the issuing lane
+    bool ok = true;
     for (int h = 0; h < NH2; ++h) {
       const int st = h % REC_STAGES, s = h >> 1;
       if ((h & 1) == 0) {
         if (s > 0 && (s & 31) == 0) { g_blk = g_nxt; g_nxt = load_g((s >> 5) + 1); }
         g = __shfl_sync(0xffffffffu, g_blk, s & 31);
       }
-      if (!mbar_wait(&bar_empty[st], ((h / REC_STAGES) & 1) ^ 1, &s_abort, &g_sm100_status, 101)) break;
-      if (elect_one()) {
+      ok = ok && mbar_wait(&bar_empty[st], ((h / REC_STAGES) & 1) ^ 1, &s_abort, &g_sm100_status, 101);
+      if (elect_one() && ok) {
         // by the lane whose arrival below releases it (to the gating warps and the MMA thread, and by theirs to the readers)
         if ((h & 1) == 0) s_g[s & 7] = g;
         const int ck = BWD ? NC - 1 - s : ck0 + s;
@@ -154,10 +156,10 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
         tma_load_3d(sl + 8192, &mapL, &bar_full[st], d0 + 64, y, bh);
         tma_load_3d(sl + 16384, &mapR, &bar_full[st], e0, y, bh);
         if (TN == 128) tma_load_3d(sl + 24576, &mapR, &bar_full[st], e0 + 64, y, bh);
+        issued = h + 1;
       }
-      issued = h + 1;
     }
-    if (lane == 0 && issued < NH2 && issued > 0) {  // error path: let the copies in flight land before the CTA retires
+    if (issued < NH2 && issued > 0) {  // error path: let the copies in flight land before the CTA retires
       for (int h = max(0, issued - REC_STAGES); h < issued; ++h)
         mbar_wait(&bar_full[h % REC_STAGES], (h / REC_STAGES) & 1, nullptr, nullptr, 0);
     }
@@ -185,10 +187,16 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
     // hand-over, which one group of eight paid for every stage (2700 cycles per chunk, the limit of the whole kernel).
     const int grp = (warp - 2) >> 2, ct = (tid - 64) & 127;
     const int row0 = ct >> 3;                      // rows row0 + 16 u of the stage, 16-byte piece ct & 7 of either box
-    bool ok = true;
+    // a lane whose wait has run out meets the others of its warp in the arrivals that are left, without arriving
+    auto stand_by = [&](int h, bool scaled) {
+      for (; h < NH2; h += 2, scaled = false) {
+        if (!scaled) warp_arrive(nullptr, false);
+        if (do_n) warp_arrive(nullptr, false);
+      }
+    };
     for (int h = grp; h < NH2; h += 2) {
       const int st = h % REC_STAGES, s = h >> 1, nb = s & 1;
-      if (!mbar_wait(&bar_full[st], (h / REC_STAGES) & 1, &s_abort, &g_sm100_status, 105)) { ok = false; break; }
+      if (!mbar_wait(&bar_full[st], (h / REC_STAGES) & 1, &s_abort, &g_sm100_status, 105)) { stand_by(h, false); break; }
       // two 64-column boxes of 64 rows x 128 B, 128-byte swizzle: the scale depends on the row only
       uint8_t* sl = smem + st * REC_STAGE_BYTES + row0 * 128 + (ct & 7) * 16;
       float sc[4];
@@ -219,10 +227,10 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
         }
       }
       fence_proxy_async_smem();
-      warp_arrive(&bar_scaled[st]);
+      warp_arrive(&bar_scaled[st], true);
       if (do_n) {   // partial column sums of this half: 16 rows of the chunk's 32
         // the n warp has read the partial sums of chunk s - 2 out of this buffer
-        if (s >= 2 && !mbar_wait(&bar_nread[nb], ((s >> 1) - 1) & 1, &s_abort, &g_sm100_status, 109)) { ok = false; break; }
+        if (s >= 2 && !mbar_wait(&bar_nread[nb], ((s >> 1) - 1) & 1, &s_abort, &g_sm100_status, 109)) { stand_by(h, true); break; }
         float* npart = reinterpret_cast<float*>(smem + REC_STAGES * REC_STAGE_BYTES) + nb * (32 * 128) + (grp * 16 + row0) * 128;
         const int lc = (ct & 7) ^ (row0 & 7);   // logical 16-byte column chunk behind the swizzle
 #pragma unroll
@@ -231,10 +239,9 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
           dst[0] = make_ulonglong2(ns[b][0], ns[b][1]);
           dst[1] = make_ulonglong2(ns[b][2], ns[b][3]);
         }
-        warp_arrive(&bar_nsum[nb]);   // (complete when both halves of chunk s are in)
+        warp_arrive(&bar_nsum[nb], true);   // (complete when both halves of chunk s are in)
       }
     }
-    (void)ok;
   } else if (warp == 18) {
     // ---------------- store warp: one TMA store per 64-column box of each staged state tile ----------------
     if (p.c_states != nullptr && elect_one()) {
@@ -265,13 +272,13 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       bool ok = true;
       for (int s = 0; s < NS; ++s) {
         const int nb = s & 1;
-        if (!mbar_wait(&bar_nsum[nb], (s >> 1) & 1, &s_abort, &g_sm100_status, 106)) { ok = false; break; }
+        ok = ok && mbar_wait(&bar_nsum[nb], (s >> 1) & 1, &s_abort, &g_sm100_status, 106);
         const float4* np4 = reinterpret_cast<const float4*>(smem + REC_STAGES * REC_STAGE_BYTES) + nb * (32 * 32) + lane;
         float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
         for (int g = 0; g < 32; ++g) { const float4 v = np4[g * 32]; cs.x += v.x; cs.y += v.y; cs.z += v.z; cs.w += v.w; }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_nread[nb]);
+        if (lane == 0 && ok) mbar_arrive(&bar_nread[nb]);
         const float g = s_g[s & 7];
         nv.x = fmaf(g, nv.x, cs.x); nv.y = fmaf(g, nv.y, cs.y); nv.z = fmaf(g, nv.z, cs.z); nv.w = fmaf(g, nv.w, cs.w);
         if (p.n_states != nullptr && d_in)
@@ -300,11 +307,13 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
     // The bf16 state tile goes to shared memory in the 128-byte-swizzled box layout and leaves with one TMA store
     // per 64-column box (coalesced, asynchronous); two staging buffers, one store group in flight.
     uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (HAS_N ? REC_NPART_BYTES : 0);
+    // (the answer of a wait counts for the arrival after it only: a flag held over the loop costs the 128-column forms
+    // register spills, and the waits after one that ran out end by the abort flag)
     int n_out = 0;   // tiles written so far
-    auto store_c = [&]() -> bool {
-      if (p.c_states == nullptr) return true;
+    auto store_c = [&]() {
+      if (p.c_states == nullptr) return;
       const int ob = n_out & 1;
-      if (n_out >= 2 && !mbar_wait(&bar_out_free[ob], ((n_out >> 1) - 1) & 1, &s_abort, &g_sm100_status, 107)) return false;
+      const bool ok = n_out < 2 || mbar_wait(&bar_out_free[ob], ((n_out >> 1) - 1) & 1, &s_abort, &g_sm100_status, 107);
       // TN = 128: each group fills its own 64-column box; TN = 64: the groups share one box (four 16-byte pieces each)
       uint8_t* rowp = stage_base + ob * REC_OUT + (TN == 128 ? half * 16384 : 0) + row * 128;
       const int piece0 = (TN == 128) ? 0 : half * 4;
@@ -316,14 +325,13 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
         *reinterpret_cast<uint4*>(rowp + (((piece0 + c) ^ (row & 7)) << 4)) = v;
       }
       fence_proxy_async_smem();
-      warp_arrive(&bar_out_full[ob]);   // the store warp ships the tile
+      warp_arrive(&bar_out_full[ob], ok);   // the store warp ships the tile
       ++n_out;
-      return true;
     };
-    bool ok = store_c();   // the state before the first step (slot 0 forward, slot NC backward)
-    for (int s = 0; s < NS && ok; ++s) {
+    store_c();   // the state before the first step (slot 0 forward, slot NC backward)
+    for (int s = 0; s < NS; ++s) {
       const int buf = s & 1;
-      if (!mbar_wait(&bar_acc_full[buf], (s >> 1) & 1, &s_abort, &g_sm100_status, 104)) { ok = false; break; }
+      const bool ok = mbar_wait(&bar_acc_full[buf], (s >> 1) & 1, &s_abort, &g_sm100_status, 104);
       tc_fence_after_sync();
       const float g = s_g[s & 7];
       const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 128 + half * HC;
@@ -336,10 +344,10 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
         for (int c = 0; c < 16; ++c) C[q4 * 16 + c] = fmaf(g, C[q4 * 16 + c], __uint_as_float(rr[c]));
       }
       tc_fence_before_sync();
-      warp_arrive(&bar_acc_free[buf]);
-      ok = store_c();
+      warp_arrive(&bar_acc_free[buf], ok);
+      store_c();
     }
-    if (ok && p.c_final) {
+    if (p.c_final) {
       float4* fd = reinterpret_cast<float4*>(p.c_final + ((size_t)bh * p.DHQK + d) * p.DHHV + ecol);
 #pragma unroll
       for (int c = 0; c < HC / 4; ++c)
@@ -659,14 +667,16 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");  // gate vectors and n visible to the element-wise warps
 
-    bool ok = true;
     // q . n_{k-1} for the denominator (H only): each thread reads half of its row of every Q slice from the
     // TMA stage (the stage is released to the producer only after these reads)
     float qn = 0.f;
     if (use_n) {
-      for (int it = 0; it < ND && ok; ++it) {
+      for (int it = 0; it < ND; ++it) {
         const int st = it % PAR_NST;
-        if (!mbar_wait(&sh.bar_full[st], (it / PAR_NST) & 1, &sh.abort, &g_sm100_status, 207)) { ok = false; break; }
+        if (!mbar_wait(&sh.bar_full[st], (it / PAR_NST) & 1, &sh.abort, &g_sm100_status, 207)) {
+          for (; it < ND; ++it) __syncwarp();   // this lane has run out of patience: it meets the others without arriving
+          break;
+        }
         const uint8_t* rowp = smem + st * PAR_STAGE + r * 128;
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
@@ -691,84 +701,82 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
 
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     float rowsum = 0.f;
-    ok = ok && mbar_wait(&sh.bar_sfull, 0, &sh.abort, &g_sm100_status, 205);
-    if (ok) {
-      tc_fence_after_sync();
-      // Tensor memory is read 16 columns at a time, the next load in flight while the current one is processed.
-      // gate the score tile; the bf16 result goes back to tensor memory as the A operand of the second product.
-      // Both warps of a quarter first read their chunks, then (after a warp-pair sync) write: the bf16 words of
-      // chunk cq land on columns [16 cq, 16 cq + 16), which the partner warp may still have to read.
-      uint32_t pk[2][16];
+    mbar_wait(&sh.bar_sfull, 0, &sh.abort, &g_sm100_status, 205);
+    tc_fence_after_sync();
+    // Tensor memory is read 16 columns at a time, the next load in flight while the current one is processed.
+    // gate the score tile; the bf16 result goes back to tensor memory as the A operand of the second product.
+    // Both warps of a quarter first read their chunks, then (after a warp-pair sync) write: the bf16 words of
+    // chunk cq land on columns [16 cq, 16 cq + 16), which the partner warp may still have to read.
+    uint32_t pk[2][16];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int cq = half + 2 * u;
-        const int c0 = cq * 32;
-        const bool skip = LOWER ? (cq > quarter) : (cq < quarter);
-        if (skip) {
+    for (int u = 0; u < 2; ++u) {
+      const int cq = half + 2 * u;
+      const int c0 = cq * 32;
+      const bool skip = LOWER ? (cq > quarter) : (cq < quarter);
+      if (skip) {
 #pragma unroll
-          for (int c = 0; c < 16; ++c) pk[u][c] = 0u;
-        } else {
-          const bool diag = (cq == quarter);   // only the diagonal chunk needs the causal mask
-          uint32_t va[16], vb[16];
-          tmem_ld16(tS + lane_base + c0, va);
-          tmem_wait_ld(va);
-          tmem_ld16(tS + lane_base + c0 + 16, vb);
+        for (int c = 0; c < 16; ++c) pk[u][c] = 0u;
+      } else {
+        const bool diag = (cq == quarter);   // only the diagonal chunk needs the causal mask
+        uint32_t va[16], vb[16];
+        tmem_ld16(tS + lane_base + c0, va);
+        tmem_wait_ld(va);
+        tmem_ld16(tS + lane_base + c0 + 16, vb);
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            if (hh == 1) tmem_wait_ld(vb);
-            const uint32_t (&v)[16] = hh ? vb : va;
-            if (diag) {
-              const float4* ce = reinterpret_cast<const float4*>(sh.s_colE + c0 + 16 * hh);
+        for (int hh = 0; hh < 2; ++hh) {
+          if (hh == 1) tmem_wait_ld(vb);
+          const uint32_t (&v)[16] = hh ? vb : va;
+          if (diag) {
+            const float4* ce = reinterpret_cast<const float4*>(sh.s_colE + c0 + 16 * hh);
 #pragma unroll
-              for (int c4 = 0; c4 < 4; ++c4) {
-                const float4 e4 = ce[c4];
-                const float ee[4] = {e4.x, e4.y, e4.z, e4.w};
-                float g4[4];
+            for (int c4 = 0; c4 < 4; ++c4) {
+              const float4 e4 = ce[c4];
+              const float ee[4] = {e4.x, e4.y, e4.z, e4.w};
+              float g4[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const int cl = 16 * hh + 4 * c4 + e;   // column inside the chunk; row inside the chunk is `lane`
-                  float val = __uint_as_float(v[4 * c4 + e]) * ex2_approx(rowE + ee[e]);
-                  if (LOWER ? (cl > lane) : (cl < lane)) val = 0.f;
-                  g4[e] = val;
-                  rowsum += val;
-                }
-                pk[u][8 * hh + 2 * c4] = Pair16<F16>::pack(g4[0], g4[1]);
-                pk[u][8 * hh + 2 * c4 + 1] = Pair16<F16>::pack(g4[2], g4[3]);
+              for (int e = 0; e < 4; ++e) {
+                const int cl = 16 * hh + 4 * c4 + e;   // column inside the chunk; row inside the chunk is `lane`
+                float val = __uint_as_float(v[4 * c4 + e]) * ex2_approx(rowE + ee[e]);
+                if (LOWER ? (cl > lane) : (cl < lane)) val = 0.f;
+                g4[e] = val;
+                rowsum += val;
               }
-            } else {
-              const float rf = ex2_approx(rowE + sh.s_colP[cq]);
-              const float4* cf = reinterpret_cast<const float4*>(sh.s_colF + c0 + 16 * hh);
+              pk[u][8 * hh + 2 * c4] = Pair16<F16>::pack(g4[0], g4[1]);
+              pk[u][8 * hh + 2 * c4 + 1] = Pair16<F16>::pack(g4[2], g4[3]);
+            }
+          } else {
+            const float rf = ex2_approx(rowE + sh.s_colP[cq]);
+            const float4* cf = reinterpret_cast<const float4*>(sh.s_colF + c0 + 16 * hh);
 #pragma unroll
-              for (int c4 = 0; c4 < 4; ++c4) {
-                const float4 f4 = cf[c4];
-                const float g0 = __uint_as_float(v[4 * c4]) * (rf * f4.x), g1 = __uint_as_float(v[4 * c4 + 1]) * (rf * f4.y);
-                const float g2 = __uint_as_float(v[4 * c4 + 2]) * (rf * f4.z), g3 = __uint_as_float(v[4 * c4 + 3]) * (rf * f4.w);
-                rowsum += (g0 + g1) + (g2 + g3);
-                pk[u][8 * hh + 2 * c4] = Pair16<F16>::pack(g0, g1);
-                pk[u][8 * hh + 2 * c4 + 1] = Pair16<F16>::pack(g2, g3);
-              }
+            for (int c4 = 0; c4 < 4; ++c4) {
+              const float4 f4 = cf[c4];
+              const float g0 = __uint_as_float(v[4 * c4]) * (rf * f4.x), g1 = __uint_as_float(v[4 * c4 + 1]) * (rf * f4.y);
+              const float g2 = __uint_as_float(v[4 * c4 + 2]) * (rf * f4.z), g3 = __uint_as_float(v[4 * c4 + 3]) * (rf * f4.w);
+              rowsum += (g0 + g1) + (g2 + g3);
+              pk[u][8 * hh + 2 * c4] = Pair16<F16>::pack(g0, g1);
+              pk[u][8 * hh + 2 * c4 + 1] = Pair16<F16>::pack(g2, g3);
             }
           }
         }
       }
-      // pair sync (bounded): both warps of the quarter have finished reading the score tile
-      tc_fence_before_sync();
-      mbar_arrive(&sh.bar_pair[quarter]);
-      ok = mbar_wait(&sh.bar_pair[quarter], 0, &sh.abort, &g_sm100_status, 210);
-      if (ok) {
-        tc_fence_after_sync();
-#pragma unroll
-        for (int u = 0; u < 2; ++u) tmem_st16(tS + lane_base + (half + 2 * u) * 16, pk[u]);
-        sh.s_part[half][r] = rowsum;
-        tmem_wait_st();
-      }
     }
+    // pair sync (bounded): both warps of the quarter have finished reading the score tile
+    tc_fence_before_sync();
+    mbar_arrive(&sh.bar_pair[quarter]);
+    mbar_wait(&sh.bar_pair[quarter], 0, &sh.abort, &g_sm100_status, 210);
+    tc_fence_after_sync();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) tmem_st16(tS + lane_base + (half + 2 * u) * 16, pk[u]);
+    sh.s_part[half][r] = rowsum;
+    tmem_wait_st();
+    // From here to the end the warps go in step whatever their waits answer (see warp_arrive).  A hand-over to the other
+    // roles takes place only if the wait before it succeeded; the element-wise warps' own barriers just count.
     // ---- per output tile: row-scale the inter-chunk product, second product, epilogue, store ----
     float inv = 1.f;
-    for (int sub = 0; sub < nsub && ok; ++sub) {
+    for (int sub = 0; sub < nsub; ++sub) {
       const int o0 = o00 + 128 * sub;
       // the inter-chunk product of this tile has usually landed by now: row-scale it in place
-      if (!mbar_wait(&sh.bar_afull, sub & 1, &sh.abort, &g_sm100_status, 214)) { ok = false; break; }
+      const bool acc_ok = mbar_wait(&sh.bar_afull, sub & 1, &sh.abort, &g_sm100_status, 214);
       tc_fence_after_sync();
 #pragma unroll 1
       for (int cq = half; cq < 4; cq += 2) {
@@ -787,8 +795,8 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       }
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&sh.bar_gated);   // (first tile: the gated score tile is in place as well)
-      if (!mbar_wait(&sh.bar_hfull, sub & 1, &sh.abort, &g_sm100_status, 206)) { ok = false; break; }
+      if (acc_ok) mbar_arrive(&sh.bar_gated);   // (first tile: the gated score tile is in place as well)
+      bool ok = mbar_wait(&sh.bar_hfull, sub & 1, &sh.abort, &g_sm100_status, 206);
       tc_fence_after_sync();
       if (sub == 0 && mode == PM_H) {
         float den = 1.f;
@@ -805,7 +813,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       const uint8_t* erow = smem;
       if (HAS_E) {
         const int lde = ldx + 1, ste = lde % PAR_NST;
-        if (!mbar_wait(&sh.bar_full[ste], (lde / PAR_NST) & 1, &sh.abort, &g_sm100_status, 208)) { ok = false; break; }
+        ok = mbar_wait(&sh.bar_full[ste], (lde / PAR_NST) & 1, &sh.abort, &g_sm100_status, 208) && ok;
         erow = smem + ste * PAR_STAGE + r * 128;
       }
       float dot4[4] = {0.f, 0.f, 0.f, 0.f};   // four partial sums: no 64-long chain of dependent FMAs
@@ -851,11 +859,11 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       }
       if (sub + 1 < nsub) {   // the accumulator tile may be overwritten by the next tile's inter-chunk product
         tc_fence_before_sync();
-        mbar_arrive(&sh.bar_accfree);
+        if (ok) mbar_arrive(&sh.bar_accfree);
       }
       const float dot = (dot4[0] + dot4[1]) + (dot4[2] + dot4[3]);
       mbar_arrive(&sh.bar_out);
-      if (!mbar_wait(&sh.bar_out, sub & 1, &sh.abort, &g_sm100_status, 211)) { ok = false; break; }
+      mbar_wait(&sh.bar_out, sub & 1, &sh.abort, &g_sm100_status, 211);
       {
         uint16_t* outp = (mode == PM_H) ? p.out_h : (mode == PM_DV) ? p.out_dv : (mode == PM_DK) ? p.out_dk : p.out_dq;
         uint8_t* gbase = reinterpret_cast<uint8_t*>(outp + out_row0 * DO + o0);
@@ -871,7 +879,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         sh.s_qn[half][r] = dot;
         mbar_arrive(&sh.bar_dot);
         if (half == 0) {
-          if (!mbar_wait(&sh.bar_dot, sub & 1, &sh.abort, &g_sm100_status, 209)) { ok = false; break; }
+          mbar_wait(&sh.bar_dot, sub & 1, &sh.abort, &g_sm100_status, 209);
           ((mode == PM_DQ) ? p.rowdot_q : p.rowdot_k)[(size_t)(o_tile0 + sub) * p.nslots + tok] = sh.s_qn[0][r] + sh.s_qn[1][r];
         }
       }
@@ -880,7 +888,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         // proxy: without this fence its data can be overtaken by this thread's own earlier (generic-proxy) staging
         // writes to the same addresses.
         fence_proxy_async_smem();
-        mbar_arrive(&sh.bar_done);
+        if (ok) mbar_arrive(&sh.bar_done);
       }
     }
   }
