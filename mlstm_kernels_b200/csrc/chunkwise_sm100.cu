@@ -450,8 +450,9 @@ struct ParShared {
 // the limit of the gating phase before: the warps of the busiest row quarter share one SM sub-partition.
 // LOOP: the CTA runs the body again for another chunk afterwards (H only): it keeps its tensor memory from the first run
 // to the last, and leaves each run with no arrival on any barrier outstanding, so that the next one can set them up anew.
+// Returns false after a run in which a wait ran out: its copies may still be on their way to barriers of that run.
 template <bool F16, bool LOOP = false>
-__device__ __forceinline__ void
+__device__ __forceinline__ bool
 par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* mapX,
          const CUtensorMap* mapSt, const CUtensorMap* mapE, const ParParams& p,
          ParShared& sh, const int o_tile0, const int nsub, const int ck, const int bh, const bool first_run = true,
@@ -895,7 +896,9 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
   if (LOOP) fence_proxy_async_smem();   // staging writes above, the next run's copies after the barrier
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1 && (!LOOP || last_run)) tmem_dealloc(tmem, 256);
+  const bool go_on = !LOOP || sh.abort == 0;   // (the next run sets it to the 0 that it is)
+  if (warp == 1 && (!LOOP || last_run || !go_on)) tmem_dealloc(tmem, 256);
+  return go_on;
 }
 
 template <bool F16>
@@ -925,7 +928,7 @@ par_fw_range_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant
   for (unsigned w = blockIdx.x; w < n_items; w += gridDim.x) {
     const int x = w % gx, ck = p.ck0 + (w / gx) % p.n_ck, bh = p.bh0 + w / (gx * p.n_ck), t0 = p.maxsub * x;
     const bool last = w + gridDim.x >= n_items;
-    par_body<F16, true>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(p.maxsub, T - t0), ck, bh, w == blockIdx.x, last);
+    if (!par_body<F16, true>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(p.maxsub, T - t0), ck, bh, w == blockIdx.x, last)) return;
   }
 }
 

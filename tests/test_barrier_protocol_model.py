@@ -10,12 +10,16 @@ random interleavings - asynchronous copies land in any order, MMA commits fire i
 the true phase count, every barrier against over-arrival, and the whole run against deadlock.
 
 It is a model, kept next to the kernel by hand: change the order of barrier operations in par_body and this file has
-to follow.  Its second test documents why a CTA does not walk several chunks with the ring running on: the MMA thread
-would then poll a stage's `full` barrier while the previous chunk's E tile is still in flight on it."""
+to follow.  One test documents why a CTA does not walk several chunks with the ring running on: the MMA thread
+would then poll a stage's `full` barrier while the previous chunk's E tile is still in flight on it.  Where a CTA does
+take several (par_fw_range_sm100), each run sets its barriers up anew, and has to leave none of its copies and commits
+behind: they would land on the next run's barriers."""
 
+import os
 import random
 
 import pytest
+
 
 class Bar:
     def __init__(self, name, count):
@@ -35,18 +39,23 @@ class Bar:
             if self.phase >= want_phase + 2: raise AssertionError(f"ALIAS hang on {self.name}: want {want_phase} at {self.phase}")
         return passes
 
-def run(mode, ND, nsub, njobs, seed, NST=3):
+def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
+    """loop: the form of a CTA that takes several chunks in runs of their own - one that starts with the producer's waits
+    for the last hand-backs and ends with nothing in flight.  lost_load: this load (its number) does not land within the
+    limit of the waits.  Returns whether the waits ran out, and the copies and commits that are still in flight."""
     rnd = random.Random(seed)
     HAS_E = mode in ("DQ", "DK")
+    USE_N = mode == "Hn"             # the element-wise warps read the A box of each score pair (q . n)
     n0 = 2 * ND + 1 + (1 if HAS_E else 0); n1 = ND + 1 + (1 if HAS_E else 0)
     n_loads = n0 + (nsub - 1) * n1
     B = {}
     for s in range(NST):
-        B[f"full{s}"] = Bar(f"full{s}", 1); B[f"empty{s}"] = Bar(f"empty{s}", 1)
+        B[f"full{s}"] = Bar(f"full{s}", 1); B[f"empty{s}"] = Bar(f"empty{s}", 1); B[f"qdone{s}"] = Bar(f"qdone{s}", 8)
     for n, c in (("sfull",1),("afull",1),("hfull",1),("gated",8),("accfree",8),("done",8),("dot",8),("out",8)):
         B[n] = Bar(n, c)
     for qd in range(4): B[f"pair{qd}"] = Bar(f"pair{qd}", 2)
     pending_async = []   # async completions: ('load', st) any order ; commits in order
+    late = []            # loads that land after the waits have run out
     commit_queue = []    # list of barrier names, fire in order
     def kind_of(sub, l):
         if sub == 0 and l < ND: return "SCORE"
@@ -55,7 +64,7 @@ def run(mode, ND, nsub, njobs, seed, NST=3):
         return "X" if ls == ND else "E"
     # generators for each role; yield ('wait', barname, phase) blocks until passes; other ops executed inline
     def producer():
-        issued = 0; rm = [0]*NST; st = 0; hist = []
+        issued = 0; rm = [0]*NST; rq = [0]*NST; st = 0; hist = []
         for job in range(njobs):
             sub = 0; l = 0
             for ld in range(n_loads):
@@ -64,16 +73,21 @@ def run(mode, ND, nsub, njobs, seed, NST=3):
                     pk, ps = hist[-3]
                     if pk in ("SCORE", "STATE") or (pk == "X" and HAS_E):
                         yield ("wait", f"empty{st}", rm[st] - 1)
+                        if USE_N and pk == "SCORE": yield ("wait", f"qdone{st}", rq[st] - 1)
                     else:
                         yield ("wait", "done", ps)
-                pending_async.append(("load", st))
+                (late if issued == lost_load else pending_async).append(("load", st))
                 if kind in ("SCORE", "STATE") or (kind == "X" and HAS_E): rm[st] += 1
+                if kind == "SCORE": rq[st] += 1
                 issued += 1
                 hist.append((kind, job * nsub + sub))
                 st = (st + 1) % NST
                 l += 1
                 if l == (n0 if sub == 0 else n1): l = 0; sub += 1
                 yield ("step",)
+        if loop:
+            for st in range(NST):
+                if rm[st] > 0: yield ("wait", f"empty{st}", rm[st] - 1)
     def mma():
         for job in range(njobs):
             lb = job * n_loads; gt0 = job * nsub
@@ -100,6 +114,10 @@ def run(mode, ND, nsub, njobs, seed, NST=3):
         for job in range(njobs):
             lb = job * n_loads; gt0 = job * nsub
             yield ("barsync",)
+            if USE_N:
+                for it in range(ND):
+                    yield ("wait", f"full{(lb + it) % NST}", (lb + it) // NST)
+                    B[f"qdone{(lb + it) % NST}"].arrive()
             yield ("wait", "sfull", job)
             B[f"pair{quarter}"].arrive()
             yield ("wait", f"pair{quarter}", job)
@@ -127,9 +145,7 @@ def run(mode, ND, nsub, njobs, seed, NST=3):
     blocked = {}
     barsync_wait = set()
     alive = set(agents)
-    steps = 0
     while alive:
-        steps += 1
         choices = []
         for a in alive:
             if a in barsync_wait: continue
@@ -170,17 +186,19 @@ def run(mode, ND, nsub, njobs, seed, NST=3):
                 if len(barsync_wait) == 8: barsync_wait.clear()
                 progressed = True; break
             progressed = True; break
+        if not progressed and lost_load is not None:
+            return True, late + pending_async + commit_queue
         if not progressed:
             raise AssertionError(f"DEADLOCK: blocked={blocked} barsync={barsync_wait} phases={{k:v.phase for k,v in B.items()}}".replace("{{","{").replace("}}","}") + str({k:v.phase for k,v in B.items()}))
-    return steps
+    return False, late + pending_async + commit_queue
 
 
 
-MODES = ("H", "DV", "DK", "DQ")   # H and DV: no E tile (the output is staged in the X tile's stage)
+MODES = ("H", "Hn", "DV", "DK", "DQ")   # H and DV: no E tile (the output is staged in the X tile's stage)
 
 
 @pytest.mark.parametrize("mode", MODES)
-@pytest.mark.parametrize("ND", [2, 4, 8])
+@pytest.mark.parametrize("ND", [1, 2, 3, 4, 8])
 @pytest.mark.parametrize("nsub", [1, 2, 3, 4, 8])
 def test_one_chunk_per_cta_protocol_has_no_aliasing_deadlock_or_over_arrival(mode, ND, nsub):
     for seed in range(40):
@@ -197,3 +215,31 @@ def test_ring_running_on_across_chunks_would_alias():
             assert "ALIAS" in str(e)
             return
     raise AssertionError("no interleaving out of 4000 showed the hazard")
+
+
+def run_range(mode, ND, nsub, runs, seed, lost_run=None, stop=True):
+    """A CTA of par_fw_range_sm100: `runs` chunks one after the other on barriers set up anew."""
+    for r in range(runs):
+        expired, in_flight = run(mode, ND, nsub, 1, seed + r, loop=True, lost_load=2 if r == lost_run else None)
+        if expired and stop:
+            return
+        if r + 1 < runs:
+            assert not in_flight, f"{in_flight} of run {r} would land on barriers of run {r + 1}"
+
+
+@pytest.mark.parametrize("ND", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("nsub", [1, 2, 3, 4])
+@pytest.mark.parametrize("mode", ["H", "Hn"])
+def test_runs_of_a_segment_leave_nothing_in_flight(mode, ND, nsub):
+    for seed in range(20):
+        run_range(mode, ND, nsub, 3, 1000 * seed)
+
+
+def test_segment_cta_stops_after_a_run_whose_waits_ran_out():
+    for seed in range(20):
+        run_range("Hn", 4, 2, 3, 1000 * seed, lost_run=1)
+    with pytest.raises(AssertionError, match="would land on barriers"):
+        run_range("Hn", 4, 2, 3, 0, lost_run=1, stop=False)
+    with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlstm_kernels_b200", "csrc",
+                           "chunkwise_sm100.cu")) as f:
+        assert "if (!par_body<F16, true>(" in f.read()
