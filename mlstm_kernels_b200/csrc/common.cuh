@@ -60,10 +60,29 @@ void note_launch();
 // Programmatic dependent launch: a kernel launched with launch_pdl may be scheduled once every CTA of the kernel before it
 // in the stream has called pdl_launch_dependents() (or has ended), so that its launch latency and set-up overlap that
 // kernel's tail; pdl_wait() then blocks until that kernel has completed and its writes are visible.  Every thread block
-// calls pdl_wait() before it touches global memory.  Saves 1-2 us per launch boundary, which is what small calls are
+// calls pdl_wait() before it touches global memory.  What such a kernel reads may be written while it is already resident,
+// so it takes its inputs as plain pointers (const __restrict__ lets the compiler read through the non-coherent path, which is
+// for memory that nothing writes during the whole kernel) and streams through ld_stream, which stays behind pdl_wait().  Saves 1-2 us per launch boundary, which is what small calls are
 // made of (a decode step of one sequence, back to back: 6.1 -> 3.7 us; the forward of 500 tokens 31.0 -> 28.5 us); overlap = false is a plain launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// evict-first loads of data that is read once
+__device__ __forceinline__ uint4 ld_stream(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 ld_stream(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.cs.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
 
 // Larger launches start plainly: their own CTAs hide the gap, and CTAs of the next kernel that are resident early would take
 // room on an SM from those of a second chain of launches.

@@ -35,8 +35,7 @@ struct GateScan {
 // NV: register-held token values per lane, NV * 32 >= L
 template <typename T, int NV>
 __global__ void __launch_bounds__(1024)
-gates_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, const float* __restrict__ n_out,
-             float* __restrict__ m_out, GateBuffers gb, GateScan sc, int S, int SP, int L, int NC, int variant, float eps) {
+gates_kernel(const T* vecI, const T* vecF, const float* n_out, float* __restrict__ m_out, GateBuffers gb, GateScan sc, int S, int SP, int L, int NC, int variant, float eps) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float s_wG[32], s_wA[32];    // totals of the warps
@@ -288,10 +287,9 @@ gate_grad_scan_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, co
 constexpr int kAnchorThreads = 512;
 template <typename T>
 __global__ void __launch_bounds__(kAnchorThreads)
-gate_grad_anchored_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, const float* __restrict__ qdq,
-                          const float* __restrict__ kdk, void* __restrict__ dI, void* __restrict__ dF,
-                          int out_dtype, int S, int SP, int variant, int nparts, size_t part_stride,
-                          const float* __restrict__ anchors, int n_anchors) {
+gate_grad_anchored_kernel(const T* vecI, const T* vecF, const float* qdq, const float* kdk, void* __restrict__ dI,
+                          void* __restrict__ dF, int out_dtype, int S, int SP, int variant, int nparts, size_t part_stride,
+                          const float* anchors, int n_anchors) {
   __shared__ float s_warp[kAnchorThreads / 32];
   const int nint = (S + kAnchorThreads - 1) / kAnchorThreads;   // 1-D grid: intervals of one (batch, head) adjacent
   const int a = blockIdx.x % nint, bh = blockIdx.x / nint, t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -331,8 +329,8 @@ gate_grad_anchored_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF
 // (a = 0 is never read).  One CTA per (anchor, batch x head); the partial sums are added in a fixed order.
 template <typename TS>
 __global__ void __launch_bounds__(256)
-state_dot_kernel(const TS* __restrict__ c_states, const TS* __restrict__ dc_states,
-                 float* __restrict__ anchors, int NC, int every, int n_anchors, size_t state_elems) {
+state_dot_kernel(const TS* c_states, const TS* dc_states, float* __restrict__ anchors, int NC, int every, int n_anchors,
+                 size_t state_elems) {
   __shared__ float s_w[8];
   const int bh = blockIdx.x / (n_anchors - 1), a = blockIdx.x % (n_anchors - 1) + 1;   // 1-D grid
   const int k = min(a * every, NC);
@@ -343,7 +341,7 @@ state_dot_kernel(const TS* __restrict__ c_states, const TS* __restrict__ dc_stat
   const uint4* pd = reinterpret_cast<const uint4*>(dc_states + off);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (size_t idx = threadIdx.x; idx < state_elems / 8; idx += 256) {
-    const uint4 x = __ldcs(pc + idx), y = __ldcs(pd + idx);
+    const uint4 x = ld_stream(pc + idx), y = ld_stream(pd + idx);
     const uint32_t xw[4] = {x.x, x.y, x.z, x.w}, yw[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {

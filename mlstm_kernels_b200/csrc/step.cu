@@ -16,12 +16,12 @@ constexpr int STEP_THREADS = 256;
 
 template <typename TS> struct Vec4;
 template <> struct Vec4<float> {
-  static __device__ __forceinline__ float4 load(const float* p) { return __ldcs(reinterpret_cast<const float4*>(p)); }
+  static __device__ __forceinline__ float4 load(const float* p) { return ld_stream(reinterpret_cast<const float4*>(p)); }
   static __device__ __forceinline__ void store(float* p, float4 v) { __stcs(reinterpret_cast<float4*>(p), v); }
 };
 template <> struct Vec4<__nv_bfloat16> {
   static __device__ __forceinline__ float4 load(const __nv_bfloat16* p) {
-    uint2 raw = __ldcs(reinterpret_cast<const uint2*>(p));
+    uint2 raw = ld_stream(reinterpret_cast<const uint2*>(p));
     __nv_bfloat162 a = *reinterpret_cast<__nv_bfloat162*>(&raw.x), b = *reinterpret_cast<__nv_bfloat162*>(&raw.y);
     return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
   }
@@ -50,10 +50,9 @@ __device__ __forceinline__ float load_gate(const void* p, size_t idx, int gate_d
 // register bound: 1.5 %).
 template <typename T, typename TS, int TV, bool PDL>
 __global__ void __launch_bounds__(STEP_THREADS)
-step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const void* __restrict__ gi,
-            const void* __restrict__ gf, int gate_dtype, const TS* __restrict__ c, const TS* __restrict__ n,
-            const TS* __restrict__ m, T* __restrict__ h, TS* __restrict__ c_new, TS* __restrict__ n_new,
-            TS* __restrict__ m_new, int DHQK, int DHHV, float eps) {
+step_kernel(const T* q, const T* k, const T* v, const void* gi, const void* gf, int gate_dtype, const TS* c, const TS* n,
+            const TS* m, T* __restrict__ h, TS* c_new, TS* __restrict__ n_new, TS* __restrict__ m_new, int DHQK, int DHHV,
+            float eps) {
   constexpr int CG = TV / 4, RG = STEP_THREADS / CG, NW = STEP_THREADS / 32, UNR = 8;
   constexpr bool EARLY = TV == 32;
   extern __shared__ float sm[];
