@@ -15,6 +15,8 @@ device).  The *_raw functions below go through the C ABI; the multi-GPU helpers 
 
 from __future__ import annotations
 
+import math
+
 import torch
 
 from . import _lib, _ops
@@ -75,6 +77,22 @@ def _f32c(t):
     return None if t is None else t.to(torch.float32).contiguous()
 
 
+def _state_f32(t, name: str, sizes: tuple[int, ...]):
+    """An initial state as the kernels read it: f32, contiguous, on the GPU, at least as many elements as `sizes`."""
+    _lib.require_cuda(t)
+    if t is not None and t.numel() < math.prod(sizes):
+        raise ValueError(f"{name} of shape {list(t.shape)} is too small for {sizes}")
+    return _f32c(t)
+
+
+def _max_state_f32(m, B: int, NH: int):
+    """m_initial: one number per (batch, head), however it is shaped."""
+    _lib.require_cuda(m)
+    if m is not None and m.numel() != B * NH:
+        raise RuntimeError(f"m_initial: shape '[{B}, {NH}]' is invalid for input of size {m.numel()}")
+    return None if m is None else _f32c(m).reshape(B, NH)
+
+
 def chunkwise_fw_raw(q, k, v, i, f, c_initial=None, n_initial=None, m_initial=None, *, chunk_size: int,
                      eps: float, variant: int, impl: str = "auto", want_last: bool = True):
     """Run the forward kernels.  Returns a dict with H, n_out, m_out, the per-chunk states and
@@ -93,8 +111,9 @@ def chunkwise_fw_raw(q, k, v, i, f, c_initial=None, n_initial=None, m_initial=No
     NC = -(-S // L)   # the last chunk may be ragged on the tcgen05 path (the library refuses it elsewhere)
     dt, gdt, im = _lib.dtype_code(q.dtype), _lib.dtype_code(i.dtype), _lib.IMPL[impl]
     q, k, v, i, f = (t.contiguous() for t in (q, k, v, i, f))
-    c0, n0 = _f32c(c_initial), _f32c(n_initial)
-    m0 = None if m_initial is None else _f32c(m_initial).reshape(B, NH)
+    c0 = _state_f32(c_initial, "c_initial", (B, NH, DHQK, DHHV))
+    n0 = _state_f32(n_initial, "n_initial", (B, NH, DHQK))
+    m0 = _max_state_f32(m_initial, B, NH)
     dev = q.device
     sdt = _lib.code_dtype(lib.mlstm_b200_chunkwise_state_dtype(S, DHQK, DHHV, L, dt, im))
     h = torch.empty((B, NH, S, DHHV), dtype=q.dtype, device=dev)
@@ -140,8 +159,8 @@ def chunkwise_states_raw(k, v, i, f, c_initial=None, m_initial=None, *, chunk_si
     if i.dtype != f.dtype:
         f = f.to(i.dtype)
     k, v, i, f = (t.contiguous() for t in (k, v, i, f))
-    c0 = _f32c(c_initial)
-    m0 = None if m_initial is None else _f32c(m_initial).reshape(B, NH)
+    c0 = _state_f32(c_initial, "c_initial", (B, NH, DHQK, DHHV))
+    m0 = _max_state_f32(m_initial, B, NH)
     dev = k.device
     sdt = _lib.code_dtype(lib.mlstm_b200_chunkwise_state_dtype(S, DHQK, DHHV, L, dt, im))
     c_states = torch.empty((B, NH, -(-S // L) + 1, DHQK, DHHV), dtype=sdt, device=dev)
@@ -175,7 +194,7 @@ def chunkwise_bw_raw(q, k, v, i, f, m_initial, c_states, n_out, dh, dc_last=None
     q, k, v, i, f = (t.contiguous() for t in (q, k, v, i, f))
     dh = dh.to(q.dtype).contiguous()
     dcl = _f32c(dc_last)
-    m0 = None if m_initial is None else _f32c(m_initial).reshape(B, NH)
+    m0 = _max_state_f32(m_initial, B, NH)
     dev = q.device
     dq = torch.empty_like(q)
     dk = torch.empty_like(k)
@@ -191,7 +210,7 @@ def chunkwise_bw_raw(q, k, v, i, f, m_initial, c_states, n_out, dh, dc_last=None
                 raise ValueError("recomputing the states inside the backward needs the forward's workspace")
             sdt = _lib.code_dtype(lib.mlstm_b200_chunkwise_state_dtype(S, DHQK, DHHV, L, dt, im))
             c_states = torch.empty((B, NH, -(-S // L) + 1, DHQK, DHHV), dtype=sdt, device=dev)
-            c0 = _f32c(recompute_c_initial)
+            c0 = _state_f32(recompute_c_initial, "c_initial", (B, NH, DHQK, DHHV))
             rc = lib.mlstm_b200_chunkwise_bw_recompute(
                 _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(i), _lib.ptr(f),
                 _lib.ptr(m0), _lib.ptr(c0), _lib.ptr(c_states), _lib.ptr(n_out), _lib.ptr(m_out),

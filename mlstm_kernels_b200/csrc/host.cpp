@@ -103,14 +103,28 @@ struct Forward {
   Tensor h, c_last, n_last, m_last, kept, states;
 };
 
+// The tensors of a chunkwise call, before anything is launched or allocated for it.  Of the states c and n the kernels read
+// as many elements as the sizes say, in memory order; m is one number per (batch, head), however it is shaped.
+void check_chunkwise(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& i, const Tensor& f, const Tensor& c0,
+                     const Tensor& n0, const Tensor& m0) {
+  const auto B = q.size(0), NH = q.size(1), S = q.size(2), DHQK = q.size(3), DHHV = v.size(3);
+  const std::array<int64_t, 3> tok_size{B, NH, S};
+  const at::IntArrayRef tok(tok_size);
+  if (k.sizes() != q.sizes() || v.sizes().slice(0, 3) != tok || i.sizes() != tok || f.sizes() != tok)
+    C10_THROW_ERROR(ValueError, "q, k, v, i, f have inconsistent shapes");
+  for (const Tensor* t : {&c0, &n0, &m0})
+    TORCH_CHECK(!t->defined() || t->is_cuda(), kNeedsCuda);
+  if (c0.defined() && c0.numel() < B * NH * DHQK * DHHV)
+    C10_THROW_ERROR(ValueError, c10::str("c_initial of shape ", c0.sizes(), " is too small for (B, NH, DHQK, DHHV)"));
+  if (n0.defined() && n0.numel() < B * NH * DHQK)
+    C10_THROW_ERROR(ValueError, c10::str("n_initial of shape ", n0.sizes(), " is too small for (B, NH, DHQK)"));
+  TORCH_CHECK(!m0.defined() || m0.numel() == B * NH, "m_initial: shape '[", B, ", ", NH, "]' is invalid for input of size ", m0.defined() ? m0.numel() : 0);
+}
+
 Forward run_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& i_, const Tensor& f_,
                     const Tensor& c0_, const Tensor& n0_, const Tensor& m0_, bool want_last, bool for_backward,
                     bool keep_states, int L, double eps, int variant, int impl) {
   const auto B = q_.size(0), NH = q_.size(1), S = q_.size(2), DHQK = q_.size(3), DHHV = v_.size(3);
-  const std::array<int64_t, 3> tok_size{B, NH, S};
-  const at::IntArrayRef tok(tok_size);
-  if (k_.sizes() != q_.sizes() || v_.sizes().slice(0, 3) != tok || i_.sizes() != tok || f_.sizes() != tok)
-    C10_THROW_ERROR(ValueError, "q, k, v, i, f have inconsistent shapes");
   if (k_.scalar_type() != q_.scalar_type() || v_.scalar_type() != q_.scalar_type())
     C10_THROW_ERROR(ValueError, "q, k, v must share one dtype");
   const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous(), i = i_.contiguous();
@@ -274,6 +288,7 @@ PyObject* py_chunkwise(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (const Tensor* t : {&q, &k, &v, &i, &f})
     TORCH_CHECK(t->is_cuda(), kNeedsCuda);
   if (q.dim() != 4 || v.dim() != 4) C10_THROW_ERROR(ValueError, "q, k, v, i, f have inconsistent shapes");
+  check_chunkwise(q, k, v, i, f, c0, n0, m0);
   std::optional<at::ScalarType> cast;
   if (at::autocast::is_autocast_enabled(at::kCUDA)) cast = kdt;
   const at::ScalarType qdt = cast && q.scalar_type() != at::kDouble ? *cast : q.scalar_type();
