@@ -341,12 +341,14 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     Tensor cn = arg(a[8], "matC_new"), nn = arg(a[9], "vecN_new"), mn = arg(a[10], "scaM_new"), h = arg(a[13], "vecH_out");
     const double eps = double_arg(a[11]);
     const at::ScalarType sdt = dtype_arg(a[12]);
-    TORCH_CHECK(q.is_cuda() && c.is_cuda(), kNeedsCuda);
+    for (const Tensor* t : {&q, &k, &v, &gi, &gf, &c, &n, &m, &cn, &nn, &mn, &h})
+      TORCH_CHECK(!t->defined() || t->is_cuda(), kNeedsCuda);
     if (q.dim() != 3) throw AssertionFailed{"q must have shape (B, NH, DHQK)"};
     const auto B = q.size(0), NH = q.size(1), DHQK = q.size(2), DHHV = v.size(-1);
     const std::array<int64_t, 3> one_size{B, NH, 1};
     const at::IntArrayRef one(one_size);
     if (k.sizes() != q.sizes()) throw AssertionFailed{"q and k must have the same shape"};
+    if (v.numel() < B * NH * DHHV) throw AssertionFailed{"vecV has wrong shape, got " + shape_text(v)};
     if (c.sizes() != at::IntArrayRef{B, NH, DHQK, DHHV}) throw AssertionFailed{"matC_old has wrong shape, got " + shape_text(c)};
     if (n.sizes() != q.sizes()) throw AssertionFailed{"vecN_old has wrong shape, got " + shape_text(n)};
     if (m.sizes() != one) throw AssertionFailed{"scaM_old has wrong shape, got " + shape_text(m)};
@@ -370,6 +372,8 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       for (const Tensor* t : {&cn, &nn, &mn})
         if (t->scalar_type() != sdt || !t->is_contiguous())
           C10_THROW_ERROR(ValueError, "output state tensors must be contiguous and of dtype_state");
+      if (cn.numel() < c.numel() || nn.numel() < n.numel() || mn.numel() < m.numel())
+        C10_THROW_ERROR(ValueError, "output state tensors are too small for the states");
     }
     if (!h.defined()) {
       h = empty(v.sizes(), qdt, dev);
@@ -401,9 +405,15 @@ PyObject* py_sequence(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   Tensor c0 = arg(a[5], "c_initial"), n0 = arg(a[6], "n_initial"), m0 = arg(a[7], "m_initial");
   const double eps = double_arg(a[8]);
   const at::ScalarType sdt = dtype_arg(a[9]);
-  for (const Tensor* t : {&q, &k, &v, &gi, &gf}) TORCH_CHECK(t->is_cuda(), kNeedsCuda);
+  for (const Tensor* t : {&q, &k, &v, &gi, &gf, &c0, &n0, &m0}) TORCH_CHECK(!t->defined() || t->is_cuda(), kNeedsCuda);
   if (q.dim() != 4) C10_THROW_ERROR(ValueError, "q must have shape (B, NH, S, DHQK)");
   const auto B = q.size(0), NH = q.size(1), S = q.size(2), DHQK = q.size(3), DHHV = v.size(-1);
+  // the kernel reads operands of these sizes in memory order, however they are shaped
+  auto fits = [](const Tensor& t, int64_t n) { return !t.defined() || t.numel() >= n; };
+  if (!fits(k, q.numel()) || !fits(v, B * NH * S * DHHV) || !fits(gi, B * NH * S) || !fits(gf, B * NH * S))
+    C10_THROW_ERROR(ValueError, "q, k, v, i, f have inconsistent shapes");
+  if (!fits(c0, B * NH * DHQK * DHHV) || !fits(n0, B * NH * DHQK) || !fits(m0, B * NH))
+    C10_THROW_ERROR(ValueError, "c_initial, n_initial or m_initial is too small for the sizes of q and v");
   const int dt = dtype_code(q.scalar_type());
   if (dt < 0) C10_THROW_ERROR(ValueError, c10::str("Unsupported kernel dtype ", q.scalar_type(), "."));
   at::NoGradGuard no_grad;

@@ -54,3 +54,50 @@ def test_states_in_host_memory_are_refused(path, name):
                 mk.mlstm_chunkwise__b200_xl_chunk(**a)
             else:
                 chunkwise_fw_raw(**a, chunk_size=128, eps=1e-6, variant=_lib.EXP)
+
+
+def step_operands():
+    e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device="cuda")  # noqa: E731
+    f32 = torch.float32
+    return dict(matC_old=e(B, NH, DHQK, DHHV, dt=f32), vecN_old=e(B, NH, DHQK, dt=f32), scaM_old=e(B, NH, 1, dt=f32),
+                vecQ=e(B, NH, DHQK), vecK=e(B, NH, DHQK), vecV=e(B, NH, DHHV), scaI=e(B, NH, 1), scaF=e(B, NH, 1),
+                matC_new=e(B, NH, DHQK, DHHV, dt=f32), vecN_new=e(B, NH, DHQK, dt=f32), scaM_new=e(B, NH, 1, dt=f32))
+
+
+@pytest.mark.parametrize("name,shape,error", [
+    ("vecK", (B, NH, DHQK - 1), AssertionError), ("vecV", (1, NH, DHHV), AssertionError),
+    ("matC_old", (B, NH, DHQK, DHHV - 1), AssertionError), ("vecN_old", (NH, DHQK), AssertionError),
+    ("scaM_old", (B, NH), AssertionError), ("scaI", (B, NH), AssertionError), ("scaF", (B, 1, 1), AssertionError),
+    ("matC_new", (B, NH, DHQK, DHHV - 1), ValueError), ("vecN_new", (NH, DHQK), ValueError), ("scaM_new", (B, 1, 1), ValueError)])
+def test_decode_step_refuses_wrong_sizes(name, shape, error):
+    from mlstm_kernels_b200.recurrent import mlstm_recurrent_step__b200_fw
+    with FakeTensorMode():
+        a = step_operands()
+        a[name] = torch.empty(*shape, dtype=a[name].dtype, device="cuda")
+        with pytest.raises(Exception) as e:
+            mlstm_recurrent_step__b200_fw(**a)
+    assert e.type is error, e.value
+
+
+@pytest.mark.parametrize("name", ["vecK", "vecV", "scaI", "scaF", "vecN_old", "scaM_old", "matC_new", "vecN_new", "scaM_new"])
+def test_decode_step_refuses_host_memory(name):
+    from mlstm_kernels_b200.recurrent import mlstm_recurrent_step__b200_fw
+    with FakeTensorMode():
+        a = step_operands()
+        a[name] = torch.empty(a[name].shape, dtype=a[name].dtype)
+        with pytest.raises(RuntimeError, match="CUDA tensors only"):
+            mlstm_recurrent_step__b200_fw(**a)
+
+
+@pytest.mark.parametrize("name,shape", [("k", (B, 1, S, DHQK)), ("v", (B, NH, S - 1, DHHV)), ("i", (B, NH, S - 1)), ("f", (B, 1, S)),
+                                        ("c_initial", (B, NH, DHQK, DHHV - 1)), ("n_initial", (NH, DHQK)), ("m_initial", (B, 1, 1))])
+def test_sequence_refuses_wrong_sizes_and_host_memory(name, shape):
+    with FakeTensorMode():
+        a = operands()
+        a[name] = torch.empty(*shape, dtype=a[name].dtype, device="cuda")
+        with pytest.raises(ValueError, match="inconsistent shapes|too small"):
+            mk.mlstm_recurrent_sequence__b200(**a)
+        a = operands()
+        a[name] = torch.empty(a[name].shape, dtype=a[name].dtype)
+        with pytest.raises(RuntimeError, match="CUDA tensors only"):
+            mk.mlstm_recurrent_sequence__b200(**a)
