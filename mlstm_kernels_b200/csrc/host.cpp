@@ -289,6 +289,10 @@ PyObject* py_chunkwise(PyObject*, PyObject* const* a, Py_ssize_t n) {
     TORCH_CHECK(t->is_cuda(), kNeedsCuda);
   if (q.dim() != 4 || v.dim() != 4) C10_THROW_ERROR(ValueError, "q, k, v, i, f have inconsistent shapes");
   check_chunkwise(q, k, v, i, f, c0, n0, m0);
+  // a forward-mode tangent would be dropped without a word
+  for (const Tensor* t : {&q, &k, &v, &i, &f, &c0, &n0, &m0})
+    if (t->defined() && t->_fw_grad(0).defined())
+      C10_THROW_ERROR(NotImplementedError, "mlstm_kernels_b200 has no forward-mode derivative of the chunkwise functions");
   std::optional<at::ScalarType> cast;
   if (at::autocast::is_autocast_enabled(at::kCUDA)) cast = kdt;
   const at::ScalarType qdt = cast && q.scalar_type() != at::kDouble ? *cast : q.scalar_type();

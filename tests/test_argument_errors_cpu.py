@@ -3,6 +3,7 @@ and multi-GPU calls), before anything is launched: checked without a GPU, on fak
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fwAD
 from torch._subclasses.fake_tensor import FakeTensorMode
 
 import mlstm_kernels_b200 as mk
@@ -54,6 +55,15 @@ def test_states_in_host_memory_are_refused(path, name):
                 mk.mlstm_chunkwise__b200_xl_chunk(**a)
             else:
                 chunkwise_fw_raw(**a, chunk_size=128, eps=1e-6, variant=_lib.EXP)
+
+
+@pytest.mark.parametrize("name", ["q", "f", "c_initial"])
+def test_forward_mode_tangents_are_refused(name):
+    with FakeTensorMode(), fwAD.dual_level():
+        a = operands()
+        a[name] = fwAD.make_dual(a[name], torch.empty_like(a[name]))
+        with pytest.raises(NotImplementedError):
+            mk.mlstm_chunkwise__b200_xl_chunk(**a)
 
 
 def step_operands():
