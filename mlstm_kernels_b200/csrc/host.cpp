@@ -279,6 +279,7 @@ PyObject* py_chunkwise(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const bool want_last = bool_arg(a[8]), recompute = bool_arg(a[12]);
   const double eps = double_arg(a[9]);
   const char* impl_name = PyUnicode_Check(a[11]) ? PyUnicode_AsUTF8(a[11]) : "?";
+  if (impl_name == nullptr) { PyErr_Clear(); impl_name = "?"; }   // text that has no UTF-8 form
   const int impl = !strcmp(impl_name, "auto") ? MLSTM_IMPL_AUTO : !strcmp(impl_name, "simt") ? MLSTM_IMPL_SIMT
                    : !strcmp(impl_name, "tcgen05") ? MLSTM_IMPL_TCGEN05 : -1;
   if (impl < 0) { PyErr_SetObject(PyExc_KeyError, a[11]); throw python_error(); }

@@ -66,6 +66,12 @@ def test_forward_mode_tangents_are_refused(name):
             mk.mlstm_chunkwise__b200_xl_chunk(**a)
 
 
+@pytest.mark.parametrize("impl", ["cutlass", "\ud800", None, 1])
+def test_unknown_implementation_is_a_key_error(impl):
+    with FakeTensorMode(), pytest.raises(KeyError):
+        mk.mlstm_chunkwise__b200_xl_chunk(**operands(), impl=impl)
+
+
 def step_operands():
     e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device="cuda")  # noqa: E731
     f32 = torch.float32
