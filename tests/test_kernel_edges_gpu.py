@@ -74,13 +74,16 @@ def test_step_slices(B, NH, DHQK, DHHV, dtype):
 
 
 def test_native_host_argument_errors():
+    """The exception types are those of the Python wrappers (every malformed operand: test_argument_errors_cpu.py)."""
     q = torch.randn(1, 2, 64, 32, device="cuda")
     i = torch.randn(1, 2, 64, device="cuda")
-    with pytest.raises((AssertionError, ValueError, RuntimeError, TypeError)):
+    with pytest.raises(ValueError, match="inconsistent shapes"):
         mk.mlstm_chunkwise__b200_xl_chunk(q, q[:, :1], q, i, i)            # other number of heads in k
-    with pytest.raises((AssertionError, ValueError, RuntimeError, TypeError)):
+    with pytest.raises(ValueError, match="inconsistent shapes"):
         mk.mlstm_chunkwise__b200_xl_chunk(q, q, q, i[:, :, :5], i)         # fewer gates than tokens
-    with pytest.raises((AssertionError, ValueError, RuntimeError, TypeError)):
+    with pytest.raises(RuntimeError, match="m_initial"):                   # one max state for two heads
+        mk.mlstm_chunkwise__b200_xl_chunk(q, q, q, i, i, m_initial=torch.zeros(1, 1, 1, device="cuda"))
+    with pytest.raises(AssertionError, match="matC_old has wrong shape"):
         mk.mlstm_recurrent_step__b200(q[:, :, 0], q[:, :, 0], q[:, :, 0], i[:, :, :1], i[:, :, :1],
                                       torch.zeros(1, 2, 32, 31, device="cuda"), torch.zeros(1, 2, 32, device="cuda"),
                                       torch.zeros(1, 2, 1, device="cuda"))
