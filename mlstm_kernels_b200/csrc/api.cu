@@ -59,6 +59,19 @@ PhaseScope::~PhaseScope() {
   if (slot < (int)g_prof_recs.size()) cudaEventRecord(g_prof_recs[slot].b, st);
 }
 
+// number of SMs of the current device (queried once per device)
+int sm_count() {
+  static int cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kB200Sms;
+  if (cached[dev] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = kB200Sms;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- the (batch, head) units as two chains of launches on two streams ---------------------------------
@@ -105,7 +118,7 @@ static SideStream* side_stream_for_current_device() {
 // while phases are being timed)
 static bool want_unit_split(const ChunkwiseDims& d, bool allow, int recurrences) {
   if (!allow || g_split_on.load(std::memory_order_relaxed) == 0 || g_prof_on || d.B * d.NH < 2) return false;
-  const long ctas = recurrences * sm100_recurrence_ctas(d), sms = sm100_sm_count();
+  const long ctas = recurrences * sm100_recurrence_ctas(d), sms = sm_count();
   const long waves = (ctas + sms - 1) / sms;
   return waves > 1 && ctas * 100 < waves * sms * 95;   // the last wave leaves more than 5 % of the SM time idle
 }

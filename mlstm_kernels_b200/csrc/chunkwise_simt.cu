@@ -8,6 +8,7 @@
 //   par_fw_kernel, par_bw_kernel  : intra-chunk gated products + inter-chunk contribution for H; deltaV, deltaK, deltaQ
 //                 fw_kernel_parallel.py:14-289, bw_kernel_parallel_dV.py, _dK.py, _dQ.py
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "launch.cuh"
 
 namespace mlstm {
@@ -26,20 +27,6 @@ constexpr int NTHR = 256;  // 16 x 16 threads, 4 x 4 outputs each
 // measured faster than one with 8 x 4 outputs per thread.  Measured 30-34 TFLOP/s at B=4 NH=4 S=2048 128/256; unbuffered
 // slices, scalar reads and a serial recurrence ran at 4.
 __device__ __forceinline__ int swz(int k, int x) { return k * TILE + (((x >> 2) ^ ((k >> 2) & 7)) << 2) + (x & 3); }
-
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
 
 __device__ __forceinline__ int row_group(int tid) { return tid >> 4; }
 __device__ __forceinline__ int col_group(int tid) { return tid & 15; }
@@ -63,8 +50,7 @@ struct Acc {   // rows 4 ty + {0..3} in pairs, columns 4 tx + {0..3}
     for (int a = 0; a < 2; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const float2 f = unpack2(v[a][b]);
-        x[2 * a][b] = f.x; x[2 * a + 1][b] = f.y;
+        unf2(v[a][b], x[2 * a][b], x[2 * a + 1][b]);
       }
   }
 };
@@ -81,11 +67,11 @@ __device__ __forceinline__ void mma_slice(Acc& acc, const float* A, const float*
       const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(pa + k * TILE);
       const float4 b = *reinterpret_cast<const float4*>(pb + k * TILE);
       const uint64_t av[2] = {a.x, a.y};
-      const uint64_t bv[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
+      const uint64_t bv[4] = {f2(b.x, b.x), f2(b.y, b.y), f2(b.z, b.z), f2(b.w, b.w)};
 #pragma unroll
       for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) fma2(acc.v[m][n], av[m], bv[n]);
+        for (int n = 0; n < 4; ++n) acc.v[m][n] = fma2(av[m], bv[n], acc.v[m][n]);
     }
   }
 }
@@ -456,8 +442,9 @@ __device__ __forceinline__ void par_tile(const ParArgs<T>& p, const int mode, in
   for (int a = 0; a < 2; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const float2 f = unpack2(acc.v[a][b]);
-      acc.v[a][b] = pack2(f.x * rs[2 * a], f.y * rs[2 * a + 1]);
+      float lo, hi;
+      unf2(acc.v[a][b], lo, hi);
+      acc.v[a][b] = f2(lo * rs[2 * a], hi * rs[2 * a + 1]);
     }
 
   const int nblk = (L + TILE - 1) / TILE;

@@ -991,7 +991,7 @@ static int set_smem_once(K kern, int bytes, bool (&done)[64]) {
 // Tensor maps depend only on (base pointer, rows, columns, box): a training loop calls with the same buffers over
 // and over, so the last few encodings are kept per thread instead of calling the driver 3-7 times per launch.
 struct MapKey { const void* base; uint64_t rows, cols, slabs; uint32_t box_rows, box_cols; bool f16; };
-// slabs == 0: plain 2-D matrix [rows x cols]; otherwise a 3-D tensor [slabs x rows x cols]; f16: IEEE half, else bf16
+// tensor [slabs x rows x cols]; f16: IEEE half, else bf16
 static bool cached_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                        uint32_t box_cols, uint64_t slabs, bool f16) {
   constexpr int N = 32;
@@ -1007,8 +1007,7 @@ static bool cached_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t
     }
   }
   auto encode = [&]() {
-    return slabs == 0 ? sm100_host::make_map_bf16(m, base, rows, cols, box_rows, box_cols, f16)
-                      : sm100_host::make_map_bf16_3d(m, base, slabs, rows, cols, box_rows, box_cols, f16);
+    return sm100_host::make_map_3d(m, base, slabs, rows, cols, box_rows, box_cols, f16);
   };
   if (!encode()) {
     // A thread whose first CUDA work this is (an autograd worker that found all its memory in the allocator's cache) has
@@ -1042,20 +1041,7 @@ static int launch_rec_tn(const CUtensorMap& mL, const CUtensorMap& mR, const CUt
   static bool attr_done[64] = {};
   if (int rc = set_smem_once(kern, rec_smem_bytes(!BWD, TN), attr_done)) return rc;
   const unsigned grid = (unsigned)((d.DHHV + TN - 1) / TN) * (unsigned)((d.DHQK + 127) / 128) * (unsigned)units;
-  return launch_ex(ur.overlap && grid <= kPdlMaxCtas, ur.started, kern, grid, REC_THREADS, rec_smem_bytes(!BWD, TN), st, mL, mR, mS, rp);
-}
-
-// number of SMs of the current device (queried once per device)
-static int sm_count() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (cached[dev] == 0) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
+  return launch_ex(ur.overlap && grid <= pdl_max_ctas(), ur.started, kern, grid, REC_THREADS, rec_smem_bytes(!BWD, TN), st, mL, mR, mS, rp);
 }
 
 // Segments of the sequence for a forward whose recurrence covers at most half of the SMs: the intra-chunk kernel of a
@@ -1077,7 +1063,6 @@ int sm100_forward_segments(const ChunkwiseDims& d) {
 long sm100_recurrence_ctas(const ChunkwiseDims& d) {
   return (long)((d.DHHV + 127) / 128) * ((d.DHQK + 127) / 128) * d.B * d.NH;
 }
-int sm100_sm_count() { return sm_count(); }
 
 struct RecMaps { CUtensorMap l, r, s; };
 static bool rec_maps(RecMaps* m, const void* left, const void* right, const void* states, const ChunkwiseDims& d) {
@@ -1118,7 +1103,7 @@ static int launch_rec_pair(const RecMaps& m, const RecParams& rp, const RecMaps&
   static bool attr_done[64] = {};
   if (int rc = set_smem_once(kern, rec_smem_bytes(false, TN), attr_done)) return rc;
   const unsigned n = (unsigned)((d.DHHV + TN - 1) / TN) * (unsigned)((d.DHQK + 127) / 128) * (unsigned)units;
-  return launch_pdl(overlap && 2 * n <= kPdlMaxCtas, kern, 2 * n, REC_THREADS, rec_smem_bytes(false, TN), st, m.l, m.r, m.s, rp, mb.l, mb.r,
+  return launch_pdl(overlap && 2 * n <= pdl_max_ctas(), kern, 2 * n, REC_THREADS, rec_smem_bytes(false, TN), st, m.l, m.r, m.s, rp, mb.l, mb.r,
                     mb.s, rpb, n);
 }
 
@@ -1205,7 +1190,7 @@ int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuf
   auto kern = f16 ? par_fw_sm100<true> : par_fw_sm100<false>;
   static bool attr_done[2][64] = {};
   if (int rc = set_smem_once(kern, PAR_SMEM, attr_done[f16])) return rc;
-  return launch_pdl(ur.overlap && grid <= kPdlMaxCtas, kern, grid, PAR_THREADS, PAR_SMEM, st, mQ, mK, mV, mC, pp);
+  return launch_pdl(ur.overlap && grid <= pdl_max_ctas(), kern, grid, PAR_THREADS, PAR_SMEM, st, mQ, mK, mV, mC, pp);
 }
 
 int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
@@ -1231,7 +1216,7 @@ int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* d
   auto ctas = [&](int m) { return ((long)ceil_div(T_dv, m) + 2 * ceil_div(T_dk, m)) * d.NC * units; };
   pp.maxsub = par_maxsub(ctas, std::max(T_dv, T_dk));
   const unsigned grid = (unsigned)ctas(pp.maxsub);
-  return launch_pdl(ur.overlap && grid <= kPdlMaxCtas, f16 ? par_bw_sm100<true> : par_bw_sm100<false>, grid, PAR_THREADS, PAR_SMEM, st,
+  return launch_pdl(ur.overlap && grid <= pdl_max_ctas(), f16 ? par_bw_sm100<true> : par_bw_sm100<false>, grid, PAR_THREADS, PAR_SMEM, st,
                     mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k, pp);
 }
 

@@ -49,6 +49,10 @@ void set_last_cuda_error(cudaError_t e, const char* where);
     }                                                  \
   } while (0)
 
+// SMs of the current device (of a B200 where there is none: sizes are asked for on hosts without a GPU too)
+constexpr int kB200Sms = 148;
+int sm_count();
+
 // every kernel launch of this library is counted (mlstm_b200_launch_count)
 void note_launch();
 #define MLSTM_LAUNCH_CHECK()                  \
@@ -86,7 +90,7 @@ __device__ __forceinline__ uint2 ld_stream(const uint2* p) {
 
 // Larger launches start plainly: their own CTAs hide the gap, and CTAs of the next kernel that are resident early would take
 // room on an SM from those of a second chain of launches.
-constexpr unsigned kPdlMaxCtas = 4 * 148;
+inline unsigned pdl_max_ctas() { return 4u * (unsigned)sm_count(); }
 
 // started (nullable): recorded once every CTA of the launch is running.
 template <typename... KArgs, typename... Args>

@@ -380,7 +380,7 @@ static int launch_gates_nv(const void* i, const void* f, const float* n_out, flo
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = cfg.gridDim.x <= kPdlMaxCtas ? 2 : 1;
+  cfg.numAttrs = cfg.gridDim.x <= pdl_max_ctas() ? 2 : 1;
   note_launch();
   MLSTM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gates_kernel<T, NV>, (const T*)i, (const T*)f, n_out, m_out, gb, sc, d.S, d.SP,
                                       d.L, d.NC, d.variant, d.eps));
@@ -516,7 +516,7 @@ static int gate_grad_scan_t(const void* i, const void* f, const float* qdq, cons
   const size_t stride = (size_t)d.B * d.NH * d.SP;
   if (anchors != nullptr && anchor_tokens == kAnchorThreads) {
     const unsigned grid = (unsigned)ceil_div(d.S, kAnchorThreads) * (unsigned)(d.B * d.NH);
-    return launch_pdl(grid <= kPdlMaxCtas, gate_grad_anchored_kernel<T>, grid, kAnchorThreads, 0, st, (const T*)i, (const T*)f, qdq,
+    return launch_pdl(grid <= pdl_max_ctas(), gate_grad_anchored_kernel<T>, grid, kAnchorThreads, 0, st, (const T*)i, (const T*)f, qdq,
                       kdk, dI, dF, out_dtype, d.S, d.SP, d.variant, nparts, stride, anchors, n_anchors);
   } else {
     gate_grad_scan_kernel<T><<<d.B * d.NH, kScanThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, out_dtype, d.S, d.SP,
@@ -544,9 +544,9 @@ int launch_state_dot(const void* c_states, const void* dc_states, float* anchors
   const unsigned grid = (unsigned)(n_anchors - 1) * (unsigned)(d.B * d.NH);
   const size_t elems = (size_t)d.DHQK * d.DHHV;
   if (d.dtype == MLSTM_F16)
-    return launch_pdl(grid <= kPdlMaxCtas, state_dot_kernel<__half>, grid, 256, 0, st, (const __half*)c_states,
+    return launch_pdl(grid <= pdl_max_ctas(), state_dot_kernel<__half>, grid, 256, 0, st, (const __half*)c_states,
                       (const __half*)dc_states, anchors, d.NC, every, n_anchors, elems);
-  return launch_pdl(grid <= kPdlMaxCtas, state_dot_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)c_states,
+  return launch_pdl(grid <= pdl_max_ctas(), state_dot_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)c_states,
                     (const __nv_bfloat16*)dc_states, anchors, d.NC, every, n_anchors, elems);
 }
 

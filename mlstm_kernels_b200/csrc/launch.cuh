@@ -61,11 +61,10 @@ int sm100_recurrent_pair(const void* k, const void* v, const float* c_initial, v
 int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
                       const void* c_states, const void* dc_states, void* dq, void* dk, void* dv, float* qdq_parts,
                       float* kdk_parts, const ChunkwiseDims& d, cudaStream_t st, UnitRange ur = UnitRange());
-// number of CTAs the recurrence launches for the whole problem with 128-column state tiles, and SMs of the device
+// number of CTAs the recurrence launches for the whole problem with 128-column state tiles
 long sm100_recurrence_ctas(const ChunkwiseDims& d);
 // segments the forward cuts the sequence into (1: none); a function of the sizes alone
 int sm100_forward_segments(const ChunkwiseDims& d);
-int sm100_sm_count();
 
 int sm100_device_status(int reset, int* status);
 int sm100_wait_expiry_selftest(unsigned limit, int code, cudaStream_t st);

@@ -354,8 +354,8 @@ int step_t(const void* q, const void* k, const void* v, const void* i, const voi
   // launches of more than one wave (four CTAs per SM) start plainly: they gain nothing from overlapping their start with
   // the last step's end
   const long ctas = (long)ceil_div(DHHV, 64) * B * NH;
-  if (ctas < 148) return STEP_RUN(32, true);
-  if (ctas <= 4 * 148) return STEP_RUN(64, true);
+  if (ctas < sm_count()) return STEP_RUN(32, true);
+  if (ctas <= 4L * sm_count()) return STEP_RUN(64, true);
   return STEP_RUN(64, false);
 #undef STEP_RUN
 }
@@ -395,7 +395,7 @@ int step_seq_rows(const void* q, const void* k, const void* v, const void* i, co
                   int B, int NH, int Tn, int DHQK, int DHHV, float eps, cudaStream_t st) {
   // 32-column slices while 64-column ones would leave SMs without a CTA: half the multiply-adds per thread and token,
   // for q, k and n prepared once more
-  const bool narrow = (long)ceil_div(DHHV, 64) * B * NH < 148;
+  const bool narrow = (long)ceil_div(DHHV, 64) * B * NH < sm_count();
 #define SEQ_CASE(R, TV) \
   if (ceil_div(DHQK, STEP_THREADS / (TV / 4)) <= R) \
     return step_seq_t<T, R, TV>(q, k, v, i, f, gate_dtype, c, n, m, h, c_new, n_new, m_new, B, NH, Tn, DHQK, DHHV, eps, st);
