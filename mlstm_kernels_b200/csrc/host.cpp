@@ -5,8 +5,9 @@
 // foreign-function call made from Python cost 15 us a step, 86 us a forward and 260 us a forward + backward, so the
 // GPU sat idle.  Here the whole call is native: tensors come straight from their Python objects, outputs from the
 // caching allocator (one scratch block per call, carved here), and the backward runs as a C++ autograd node that needs
-// no interpreter lock.  Signatures, defaults, return conventions and error texts are those of the Python wrappers
-// (chunkwise.py, recurrent.py), which hand over to this module.
+// no interpreter lock.  Signatures, defaults, return conventions and exception types are those of the Python wrappers
+// (chunkwise.py, recurrent.py), which hand over to this module; the operands' sizes and memory are checked before anything
+// touches the device.
 #include <Python.h>
 
 #include <ATen/ATen.h>

@@ -58,7 +58,8 @@ def mlstm_recurrent_step__b200_fw(
 ):
     """One decode step.  `validate=False` is for decode loops that own all their buffers: every tensor (the new-state
     and `vecH_out` buffers included) must then be a contiguous CUDA tensor of the expected shape and element type on
-    the current device; nothing is checked or converted and the call costs little more than the launch itself."""
+    the current device; nothing is checked or converted.  (The call goes through ctypes: 6.3 us per step at batch 1, where
+    the checked call, which is native, takes 4.2.)"""
     if not validate:
         B, NH, DHQK = vecQ.shape
         codes = _lib._DTYPE_CODE
