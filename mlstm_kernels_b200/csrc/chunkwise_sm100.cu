@@ -159,10 +159,9 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
         issued = h + 1;
       }
     }
-    if (issued < NH2 && issued > 0) {  // error path: let the copies in flight land before the CTA retires
-      for (int h = max(0, issued - REC_STAGES); h < issued; ++h)
-        mbar_wait(&bar_full[h % REC_STAGES], (h / REC_STAGES) & 1, nullptr, nullptr, 0);
-    }
+    // the copies in flight land before the CTA retires, whichever role may have given up (the other lanes have issued none)
+    for (int h = max(0, issued - REC_STAGES); h < issued; ++h)
+      mbar_wait(&bar_full[h % REC_STAGES], (h / REC_STAGES) & 1, nullptr, nullptr, 0);
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
@@ -427,6 +426,7 @@ struct ParShared {
   uint64_t bar_full[PAR_NST], bar_empty[PAR_NST], bar_qdone[PAR_NST], bar_sfull, bar_afull, bar_gated, bar_hfull, bar_accfree, bar_done, bar_dot,
       bar_pair[4], bar_out;
   uint32_t tmem;
+  int issued;                      // loads the producer has issued
   int abort;                       // set by the first wait of this CTA that runs out; every other wait polls it
   __align__(16) float s_colE[CL];  // per-column term of the gate exponent, base 2 (see par_body)
   __align__(16) float s_colF[CL];  // 2^(colE_c - colP of the column's 32-column block)
@@ -480,7 +480,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       mbar_inval(&sh.bar_sfull); mbar_inval(&sh.bar_afull); mbar_inval(&sh.bar_gated); mbar_inval(&sh.bar_hfull); mbar_inval(&sh.bar_dot);
       mbar_inval(&sh.bar_out); mbar_inval(&sh.bar_accfree); mbar_inval(&sh.bar_done);
     }
-    sh.abort = 0;
+    sh.abort = 0; sh.issued = 0;
     for (int s = 0; s < PAR_NST; ++s) {
       mbar_init(&sh.bar_full[s], 1); mbar_init(&sh.bar_empty[s], 1); mbar_init(&sh.bar_qdone[s], 8);
     }
@@ -577,10 +577,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         st = st == PAR_NST - 1 ? 0 : st + 1;
         if (++l == (sub == 0 ? n0 : n1)) { l = 0; ++sub; }
       }
-      if (issued < n_loads && issued > 0) {  // error path: let the copies in flight land before the CTA retires
-        for (int ld = max(0, issued - PAR_NST); ld < issued; ++ld)
-          mbar_wait(&sh.bar_full[ld % PAR_NST], (ld / PAR_NST) & 1, nullptr, nullptr, 0);
-      }
+      sh.issued = issued;
       if (LOOP && issued == n_loads) {   // the hand-backs of the last uses, which nobody else waits for
         if (rm0 > 0) mbar_wait(&sh.bar_empty[0], (rm0 - 1) & 1, &sh.abort, &g_sm100_status, 217);
         if (rm1 > 0) mbar_wait(&sh.bar_empty[1], (rm1 - 1) & 1, &sh.abort, &g_sm100_status, 217);
@@ -771,7 +768,8 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     sh.s_part[half][r] = rowsum;
     tmem_wait_st();
     // From here to the end the warps go in step whatever their waits answer (see warp_arrive).  A hand-over to the other
-    // roles takes place only if the wait before it succeeded; the element-wise warps' own barriers just count.
+    // roles takes place only if no wait has run out (the flag is read where it is needed: kept in a register over the epilogue
+    // it costs the kernel 1-2 %); the element-wise warps' own barriers just count.
     // ---- per output tile: row-scale the inter-chunk product, second product, epilogue, store ----
     float inv = 1.f;
     for (int sub = 0; sub < nsub; ++sub) {
@@ -797,7 +795,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       tmem_wait_st();
       tc_fence_before_sync();
       if (acc_ok) mbar_arrive(&sh.bar_gated);   // (first tile: the gated score tile is in place as well)
-      bool ok = mbar_wait(&sh.bar_hfull, sub & 1, &sh.abort, &g_sm100_status, 206);
+      mbar_wait(&sh.bar_hfull, sub & 1, &sh.abort, &g_sm100_status, 206);
       tc_fence_after_sync();
       if (sub == 0 && mode == PM_H) {
         float den = 1.f;
@@ -814,7 +812,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       const uint8_t* erow = smem;
       if (HAS_E) {
         const int lde = ldx + 1, ste = lde % PAR_NST;
-        ok = mbar_wait(&sh.bar_full[ste], (lde / PAR_NST) & 1, &sh.abort, &g_sm100_status, 208) && ok;
+        mbar_wait(&sh.bar_full[ste], (lde / PAR_NST) & 1, &sh.abort, &g_sm100_status, 208);
         erow = smem + ste * PAR_STAGE + r * 128;
       }
       float dot4[4] = {0.f, 0.f, 0.f, 0.f};   // four partial sums: no 64-long chain of dependent FMAs
@@ -860,7 +858,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       }
       if (sub + 1 < nsub) {   // the accumulator tile may be overwritten by the next tile's inter-chunk product
         tc_fence_before_sync();
-        if (ok) mbar_arrive(&sh.bar_accfree);
+        if (!aborted(&sh.abort)) mbar_arrive(&sh.bar_accfree);
       }
       const float dot = (dot4[0] + dot4[1]) + (dot4[2] + dot4[3]);
       mbar_arrive(&sh.bar_out);
@@ -889,14 +887,19 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         // proxy: without this fence its data can be overtaken by this thread's own earlier (generic-proxy) staging
         // writes to the same addresses.
         fence_proxy_async_smem();
-        if (ok) mbar_arrive(&sh.bar_done);
+        if (!aborted(&sh.abort)) mbar_arrive(&sh.bar_done);
       }
     }
   }
   if (LOOP) fence_proxy_async_smem();   // staging writes above, the next run's copies after the barrier
   tc_fence_before_sync();
   __syncthreads();
-  const bool go_on = !LOOP || sh.abort == 0;   // (the next run sets it to the 0 that it is)
+  const bool go_on = sh.abort == 0;   // (the next run sets it to the 0 that it is)
+  // Whichever role gave up: the copies in flight land before the CTA retires.  (Where the producer waits for them on every
+  // way out, as in the recurrence, its polling costs the backward 2 %.)
+  if (tid == 0 && !go_on)
+    for (int ld = max(0, sh.issued - PAR_NST); ld < sh.issued; ++ld)
+      mbar_wait(&sh.bar_full[ld % PAR_NST], (ld / PAR_NST) & 1, nullptr, nullptr, 0);
   if (warp == 1 && (!LOOP || last_run || !go_on)) tmem_dealloc(tmem, 256);
   return go_on;
 }

@@ -46,17 +46,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // early, used where the CTA must wait for copies still in flight), `status` is the device-wide word the host reads:
 // it keeps the code of the FIRST wait that ran out and is never consulted by a kernel, so one expired wait does not
 // make later launches give up.
+__device__ __forceinline__ bool aborted(const int* abort) {
+  uint32_t a;
+  asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(a) : "r"(smem_u32(abort)) : "memory");
+  return a != 0;
+}
 constexpr uint32_t kWaitLimit = 20u * 1000u * 1000u;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* abort, int* status, int code,
                                           uint32_t limit = kWaitLimit) {
   for (uint32_t it = 0; it < limit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if (it > 64) __nanosleep(32);
-    if (abort != nullptr && (it & 1023) == 1023) {
-      uint32_t a;
-      asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(a) : "r"(smem_u32(abort)) : "memory");
-      if (a != 0) return false;
-    }
+    if (abort != nullptr && (it & 1023) == 1023 && aborted(abort)) return false;
   }
   if (abort != nullptr) asm volatile("st.volatile.shared::cta.u32 [%0], %1;" :: "r"(smem_u32(abort)), "r"(1u) : "memory");
   if (status != nullptr) atomicCAS(status, 0, code);

@@ -17,6 +17,7 @@ behind: they would land on the next run's barriers."""
 
 import os
 import random
+import re
 
 import pytest
 
@@ -42,7 +43,8 @@ class Bar:
 def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
     """loop: the form of a CTA that takes several chunks in runs of their own - one that starts with the producer's waits
     for the last hand-backs and ends with nothing in flight.  lost_load: this load (its number) does not land within the
-    limit of the waits.  Returns whether the waits ran out, and the copies and commits that are still in flight."""
+    limit of the waits.  Returns whether the waits ran out, the copies and commits that are still in flight, and the
+    number of loads issued."""
     rnd = random.Random(seed)
     HAS_E = mode in ("DQ", "DK")
     USE_N = mode == "Hn"             # the element-wise warps read the A box of each score pair (q . n)
@@ -55,6 +57,7 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
         B[n] = Bar(n, c)
     for qd in range(4): B[f"pair{qd}"] = Bar(f"pair{qd}", 2)
     pending_async = []   # async completions: ('load', st) any order ; commits in order
+    issued = 0
     late = []            # loads that land after the waits have run out
     commit_queue = []    # list of barrier names, fire in order
     def kind_of(sub, l):
@@ -64,7 +67,8 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
         return "X" if ls == ND else "E"
     # generators for each role; yield ('wait', barname, phase) blocks until passes; other ops executed inline
     def producer():
-        issued = 0; rm = [0]*NST; rq = [0]*NST; st = 0; hist = []
+        nonlocal issued
+        rm = [0]*NST; rq = [0]*NST; st = 0; hist = []
         for job in range(njobs):
             sub = 0; l = 0
             for ld in range(n_loads):
@@ -187,10 +191,10 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
                 progressed = True; break
             progressed = True; break
         if not progressed and lost_load is not None:
-            return True, late + pending_async + commit_queue
+            return True, late + pending_async + commit_queue, issued
         if not progressed:
             raise AssertionError(f"DEADLOCK: blocked={blocked} barsync={barsync_wait} phases={{k:v.phase for k,v in B.items()}}".replace("{{","{").replace("}}","}") + str({k:v.phase for k,v in B.items()}))
-    return False, late + pending_async + commit_queue
+    return False, late + pending_async + commit_queue, issued
 
 
 
@@ -220,7 +224,7 @@ def test_ring_running_on_across_chunks_would_alias():
 def run_range(mode, ND, nsub, runs, seed, lost_run=None, stop=True):
     """A CTA of par_fw_range_sm100: `runs` chunks one after the other on barriers set up anew."""
     for r in range(runs):
-        expired, in_flight = run(mode, ND, nsub, 1, seed + r, loop=True, lost_load=2 if r == lost_run else None)
+        expired, in_flight, _ = run(mode, ND, nsub, 1, seed + r, loop=True, lost_load=2 if r == lost_run else None)
         if expired and stop:
             return
         if r + 1 < runs:
@@ -243,3 +247,24 @@ def test_segment_cta_stops_after_a_run_whose_waits_ran_out():
     with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlstm_kernels_b200", "csrc",
                            "chunkwise_sm100.cu")) as f:
         assert "if (!par_body<F16, true>(" in f.read()
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("ND,nsub", [(1, 1), (2, 2), (4, 3)])
+def test_a_load_that_is_late_is_among_the_last_of_its_ring(mode, ND, nsub):
+    """After a wait of any role has run out, thread 0 waits for the last PAR_NST loads issued before the CTA retires: a late
+    one is always among them, also where the producer had issued everything and another role gave up."""
+    extra = 1 if mode in ("DQ", "DK") else 0
+    n_loads = (2 * ND + 1 + extra) + (nsub - 1) * (ND + 1 + extra)
+    for lost in range(n_loads):
+        expired, in_flight, issued = run(mode, ND, nsub, 1, lost, lost_load=lost)
+        assert expired and ("load", lost % 3) in in_flight
+        assert issued - 3 <= lost < issued
+    with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlstm_kernels_b200", "csrc",
+                           "chunkwise_sm100.cu")) as f:
+        src = f.read()
+    # the intra-chunk kernels wait behind the barrier that all roles reach, on the abort flag alone; the recurrence's
+    # producer on every way out
+    assert re.search(r"__syncthreads\(\);\n  const bool go_on = sh\.abort == 0;.*\n(?:  //.*\n)*  if \(tid == 0 && !go_on\)\n"
+                     r"    for \(int ld = max\(0, sh\.issued - PAR_NST\); ld < sh\.issued; \+\+ld\)\n      mbar_wait\(&sh\.bar_full", src)
+    assert re.search(r"\n    for \(int h = max\(0, issued - REC_STAGES\); h < issued; \+\+h\)\n      mbar_wait\(&bar_full", src)

@@ -15,11 +15,11 @@ LANES, POLLS, ROUNDS = 4, 6, 3
 def lane(i, state, on_failure):
     """One lane: rounds of (bounded wait, warp-wide operation, arrival of lane 0).  Yields "operation" where the whole
     warp has to come together; the polls of the lanes interleave freely.  After a failed wait the lane leaves, or goes on
-    without waits and arrivals ("flag"), or without the arrival that follows the wait ("answer"), or only meets the
-    others in the operations that are left ("stand by")."""
+    without waits and arrivals ("flag"), or without the arrival that follows the wait ("answer"), or without arrivals
+    once any wait has run out ("abort flag"), or only meets the others in the operations that are left ("stand by")."""
     ok = True
     for round_ in range(ROUNDS):
-        if ok or on_failure == "answer":
+        if ok or on_failure in ("answer", "abort flag"):
             ok = False
             for poll in range(POLLS):
                 yield "poll"                            # another lane, or the barrier, may move here
@@ -37,7 +37,7 @@ def lane(i, state, on_failure):
                     yield "operation"
                 return
         yield "operation"                               # elect, shuffle, tensor-memory access
-        if i == 0 and ok:
+        if i == 0 and (not state["abort"] if on_failure == "abort flag" else ok):
             assert state["complete"] > round_, "arrival without the phase that it follows"
             state["arrivals"] += 1
 
@@ -69,7 +69,7 @@ def run(seed, on_failure):
     return state
 
 
-@pytest.mark.parametrize("on_failure", ["flag", "answer", "stand by"])
+@pytest.mark.parametrize("on_failure", ["flag", "answer", "abort flag", "stand by"])
 def test_lanes_that_go_on_end_together(on_failure):
     expired = 0
     for seed in range(4000):
@@ -101,7 +101,7 @@ def test_no_lane_leaves_a_warp_alone():
         stands_by = "stand_by(h, " in after or "__syncwarp();" in next_line
         assert stands_by or (not left and "if (!" not in before), f"wait with status code {code}"
     # hand-overs to other roles depend on the wait before them
-    for bar, flag in (("gated", "acc_ok"), ("accfree", "ok"), ("done", "ok")):
+    for bar, flag in (("gated", "acc_ok"), ("accfree", r"!aborted\(&sh\.abort\)"), ("done", r"!aborted\(&sh\.abort\)")):
         assert re.findall(rf"(.*)mbar_arrive\(&sh\.bar_{bar}\)", src) == [re.search(rf" *if \({flag}\) (?=mbar_arrive\(&sh\.bar_{bar}\))", src).group(0)]
     for bar in ("out_full", "acc_free"):
         assert re.search(rf"warp_arrive\(&bar_{bar}\[\w+\], ok\)", src)
