@@ -858,7 +858,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       }
       if (sub + 1 < nsub) {   // the accumulator tile may be overwritten by the next tile's inter-chunk product
         tc_fence_before_sync();
-        if (!aborted(&sh.abort)) mbar_arrive(&sh.bar_accfree);
+        if (!aborted(smem_u32(&sh.abort))) mbar_arrive(&sh.bar_accfree);
       }
       const float dot = (dot4[0] + dot4[1]) + (dot4[2] + dot4[3]);
       mbar_arrive(&sh.bar_out);
@@ -887,7 +887,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         // proxy: without this fence its data can be overtaken by this thread's own earlier (generic-proxy) staging
         // writes to the same addresses.
         fence_proxy_async_smem();
-        if (!aborted(&sh.abort)) mbar_arrive(&sh.bar_done);
+        if (!aborted(smem_u32(&sh.abort))) mbar_arrive(&sh.bar_done);
       }
     }
   }
