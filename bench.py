@@ -957,7 +957,7 @@ def bench_portable(torch, mk, dev):
     ffw = fw_flops(B, NH, S, DHQK, DHHV, L)
     ffb = ffw + bw_flops(B, NH, S, DHQK, DHHV, L)
     return dict(fw_ms=ms_fw, fw_tflops=ffw / ms_fw / 1e9, fwbw_ms=ms_fwbw, fwbw_tflops=ffb / ms_fwbw / 1e9,
-                note="exact f32 arithmetic on CUDA cores (coverage path, not tuned)")
+                note="exact f32 arithmetic on CUDA cores")
 
 
 def bench_head_dims(torch, mk, dev):

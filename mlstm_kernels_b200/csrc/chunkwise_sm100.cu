@@ -423,7 +423,7 @@ constexpr int PAR_SMEM = PAR_NST * PAR_STAGE + 1024;
 
 // Shared-memory control block of one intra-chunk CTA (the operand ring lives in dynamic shared memory).
 struct ParShared {
-  uint64_t bar_full[PAR_NST], bar_empty[PAR_NST], bar_qdone[PAR_NST], bar_sfull, bar_afull, bar_gated, bar_hfull, bar_accfree, bar_done, bar_dot,
+  uint64_t bar_full[PAR_NST], bar_empty[PAR_NST], bar_qdone[PAR_NST], bar_sfull, bar_afull, bar_gated, bar_hfull, bar_accfree, bar_done[2], bar_dot,
       bar_pair[4], bar_out;
   uint32_t tmem;
   int issued;                      // loads the producer has issued
@@ -478,7 +478,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       for (int s = 0; s < PAR_NST; ++s) { mbar_inval(&sh.bar_full[s]); mbar_inval(&sh.bar_empty[s]); mbar_inval(&sh.bar_qdone[s]); }
       for (int s = 0; s < 4; ++s) mbar_inval(&sh.bar_pair[s]);
       mbar_inval(&sh.bar_sfull); mbar_inval(&sh.bar_afull); mbar_inval(&sh.bar_gated); mbar_inval(&sh.bar_hfull); mbar_inval(&sh.bar_dot);
-      mbar_inval(&sh.bar_out); mbar_inval(&sh.bar_accfree); mbar_inval(&sh.bar_done);
+      mbar_inval(&sh.bar_out); mbar_inval(&sh.bar_accfree); mbar_inval(&sh.bar_done[0]); mbar_inval(&sh.bar_done[1]);
     }
     sh.abort = 0; sh.issued = 0;
     for (int s = 0; s < PAR_NST; ++s) {
@@ -486,7 +486,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     }
     mbar_init(&sh.bar_sfull, 1); mbar_init(&sh.bar_afull, 1); mbar_init(&sh.bar_gated, 256); mbar_init(&sh.bar_hfull, 1); mbar_init(&sh.bar_dot, 256);
     for (int s = 0; s < 4; ++s) mbar_init(&sh.bar_pair[s], 64);
-    mbar_init(&sh.bar_out, 256); mbar_init(&sh.bar_accfree, 256); mbar_init(&sh.bar_done, 256);
+    mbar_init(&sh.bar_out, 256); mbar_init(&sh.bar_accfree, 256); mbar_init(&sh.bar_done[0], 256); mbar_init(&sh.bar_done[1], 256);
     fence_barrier_init();
     tma_prefetch_desc(mapA); tma_prefetch_desc(mapB); tma_prefetch_desc(mapX); tma_prefetch_desc(mapSt);
     if (HAS_E) tma_prefetch_desc(mapE);
@@ -546,8 +546,11 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
               const int rq = st == 0 ? rq0 : (st == 1 ? rq1 : rq2);
               okw = mbar_wait(&sh.bar_qdone[st], (rq - 1) & 1, &sh.abort, &g_sm100_status, 212);
             }
-          } else {   // the staging buffer of a tile (its E stage, or its X stage in the modes without E) is handed
-            okw = mbar_wait(&sh.bar_done, psub & 1, &sh.abort, &g_sm100_status, 215);   // back when the tile has been stored
+          } else {
+            // The staging buffer of a tile (its E stage, or its X stage in the modes without E) is handed back when the tile
+            // has been stored.  Two barriers, for every other tile: with one operand slice (DHQK <= 64) a tile's loads are two
+            // and the ring holds three, so that the next tile, too, can be done before this wait looks.
+            okw = mbar_wait(&sh.bar_done[psub & 1], (psub >> 1) & 1, &sh.abort, &g_sm100_status, 215);
           }
           if (!okw) break;
         }
@@ -887,7 +890,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         // proxy: without this fence its data can be overtaken by this thread's own earlier (generic-proxy) staging
         // writes to the same addresses.
         fence_proxy_async_smem();
-        if (!aborted(smem_u32(&sh.abort))) mbar_arrive(&sh.bar_done);
+        if (!aborted(smem_u32(&sh.abort))) mbar_arrive(&sh.bar_done[sub & 1]);
       }
     }
   }

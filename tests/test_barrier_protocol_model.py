@@ -40,10 +40,11 @@ class Bar:
             if self.phase >= want_phase + 2: raise AssertionError(f"ALIAS hang on {self.name}: want {want_phase} at {self.phase}")
         return passes
 
-def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
+def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None, slow=None, two_done=True):
     """loop: the form of a CTA that takes several chunks in runs of their own - one that starts with the producer's waits
     for the last hand-backs and ends with nothing in flight.  lost_load: this load (its number) does not land within the
-    limit of the waits.  Returns whether the waits ran out, the copies and commits that are still in flight, and the
+    limit of the waits.  slow: a role that gets its turn late.  two_done: the tiles are handed back on two barriers in
+    turn.  Returns whether the waits ran out, the copies and commits that are still in flight, and the
     number of loads issued."""
     rnd = random.Random(seed)
     HAS_E = mode in ("DQ", "DK")
@@ -53,7 +54,7 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
     B = {}
     for s in range(NST):
         B[f"full{s}"] = Bar(f"full{s}", 1); B[f"empty{s}"] = Bar(f"empty{s}", 1); B[f"qdone{s}"] = Bar(f"qdone{s}", 8)
-    for n, c in (("sfull",1),("afull",1),("hfull",1),("gated",8),("accfree",8),("done",8),("dot",8),("out",8)):
+    for n, c in (("sfull",1),("afull",1),("hfull",1),("gated",8),("accfree",8),("done0",8),("done1",8),("dot",8),("out",8)):
         B[n] = Bar(n, c)
     for qd in range(4): B[f"pair{qd}"] = Bar(f"pair{qd}", 2)
     pending_async = []   # async completions: ('load', st) any order ; commits in order
@@ -79,7 +80,7 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
                         yield ("wait", f"empty{st}", rm[st] - 1)
                         if USE_N and pk == "SCORE": yield ("wait", f"qdone{st}", rq[st] - 1)
                     else:
-                        yield ("wait", "done", ps)
+                        yield ("wait", f"done{ps & 1}" if two_done else "done0", ps >> 1 if two_done else ps)
                 (late if issued == lost_load else pending_async).append(("load", st))
                 if kind in ("SCORE", "STATE") or (kind == "X" and HAS_E): rm[st] += 1
                 if kind == "SCORE": rq[st] += 1
@@ -142,13 +143,13 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
                 if HAS_E:
                     B["dot"].arrive()
                     if half == 0: yield ("wait", "dot", gt)
-                if njobs > 1 or sub + 1 < nsub: B["done"].arrive()
+                if njobs > 1 or sub + 1 < nsub: B[f"done{gt & 1}" if two_done else "done0"].arrive()
     agents = {"prod": producer(), "mma": mma()}
     for qd in range(4):
         for h in range(2): agents[f"ew{qd}{h}"] = ew(qd, h)
     blocked = {}
     barsync_wait = set()
-    alive = set(agents)
+    alive = dict.fromkeys(agents)    # (in a fixed order: a run depends on its seed alone)
     while alive:
         choices = []
         for a in alive:
@@ -158,6 +159,8 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
         if commit_queue: choices.append(("commit", None))
         # try a random choice; if agent blocked, it stays blocked
         rnd.shuffle(choices)
+        if slow is not None and rnd.random() < 0.95:
+            choices.sort(key=lambda ch: ch[1] == slow)
         progressed = False
         for ch in choices:
             if ch[0] == "async_load":
@@ -177,7 +180,7 @@ def run(mode, ND, nsub, njobs, seed, NST=3, loop=False, lost_load=None):
             try:
                 op = next(agents[a])
             except StopIteration:
-                alive.discard(a); progressed = True; break
+                del alive[a]; progressed = True; break
             if op[0] == "wait":
                 try:
                     okk = B[op[1]].test(op[2])
@@ -205,8 +208,26 @@ MODES = ("H", "Hn", "DV", "DK", "DQ")   # H and DV: no E tile (the output is sta
 @pytest.mark.parametrize("ND", [1, 2, 3, 4, 8])
 @pytest.mark.parametrize("nsub", [1, 2, 3, 4, 8])
 def test_one_chunk_per_cta_protocol_has_no_aliasing_deadlock_or_over_arrival(mode, ND, nsub):
-    for seed in range(40):
+    for seed in range(60):
         run(mode, ND, nsub, 1, seed)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("ND", [1, 2, 3, 4])
+@pytest.mark.parametrize("slow", ["prod", "mma", "ew00", "ew31"])
+def test_a_role_that_falls_behind_meets_no_barrier_two_phases_on(mode, ND, slow):
+    for seed in range(30):
+        run(mode, ND, 4, 1, seed, slow=slow)
+
+
+def test_one_done_barrier_would_run_away_from_the_producer_at_one_operand_slice():
+    for seed in range(200):
+        try:
+            run("H", 1, 4, 1, seed, slow="prod", two_done=False)
+        except AssertionError as e:
+            assert "ALIAS hang on done" in str(e)
+            return
+    raise AssertionError("no interleaving out of 200 showed the hazard")
 
 
 def test_ring_running_on_across_chunks_would_alias():

@@ -101,7 +101,7 @@ def test_no_lane_leaves_a_warp_alone():
         stands_by = "stand_by(h, " in after or "__syncwarp();" in next_line
         assert stands_by or (not left and "if (!" not in before), f"wait with status code {code}"
     # hand-overs to other roles depend on the wait before them
-    for bar, flag in (("gated", "acc_ok"), ("accfree", r"!aborted\(smem_u32\(&sh\.abort\)\)"), ("done", r"!aborted\(smem_u32\(&sh\.abort\)\)")):
+    for bar, flag in (("gated", "acc_ok"), ("accfree", r"!aborted\(smem_u32\(&sh\.abort\)\)"), (r"done\[sub & 1\]", r"!aborted\(smem_u32\(&sh\.abort\)\)")):
         assert re.findall(rf"(.*)mbar_arrive\(&sh\.bar_{bar}\)", src) == [re.search(rf" *if \({flag}\) (?=mbar_arrive\(&sh\.bar_{bar}\))", src).group(0)]
     for bar in ("out_full", "acc_free"):
         assert re.search(rf"warp_arrive\(&bar_{bar}\[\w+\], ok\)", src)

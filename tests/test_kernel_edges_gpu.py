@@ -54,6 +54,21 @@ def test_tile_splits(B, NH, S, DHQK, DHHV, dtype):
     check(run_cuda_fwbw(inp, 128, dtype), run_oracle_fwbw(inp, math.gcd(S, 128), dtype), 2e-2)
 
 
+@pytest.mark.parametrize("DHQK, DHHV", [(64, 512), (40, 384), (64, 1024)])
+@pytest.mark.parametrize("siging", [False, True])
+def test_one_operand_slice_and_several_output_tiles(DHQK, DHHV, siging):
+    """A head dim of one 64-column slice in a launch that fills the GPU: a CTA takes three or four output tiles, with two
+    loads each.  Two of the 32 units against the oracle; bounds as in the other 16-bit parity tests."""
+    B, NH, S, units = 2, 16, 1344, (3, 30)
+    inp = case_inputs(DHQK + DHHV, B, NH, S, DHQK, DHHV)
+    got = run_cuda_fwbw(inp, 128, torch.bfloat16, siging=siging)
+    one = {k: v.reshape(1, B * NH, *v.shape[2:])[:, list(units)] if v is not None and v.ndim >= 3 else v for k, v in inp.items()}
+    ref = run_oracle_fwbw(one, 64, torch.bfloat16, siging=siging)
+    for key in ("H", "dQ", "dK", "dV", "dI", "dF"):
+        x = got[key].reshape(1, B * NH, *got[key].shape[2:])[:, list(units)]
+        assert max_rel_err(x, ref[key]) < 2e-2, key
+
+
 @pytest.mark.parametrize("B, NH, DHQK, DHHV", [(1, 1, 8, 8), (1, 3, 100, 36), (1, 5, 512, 28), (4, 9, 256, 68), (6, 16, 128, 100), (40, 9, 64, 64)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_step_slices(B, NH, DHQK, DHHV, dtype):

@@ -58,7 +58,8 @@ class Bar:
         return passes
 
 
-def run(NC, do_n, store_states, seed, stages, decay_writer="issuing lane"):
+def run(NC, do_n, store_states, seed, stages, decay_writer="issuing lane", slow=None):
+    """slow: a role that gets its turn late."""
     rnd = random.Random(seed)
     NH2 = 2 * NC
     B = {}
@@ -172,7 +173,7 @@ def run(NC, do_n, store_states, seed, stages, decay_writer="issuing lane"):
     if do_n:
         agents["n"] = n_warp()
     clocks.update({a: {} for a in [*agents, "prod other lane"]})
-    blocked, alive = {}, set(agents)
+    blocked, alive = {}, dict.fromkeys(agents)    # (in a fixed order: a run depends on its seed alone)
 
     def acquire(a, bar, phase):
         if phase < 0:
@@ -187,6 +188,8 @@ def run(NC, do_n, store_states, seed, stages, decay_writer="issuing lane"):
         if commits:
             choices.append(("commit", None))
         rnd.shuffle(choices)
+        if slow is not None and rnd.random() < 0.95:
+            choices.sort(key=lambda c: c[1] == slow)
         progressed = False
         for kind, a in choices:
             if kind == "load":
@@ -208,7 +211,7 @@ def run(NC, do_n, store_states, seed, stages, decay_writer="issuing lane"):
             try:
                 op = next(agents[a])
             except StopIteration:
-                alive.discard(a)
+                del alive[a]
                 progressed = True
                 break
             if op[0] == "wait":
@@ -231,6 +234,14 @@ DEPTHS = ring_depths()
 def test_recurrence_protocol_has_no_aliasing_deadlock_or_over_arrival(NC, do_n, store_states, stages):
     for seed in range(25):
         run(NC, do_n, store_states, seed, stages)
+
+
+@pytest.mark.parametrize("slow", ["prod", "mma", "gate0", "gate5", "state0", "state7", "store", "n"])
+@pytest.mark.parametrize("stages", DEPTHS)
+def test_a_role_that_falls_behind_meets_no_barrier_two_phases_on(stages, slow):
+    for seed in range(20):
+        run(12, True, True, seed, stages, slow=slow)
+        run(12, False, True, seed, stages, slow=slow)
 
 
 @pytest.mark.parametrize("stages", [5, 7])
