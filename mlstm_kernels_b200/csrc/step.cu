@@ -171,8 +171,8 @@ step_kernel(const T* q, const T* k, const T* v, const void* gi, const void* gf, 
 // three barriers per block), the token loop itself runs on registers and broadcast shared-memory reads without a
 // barrier, and the partial h of the block's tokens are summed over the warps together.  Token by token with five
 // barriers and a load latency each it took 4.3 us per token (4 sequences x 13 tokens, 8 heads 256/512: 56.5 us, of which
-// the state traffic is 5.3); in blocks 24.3 us.  Bound by latency: a block's loads, preparation, token loop and reduction
-// follow one another (the multiply-adds of 13 tokens are 5 us of issue slots; no unit of the SM is busier than 22 %).
+// the state traffic is 5.3); in blocks 24.1 us.  Bound by latency: a block's loads, preparation, token loop and reduction
+// follow one another (issue slots 42 % busy, the FMA pipe 26 %, memory less).
 constexpr int SEQ_TB = 8;
 
 template <typename T, int ROWS, int TV>
