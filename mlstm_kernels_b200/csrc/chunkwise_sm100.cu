@@ -7,13 +7,13 @@
 //                    (gated left)^T x right contraction on the tensor cores into a double-buffered TMEM
 //                    accumulator, decay + accumulate of the running state in registers, bf16 state store.
 //                    mlstm_kernels/triton/chunkwise/xl_chunk/fw_kernel_recurrent.py:14-230, bw_kernel_recurrent.py:15-181
-//   par_body         intra-chunk kernel (par_fw_sm100, par_bw_sm100) for H, deltaV, deltaK, deltaQ.  Per (batch, head, chunk, 128-wide output tile):
+//   par_body         intra-chunk kernel of the forward (par_fw_sm100, par_fw_range_sm100).  Per (batch, head, chunk, 128-wide output tile):
 //                    score = A B^T (TMEM) -> gate matrix applied by the CUDA cores, bf16 result written back to
 //                    TMEM and used as the A operand of score x X; the inter-chunk term A x state is accumulated
 //                    into the same TMEM tile first and row-scaled in place.  The L x L gate matrix never
 //                    leaves the SM.
-//                    fw_kernel_parallel.py:14-289, bw_kernel_parallel_dV.py, bw_kernel_parallel_dK.py, bw_kernel_parallel_dQ.py
-// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four or six half-chunk stages in the recurrence, three stages in the intra-chunk kernels); one warp produces,
+//                    fw_kernel_parallel.py:14-289
+// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four or six half-chunk stages in the recurrence, three stages in the intra-chunk kernel); one warp produces,
 // one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded
 // and a lane whose wait has run out keeps its warp company to the end of the role, without arriving anywhere: see warp_arrive.
 #include <algorithm>
@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "launch.cuh"
 #include "sm100.cuh"
+#include "tensor_maps.cuh"
 
 namespace mlstm {
 
@@ -380,16 +381,9 @@ rec_pair_sm100(const __grid_constant__ CUtensorMap mL, const __grid_constant__ C
 
 // =====================================================================================================
 // Intra-chunk kernel.  Output tile rows r = tokens of one chunk, 128 output columns.
-//   out[r,:] = sum_c G[r,c] X[c,:] + rowscale_r * (A[r,:] . State)
-//   G[r,c]   = gate(r,c) * (A[r,:] . B[c,:])
-//   mode  A    B    contraction  gate   X    State operand                  rowscale            out
-//   H     Q    K    DHQK         lower  V    C_k        [DHQK x DHHV]       s*bbar_r            H (divided by den)
-//   DV    K    Q    DHQK         upper  dH   dC_{k+1}   [DHQK x DHHV]       abar_r              dV
-//   DK    V    dH   DHHV         upper  Q    dC_{k+1}^T (rows d, cols e)    abar_r              dK
-//   DQ    dH   V    DHHV         lower  K    C_k^T      (rows d, cols e)    s*bbar_r/(den_r+e)  dQ
-// lower: c <= r, (i,j) = (r,c); upper: c >= r, (i,j) = (c,r);
-// gate = s * exp((b_i - b_j) + iota_j - m_i) [* 1/(den_i+eps) in the three backward modes].
-// grid (ceil(DO / 128 / PAR_MAXSUB), NC, B*NH), two CTAs per SM; 320 threads: warp 0 TMA, warp 1 MMA, warps 2..9
+//   H[r,:] = (sum_{c <= r} G[r,c] V[c,:] + s * bbar_r * (Q[r,:] . C_k)) / (den_r + eps)
+//   G[r,c] = gate(r,c) * (Q[r,:] . K[c,:]),   gate = s * exp((b_r - b_c) + iota_c - m_r)
+// grid (ceil(DHHV / 128 / PAR_MAXSUB), NC, B*NH), two CTAs per SM; 320 threads: warp 0 TMA, warp 1 MMA, warps 2..9
 // element-wise (two warps per 32-row quarter of the tile, each owning two 32-column chunks).  One CTA produces up to
 // PAR_MAXSUB neighbouring output tiles of its chunk and mode, one after the other, from a single score tile.
 // Time line of a CTA's first tile (measured with time stamps at the benchmark size, two CTAs sharing an SM): first
@@ -398,16 +392,12 @@ rec_pair_sm100(const __grid_constant__ CUtensorMap mL, const __grid_constant__ C
 // Within a tile the kernel is bound by this chain of dependent steps (the same kernel with every operand resident in
 // L2 runs at the same speed); the forward kernel as a whole runs at the HBM copy bandwidth.
 // =====================================================================================================
-enum { PM_H = 0, PM_DV = 1, PM_DK = 2, PM_DQ = 3 };
-
 struct ParParams {
-  const float *vecB, *iota, *m_tok, *abar, *bbar, *inv_den;  // per token, f32
-  const float* n_states;                                     // H only
-  uint16_t *out_h, *out_dv, *out_dk, *out_dq;   // 16-bit elements of the input type
-  float* n_out;               // H only: denominator per token, or nullptr
-  float* inv_den_out;         // H only: 1 / (denominator + eps) per slot (0 past the sequence end), or nullptr
-  float *rowdot_q, *rowdot_k; // sum_d q dq (from DQ), sum_d k dk (from DK); one partial per output tile: [DHQK/128][tokens]
-  size_t nslots;              // B * NH * SP
+  const float *vecB, *iota, *m_tok, *bbar;   // per token, f32
+  const float* n_states;
+  uint16_t* out_h;            // 16-bit elements of the input type
+  float* n_out;               // denominator per token, or nullptr
+  float* inv_den_out;         // 1 / (denominator + eps) per slot (0 past the sequence end), or nullptr
   int S, SP, NC, DHQK, DHHV, variant;   // SP = NC * 128: slots per (batch, head) of the per-token gate vectors
   float eps, qk_scale;
   int bh0;                    // first (batch, head) unit of this launch
@@ -423,7 +413,7 @@ constexpr int PAR_SMEM = PAR_NST * PAR_STAGE + 1024;
 
 // Shared-memory control block of one intra-chunk CTA (the operand ring lives in dynamic shared memory).
 struct ParShared {
-  uint64_t bar_full[PAR_NST], bar_empty[PAR_NST], bar_qdone[PAR_NST], bar_sfull, bar_afull, bar_gated, bar_hfull, bar_accfree, bar_done[2], bar_dot,
+  uint64_t bar_full[PAR_NST], bar_empty[PAR_NST], bar_qdone[PAR_NST], bar_sfull, bar_afull, bar_gated, bar_hfull, bar_accfree, bar_done[2],
       bar_pair[4], bar_out;
   uint32_t tmem;
   int issued;                      // loads the producer has issued
@@ -436,60 +426,51 @@ struct ParShared {
   float s_n[512];
 };
 
-// One body for the four modes; `mode` is uniform over the CTA, so every branch on it is uniform (a single copy of the
-// code keeps the instruction cache warm when CTAs of different modes share an SM).
-// Gate factor of element (r, c): 2^(rowE_r + colE_c), every positive factor folded into the exponent:
-//   lower (H, DQ), valid c <= r:  rowE = (b_r - m_r) log2e + log2(s [/(den_r+eps)]),   colE = (iota_c - b_c) log2e
-//   upper (DV, DK), valid c >= r: rowE = (iota_r - b_r) log2e + log2(s),               colE = (b_c - m_c) log2e - log2(den_c+eps)
+// Gate factor of element (r, c), c <= r: 2^(rowE_r + colE_c), every positive factor folded into the exponent:
+//   rowE = (b_r - m_r) log2e + log2(s),   colE = (iota_c - b_c) log2e
 // A 32 x 32 block off the diagonal is gated without a transcendental per element: with colP = the largest colE of
 // the block's columns, 2^(rowE_r + colE_c) = 2^(rowE_r + colP) * 2^(colE_c - colP); the column factors (one ex2 per
 // column and CTA) lie in (0, 1], and the row factor (one ex2 per row and block) cannot overflow because every
-// element of an off-diagonal block is a valid gate entry, bounded by s / (den + eps).  Where a column factor
+// element of an off-diagonal block is a valid gate entry, bounded by s.  Where a column factor
 // underflows the exact value is below 2^-100 as well.  The diagonal block keeps the exact per-element form (its
 // masked columns may carry arbitrarily large colE).  The special-function unit (16 results per clock and SM) was
 // the limit of the gating phase before: the warps of the busiest row quarter share one SM sub-partition.
-// LOOP: the CTA runs the body again for another chunk afterwards (H only): it keeps its tensor memory from the first run
+// LOOP: the CTA runs the body again for another chunk afterwards: it keeps its tensor memory from the first run
 // to the last, and leaves each run with no arrival on any barrier outstanding, so that the next one can set them up anew.
 // Returns false after a run in which a wait ran out: its copies may still be on their way to barriers of that run.
 template <bool F16, bool LOOP = false>
 __device__ __forceinline__ bool
-par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* mapX,
-         const CUtensorMap* mapSt, const CUtensorMap* mapE, const ParParams& p,
+par_body(const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* mapX, const CUtensorMap* mapSt, const ParParams& p,
          ParShared& sh, const int o_tile0, const int nsub, const int ck, const int bh, const bool first_run = true,
          const bool last_run = true) {
-  const bool LOWER = (mode == PM_H || mode == PM_DQ);
-  const bool ST_MN = (mode == PM_H || mode == PM_DV);  // state operand N-contiguous in shared memory
-  const bool HAS_E = (mode == PM_DQ || mode == PM_DK);  // extra tile for the gate-gradient row sums
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int o00 = o_tile0 * 128;   // first output column of the CTA's first tile
-  const int DI = (mode == PM_H || mode == PM_DV) ? p.DHQK : p.DHHV;   // contraction dim of the score product
-  const int DO = (mode == PM_H || mode == PM_DV) ? p.DHHV : p.DHQK;   // output width
-  const int NC = p.NC, ND = (DI + 63) / 64;   // slices of 64 columns; a last partial slice is padded with zeros by TMA
+  const int DO = p.DHHV;                      // output width
+  const int NC = p.NC, ND = (p.DHQK + 63) / 64;   // slices of 64 columns; a last partial slice is padded with zeros by TMA
   const int y0 = ck * CL;                         // first token of the chunk inside its sequence
   const int valid = min(CL, p.S - y0);            // tokens of the chunk that exist (ragged last chunk: < 128)
   const size_t out_row0 = (size_t)bh * p.S + y0;  // first row of the chunk in the (B*NH*S)-row token tensors
-  const bool use_n = (mode == PM_H) && p.variant != MLSTM_SIG_NONORM && p.n_states != nullptr;
+  const bool use_n = p.variant != MLSTM_SIG_NONORM && p.n_states != nullptr;
 
   if (tid == 0) {
     if (LOOP && !first_run) {
       for (int s = 0; s < PAR_NST; ++s) { mbar_inval(&sh.bar_full[s]); mbar_inval(&sh.bar_empty[s]); mbar_inval(&sh.bar_qdone[s]); }
       for (int s = 0; s < 4; ++s) mbar_inval(&sh.bar_pair[s]);
-      mbar_inval(&sh.bar_sfull); mbar_inval(&sh.bar_afull); mbar_inval(&sh.bar_gated); mbar_inval(&sh.bar_hfull); mbar_inval(&sh.bar_dot);
+      mbar_inval(&sh.bar_sfull); mbar_inval(&sh.bar_afull); mbar_inval(&sh.bar_gated); mbar_inval(&sh.bar_hfull);
       mbar_inval(&sh.bar_out); mbar_inval(&sh.bar_accfree); mbar_inval(&sh.bar_done[0]); mbar_inval(&sh.bar_done[1]);
     }
     sh.abort = 0; sh.issued = 0;
     for (int s = 0; s < PAR_NST; ++s) {
       mbar_init(&sh.bar_full[s], 1); mbar_init(&sh.bar_empty[s], 1); mbar_init(&sh.bar_qdone[s], 8);
     }
-    mbar_init(&sh.bar_sfull, 1); mbar_init(&sh.bar_afull, 1); mbar_init(&sh.bar_gated, 256); mbar_init(&sh.bar_hfull, 1); mbar_init(&sh.bar_dot, 256);
+    mbar_init(&sh.bar_sfull, 1); mbar_init(&sh.bar_afull, 1); mbar_init(&sh.bar_gated, 256); mbar_init(&sh.bar_hfull, 1);
     for (int s = 0; s < 4; ++s) mbar_init(&sh.bar_pair[s], 64);
     mbar_init(&sh.bar_out, 256); mbar_init(&sh.bar_accfree, 256); mbar_init(&sh.bar_done[0], 256); mbar_init(&sh.bar_done[1], 256);
     fence_barrier_init();
     tma_prefetch_desc(mapA); tma_prefetch_desc(mapB); tma_prefetch_desc(mapX); tma_prefetch_desc(mapSt);
-    if (HAS_E) tma_prefetch_desc(mapE);
   }
   if (warp == 1 && (!LOOP || first_run)) { tmem_alloc(&sh.tmem, 256); tmem_relinquish(); }
   tc_fence_before_sync();
@@ -500,30 +481,29 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
   pdl_launch_dependents();
   pdl_wait();
   // Ring loads, in order: ND (A, B) slice pairs for the score product, ND (A, state) slice pairs for the inter-chunk
-  // product (A comes from L2 the second time), the X tile, the E tile.  The score is complete - and the element-wise
+  // product (A comes from L2 the second time), the X tile.  The score is complete - and the element-wise
   // warps start gating - while the second group is still arriving.
   // A CTA produces `nsub` (1 .. PAR_MAXSUB) neighbouring 128-column output tiles of the same chunk and mode.  The
   // score tile and its gated form are the same for all of them, so every tile after the first only needs its own
-  // state slices, X and E tiles: the gated tile stays in tensor memory, the accumulator is reused once the previous
+  // state slices and X tile: the gated tile stays in tensor memory, the accumulator is reused once the previous
   // tile's epilogue has read it.
-  const int n0 = 2 * ND + 1 + (HAS_E ? 1 : 0);          // loads of the first tile
-  const int n1 = ND + 1 + (HAS_E ? 1 : 0);              // loads of every further tile
+  const int n0 = 2 * ND + 1;          // loads of the first tile
+  const int n1 = ND + 1;              // loads of every further tile
   const int n_loads = n0 + (nsub - 1) * n1;
-  enum { LK_SCORE = 0, LK_STATE = 1, LK_X = 2, LK_E = 3 };
+  enum { LK_SCORE = 0, LK_STATE = 1, LK_X = 2 };
   // kind of the load at position l of tile `sub` (no divisions: this runs on the load-issue path)
   auto load_kind = [&](int sub, int l, int& it) -> int {
     if (sub == 0 && l < ND) { it = l; return LK_SCORE; }
     const int ls = l - (sub == 0 ? ND : 0);
     if (ls < ND) { it = ls; return LK_STATE; }
     it = 0;
-    return ls == ND ? LK_X : LK_E;
+    return LK_X;
   };
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (elect_one()) {
-      const int slot = LOWER ? ck : ck + 1;
-      const int sz = bh * (NC + 1) + slot;   // slab of the state tensor (one DHQK x DHHV matrix per chunk boundary)
+      const int sz = bh * (NC + 1) + ck;   // slab of the state tensor (one DHQK x DHHV matrix per chunk boundary)
       int issued = 0;
       // Per stage: uses handed back by an MMA commit so far (phase counter of bar_empty) and score pairs read for
       // q . n so far (phase counter of bar_qdone).  Scalars picked by comparisons, not arrays: a dynamically indexed
@@ -538,7 +518,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         if (ld >= PAR_NST) {   // the stage's previous occupant (three loads back) must be gone
           const int pkind = pk3, psub = ps3;
           bool okw;
-          if (pkind == LK_SCORE || pkind == LK_STATE || (pkind == LK_X && HAS_E)) {
+          if (pkind == LK_SCORE || pkind == LK_STATE) {
             const int rm = st == 0 ? rm0 : (st == 1 ? rm1 : rm2);
             okw = mbar_wait(&sh.bar_empty[st], (rm - 1) & 1, &sh.abort, &g_sm100_status, 201);
             // the element-wise warps read the A box of a score pair (q . n)
@@ -547,8 +527,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
               okw = mbar_wait(&sh.bar_qdone[st], (rq - 1) & 1, &sh.abort, &g_sm100_status, 212);
             }
           } else {
-            // The staging buffer of a tile (its E stage, or its X stage in the modes without E) is handed back when the tile
-            // has been stored.  Two barriers, for every other tile: with one operand slice (DHQK <= 64) a tile's loads are two
+            // The staging buffer of a tile (its X stage) is handed back when the tile has been stored.  Two barriers, for every other tile: with one operand slice (DHQK <= 64) a tile's loads are two
             // and the ring holds three, so that the next tile, too, can be done before this wait looks.
             okw = mbar_wait(&sh.bar_done[psub & 1], (psub >> 1) & 1, &sh.abort, &g_sm100_status, 215);
           }
@@ -562,18 +541,13 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
           tma_load_3d(sb + 16384, mapB, &sh.bar_full[st], 64 * it, y0, bh);
         } else if (kind == LK_STATE) {
           tma_load_3d(sb, mapA, &sh.bar_full[st], 64 * it, y0, bh);
-          if (ST_MN) {
-            tma_load_3d(sb + 16384, mapSt, &sh.bar_full[st], o0, 64 * it, sz);
-            tma_load_3d(sb + 16384 + 8192, mapSt, &sh.bar_full[st], o0 + 64, 64 * it, sz);
-          } else {
-            tma_load_3d(sb + 16384, mapSt, &sh.bar_full[st], 64 * it, o0, sz);
-          }
+          tma_load_3d(sb + 16384, mapSt, &sh.bar_full[st], o0, 64 * it, sz);
+          tma_load_3d(sb + 16384 + 8192, mapSt, &sh.bar_full[st], o0 + 64, 64 * it, sz);
         } else {
-          const CUtensorMap* m = (kind == LK_X) ? mapX : mapE;
-          tma_load_3d(sb, m, &sh.bar_full[st], o0, y0, bh);
-          tma_load_3d(sb + 16384, m, &sh.bar_full[st], o0 + 64, y0, bh);
+          tma_load_3d(sb, mapX, &sh.bar_full[st], o0, y0, bh);
+          tma_load_3d(sb + 16384, mapX, &sh.bar_full[st], o0 + 64, y0, bh);
         }
-        if (kind == LK_SCORE || kind == LK_STATE || (kind == LK_X && HAS_E)) { rm0 += (st == 0); rm1 += (st == 1); rm2 += (st == 2); }
+        if (kind == LK_SCORE || kind == LK_STATE) { rm0 += (st == 0); rm1 += (st == 1); rm2 += (st == 2); }
         if (kind == LK_SCORE) { rq0 += (st == 0); rq1 += (st == 1); rq2 += (st == 2); }
         issued = ld + 1;
         pk3 = pk2; pk2 = pk1; pk1 = kind; ps3 = ps2; ps2 = ps1; ps1 = sub;
@@ -591,7 +565,6 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_16(F16, 128, 128, 0, 0);
-      const uint32_t idesc_st = ST_MN ? umma_idesc_16(F16, 128, 128, 0, 1) : umma_idesc_16(F16, 128, 128, 0, 0);
       constexpr uint32_t idesc_x = umma_idesc_16(F16, 128, 128, 0, 1);
       bool ok = true;
       for (int ld = 0; ld < ND; ++ld) {            // score: S = A . B^T
@@ -618,8 +591,8 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
           const uint32_t sa = smem_u32(smem + st * PAR_STAGE), ss = sa + 16384;
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
-            const uint64_t bdesc = ST_MN ? umma_desc_sw128(ss + kk * 2048, 8192, 1024) : umma_desc_sw128(ss + kk * 32, 16, 1024);
-            umma_ss(tAcc, umma_desc_sw128(sa + kk * 32, 16, 1024), bdesc, idesc_st, (it > 0 || kk > 0) ? 1u : 0u);
+            umma_ss(tAcc, umma_desc_sw128(sa + kk * 32, 16, 1024), umma_desc_sw128(ss + kk * 2048, 8192, 1024), idesc_x,
+                    (it > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&sh.bar_empty[st]);
         }
@@ -634,7 +607,6 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           umma_ts(tAcc, tS + kk * 8, umma_desc_sw128(sx + kk * 2048, 16384, 1024), idesc_x, 1u);
-        if (HAS_E) umma_commit(&sh.bar_empty[stx]);   // the output is staged in the E stage: X's stage is free again
         umma_commit(&sh.bar_hfull);
       }
     }
@@ -644,12 +616,10 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     const int r = quarter * 32 + lane;
     const size_t tok = (size_t)bh * p.SP + y0 + r;   // slot of this row in the per-token gate vectors
     const float b_r = p.vecB[tok], iota_r = p.iota[tok], m_r = p.m_tok[tok];
-    const float inv_r = (mode == PM_H) ? 1.f : p.inv_den[tok];
     constexpr float kLog2e = 1.4426950408889634f;
-    const float rowE = (LOWER ? (b_r - m_r) : (iota_r - b_r)) * kLog2e +
-                       __log2f((mode == PM_DQ) ? p.qk_scale * inv_r : p.qk_scale);
+    const float rowE = (b_r - m_r) * kLog2e + __log2f(p.qk_scale);
     if (half == 0) {   // this thread's row in its role as a column of the gate matrix
-      const float colE = LOWER ? (iota_r - b_r) * kLog2e : (b_r - m_r) * kLog2e + __log2f(inv_r);
+      const float colE = (iota_r - b_r) * kLog2e;
       float colP = colE;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) colP = fmaxf(colP, __shfl_xor_sync(0xffffffffu, colP, o));
@@ -658,17 +628,14 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       sh.s_colF[r] = ex2_approx(colE - colP);
       if (lane == 0) sh.s_colP[quarter] = colP;
     }
-    float rowscale;
-    if (mode == PM_H) rowscale = p.qk_scale * p.bbar[tok];
-    else if (mode == PM_DQ) rowscale = p.qk_scale * p.bbar[tok] * inv_r;
-    else rowscale = p.abar[tok];
+    const float rowscale = p.qk_scale * p.bbar[tok];
     if (use_n) {
       const float* nsrc = p.n_states + ((size_t)bh * (NC + 1) + ck) * p.DHQK;
       for (int dd = tid - 64; dd < ND * 64; dd += 256) sh.s_n[dd] = dd < p.DHQK ? nsrc[dd] : 0.f;   // zero padding
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");  // gate vectors and n visible to the element-wise warps
 
-    // q . n_{k-1} for the denominator (H only): each thread reads half of its row of every Q slice from the
+    // q . n_{k-1} for the denominator: each thread reads half of its row of every Q slice from the
     // TMA stage (the stage is released to the producer only after these reads)
     float qn = 0.f;
     if (use_n) {
@@ -713,7 +680,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
     for (int u = 0; u < 2; ++u) {
       const int cq = half + 2 * u;
       const int c0 = cq * 32;
-      const bool skip = LOWER ? (cq > quarter) : (cq < quarter);
+      const bool skip = cq > quarter;
       if (skip) {
 #pragma unroll
         for (int c = 0; c < 16; ++c) pk[u][c] = 0u;
@@ -738,7 +705,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
               for (int e = 0; e < 4; ++e) {
                 const int cl = 16 * hh + 4 * c4 + e;   // column inside the chunk; row inside the chunk is `lane`
                 float val = __uint_as_float(v[4 * c4 + e]) * ex2_approx(rowE + ee[e]);
-                if (LOWER ? (cl > lane) : (cl < lane)) val = 0.f;
+                if (cl > lane) val = 0.f;
                 g4[e] = val;
                 rowsum += val;
               }
@@ -800,7 +767,7 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
       if (acc_ok) mbar_arrive(&sh.bar_gated);   // (first tile: the gated score tile is in place as well)
       mbar_wait(&sh.bar_hfull, sub & 1, &sh.abort, &g_sm100_status, 206);
       tc_fence_after_sync();
-      if (sub == 0 && mode == PM_H) {
+      if (sub == 0) {
         float den = 1.f;
         const float nn = (sh.s_part[0][r] + sh.s_part[1][r]) + rowscale * (use_n ? (sh.s_qn[0][r] + sh.s_qn[1][r]) : 0.f);
         if (p.variant == MLSTM_EXP) den = fmaxf(fabsf(nn), __expf(-m_r));
@@ -811,21 +778,12 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
           if (p.inv_den_out != nullptr) p.inv_den_out[tok] = r < valid ? inv : 0.f;
         }
       }
-      const int ldx = (sub == 0 ? 2 * ND : n0 + (sub - 1) * n1 + ND);    // ring index of this tile's X load; E follows it
-      const uint8_t* erow = smem;
-      if (HAS_E) {
-        const int lde = ldx + 1, ste = lde % PAR_NST;
-        mbar_wait(&sh.bar_full[ste], (lde / PAR_NST) & 1, &sh.abort, &g_sm100_status, 208);
-        erow = smem + ste * PAR_STAGE + r * 128;
-      }
-      float dot4[4] = {0.f, 0.f, 0.f, 0.f};   // four partial sums: no 64-long chain of dependent FMAs
+      const int ldx = (sub == 0 ? 2 * ND : n0 + (sub - 1) * n1 + ND);    // ring index of this tile's X load
       // The output tile is staged (bf16, two boxes of 128 rows x 128 bytes, 16-byte pieces XOR-swizzled by the row)
-      // in the ring stage of the E tile - which arrives in exactly this layout, so a thread reads its E piece and
-      // writes its output piece to the same 16 bytes - or, in the modes without E, in the stage the X tile occupied
-      // (every MMA that read it has completed).  It is then written out by all element-wise warps together, each warp
-      // instruction covering two full 256-byte rows of the tile.  Plain stores are posted, so the CTA retires without
-      // waiting for them.
-      uint8_t* ostage = smem + ((ldx + (HAS_E ? 1 : 0)) % PAR_NST) * PAR_STAGE;
+      // in the ring stage the X tile occupied (every MMA that read it has completed).  It is then written out by all element-wise
+      // warps together, each warp instruction covering two full 256-byte rows of the tile.  Plain stores are posted, so the CTA
+      // retires without waiting for them.
+      uint8_t* ostage = smem + (ldx % PAR_NST) * PAR_STAGE;
 #pragma unroll 1
       for (int cq = half; cq < 4; cq += 2) {
         uint32_t va[16], vb[16];
@@ -842,17 +800,6 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
 #pragma unroll
           for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[8 * (c & 1) + e]) * inv;
           const int sw = (((cq & 1) * 4 + c) ^ (r & 7)) << 4;   // 16-byte chunk (cq*4 + c) of the row, swizzled
-          if (HAS_E) {
-            const uint4 ev = *reinterpret_cast<const uint4*>(erow + (cq >> 1) * 16384 + sw);
-            const uint32_t w[4] = {ev.x, ev.y, ev.z, ev.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float lo, hi;
-              Pair16<F16>::unpack(w[e], lo, hi);
-              dot4[e] = fmaf(lo, x[2 * e], dot4[e]);
-              dot4[e] = fmaf(hi, x[2 * e + 1], dot4[e]);
-            }
-          }
           uint4 o;
           o.x = Pair16<F16>::pack(x[0], x[1]); o.y = Pair16<F16>::pack(x[2], x[3]);
           o.z = Pair16<F16>::pack(x[4], x[5]); o.w = Pair16<F16>::pack(x[6], x[7]);
@@ -863,26 +810,16 @@ par_body(const int mode, const CUtensorMap* mapA, const CUtensorMap* mapB, const
         tc_fence_before_sync();
         if (!aborted(smem_u32(&sh.abort))) mbar_arrive(&sh.bar_accfree);
       }
-      const float dot = (dot4[0] + dot4[1]) + (dot4[2] + dot4[3]);
       mbar_arrive(&sh.bar_out);
       mbar_wait(&sh.bar_out, sub & 1, &sh.abort, &g_sm100_status, 211);
       {
-        uint16_t* outp = (mode == PM_H) ? p.out_h : (mode == PM_DV) ? p.out_dv : (mode == PM_DK) ? p.out_dk : p.out_dq;
-        uint8_t* gbase = reinterpret_cast<uint8_t*>(outp + out_row0 * DO + o0);
+        uint8_t* gbase = reinterpret_cast<uint8_t*>(p.out_h + out_row0 * DO + o0);
         const int ew = warp - 2, j = lane & 15;          // 16-byte piece j of the 256-byte tile row
 #pragma unroll
         for (int i2 = 0; i2 < 8; ++i2) {
           const int orow_i = 16 * i2 + 2 * ew + (lane >> 4);
           const uint4 o = *reinterpret_cast<const uint4*>(ostage + (j >> 3) * 16384 + orow_i * 128 + (((j & 7) ^ (orow_i & 7)) << 4));
           if (orow_i < valid && o0 + j * 8 < DO) *reinterpret_cast<uint4*>(gbase + (size_t)orow_i * DO * 2 + j * 16) = o;
-        }
-      }
-      if (HAS_E) {
-        sh.s_qn[half][r] = dot;
-        mbar_arrive(&sh.bar_dot);
-        if (half == 0) {
-          mbar_wait(&sh.bar_dot, sub & 1, &sh.abort, &g_sm100_status, 209);
-          ((mode == PM_DQ) ? p.rowdot_q : p.rowdot_k)[(size_t)(o_tile0 + sub) * p.nslots + tok] = sh.s_qn[0][r] + sh.s_qn[1][r];
         }
       }
       if (sub + 1 < nsub) {
@@ -918,7 +855,7 @@ par_fw_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUt
   const int gx = (T + p.maxsub - 1) / p.maxsub;
   const int x = blockIdx.x % gx, ck = p.ck0 + (blockIdx.x / gx) % p.n_ck, bh = p.bh0 + blockIdx.x / (gx * p.n_ck);
   const int t0 = p.maxsub * x;
-  par_body<F16>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(p.maxsub, T - t0), ck, bh);
+  par_body<F16>(&mQ, &mK, &mV, &mC, p, sh, t0, min(p.maxsub, T - t0), ck, bh);
 }
 
 // The same for a range of chunks, beside the recurrence of the following chunks: one CTA per resident place on the SMs that
@@ -934,31 +871,8 @@ par_fw_range_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant
   for (unsigned w = blockIdx.x; w < n_items; w += gridDim.x) {
     const int x = w % gx, ck = p.ck0 + (w / gx) % p.n_ck, bh = p.bh0 + w / (gx * p.n_ck), t0 = p.maxsub * x;
     const bool last = w + gridDim.x >= n_items;
-    if (!par_body<F16, true>(PM_H, &mQ, &mK, &mV, &mC, &mV, p, sh, t0, min(p.maxsub, T - t0), ck, bh, w == blockIdx.x, last)) return;
+    if (!par_body<F16, true>(&mQ, &mK, &mV, &mC, p, sh, t0, min(p.maxsub, T - t0), ck, bh, w == blockIdx.x, last)) return;
   }
-}
-
-// deltaV, deltaK and deltaQ of one chunk in ONE launch: blockIdx.x enumerates the 128-wide output tiles of the three
-// results, so the CTAs that read the same q, k, v, deltaH and state tiles of a chunk are scheduled next to each other
-// and share them through L2 instead of re-reading them from HBM in three separate launches.
-template <bool F16>
-__global__ void __launch_bounds__(PAR_THREADS, 2)
-par_bw_sm100(const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mK,
-             const __grid_constant__ CUtensorMap mV, const __grid_constant__ CUtensorMap mDH,
-             const __grid_constant__ CUtensorMap mC_k, const __grid_constant__ CUtensorMap mdC_mn,
-             const __grid_constant__ CUtensorMap mdC_k,
-             const __grid_constant__ ParParams p) {
-  __shared__ ParShared sh;
-  const int T_dv = (p.DHHV + 127) / 128, T_dk = (p.DHQK + 127) / 128;   // output tiles per chunk of dV, and of dK / dQ
-  const int c_dv = (T_dv + p.maxsub - 1) / p.maxsub, c_dk = (T_dk + p.maxsub - 1) / p.maxsub;   // CTAs per mode
-  const int gx = c_dv + 2 * c_dk;   // 1-D grid in the order (mode and tile group, chunk, batch x head)
-  const int x = blockIdx.x % gx, ck = p.ck0 + (blockIdx.x / gx) % p.n_ck, bh = p.bh0 + blockIdx.x / (gx * p.n_ck);
-  int mode, pair, T;
-  const CUtensorMap *a, *b, *xm, *stm, *e;
-  if (x < c_dv) { mode = PM_DV; pair = x; T = T_dv; a = &mK; b = &mQ; xm = &mDH; stm = &mdC_mn; e = &mDH; }
-  else if (x < c_dv + c_dk) { mode = PM_DK; pair = x - c_dv; T = T_dk; a = &mV; b = &mDH; xm = &mQ; stm = &mdC_k; e = &mK; }
-  else { mode = PM_DQ; pair = x - c_dv - c_dk; T = T_dk; a = &mDH; b = &mV; xm = &mK; stm = &mC_k; e = &mQ; }
-  par_body<F16>(mode, a, b, xm, stm, e, p, sh, p.maxsub * pair, min(p.maxsub, T - p.maxsub * pair), ck, bh);
 }
 
 // =====================================================================================================
@@ -980,18 +894,6 @@ bool sm100_sizes_ok(int B, int NH, int S, int DHQK, int DHHV) {
   const uint64_t tiles = (uint64_t)((DHHV + 127) / 128 + 2 * ((DHQK + 127) / 128));
   return bnh * S < lim && bnh * (nc + 1) * DHQK < lim && bnh * nc * tiles < lim &&
          bnh * (uint64_t)((DHHV + 63) / 64) * ((DHQK + 127) / 128) < lim;
-}
-
-// cudaFuncSetAttribute once per kernel and device instead of on every call
-template <typename K>
-static int set_smem_once(K kern, int bytes, bool (&done)[64]) {
-  int dev = 0;
-  MLSTM_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !done[dev]) {
-    MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if (dev >= 0 && dev < 64) done[dev] = true;
-  }
-  return MLSTM_OK;
 }
 
 // Tensor maps depend only on (base pointer, rows, columns, box): a training loop calls with the same buffers over
@@ -1028,14 +930,10 @@ static bool cached_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t
   return true;
 }
 
-// token tensors (q, k, v, deltaH): one slab of S rows per (batch, head), so that a box hanging over the end of a
-// sequence (ragged last chunk) reads zeros instead of the next head's tokens
-static bool tok_map(CUtensorMap* m, const void* base, const ChunkwiseDims& d, int cols, int box_rows = 128) {
+bool tok_map(CUtensorMap* m, const void* base, const ChunkwiseDims& d, int cols, int box_rows) {
   return cached_map(m, base, (uint64_t)d.S, (uint64_t)cols, box_rows, 64, (uint64_t)d.B * d.NH, d.dtype == MLSTM_F16);
 }
-// per-chunk states: one slab of DHQK x DHHV per (batch, head, chunk boundary), so that a tile hanging over the edge of
-// a head dim reads zeros (and is clipped on the way out) instead of touching the next slab
-static bool state_map(CUtensorMap* m, const void* base, const ChunkwiseDims& d, int box_rows) {
+bool state_map(CUtensorMap* m, const void* base, const ChunkwiseDims& d, int box_rows) {
   return cached_map(m, base, (uint64_t)d.DHQK, (uint64_t)d.DHHV, box_rows, 64, (uint64_t)d.B * d.NH * (d.NC + 1),
                     d.dtype == MLSTM_F16);
 }
@@ -1152,9 +1050,7 @@ int sm100_recurrent_pair(const void* k, const void* v, const float* c_initial, v
 
 static ParParams base_params(const GateBuffers& gb, const ChunkwiseDims& d) {
   ParParams pp{};
-  pp.vecB = gb.vecB; pp.iota = gb.iota; pp.m_tok = gb.m_tok; pp.abar = gb.abar; pp.bbar = gb.bbar;
-  pp.inv_den = gb.inv_den;
-  pp.nslots = (size_t)d.B * d.NH * d.SP;
+  pp.vecB = gb.vecB; pp.iota = gb.iota; pp.m_tok = gb.m_tok; pp.bbar = gb.bbar;
   pp.S = d.S; pp.SP = d.SP; pp.NC = d.NC; pp.DHQK = d.DHQK; pp.DHHV = d.DHHV; pp.variant = d.variant; pp.eps = d.eps;
   pp.qk_scale = d.qk_scale;
   return pp;
@@ -1201,33 +1097,6 @@ int sm100_parallel_fw(const void* q, const void* k, const void* v, const GateBuf
   return launch_pdl(ur.overlap && grid <= pdl_max_ctas(), kern, grid, PAR_THREADS, PAR_SMEM, st, mQ, mK, mV, mC, pp);
 }
 
-int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
-                      const void* c_states, const void* dc_states, void* dq, void* dk, void* dv, float* qdq_parts,
-                      float* kdk_parts, const ChunkwiseDims& d, cudaStream_t st, UnitRange ur) {
-  const int units = ur.count < 0 ? d.B * d.NH - ur.first : ur.count;
-  if (units <= 0) return MLSTM_OK;
-  PhaseScope ps(PH_PAR_BW, st);
-  CUtensorMap mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k;
-  if (!tok_map(&mQ, q, d, d.DHQK) || !tok_map(&mK, k, d, d.DHQK) || !tok_map(&mV, v, d, d.DHHV) ||
-      !tok_map(&mDH, dh, d, d.DHHV) || !state_map(&mC_k, c_states, d, 128) || !state_map(&mdC_mn, dc_states, d, 64) ||
-      !state_map(&mdC_k, dc_states, d, 128))
-    return MLSTM_ERR_CUDA;
-  ParParams pp = base_params(gb, d);
-  pp.out_dv = (uint16_t*)dv; pp.out_dk = (uint16_t*)dk; pp.out_dq = (uint16_t*)dq;
-  pp.rowdot_q = qdq_parts; pp.rowdot_k = kdk_parts;
-  pp.bh0 = ur.first; pp.n_ck = d.NC;
-  const bool f16 = d.dtype == MLSTM_F16;
-  static bool attr_done[2][64] = {};
-  if (int rc = f16 ? set_smem_once(par_bw_sm100<true>, PAR_SMEM, attr_done[1])
-                   : set_smem_once(par_bw_sm100<false>, PAR_SMEM, attr_done[0])) return rc;
-  const int T_dv = (d.DHHV + 127) / 128, T_dk = (d.DHQK + 127) / 128;
-  auto ctas = [&](int m) { return ((long)ceil_div(T_dv, m) + 2 * ceil_div(T_dk, m)) * d.NC * units; };
-  pp.maxsub = par_maxsub(ctas, std::max(T_dv, T_dk));
-  const unsigned grid = (unsigned)ctas(pp.maxsub);
-  return launch_pdl(ur.overlap && grid <= pdl_max_ctas(), f16 ? par_bw_sm100<true> : par_bw_sm100<false>, grid, PAR_THREADS, PAR_SMEM, st,
-                    mQ, mK, mV, mDH, mC_k, mdC_mn, mdC_k, pp);
-}
-
 // Self-test of the bounded wait: one thread waits, for at most `limit` polls, on an mbarrier that nothing arrives
 // at.  No copy is in flight and no tensor memory is held, so giving up is all that happens: the wait records
 // `code` in the status word and the kernel returns.
@@ -1268,7 +1137,10 @@ int sm100_device_status(int reset, int* status) {
     const int zero = 0;
     MLSTM_CUDA_CHECK(cudaMemcpyToSymbol(g_sm100_status, &zero, sizeof(int)));
   }
-  return MLSTM_OK;
+  int bw = 0;
+  const int rc = par_bw_status(reset, &bw);
+  if (*status == 0) *status = bw;
+  return rc;
 }
 
 }  // namespace mlstm

@@ -67,6 +67,7 @@ long sm100_recurrence_ctas(const ChunkwiseDims& d);
 int sm100_forward_segments(const ChunkwiseDims& d);
 
 int sm100_device_status(int reset, int* status);
+int par_bw_status(int reset, int* status);   // (the part of it that chunkwise_bw_sm100.cu keeps)
 int sm100_wait_expiry_selftest(unsigned limit, int code, cudaStream_t st);
 // make the runtime load the forward kernels' code on the current device now (CUDA loads modules lazily, on first use)
 int sm100_force_load();
