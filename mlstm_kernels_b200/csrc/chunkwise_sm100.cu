@@ -13,7 +13,7 @@
 //                    into the same TMEM tile first and row-scaled in place.  The L x L gate matrix never
 //                    leaves the SM.
 //                    fw_kernel_parallel.py:14-289
-// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (four or six half-chunk stages in the recurrence, three stages in the intra-chunk kernel); one warp produces,
+// Operands arrive by TMA (128-byte swizzle, no multicast) through mbarrier rings (half-chunk stages in the recurrence, three stages in the intra-chunk kernel); one warp produces,
 // one thread issues the MMAs, the remaining warps do the element-wise work.  Every wait is bounded
 // and a lane whose wait has run out keeps its warp company to the end of the role, without arriving anywhere: see warp_arrive.
 #include <algorithm>
@@ -51,25 +51,26 @@ struct RecParams {
   int ck0, n_ck;               // forward: first chunk and number of chunks of this launch (backward: all of them)
 };
 
-constexpr int REC_THREADS = 640;                 // warp 0 TMA, 1 MMA, 2..9 gate the left tile, 10..17 own the state, 18 stores it, 19 keeps n
+constexpr int REC_THREADS = 640;                 // warp 0 TMA (left), 1 MMA, 2..9 gate the left tile, 10..17 own the state, 18 stores it and keeps n, 19 TMA (right)
 constexpr int REC_HALF = 64;                     // tokens per ring stage: half a chunk
-constexpr int REC_NPART_BYTES = 2 * 32 * 128 * 4;   // double-buffered partial column sums of the gated left tile
-constexpr int rec_stage_bytes(int TN) { return 16384 + TN * 128; }    // 64 tokens: left tile 16 KB + right tile
+constexpr int REC_NPART_BYTES = 2 * 2 * 128 * 4; // column sums of the gated left tile, per half chunk, double-buffered
+constexpr int REC_LBUF = 8;                      // gated left tiles in tensor memory, 32 columns each
+constexpr int rec_right_bytes(int TN) { return TN * 128; }            // 64 tokens of the right operand (16 KB of the left one)
 constexpr int rec_out_bytes(int TN) { return TN * 256; }              // 16-bit state tile staged for the TMA store (two of them)
-// Operand ring depth.  A stage comes round in about 4600 cycles (load 2500, gating and hand-over 1300, MMA and hand-back
-// 800), so the 64-column form with its smaller stages runs three chunks ahead.  The depth is even, so that a stage always
-// goes to the same group of gating warps: a wait sees the parity of a phase only, and in an odd ring a group would come back
-// to a stage two phases later, where the load before the other group's last one passes for its own.  (The 64-column form
-// without n has room for a seventh stage, which measured the same: 4 x 4 x 1024, 96/192, the call 88.4 and 88.8 us.)
+// Depths of the two operand rings: a stage of the left operand goes back as soon as it has been gated, one of the right when
+// the product that reads it is done.  The left ring's depth is even, so that a stage always goes to the same group of gating
+// warps: a wait sees the parity of a phase only, and in an odd ring a group would come back to a stage two phases later, where
+// the load before the other group's last one passes for its own.  With 64-column tiles the right operand is small: both travel as
+// one stage, which saves the MMA thread a wait per half chunk (128 CTAs of 8 heads 256/512, 131072 tokens: 1096 us with two
+// rings, 973 with one; with 128-column tiles, 8 x 8192 tokens, 16 heads 256/256: 373 and 390).
 constexpr int rec_stages(int TN) { return TN == 128 ? 4 : 6; }
-constexpr int rec_smem_bytes(bool has_n, int TN) {
-  return rec_stages(TN) * rec_stage_bytes(TN) + (has_n ? REC_NPART_BYTES : 0) + 2 * rec_out_bytes(TN) + 1024;
-}
+constexpr int rec_right_stages(int TN) { return TN == 128 ? 5 : 6; }
+constexpr int rec_npart_offset(int TN) { return rec_stages(TN) * 16384 + rec_right_stages(TN) * rec_right_bytes(TN); }
+constexpr int rec_smem_bytes(bool has_n, int TN) { return rec_npart_offset(TN) + (has_n ? REC_NPART_BYTES : 0) + 2 * rec_out_bytes(TN) + 1024; }
 
-// One ring stage holds 64 tokens of the left and of the right operand (boxes of 64 rows x 64 columns, 8 KB each:
-// left columns d0.., d0+64.., right columns e0.., e0+64..).  A chunk is two stages; the product of a chunk is
-// accumulated over both before the state warps fold it in.  The ring is deeper than one chunk so that the load of
-// chunk s+2 is already in flight while chunk s is being gated and multiplied.
+// A stage holds 64 tokens of one operand (boxes of 64 rows x 64 columns, 8 KB each: left columns d0.., d0+64.., right
+// columns e0.., e0+64..).  A chunk is two stages of either; the product of a chunk is accumulated over both before the state
+// warps fold it in.
 // TN = columns of the state tile (128, or 64 for small problems: twice as many CTAs, so that a launch with few
 // (batch, head) units still covers the GPU).
 // F16: the 16-bit element type is IEEE half instead of bf16 (operands, gated tiles, stored states, outputs).
@@ -79,15 +80,21 @@ __device__ __forceinline__ void
 rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& mapS, const RecParams& p, const unsigned block) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int REC_STAGES = rec_stages(TN), REC_STAGE_BYTES = rec_stage_bytes(TN), REC_OUT = rec_out_bytes(TN);
+  constexpr int REC_STAGES = rec_stages(TN), RIGHT_STAGES = rec_right_stages(TN), RIGHT_BYTES = rec_right_bytes(TN), REC_OUT = rec_out_bytes(TN);
+  uint8_t* smem_r = smem + REC_STAGES * 16384;
+  constexpr int G_RING = 16;
+  constexpr bool JOINT = TN == 64;   // one ring: a stage holds both operands and is free when its product is done
+  static_assert(!JOINT || RIGHT_STAGES == REC_STAGES, "one ring");
   // (separate arrays: members of one shared struct cost 68 bytes of register spills in the 128-column forward)
-  __shared__ uint64_t bar_full[REC_STAGES], bar_empty[REC_STAGES], bar_scaled[REC_STAGES], bar_acc_full[2], bar_acc_free[2], bar_nsum[2],
+  __shared__ uint64_t bar_full[REC_STAGES], bar_empty[REC_STAGES], bar_rfull[RIGHT_STAGES],
+      bar_scaled[REC_LBUF], bar_done[REC_LBUF], bar_acc_free[2], bar_nsum[2],
       bar_nread[2], bar_out_full[2], bar_out_free[2];
+  // Decay of the chunk.  The thread that writes it is at most STAGES / 2 + REC_LBUF / 2 + 3 <= 10 chunks ahead of its last reader: ring of 16.
+  __shared__ float s_g[G_RING];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;   // set by the first wait of this CTA that runs out; every other wait polls it
   // per-row scale factors of the left tile, copied with the stage (backward: two factors per row)
   __shared__ __align__(16) float s_scale[REC_STAGES][REC_HALF], s_scale2[BWD ? REC_STAGES : 1][REC_HALF];
-  __shared__ float s_g[8];  // decay of the chunk, ring of eight (outlives the operand ring)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 1-D grid (no 65535 limit on batch x heads), state tiles of one (batch, head) next to each other
@@ -105,187 +112,227 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
 
   if (tid == 0) {
     s_abort = 0;
-    for (int s = 0; s < REC_STAGES; ++s) {
-      mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); mbar_init(&bar_scaled[s], 4);   // (arrivals once per warp)
-    }
+    for (int s = 0; s < REC_STAGES; ++s) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 4); }   // (arrivals once per warp)
+    for (int s = 0; s < RIGHT_STAGES; ++s) mbar_init(&bar_rfull[s], 1);
+    for (int s = 0; s < REC_LBUF; ++s) { mbar_init(&bar_scaled[s], 4); mbar_init(&bar_done[s], 1); }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&bar_acc_full[s], 1); mbar_init(&bar_acc_free[s], 8); mbar_init(&bar_nsum[s], 8); mbar_init(&bar_nread[s], 1);
+      mbar_init(&bar_acc_free[s], 8); mbar_init(&bar_nsum[s], 8); mbar_init(&bar_nread[s], 1);
       mbar_init(&bar_out_full[s], 8); mbar_init(&bar_out_free[s], 1);
     }
     fence_barrier_init();
     tma_prefetch_desc(&mapL); tma_prefetch_desc(&mapR); tma_prefetch_desc(&mapS);
   }
-  if (warp == 1) { tmem_alloc(&s_tmem, 256); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(&s_tmem, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = s_tmem;
+  // two accumulators of 128 columns, then the gated left tiles (64 tokens, 32 columns each)
+  const uint32_t tmem = s_tmem, tL = tmem + 256;
   pdl_launch_dependents();
   pdl_wait();
 
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    // The per-row scale vectors travel with the stage (bulk copies on the same barrier).  The decay of a chunk is a
-    // single float: the warp keeps the values of 32 consecutive steps in its lanes and fetches the next 32 a whole
-    // block ahead, so no global-memory latency sits between a stage becoming free and the next issue.
-    auto load_g = [&](int blk) -> float {
-      const int s = blk * 32 + lane;
-      return s < NS ? p.gbar[(size_t)bh * NC + (BWD ? NC - 1 - s : ck0 + s)] : 0.f;
-    };
-    float g_blk = load_g(0), g_nxt = load_g(1), g = 0.f;
+    // ---------------- TMA producer of the left operand ----------------
+    // The per-row scale vectors travel with the stage (bulk copies on the same barrier).  Stage, phase and addresses are carried
+    // along: the thread issues four copies per stage, and what it computes in between is in every stage's way.
     int issued = 0;   // by the issuing lane
-    bool ok = true;
-    for (int h = 0; h < NH2; ++h) {
-      const int st = h % REC_STAGES, s = h >> 1;
-      if ((h & 1) == 0) {
-        if (s > 0 && (s & 31) == 0) { g_blk = g_nxt; g_nxt = load_g((s >> 5) + 1); }
-        g = __shfl_sync(0xffffffffu, g_blk, s & 31);
-      }
-      ok = ok && mbar_wait(&bar_empty[st], ((h / REC_STAGES) & 1) ^ 1, &s_abort, &g_sm100_status, 101);
-      if (elect_one() && ok) {
-        // by the lane whose arrival below releases it (to the gating warps and the MMA thread, and by theirs to the readers)
-        if ((h & 1) == 0) s_g[s & 7] = g;
-        const int ck = BWD ? NC - 1 - s : ck0 + s;
-        // token rows past the end of the sequence (ragged last chunk) arrive as zeros; their scale slots hold zeros
-        const int y = ck * CL + (h & 1) * REC_HALF;          // first token of this half chunk inside the sequence
-        const size_t slot0 = (size_t)bh * p.SP + y;
-        uint8_t* sl = smem + st * REC_STAGE_BYTES;
-        mbar_expect_tx(&bar_full[st], 16384 + TN * 128 + (BWD ? 2 : 1) * REC_HALF * 4);
-        bulk_load(s_scale[st], p.lscale + slot0, REC_HALF * 4, &bar_full[st]);
-        if (BWD) bulk_load(s_scale2[st], p.rscale + slot0, REC_HALF * 4, &bar_full[st]);
-        tma_load_3d(sl, &mapL, &bar_full[st], d0, y, bh);
-        tma_load_3d(sl + 8192, &mapL, &bar_full[st], d0 + 64, y, bh);
-        tma_load_3d(sl + 16384, &mapR, &bar_full[st], e0, y, bh);
-        if (TN == 128) tma_load_3d(sl + 24576, &mapR, &bar_full[st], e0 + 64, y, bh);
-        issued = h + 1;
+    if (elect_one()) {
+      int st = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      int y = (BWD ? NC - 1 : ck0) * CL;                    // first token of the half chunk inside the sequence
+      const float* gbar = p.gbar + (size_t)bh * NC + (BWD ? NC - 1 : ck0);
+      float g = gbar[0];                                    // asked for a chunk ahead
+      const float *ls = p.lscale + (size_t)bh * p.SP, *rs = BWD ? p.rscale + (size_t)bh * p.SP : nullptr;
+      for (int h = 0; h < NH2; ++h) {
+        if (JOINT) ok = ok && (h < REC_STAGES || mbar_wait(&bar_done[(h - REC_STAGES) & (REC_LBUF - 1)], ((h - REC_STAGES) / REC_LBUF) & 1, &s_abort, &g_sm100_status, 113));
+        else ok = ok && mbar_wait(&bar_empty[st], ph, &s_abort, &g_sm100_status, 101);
+        if ((h & 1) == 0) {   // (the arrival below releases it to the gating warps, theirs to the MMA thread, and its to the readers)
+          const int s = h >> 1;
+          s_g[s & (G_RING - 1)] = g;
+          if (s + 1 < NS) g = gbar[BWD ? -(s + 1) : s + 1];
+        }
+        if (ok) {
+          // token rows past the end of the sequence (ragged last chunk) arrive as zeros; their scale slots hold zeros
+          uint8_t* sl = smem + st * 16384;
+          mbar_expect_tx(&bar_full[st], 16384 + (JOINT ? RIGHT_BYTES : 0) + (BWD ? 2 : 1) * REC_HALF * 4);
+          bulk_load(s_scale[st], ls + y, REC_HALF * 4, &bar_full[st]);
+          if (BWD) bulk_load(s_scale2[st], rs + y, REC_HALF * 4, &bar_full[st]);
+          tma_load_3d(sl, &mapL, &bar_full[st], d0, y, bh);
+          tma_load_3d(sl + 8192, &mapL, &bar_full[st], d0 + 64, y, bh);
+          if (JOINT) tma_load_3d(smem_r + st * RIGHT_BYTES, &mapR, &bar_full[st], e0, y, bh);
+          issued = h + 1;
+        }
+        y += (BWD && (h & 1)) ? -CL - REC_HALF : REC_HALF;
+        if (++st == REC_STAGES) { st = 0; ph ^= 1; }
       }
     }
     // the copies in flight land before the CTA retires, whichever role may have given up (the other lanes have issued none)
     for (int h = max(0, issued - REC_STAGES); h < issued; ++h)
       mbar_wait(&bar_full[h % REC_STAGES], (h / REC_STAGES) & 1, nullptr, nullptr, 0);
+  } else if (warp == 19) {
+    // ---------------- TMA producer of the right operand, where it has a ring of its own ----------------
+    int issued = 0;
+    if (!JOINT && elect_one()) {
+      int st = 0;
+      bool ok = true;
+      int y = (BWD ? NC - 1 : ck0) * CL;
+      for (int h = 0; h < NH2; ++h) {
+        // the product of RIGHT_STAGES half chunks ago is done
+        const int hb = h - RIGHT_STAGES;
+        ok = ok && (hb < 0 || mbar_wait(&bar_done[hb & (REC_LBUF - 1)], (hb / REC_LBUF) & 1, &s_abort, &g_sm100_status, 110));
+        if (ok) {
+          uint8_t* sr = smem_r + st * RIGHT_BYTES;
+          mbar_expect_tx(&bar_rfull[st], RIGHT_BYTES);
+          tma_load_3d(sr, &mapR, &bar_rfull[st], e0, y, bh);
+          tma_load_3d(sr + 8192, &mapR, &bar_rfull[st], e0 + 64, y, bh);
+          issued = h + 1;
+        }
+        y += (BWD && (h & 1)) ? -CL - REC_HALF : REC_HALF;
+        if (++st == RIGHT_STAGES) st = 0;
+      }
+    }
+    for (int h = max(0, issued - RIGHT_STAGES); h < issued; ++h)
+      mbar_wait(&bar_rfull[h % RIGHT_STAGES], (h / RIGHT_STAGES) & 1, nullptr, nullptr, 0);
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_16(F16, 128, TN, 1, 1);
-      for (int h = 0; h < NH2; ++h) {
-        const int st = h % REC_STAGES, s = h >> 1, buf = s & 1;
-        if (!mbar_wait(&bar_scaled[st], (h / REC_STAGES) & 1, &s_abort, &g_sm100_status, 102)) break;
-        if ((h & 1) == 0 && !mbar_wait(&bar_acc_free[buf], ((s >> 1) & 1) ^ 1, &s_abort, &g_sm100_status, 103)) break;
-        tc_fence_after_sync();
-        const uint32_t sl = smem_u32(smem + st * REC_STAGE_BYTES), sr = sl + 16384;
+      constexpr uint32_t idesc = umma_idesc_16(F16, 128, TN, 0, 1);
+      constexpr uint32_t desc_hi = umma_desc_hi(1024);
+      const uint32_t desc0 = umma_desc_lo(smem_u32(smem_r), 8192);
+      int st = 0;
+      uint32_t ph = 0, desc = desc0;
+      bool ok = true;
+      for (int s = 0; s < NS && ok; ++s) {
+        const int buf = s & 1;
+        if (!(ok = mbar_wait(&bar_acc_free[buf], ((s >> 1) & 1) ^ 1, &s_abort, &g_sm100_status, 103))) break;
 #pragma unroll
-        for (int kk = 0; kk < REC_HALF / 16; ++kk)
-          umma_ss(tmem + buf * 128, umma_desc_sw128(sl + kk * 2048, 8192, 1024),
-                  umma_desc_sw128(sr + kk * 2048, 8192, 1024), idesc, ((h & 1) || kk > 0) ? 1u : 0u);
-        umma_commit(&bar_empty[st]);
-        if (h & 1) umma_commit(&bar_acc_full[buf]);
+        for (int hf = 0; hf < 2; ++hf) {
+          const int lb = (2 * s + hf) & (REC_LBUF - 1);
+          ok = ok && (JOINT || mbar_wait(&bar_rfull[st], ph, &s_abort, &g_sm100_status, 111));
+          ok = ok && mbar_wait(&bar_scaled[lb], ((2 * s + hf) / REC_LBUF) & 1, &s_abort, &g_sm100_status, 102);
+          tc_fence_after_sync();
+          if (!ok) break;
+#pragma unroll
+          for (int kk = 0; kk < REC_HALF / 16; ++kk)
+            umma_ts(tmem + buf * 128, tL + lb * 32 + kk * 8, umma_desc(desc + kk * (2048 >> 4), desc_hi), idesc, (hf > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(&bar_done[lb]);
+          desc += RIGHT_BYTES >> 4;
+          if (++st == RIGHT_STAGES) { st = 0; ph ^= 1; desc = desc0; }
+        }
       }
     }
   } else if (warp < 10) {
-    // ---------------- gating warps: scale the rows of the left tile in place; column sums give n ----------------
-    // Two groups of four warps take the half chunks in turn: a stage costs 750 cycles of dependent work and 500 of waits and
-    // hand-over, which one group of eight paid for every stage (2700 cycles per chunk, the limit of the whole kernel).
-    const int grp = (warp - 2) >> 2, ct = (tid - 64) & 127;
-    const int row0 = ct >> 3;                      // rows row0 + 16 u of the stage, 16-byte piece ct & 7 of either box
-    // a lane whose wait has run out meets the others of its warp in the arrivals that are left, without arriving
-    auto stand_by = [&](int h, bool scaled) {
-      for (; h < NH2; h += 2, scaled = false) {
-        if (!scaled) warp_arrive(nullptr, false);
-        if (do_n) warp_arrive(nullptr, false);
-      }
-    };
+    // ---------------- gating warps: left tile, scaled and transposed, into tensor memory; column sums give n ----------------
+    // Two groups of four warps take the half chunks in turn: a stage costs hundreds of cycles of dependent work and of waits and
+    // hand-over, which one group would pay for every stage.  A warp reads its 32 columns (state rows d) of all 64 tokens with
+    // transposing loads, so that a lane holds pairs of tokens of one d, and writes them where the MMA reads its A operand: the
+    // shared-memory port, the busiest unit of this kernel, carries the left tile once instead of three times (read, rewritten in
+    // place, read by the MMA; 288 -> 192 KB per chunk and 128 x 128 tile), and no writes have to be made visible to the tensor
+    // core's proxy.  All reads go out before the first is used, and the stage is handed back then.  Measured (first rewriting in
+    // place, then this): 8 x 8192 tokens, 16 heads 256/256, 402 -> 374 us (HBM at 0.82 of the copy rate), gradient 397 -> 362;
+    // 8 heads 256/512, 131072 tokens 1135 -> 964 (narrow tiles: the chain of one half chunk after the other through gating,
+    // product and fold); 4 x 4 x 1024, 96/192 18.8 -> 16.5.
+    const int grp = (warp - 2) >> 2, quarter = warp & 3;
+    // tile m = lane / 8 of a transposing load: columns 8 m of the warp's 32; row lane % 8, 16-byte pieces XOR-swizzled by the row
+    const uint32_t src0 = smem_u32(smem) + (quarter >> 1) * 8192 + (lane & 7) * 128 + ((((quarter & 1) * 4 + (lane >> 3)) ^ (lane & 7)) << 4);
+    const int tok2 = 2 * (lane & 3);               // first of the lane's two tokens in every eight
+    // (a lane whose wait has run out goes on with its warp, and does not arrive: see warp_arrive)
     for (int h = grp; h < NH2; h += 2) {
-      const int st = h % REC_STAGES, s = h >> 1, nb = s & 1;
-      if (!mbar_wait(&bar_full[st], (h / REC_STAGES) & 1, &s_abort, &g_sm100_status, 105)) { stand_by(h, false); break; }
-      // two 64-column boxes of 64 rows x 128 B, 128-byte swizzle: the scale depends on the row only
-      uint8_t* sl = smem + st * REC_STAGE_BYTES + row0 * 128 + (ct & 7) * 16;
-      float sc[4];
+      const int st = h % REC_STAGES, lb = h & (REC_LBUF - 1), s = h >> 1, nb = s & 1;
+      bool ok = mbar_wait(&bar_full[st], (h / REC_STAGES) & 1, &s_abort, &g_sm100_status, 105);
+      uint32_t x[REC_HALF / 8][4];
+      float2 sc[REC_HALF / 8], sc2[BWD ? REC_HALF / 8 : 1];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        sc[u] = s_scale[st][row0 + 16 * u] * p.lmul;
-        if (BWD) sc[u] *= s_scale2[st][row0 + 16 * u];
+      for (int tb = 0; tb < REC_HALF / 8; ++tb) ldmatrix_x4_trans(src0 + st * 16384 + tb * 1024, x[tb]);
+#pragma unroll
+      for (int tb = 0; tb < REC_HALF / 8; ++tb) {
+        sc[tb] = *reinterpret_cast<const float2*>(&s_scale[st][8 * tb + tok2]);
+        if (BWD) sc2[tb] = *reinterpret_cast<const float2*>(&s_scale2[st][8 * tb + tok2]);
       }
-      uint64_t ns[2][4];
+      if (!JOINT) warp_arrive(&bar_empty[st], ok);
+      uint32_t w[2][16];
+      uint64_t ns[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        uint4 v[4];
+      for (int tb = 0; tb < REC_HALF / 8; ++tb) {
+        uint64_t ss = mul2(f2(sc[tb].x, sc[tb].y), f2(p.lmul, p.lmul));
+        if (BWD) ss = mul2(ss, f2(sc2[tb].x, sc2[tb].y));
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint4*>(sl + b * 8192 + u * 2048);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ns[b][e] = 0ull;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint64_t ss = f2(sc[u], sc[u]);
-          uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint64_t x = mul2(unpack2<F16>(w[e]), ss);
-            ns[b][e] = add2(ns[b][e], x);
-            w[e] = pack2<F16>(x);
-          }
-          *reinterpret_cast<uint4*>(sl + b * 8192 + u * 2048) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int m = 0; m < 4; ++m) {
+          const uint64_t y = mul2(unpack2<F16>(x[tb][m]), ss);
+          if (HAS_N) ns[m] = add2(ns[m], y);
+          w[m >> 1][2 * tb + (m & 1)] = pack2<F16>(y);
         }
       }
-      fence_proxy_async_smem();
-      warp_arrive(&bar_scaled[st], true);
-      if (do_n) {   // partial column sums of this half: 16 rows of the chunk's 32
-        // the n warp has read the partial sums of chunk s - 2 out of this buffer
-        if (s >= 2 && !mbar_wait(&bar_nread[nb], ((s >> 1) - 1) & 1, &s_abort, &g_sm100_status, 109)) { stand_by(h, true); break; }
-        float* npart = reinterpret_cast<float*>(smem + REC_STAGES * REC_STAGE_BYTES) + nb * (32 * 128) + (grp * 16 + row0) * 128;
-        const int lc = (ct & 7) ^ (row0 & 7);   // logical 16-byte column chunk behind the swizzle
+      // the product that read this buffer last is done (with one ring it was before the stage could be loaded)
+      const bool free_ok = JOINT || h < REC_LBUF || mbar_wait(&bar_done[lb], ((h / REC_LBUF) - 1) & 1, &s_abort, &g_sm100_status, 112);
+      tc_fence_after_sync();
+      const uint32_t dst = tL + lb * 32 + ((uint32_t)(quarter * 32) << 16);
+      tmem_st_16x128b_x8(dst, w[0]);
+      tmem_st_16x128b_x8(dst + (16u << 16), w[1]);
+      tmem_wait_st();
+      tc_fence_before_sync();
+      ok = ok && free_ok;
+      warp_arrive(&bar_scaled[lb], ok);
+      if (do_n) {   // column sums of this half chunk: the four lanes of a d hold the sums over their tokens
+        float v[4];
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          ulonglong2* dst = reinterpret_cast<ulonglong2*>(npart + b * 64 + lc * 8);
-          dst[0] = make_ulonglong2(ns[b][0], ns[b][1]);
-          dst[1] = make_ulonglong2(ns[b][2], ns[b][3]);
+        for (int m = 0; m < 4; ++m) {
+          float lo, hi;
+          unf2(ns[m], lo, hi);
+          v[m] = lo + hi;
+          v[m] += __shfl_xor_sync(0xffffffffu, v[m], 1);
+          v[m] += __shfl_xor_sync(0xffffffffu, v[m], 2);
         }
-        warp_arrive(&bar_nsum[nb], true);   // (complete when both halves of chunk s are in)
+        // the n warp has read the sums of chunk s - 2 out of this buffer
+        const bool nok = s < 2 || mbar_wait(&bar_nread[nb], ((s >> 1) - 1) & 1, &s_abort, &g_sm100_status, 109);
+        float* npart = reinterpret_cast<float*>(smem + rec_npart_offset(TN)) + (nb * 2 + grp) * 128;
+        const int m = lane & 3;
+        npart[quarter * 32 + m * 8 + (lane >> 2)] = m == 0 ? v[0] : (m == 1 ? v[1] : (m == 2 ? v[2] : v[3]));
+        warp_arrive(&bar_nsum[nb], ok && nok);   // (complete when both halves of chunk s are in)
       }
     }
   } else if (warp == 18) {
-    // ---------------- store warp: one TMA store per 64-column box of each staged state tile ----------------
-    if (p.c_states != nullptr && elect_one()) {
-      uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (HAS_N ? REC_NPART_BYTES : 0);
-      for (int n = 0; n <= NS; ++n) {
+    // ---------------- store and n warp ----------------
+    // Per chunk boundary one TMA store per 64-column box of the staged state tile; then n_{s+1} = gbar n_s + column sums of the
+    // gated left tile (no tensor cores needed), four columns per lane.
+    const bool store = p.c_states != nullptr;
+    uint8_t* stage_base = smem + rec_npart_offset(TN) + (HAS_N ? REC_NPART_BYTES : 0);
+    float4 nv = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool d_in = do_n && d0 + 4 * lane < p.DHQK;   // the lane's four rows exist (DHQK is a multiple of 8)
+    if (p.n_init && d_in) nv = *reinterpret_cast<const float4*>(p.n_init + (size_t)bh * p.DHQK + d0 + 4 * lane);
+    if (p.n_states != nullptr && d_in)
+      *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1) + ck0) * p.DHQK + d0 + 4 * lane) = nv;
+    bool ok = true;
+    for (int n = 0; n <= NS; ++n) {
+      if (store) {
         const int ob = n & 1;
-        if (!mbar_wait(&bar_out_full[ob], (n >> 1) & 1, &s_abort, &g_sm100_status, 108)) break;
-        const int slot = BWD ? NC - n : ck0 + n;
-        const int z = bh * (NC + 1) + slot;
-        tma_store_3d(&mapS, stage_base + ob * REC_OUT, e0, d0, z);
-        if (TN == 128 && e0 + 64 < p.DHHV) tma_store_3d(&mapS, stage_base + ob * REC_OUT + 16384, e0 + 64, d0, z);
-        tma_store_commit();
-        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the previous tile has left its buffer
-        if (n >= 1) mbar_arrive(&bar_out_free[ob ^ 1]);
+        ok = ok && mbar_wait(&bar_out_full[ob], (n >> 1) & 1, &s_abort, &g_sm100_status, 108);
+        if (lane == 0 && ok) {
+          const int z = bh * (NC + 1) + (BWD ? NC - n : ck0 + n);
+          tma_store_3d(&mapS, stage_base + ob * REC_OUT, e0, d0, z);
+          if (TN == 128 && e0 + 64 < p.DHHV) tma_store_3d(&mapS, stage_base + ob * REC_OUT + 16384, e0 + 64, d0, z);
+          tma_store_commit();
+          asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the previous tile has left its buffer
+          if (n >= 1) mbar_arrive(&bar_out_free[ob ^ 1]);
+        }
       }
-      tma_store_wait_all();   // all state tiles have been written before the CTA retires
-    }
-  } else if (warp == 19) {
-    // ---------------- n warp: n_{s+1} = gbar n_s + column sums of the gated left tile (no tensor cores needed) ----
-    // Four columns per lane; the 32 partial sums of a column are added in a fixed order, so the result does not
-    // depend on scheduling.
-    if (do_n) {
-      float4 nv = make_float4(0.f, 0.f, 0.f, 0.f);
-      const bool d_in = d0 + 4 * lane < p.DHQK;   // the lane's four rows exist (DHQK is a multiple of 8)
-      if (p.n_init && d_in) nv = *reinterpret_cast<const float4*>(p.n_init + (size_t)bh * p.DHQK + d0 + 4 * lane);
+      if (!do_n || n == NS) continue;
+      const int nb = n & 1;
+      ok = ok && mbar_wait(&bar_nsum[nb], (n >> 1) & 1, &s_abort, &g_sm100_status, 106);
+      const float4* np4 = reinterpret_cast<const float4*>(smem + rec_npart_offset(TN)) + nb * 64 + lane;
+      float4 cs = np4[0];
+      const float4 c1 = np4[32];
+      cs.x += c1.x; cs.y += c1.y; cs.z += c1.z; cs.w += c1.w;
+      const float g = s_g[n & (G_RING - 1)];
+      __syncwarp();
+      if (lane == 0 && ok) mbar_arrive(&bar_nread[nb]);
+      nv.x = fmaf(g, nv.x, cs.x); nv.y = fmaf(g, nv.y, cs.y); nv.z = fmaf(g, nv.z, cs.z); nv.w = fmaf(g, nv.w, cs.w);
       if (p.n_states != nullptr && d_in)
-        *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1) + ck0) * p.DHQK + d0 + 4 * lane) = nv;
-      bool ok = true;
-      for (int s = 0; s < NS; ++s) {
-        const int nb = s & 1;
-        ok = ok && mbar_wait(&bar_nsum[nb], (s >> 1) & 1, &s_abort, &g_sm100_status, 106);
-        const float4* np4 = reinterpret_cast<const float4*>(smem + REC_STAGES * REC_STAGE_BYTES) + nb * (32 * 32) + lane;
-        float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (int g = 0; g < 32; ++g) { const float4 v = np4[g * 32]; cs.x += v.x; cs.y += v.y; cs.z += v.z; cs.w += v.w; }
-        __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(&bar_nread[nb]);
-        const float g = s_g[s & 7];
-        nv.x = fmaf(g, nv.x, cs.x); nv.y = fmaf(g, nv.y, cs.y); nv.z = fmaf(g, nv.z, cs.z); nv.w = fmaf(g, nv.w, cs.w);
-        if (p.n_states != nullptr && d_in)
-          *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1) + ck0 + s + 1) * p.DHQK + d0 + 4 * lane) = nv;
-      }
-      if (ok && p.n_final && d_in) *reinterpret_cast<float4*>(p.n_final + (size_t)bh * p.DHQK + d0 + 4 * lane) = nv;
+        *reinterpret_cast<float4*>(p.n_states + ((size_t)bh * (NC + 1) + ck0 + n + 1) * p.DHQK + d0 + 4 * lane) = nv;
     }
+    if (ok && p.n_final && d_in) *reinterpret_cast<float4*>(p.n_final + (size_t)bh * p.DHQK + d0 + 4 * lane) = nv;
+    if (store && lane == 0) tma_store_wait_all();   // all state tiles have been written before the CTA retires
   } else {
     // ---------------- state warps: fold each chunk's product into the running state, store it ----------------
     const int quarter = warp & 3, half = (warp - 10) >> 2;
@@ -306,11 +353,10 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
     }
     // The bf16 state tile goes to shared memory in the 128-byte-swizzled box layout and leaves with one TMA store
     // per 64-column box (coalesced, asynchronous); two staging buffers, one store group in flight.
-    uint8_t* stage_base = smem + REC_STAGES * REC_STAGE_BYTES + (HAS_N ? REC_NPART_BYTES : 0);
+    uint8_t* stage_base = smem + rec_npart_offset(TN) + (HAS_N ? REC_NPART_BYTES : 0);
     // (the answer of a wait counts for the arrival after it only: a flag held over the loop costs the 128-column forms
     // register spills, and the waits after one that ran out end by the abort flag)
-    int n_out = 0;   // tiles written so far
-    auto store_c = [&]() {
+    auto store_c = [&](const int n_out) {   // n_out: tiles written before this one
       if (p.c_states == nullptr) return;
       const int ob = n_out & 1;
       const bool ok = n_out < 2 || mbar_wait(&bar_out_free[ob], ((n_out >> 1) - 1) & 1, &s_abort, &g_sm100_status, 107);
@@ -326,14 +372,13 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       }
       fence_proxy_async_smem();
       warp_arrive(&bar_out_full[ob], ok);   // the store warp ships the tile
-      ++n_out;
     };
-    store_c();   // the state before the first step (slot 0 forward, slot NC backward)
+    store_c(0);   // the state before the first step (slot 0 forward, slot NC backward)
     for (int s = 0; s < NS; ++s) {
       const int buf = s & 1;
-      const bool ok = mbar_wait(&bar_acc_full[buf], (s >> 1) & 1, &s_abort, &g_sm100_status, 104);
+      const bool ok = mbar_wait(&bar_done[(2 * s + 1) & (REC_LBUF - 1)], ((2 * s + 1) / REC_LBUF) & 1, &s_abort, &g_sm100_status, 104);
       tc_fence_after_sync();
-      const float g = s_g[s & 7];
+      const float g = s_g[s & (G_RING - 1)];
       const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 128 + half * HC;
 #pragma unroll
       for (int q4 = 0; q4 < HC / 16; ++q4) {
@@ -345,7 +390,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
       }
       tc_fence_before_sync();
       warp_arrive(&bar_acc_free[buf], ok);
-      store_c();
+      store_c(s + 1);
     }
     if (p.c_final) {
       float4* fd = reinterpret_cast<float4*>(p.c_final + ((size_t)bh * p.DHQK + d) * p.DHHV + ecol);
@@ -356,7 +401,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, 256);
+  if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
 template <bool BWD, int TN, bool F16>
