@@ -216,15 +216,19 @@ par_bw_run_sm100(const __grid_constant__ BwMaps maps, const __grid_constant__ Bw
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
       constexpr uint32_t idesc_kk = umma_idesc_16(F16, 128, 128, 0, 0), idesc_kn = umma_idesc_16(F16, 128, 128, 0, 1);
+      constexpr uint32_t hi = umma_desc_hi(1024);
       const uint32_t tS = tmem, tG = tmem + 128, tA = tmem + 256;
+      const uint32_t base = smem_u32(smem) >> 4;
       int st = 0;
       uint32_t ph = 0;
       bool ok = true;
-      auto arrived = [&]() -> uint32_t {   // the next stage of the ring
+      // low word of the descriptor of the next stage of the ring (its leading-dimension field still empty: unused with K-major operands)
+      auto arrived = [&]() -> uint32_t {
         ok = ok && mbar_wait(&sh.full[st], ph, &sh.abort, &g_par_bw_status, 302);
         tc_fence_after_sync();
-        return smem_u32(smem + st * STAGE);
+        return base + st * (STAGE >> 4);
       };
+      constexpr uint32_t lbo8 = (8192u >> 4) << 16, lbo16 = (16384u >> 4) << 16;
       auto release = [&]() {
         umma_commit(&sh.empty[st]);
         if (++st == NST) { st = 0; ph ^= 1; }
@@ -239,21 +243,22 @@ par_bw_run_sm100(const __grid_constant__ BwMaps maps, const __grid_constant__ Bw
         tc_fence_after_sync();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          umma_ts(tA + (tp & 1) * 128, tG + (n & 1) * 64 + kk * 8, umma_desc_sw128(sx + kk * 2048, 16384, 1024), idesc_kn, 1u);
+          umma_ts(tA + (tp & 1) * 128, tG + (n & 1) * 64 + kk * 8, umma_desc((sx | lbo16) + kk * (2048 >> 4), hi), idesc_kn, 1u);
         release();
         umma_commit(&sh.hfull[tp & 1]);
       };
       int n = 0, before = 0;   // items begun; tiles of the item before
       for (; it.left > 0 && ok; it.next(p), ++n) {
         const int nd = it.slices(p), nsub = it.tiles(p);
-        const bool mn = it.mode(p) == PM_DV;
+        const bool mn = it.mode(p) == PM_DV;          // the state operand is N-contiguous in shared memory
+        const uint32_t step = (mn ? 2048 : 32) >> 4, idesc = mn ? idesc_kn : idesc_kk;
         if (n > 0 && !(ok = mbar_wait(&sh.sread, (n - 1) & 1, &sh.abort, &g_par_bw_status, 305))) break;
         for (int i = 0; i < nd; ++i) {            // score: S = A . B^T
-          const uint32_t sa = arrived(), sb = sa + 16384;
+          const uint32_t sa = arrived(), sb = sa + (16384 >> 4);
           if (!ok) break;
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            umma_ss(tS, umma_desc_sw128(sa + kk * 32, 16, 1024), umma_desc_sw128(sb + kk * 32, 16, 1024), idesc_kk, (i > 0 || kk > 0) ? 1u : 0u);
+            umma_ss(tS, umma_desc(sa + kk * (32 >> 4), hi), umma_desc(sb + kk * (32 >> 4), hi), idesc_kk, (i > 0 || kk > 0) ? 1u : 0u);
           release();
         }
         if (!ok) break;
@@ -265,13 +270,11 @@ par_bw_run_sm100(const __grid_constant__ BwMaps maps, const __grid_constant__ Bw
           tc_fence_after_sync();
           const uint32_t acc = tA + (t & 1) * 128;
           for (int i = 0; i < nd; ++i) {           // inter-chunk term: Acc = A . State
-            const uint32_t sa = arrived(), ss = sa + 16384;
+            const uint32_t sa = arrived(), ss = (sa + (16384 >> 4)) | (mn ? lbo8 : 0u);
             if (!ok) break;
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              const uint64_t bd = mn ? umma_desc_sw128(ss + kk * 2048, 8192, 1024) : umma_desc_sw128(ss + kk * 32, 16, 1024);
-              umma_ss(acc, umma_desc_sw128(sa + kk * 32, 16, 1024), bd, mn ? idesc_kn : idesc_kk, (i > 0 || kk > 0) ? 1u : 0u);
-            }
+            for (int kk = 0; kk < 4; ++kk)
+              umma_ss(acc, umma_desc(sa + kk * (32 >> 4), hi), umma_desc(ss + kk * step, hi), idesc, (i > 0 || kk > 0) ? 1u : 0u);
             release();
           }
           if (!ok) break;

@@ -610,17 +610,18 @@ par_body(const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* ma
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_16(F16, 128, 128, 0, 0);
-      constexpr uint32_t idesc_x = umma_idesc_16(F16, 128, 128, 0, 1);
+      constexpr uint32_t idesc_x = umma_idesc_16(F16, 128, 128, 0, 1), hi = umma_desc_hi(1024);
+      constexpr uint32_t lbo8 = (8192u >> 4) << 16, lbo16 = (16384u >> 4) << 16;   // (unused with K-major operands)
+      const uint32_t base = smem_u32(smem) >> 4;
       bool ok = true;
       for (int ld = 0; ld < ND; ++ld) {            // score: S = A . B^T
         const int st = ld % PAR_NST;
         if (!mbar_wait(&sh.bar_full[st], (ld / PAR_NST) & 1, &sh.abort, &g_sm100_status, 202)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t sa = smem_u32(smem + st * PAR_STAGE), sb = sa + 16384;
+        const uint32_t sa = base + st * (PAR_STAGE >> 4), sb = sa + (16384 >> 4);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma_ss(tS, umma_desc_sw128(sa + kk * 32, 16, 1024), umma_desc_sw128(sb + kk * 32, 16, 1024), idesc_s,
-                  (ld > 0 || kk > 0) ? 1u : 0u);
+          umma_ss(tS, umma_desc(sa + kk * (32 >> 4), hi), umma_desc(sb + kk * (32 >> 4), hi), idesc_s, (ld > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&sh.bar_empty[st]);
       }
       if (ok) umma_commit(&sh.bar_sfull);
@@ -633,12 +634,10 @@ par_body(const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* ma
           const int ld = lbase + it, st = ld % PAR_NST;
           if (!mbar_wait(&sh.bar_full[st], (ld / PAR_NST) & 1, &sh.abort, &g_sm100_status, 213)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + st * PAR_STAGE), ss = sa + 16384;
+          const uint32_t sa = base + st * (PAR_STAGE >> 4), ss = (sa + (16384 >> 4)) | lbo8;
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            umma_ss(tAcc, umma_desc_sw128(sa + kk * 32, 16, 1024), umma_desc_sw128(ss + kk * 2048, 8192, 1024), idesc_x,
-                    (it > 0 || kk > 0) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < 4; ++kk)
+            umma_ss(tAcc, umma_desc(sa + kk * (32 >> 4), hi), umma_desc(ss + kk * (2048 >> 4), hi), idesc_x, (it > 0 || kk > 0) ? 1u : 0u);
           umma_commit(&sh.bar_empty[st]);
         }
         if (!ok) break;
@@ -648,10 +647,10 @@ par_body(const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* ma
              mbar_wait(&sh.bar_gated, sub & 1, &sh.abort, &g_sm100_status, 204);
         if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t sx = smem_u32(smem + stx * PAR_STAGE);
+        const uint32_t sx = (base + stx * (PAR_STAGE >> 4)) | lbo16;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          umma_ts(tAcc, tS + kk * 8, umma_desc_sw128(sx + kk * 2048, 16384, 1024), idesc_x, 1u);
+          umma_ts(tAcc, tS + kk * 8, umma_desc(sx + kk * (2048 >> 4), hi), idesc_x, 1u);
         umma_commit(&sh.bar_hfull);
       }
     }
