@@ -443,6 +443,13 @@ size_t fw_bytes_one_stream(const CallDims& c) {
   return carve_fw(nullptr, c.B * c.NH, NC * c.L, NC).bytes;
 }
 
+size_t score_scratch_bytes(const CallDims& c, bool backward) {
+  bool use_sm100 = false;
+  if (check_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L) != MLSTM_OK ||
+      resolve_impl(c.impl, c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, &use_sm100) != MLSTM_OK || use_sm100) return 0;
+  return simt_score_bytes(make_dims(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.variant, 0.f, c.dtype), backward);
+}
+
 int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
   int rc = check_call(c);
   if (rc != MLSTM_OK) return rc;
@@ -474,8 +481,9 @@ int run_chunkwise_fw(const FwCall& a, const CallDims& c) {
     if (ch.split() && (rc = sm100_parallel_fw(a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, d, ch.second_stream(), ch.second())) != MLSTM_OK) return rc;
     if ((rc = ch.join()) != MLSTM_OK) return rc;
   } else {
-    if ((rc = simt_recurrent_fw(c.dtype, a.k, a.v, lay.gb, a.c_initial, a.n_initial, a.c_states, a.n_states, a.c_last, a.n_last, d, st)) != MLSTM_OK) return rc;
-    if ((rc = simt_parallel_fw(c.dtype, a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, d, st)) != MLSTM_OK) return rc;
+    float* scores = static_cast<float*>(a.scores);
+    if ((rc = simt_recurrent_fw(c.dtype, a.q, a.k, a.v, lay.gb, a.c_initial, a.n_initial, a.c_states, a.n_states, a.c_last, a.n_last, scores, d, st)) != MLSTM_OK) return rc;
+    if ((rc = simt_parallel_fw(c.dtype, a.q, a.k, a.v, lay.gb, a.c_states, a.n_states, a.h, a.n_out, scores, d, st)) != MLSTM_OK) return rc;
   }
   return MLSTM_OK;
 }
@@ -538,10 +546,9 @@ int run_chunkwise_bw(const BwCall& a, const CallDims& c) {
                                       lay.anchors, n_anchors, kAnchorEvery * c.L)) != MLSTM_OK) return rc;
     }
   } else {
-    if (a.recompute_into &&
-        (rc = simt_recurrent_fw(c.dtype, a.k, a.v, lay.gb, a.recompute_c_initial, nullptr, a.recompute_into, nullptr, nullptr, nullptr, d, st)) != MLSTM_OK) return rc;
-    if ((rc = simt_recurrent_bw(c.dtype, a.q, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, d, st)) != MLSTM_OK) return rc;
-    if ((rc = simt_parallel_bw(c.dtype, a.q, a.k, a.v, a.dh, lay.gb, c_states, lay.dc_states, a.dq, a.dk, a.dv, d, st)) != MLSTM_OK) return rc;
+    float* scores = static_cast<float*>(a.scores);
+    if ((rc = simt_recurrent_bw(c.dtype, a.q, a.k, a.v, a.dh, lay.gb, a.dc_last, lay.dc_states, a.dc_initial, a.recompute_c_initial, a.recompute_into, scores, d, st)) != MLSTM_OK) return rc;
+    if ((rc = simt_parallel_bw(c.dtype, a.q, a.k, a.v, a.dh, lay.gb, c_states, lay.dc_states, a.dq, a.dk, a.dv, scores, d, st)) != MLSTM_OK) return rc;
     if ((rc = launch_gate_grads(c.dtype, c.gate_dtype, a.q, a.k, a.dq, a.dk, a.i, a.f, lay.acc, lay.kdk, a.di, a.df, a.grad_gate_dtype, d, st)) != MLSTM_OK) return rc;
   }
   return MLSTM_OK;
@@ -621,7 +628,7 @@ int mlstm_b200_chunkwise_states(const void* k, const void* v, const void* i, con
     if ((rc = launch_gates(gate_dtype, i, f, variant == MLSTM_EXP ? m_initial : nullptr, nullptr, nullptr, gb, lay.m_states, nullptr, d, st)) != MLSTM_OK) return rc;
   }
   if (use_sm100) return sm100_recurrent_fw(k, v, gb, c_initial, nullptr, c_states, nullptr, nullptr, nullptr, d, st);
-  return simt_recurrent_fw(dtype, k, v, gb, c_initial, nullptr, c_states, nullptr, nullptr, nullptr, d, st);
+  return simt_recurrent_fw(dtype, nullptr, k, v, gb, c_initial, nullptr, c_states, nullptr, nullptr, nullptr, nullptr, d, st);
 }
 
 int mlstm_b200_chunkwise_dc_summary(const void* q, const void* dh, const float* n_out, const void* fw_workspace,
@@ -648,7 +655,7 @@ int mlstm_b200_chunkwise_dc_summary(const void* q, const void* dh, const float* 
   gb.inv_den = static_cast<float*>(workspace);
   if ((rc = launch_inv_den(n_out, gb.inv_den, d, st)) != MLSTM_OK) return rc;
   if (use_sm100) return sm100_recurrent_bw(q, dh, gb, nullptr, nullptr, dc_initial, d, st);
-  return simt_recurrent_bw(dtype, q, dh, gb, nullptr, nullptr, dc_initial, d, st);
+  return simt_recurrent_bw(dtype, q, nullptr, nullptr, dh, gb, nullptr, nullptr, dc_initial, nullptr, nullptr, nullptr, d, st);
 }
 
 int mlstm_b200_chunkwise_summary(const void* k, const void* v, const void* i, const void* f, float* c_last,
@@ -675,7 +682,7 @@ int mlstm_b200_chunkwise_summary(const void* k, const void* v, const void* i, co
   if (use_sm100) {
     if ((rc = sm100_recurrent_fw(k, v, lay.gb, nullptr, nullptr, nullptr, nullptr, c_last, n_last, d, st)) != MLSTM_OK) return rc;
   } else {
-    if ((rc = simt_recurrent_fw(dtype, k, v, lay.gb, nullptr, nullptr, nullptr, nullptr, c_last, n_last, d, st)) != MLSTM_OK) return rc;
+    if ((rc = simt_recurrent_fw(dtype, nullptr, k, v, lay.gb, nullptr, nullptr, nullptr, nullptr, c_last, n_last, nullptr, d, st)) != MLSTM_OK) return rc;
   }
   return MLSTM_OK;
 }

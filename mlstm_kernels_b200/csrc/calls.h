@@ -25,6 +25,7 @@ struct FwCall {
   void* workspace;
   size_t workspace_bytes;
   bool allow_split;            // false: every launch stays on the caller's stream
+  void* scores;                // scratch of score_scratch_bytes(), or null: slower without
 };
 
 struct BwCall {
@@ -45,6 +46,7 @@ struct BwCall {
   float* dc_initial;
   void* workspace;
   size_t workspace_bytes;
+  void* scores;                // as in FwCall
 };
 
 #if defined(__GNUC__)
@@ -52,6 +54,8 @@ struct BwCall {
 #endif
 // scratch of a forward with allow_split = false (0: sizes it does not take)
 size_t fw_bytes_one_stream(const CallDims& c);
+// further scratch that a forward or backward call can use (0: none)
+size_t score_scratch_bytes(const CallDims& c, bool backward);
 int run_chunkwise_fw(const FwCall& a, const CallDims& c);
 int run_chunkwise_bw(const BwCall& a, const CallDims& c);
 #if defined(__GNUC__)

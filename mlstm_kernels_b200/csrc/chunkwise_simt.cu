@@ -2,7 +2,8 @@
 // dimension, f32 / bf16 / f16 inputs, exact f32 arithmetic).  It covers the shapes the tcgen05 path
 // does not (small chunks, odd head dims, f32 inputs) and is the on-device cross-check for it.
 //
-//   rec_part_kernel, rec_scan_kernel, rec_final_kernel : inter-chunk recurrence, forward (C_k, n_k) and backward (deltaC_k)
+//   part_kernel, rec_scan_kernel, rec_final_kernel : inter-chunk recurrence, forward (C_k, n_k) and backward (deltaC_k);
+//                 part_kernel also computes the gated score blocks that the output tiles of a chunk share
 //                 mlstm_kernels/triton/chunkwise/xl_chunk/fw_kernel_recurrent.py:14-230,
 //                 bw_kernel_recurrent.py:15-181
 //   par_fw_kernel, par_bw_kernel  : intra-chunk gated products + inter-chunk contribution for H; deltaV, deltaK, deltaQ
@@ -185,7 +186,7 @@ struct NoEach { __device__ __forceinline__ void operator()(const float*, int) co
 //   forward : left = K, lscale = abar, right = V;  also n <- gbar n + sum_j abar_j k_j
 //   backward: left = Q, lscale = bbar, lmul = qk_scale, right = deltaH, rscale = 1/(den+eps); chunks reversed
 // Where the per-chunk states are wanted, the chunks' contributions are independent CTAs that leave them in the state
-// buffer itself (rec_part_kernel), and an element-wise scan over the chunks turns them into states in place
+// buffer itself (part_kernel), and an element-wise scan over the chunks turns them into states in place
 // (rec_scan_kernel, one thread per four elements): a CTA that walks a whole sequence took 9.6 us per chunk of 64 tokens
 // while most SMs idled.  Without a state buffer (segment summaries) rec_final_kernel walks the chunks of its tile.
 // =====================================================================================================
@@ -223,20 +224,20 @@ __device__ __forceinline__ void chunk_part(const RecArgs<T>& p, int bh, int ck, 
   }
 }
 
-template <typename T, bool BWD, bool VEC>
-__global__ void __launch_bounds__(NTHR) rec_part_kernel(RecArgs<T> p) {
-  __shared__ __align__(16) float buf[4 * SLICE];
-  // 1-D grid: the tiles of one chunk next to each other (they share its operands through L2)
+// One tile of one chunk's contribution to the state, of the forward's recurrence or (bwd) the gradient's.
+template <typename T, bool VEC>
+__device__ __forceinline__ void rec_part_tile(const RecArgs<T>& p, const bool bwd, const unsigned block, float* buf) {
+  // the tiles of one chunk next to each other (they share its operands through L2)
   const int n_et = (p.DHHV + TILE - 1) / TILE, n_dt = (p.DHQK + TILE - 1) / TILE;
-  const int et = blockIdx.x % n_et, dt = (blockIdx.x / n_et) % n_dt, bc = blockIdx.x / (n_et * n_dt);
+  const int et = block % n_et, dt = (block / n_et) % n_dt, bc = block / (n_et * n_dt);
   const int bh = bc / p.NC, ck = bc % p.NC, e0 = et * TILE, d0 = dt * TILE;
-  const bool do_n = !BWD && et == 0 && p.n_states != nullptr;
+  const bool do_n = !bwd && et == 0 && p.n_states != nullptr;
   const int ty = row_group(threadIdx.x), tx = col_group(threadIdx.x);
   Acc acc;
   float ns[4], x[4][4];
   chunk_part<T, VEC>(p, bh, ck, d0, e0, do_n, buf, acc, ns);
   acc.get(x);
-  const size_t slot = (size_t)bh * (p.NC + 1) + (BWD ? ck : ck + 1);
+  const size_t slot = (size_t)bh * (p.NC + 1) + (bwd ? ck : ck + 1);
   float* out = p.c_states + slot * p.DHQK * p.DHHV;
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
@@ -245,6 +246,89 @@ __global__ void __launch_bounds__(NTHR) rec_part_kernel(RecArgs<T> p) {
       store4(out + (size_t)d * p.DHHV, e0 + 4 * tx, p.DHHV, VEC,
              make_float4(x[a][0] * p.lmul, x[a][1] * p.lmul, x[a][2] * p.lmul, x[a][3] * p.lmul));
     if (do_n && tx == 0 && d < p.DHQK) p.n_states[slot * p.DHQK + d] = ns[a];
+  }
+}
+
+// ---- gated score blocks ------------------------------------------------------------------------------
+// block[i][j] = qk_scale * (a_i . b_j) * D(i,j) for j <= i, else 0: 64 x 64 tokens of one chunk.
+template <typename T>
+struct ScoreArgs {
+  const T *a, *b;          // rows i and j
+  const float* a_scale;    // per token or null
+  float* out;              // [chunk][pair of 64-token blocks, (0,0), (1,0), (1,1), ..][64][64]
+  int D;                   // contraction
+};
+struct ScoreGate {
+  const float *vecB, *iota, *m_tok;
+  int S, L, NC;
+  float qk_scale;
+};
+__host__ __device__ constexpr int score_pairs(int L) { const int nb = (L + TILE - 1) / TILE; return nb * (nb + 1) / 2; }
+__device__ __forceinline__ int score_pair(int rb, int cb) { return rb * (rb + 1) / 2 + cb; }
+
+__device__ __forceinline__ float gate_score(float s, float qk_scale, float b_i, float b_j, float iota_j, float m_i) {
+  return qk_scale * s * expf((b_i - b_j) + iota_j - m_i);
+}
+
+template <typename T, bool VEC>
+__device__ __forceinline__ void score_tile(const ScoreArgs<T>& p, const ScoreGate& g, const unsigned block, float* buf) {
+  const int np = score_pairs(g.L), pair = block % np, bc = block / np, bh = bc / g.NC, ck = bc % g.NC;
+  int rb = 0;
+  while (score_pair(rb + 1, 0) <= pair) ++rb;
+  const int r0 = rb * TILE, c0 = (pair - score_pair(rb, 0)) * TILE;
+  const int tid = threadIdx.x, ty = row_group(tid), tx = col_group(tid);
+  const size_t tok0 = (size_t)bh * g.S + (size_t)ck * g.L;
+  const Mat<T> A{p.a + tok0 * p.D, p.a_scale ? p.a_scale + tok0 : nullptr, g.L, p.D, p.D}, B{p.b + tok0 * p.D, nullptr, g.L, p.D, p.D};
+  Acc pr;
+  pr.zero();
+  tile_product<VEC, true, true>(pr, A, r0, B, c0, p.D, buf, tid, NoEach());
+  float s[4][4], b_j[4], iota_j[4];
+  pr.get(s);
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const int c = c0 + 4 * tx + b;
+    b_j[b] = c < g.L ? g.vecB[tok0 + c] : 0.f;
+    iota_j[b] = c < g.L ? g.iota[tok0 + c] : 0.f;
+  }
+  float* out = p.out + (size_t)block * TILE * TILE;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int r = r0 + 4 * ty + a;
+    const float b_i = r < g.L ? g.vecB[tok0 + r] : 0.f, m_i = r < g.L ? g.m_tok[tok0 + r] : 0.f;
+    float v[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int c = c0 + 4 * tx + b;
+      v[b] = r < g.L && c <= r ? gate_score(s[a][b], g.qk_scale, b_i, b_j[b], iota_j[b], m_i) : 0.f;
+    }
+    *reinterpret_cast<float4*>(out + (4 * ty + a) * TILE + 4 * tx) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+// The products that need nothing but inputs and gate vectors, in one launch: the score blocks (the longer ones, first) and the
+// chunks' contributions of one recurrence or two.  Alone each of them is a launch of one wave or less, bound by load and
+// barrier latency; the score blocks ran in every output tile of their chunk, a quarter of the forward's multiply-adds and 43 % of
+// the backward's (B=2 NH=4 S=512 128/256, chunk 64, forward and backward phases in us: recurrences 42 and 21, now, with the
+// scores, 25 and 37; intra-chunk 35 and 81, now 23 and 50; the call 180 -> 136, same bits).
+template <typename T>
+struct PartArgs {
+  ScoreArgs<T> sc[2];
+  RecArgs<T> rec[2];
+  ScoreGate gate;
+  unsigned end[4];         // CTAs up to and with: sc[0], sc[1], rec[0], rec[1]
+  bool bwd[2];             // rec[i] is the state gradient's
+};
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(NTHR) part_kernel(const __grid_constant__ PartArgs<T> p) {
+  __shared__ __align__(16) float buf[4 * SLICE];
+  const unsigned x = blockIdx.x;
+  if (x < p.end[1]) {
+    const int i = x >= p.end[0];
+    score_tile<T, VEC>(p.sc[i], p.gate, i ? x - p.end[0] : x, buf);
+  } else {
+    const int i = x >= p.end[2];
+    rec_part_tile<T, VEC>(p.rec[i], p.bwd[i], x - p.end[1 + i], buf);
   }
 }
 
@@ -290,20 +374,33 @@ __device__ __forceinline__ void scan_elements(float* states, const float* init, 
   if (fin) c.store(fin + e);
 }
 
+struct ScanArgs {
+  float* c_states;
+  const float* c_init;
+  float *c_final, *n_states;
+  const float* n_init;
+  float* n_final;
+  int nblk;                // CTAs per (batch, head)
+};
 template <int V, bool BWD>
-__global__ void __launch_bounds__(128)
-rec_scan_kernel(float* c_states, const float* c_init, float* c_final, float* n_states, const float* n_init, float* n_final,
-                const float* gbar, int NC, int DHQK, int DHHV, int nblk) {
-  const int bh = blockIdx.x / nblk;
-  const size_t E = (size_t)DHQK * DHHV, t = (size_t)(blockIdx.x % nblk) * 128 + threadIdx.x;
+__device__ __forceinline__ void scan_tile(const ScanArgs& a, const float* gbar, int NC, int DHQK, int DHHV, const unsigned block) {
+  const int bh = block / a.nblk;
+  const size_t E = (size_t)DHQK * DHHV, t = (size_t)(block % a.nblk) * 128 + threadIdx.x;
   const float* g = gbar + (size_t)bh * NC;
   if (t * V < E) {
-    scan_elements<V, BWD>(c_states + (size_t)bh * (NC + 1) * E, c_init ? c_init + bh * E : nullptr,
-                          c_final ? c_final + bh * E : nullptr, g, E, t * V, NC);
-  } else if (!BWD && n_states != nullptr && t - (E + V - 1) / V < (size_t)DHQK) {   // threads past the tiles: n
-    scan_elements<1, BWD>(n_states + (size_t)bh * (NC + 1) * DHQK, n_init ? n_init + (size_t)bh * DHQK : nullptr,
-                          n_final ? n_final + (size_t)bh * DHQK : nullptr, g, DHQK, t - (E + V - 1) / V, NC);
+    scan_elements<V, BWD>(a.c_states + (size_t)bh * (NC + 1) * E, a.c_init ? a.c_init + bh * E : nullptr,
+                          a.c_final ? a.c_final + bh * E : nullptr, g, E, t * V, NC);
+  } else if (!BWD && a.n_states != nullptr && t - (E + V - 1) / V < (size_t)DHQK) {   // threads past the tiles: n
+    scan_elements<1, BWD>(a.n_states + (size_t)bh * (NC + 1) * DHQK, a.n_init ? a.n_init + (size_t)bh * DHQK : nullptr,
+                          a.n_final ? a.n_final + (size_t)bh * DHQK : nullptr, g, DHQK, t - (E + V - 1) / V, NC);
   }
+}
+// the first n_fw CTAs scan the forward's states, the others the gradient's
+template <int V>
+__global__ void __launch_bounds__(128)
+rec_scan_kernel(const ScanArgs fw, const ScanArgs bw, const unsigned n_fw, const float* gbar, int NC, int DHQK, int DHHV) {
+  if (blockIdx.x < n_fw) scan_tile<V, false>(fw, gbar, NC, DHQK, DHHV, blockIdx.x);
+  else scan_tile<V, true>(bw, gbar, NC, DHQK, DHHV, blockIdx.x - n_fw);
 }
 
 // Final state only, one CTA per tile walking the chunks.
@@ -370,6 +467,7 @@ struct ParArgs {
   const float* c_states;   // slot k used by H and DQ
   const float* dc_states;  // slot k+1 used by DV and DK
   const float* n_states;
+  const float *qk_blocks, *vh_blocks;   // gated score blocks (score_tile) of Q K^T and dHbar V^T, or null: computed by every output tile anew
   T *out_h, *out_dv, *out_dk, *out_dq;
   float* n_out;            // H only, may be null
   float* inv_den_out;      // H only, may be null
@@ -447,11 +545,45 @@ __device__ __forceinline__ void par_tile(const ParArgs<T>& p, const int mode, in
       acc.v[a][b] = f2(lo * rs[2 * a], hi * rs[2 * a + 1]);
     }
 
+  const float* blocks = QK ? p.qk_blocks : p.vh_blocks;
   const int nblk = (L + TILE - 1) / TILE;
   const int cb_lo = LOWER ? 0 : rb, cb_hi = LOWER ? rb : nblk - 1;
   for (int cb = cb_lo; cb <= cb_hi; ++cb) {
     const int c0 = cb * TILE;
     __syncthreads();   // the slices and the gated block of the previous round have been read
+    Slice<T, false, VEC> x0, x1;
+    if (blocks != nullptr) {
+      const Mat<float> P{blocks + ((size_t)bc * score_pairs(L) + (LOWER ? score_pair(rb, cb) : score_pair(cb, rb))) * TILE * TILE, nullptr,
+                         TILE, TILE, TILE};
+      x0.fetch(X, o0, c0, tid);
+      x1.fetch(X, o0, c0 + KSL, tid);
+      if (LOWER) {   // [i][j] -> [c = j][r = i]
+        Slice<float, true, true> p0, p1;
+        p0.fetch(P, 0, 0, tid);
+        p1.fetch(P, 0, KSL, tid);
+        p0.put(Ps, tid);
+        p1.put(Ps + SLICE, tid);
+      } else {       // [i][j] = [c][r]
+        Slice<float, false, true> p0, p1;
+        p0.fetch(P, 0, 0, tid);
+        p1.fetch(P, 0, KSL, tid);
+        p0.put(Ps, tid);
+        p1.put(Ps + SLICE, tid);
+      }
+      x0.put(buf, tid);
+      x1.put(buf + SLICE, tid);
+      __syncthreads();
+      if (FW) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const float4 v = *reinterpret_cast<const float4*>(Ps + swz(4 * tx + b, 4 * ty));
+          rowsum[0] += v.x; rowsum[1] += v.y; rowsum[2] += v.z; rowsum[3] += v.w;
+        }
+      }
+#pragma unroll 1
+      for (int u = 0; u < 2; ++u) mma_slice(acc, Ps + u * SLICE, buf + u * SLICE, ty, tx);
+      continue;
+    }
     Acc pr;
     pr.zero();
     tile_product<VEC, true, true>(pr, U, r0, W, c0, DI, buf, tid, NoEach());
@@ -466,7 +598,7 @@ __device__ __forceinline__ void par_tile(const ParArgs<T>& p, const int mode, in
         float val = 0.f;
         if (valid) {
           const int ii = LOWER ? r : c, jj = LOWER ? c : r;
-          val = p.qk_scale * s[a][b] * expf((s_b[ii] - s_b[jj]) + s_iota[jj] - s_m[ii]);
+          val = gate_score(s[a][b], p.qk_scale, s_b[ii], s_b[jj], s_iota[jj], s_m[ii]);
         }
         s[a][b] = val;
         if (FW) rowsum[a] += val;
@@ -475,7 +607,6 @@ __device__ __forceinline__ void par_tile(const ParArgs<T>& p, const int mode, in
     for (int b = 0; b < 4; ++b) {
       *reinterpret_cast<float4*>(Ps + swz(4 * tx + b, 4 * ty)) = make_float4(s[0][b], s[1][b], s[2][b], s[3][b]);
     }
-    Slice<T, false, VEC> x0, x1;
     x0.fetch(X, o0, c0, tid);
     x1.fetch(X, o0, c0 + KSL, tid);
     __syncthreads();   // every thread has left the score product: its slices are free
@@ -541,33 +672,44 @@ static size_t par_smem_bytes(int L, int DHQK) {
 // ---- launchers ----------------------------------------------------------------------------------------
 static bool vec_dims(const ChunkwiseDims& d) { return d.DHQK % 4 == 0 && d.DHHV % 4 == 0; }
 
-template <bool BWD>
-static int launch_rec_scan(float* c_states, const float* c_init, float* c_final, float* n_states, const float* n_init,
-                           float* n_final, const float* gbar, const ChunkwiseDims& d, cudaStream_t st) {
+// The chunks' contributions of one or two recurrences and the score blocks wanted, then the scans over the chunks.
+template <typename T>
+static int parts_t(PartArgs<T> a, int n_rec, const ChunkwiseDims& d, cudaStream_t st) {
+  PhaseScope ps(a.bwd[n_rec - 1] ? PH_REC_BW : PH_REC_FW, st);
+  const unsigned bnc = (unsigned)(d.B * d.NH) * (unsigned)d.NC;
+  const unsigned tiles = (unsigned)ceil_div(d.DHHV, TILE) * ceil_div(d.DHQK, TILE) * bnc, pairs = (unsigned)score_pairs(d.L) * bnc;
+  a.end[0] = a.sc[0].out ? pairs : 0;
+  a.end[1] = a.end[0] + (a.sc[1].out ? pairs : 0);
+  a.end[2] = a.end[1] + tiles;
+  a.end[3] = a.end[2] + (n_rec > 1 ? tiles : 0);
+  if (vec_dims(d)) part_kernel<T, true><<<a.end[3], NTHR, 0, st>>>(a);
+  else part_kernel<T, false><<<a.end[3], NTHR, 0, st>>>(a);
+  MLSTM_LAUNCH_CHECK();
   const size_t E = (size_t)d.DHQK * d.DHHV;
   const int V = E % 4 == 0 ? 4 : 1;
-  const int nblk = (int)((E / V + (n_states ? d.DHQK : 0) + 127) / 128);
-  const unsigned grid = (unsigned)nblk * (unsigned)(d.B * d.NH);
-  if (V == 4) rec_scan_kernel<4, BWD><<<grid, 128, 0, st>>>(c_states, c_init, c_final, n_states, n_init, n_final, gbar, d.NC, d.DHQK, d.DHHV, nblk);
-  else rec_scan_kernel<1, BWD><<<grid, 128, 0, st>>>(c_states, c_init, c_final, n_states, n_init, n_final, gbar, d.NC, d.DHQK, d.DHHV, nblk);
+  ScanArgs scan[2] = {};   // forward, backward
+  unsigned n[2] = {0, 0};
+  const float* gbar = a.rec[0].gbar;
+  for (int i = 0; i < n_rec; ++i) {
+    const RecArgs<T>& r = a.rec[i];
+    const int nblk = (int)((E / V + (!a.bwd[i] && r.n_states ? d.DHQK : 0) + 127) / 128);
+    scan[a.bwd[i]] = ScanArgs{r.c_states, r.c_init, r.c_final, r.n_states, r.n_init, r.n_final, nblk};
+    n[a.bwd[i]] = (unsigned)nblk * (unsigned)(d.B * d.NH);
+  }
+  if (V == 4) rec_scan_kernel<4><<<n[0] + n[1], 128, 0, st>>>(scan[0], scan[1], n[0], gbar, d.NC, d.DHQK, d.DHHV);
+  else rec_scan_kernel<1><<<n[0] + n[1], 128, 0, st>>>(scan[0], scan[1], n[0], gbar, d.NC, d.DHQK, d.DHHV);
   MLSTM_LAUNCH_CHECK();
   return MLSTM_OK;
 }
 
 template <typename T, bool BWD>
-static int rec_t(const RecArgs<T>& a, const ChunkwiseDims& d, cudaStream_t st) {
+static int rec_final_t(const RecArgs<T>& a, const ChunkwiseDims& d, cudaStream_t st) {
   PhaseScope ps(BWD ? PH_REC_BW : PH_REC_FW, st);
   const unsigned tiles = (unsigned)ceil_div(d.DHHV, TILE) * ceil_div(d.DHQK, TILE) * (unsigned)(d.B * d.NH);
-  if (a.c_states == nullptr) {
-    if (vec_dims(d)) rec_final_kernel<T, BWD, true><<<tiles, NTHR, 0, st>>>(a);
-    else rec_final_kernel<T, BWD, false><<<tiles, NTHR, 0, st>>>(a);
-    MLSTM_LAUNCH_CHECK();
-    return MLSTM_OK;
-  }
-  if (vec_dims(d)) rec_part_kernel<T, BWD, true><<<tiles * (unsigned)d.NC, NTHR, 0, st>>>(a);
-  else rec_part_kernel<T, BWD, false><<<tiles * (unsigned)d.NC, NTHR, 0, st>>>(a);
+  if (vec_dims(d)) rec_final_kernel<T, BWD, true><<<tiles, NTHR, 0, st>>>(a);
+  else rec_final_kernel<T, BWD, false><<<tiles, NTHR, 0, st>>>(a);
   MLSTM_LAUNCH_CHECK();
-  return launch_rec_scan<BWD>(a.c_states, a.c_init, a.c_final, a.n_states, a.n_init, a.n_final, a.gbar, d, st);
+  return MLSTM_OK;
 }
 
 template <typename T>
@@ -604,36 +746,70 @@ static ParArgs<T> par_args(const void* q, const void* k, const void* v, const Ga
   }                                                                         \
   return MLSTM_ERR_DTYPE;
 
-int simt_recurrent_fw(int dtype, const void* k, const void* v, const GateBuffers& gb, const float* c_initial,
-                      const float* n_initial, void* c_states, float* n_states, float* c_last, float* n_last,
+// Scratch for the score blocks of a forward (one product) or a backward (two); 0 where they are not used.  A chunk of 64 or 128
+// tokens has one or three blocks of 16 KB, used by every output tile of it.  Shorter chunks would mostly store padding, longer
+// ones and small head dims would need more room than their states.
+size_t simt_score_bytes(const ChunkwiseDims& d, bool backward) {
+  if ((d.L != TILE && d.L != 2 * TILE) || d.DHQK * d.DHHV < score_pairs(d.L) * TILE * TILE) return 0;
+  return (size_t)(backward ? 2 : 1) * d.B * d.NH * d.NC * score_pairs(d.L) * TILE * TILE * sizeof(float);
+}
+
+static ScoreGate score_gate(const GateBuffers& gb, const ChunkwiseDims& d) {
+  return ScoreGate{gb.vecB, gb.iota, gb.m_tok, d.S, d.L, d.NC, d.qk_scale};
+}
+
+int simt_recurrent_fw(int dtype, const void* q, const void* k, const void* v, const GateBuffers& gb, const float* c_initial,
+                      const float* n_initial, void* c_states, float* n_states, float* c_last, float* n_last, float* scores,
                       const ChunkwiseDims& d, cudaStream_t st) {
   MLSTM_DISPATCH(dtype, {
-    return rec_t<T, false>(RecArgs<T>{(const T*)k, (const T*)v, gb.abar, nullptr, gb.gbar, 1.f, c_initial, n_initial,
-                                      (float*)c_states, n_states, c_last, n_last, d.S, d.L, d.NC, d.DHQK, d.DHHV}, d, st);
+    const RecArgs<T> r{(const T*)k, (const T*)v, gb.abar, nullptr, gb.gbar, 1.f, c_initial, n_initial,
+                       (float*)c_states, n_states, c_last, n_last, d.S, d.L, d.NC, d.DHQK, d.DHHV};
+    if (c_states == nullptr) return rec_final_t<T, false>(r, d, st);
+    PartArgs<T> a{};
+    a.rec[0] = r;
+    a.gate = score_gate(gb, d);
+    a.sc[0] = ScoreArgs<T>{(const T*)q, (const T*)k, nullptr, scores, d.DHQK};
+    return parts_t<T>(a, 1, d, st);
   })
 }
 int simt_parallel_fw(int dtype, const void* q, const void* k, const void* v, const GateBuffers& gb, const void* c_states,
-                     const float* n_states, void* h, float* n_out, const ChunkwiseDims& d, cudaStream_t st) {
+                     const float* n_states, void* h, float* n_out, const float* scores, const ChunkwiseDims& d, cudaStream_t st) {
   MLSTM_DISPATCH(dtype, {
     auto a = par_args<T>(q, k, v, gb, c_states, d);
-    a.n_states = n_states; a.out_h = (T*)h; a.n_out = n_out; a.inv_den_out = gb.inv_den;
+    a.n_states = n_states; a.out_h = (T*)h; a.n_out = n_out; a.inv_den_out = gb.inv_den; a.qk_blocks = scores;
     return par_t<T>(a, false, d, st);
   })
 }
-int simt_recurrent_bw(int dtype, const void* q, const void* dh, const GateBuffers& gb, const float* dc_last, void* dc_states,
-                      float* dc_initial, const ChunkwiseDims& d, cudaStream_t st) {
+int simt_recurrent_bw(int dtype, const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb, const float* dc_last,
+                      void* dc_states, float* dc_initial, const float* c_initial, void* c_states, float* scores,
+                      const ChunkwiseDims& d, cudaStream_t st) {
   MLSTM_DISPATCH(dtype, {
-    return rec_t<T, true>(RecArgs<T>{(const T*)q, (const T*)dh, gb.bbar, gb.inv_den, gb.gbar, d.qk_scale, dc_last, nullptr,
-                                     (float*)dc_states, nullptr, dc_initial, nullptr, d.S, d.L, d.NC, d.DHQK, d.DHHV}, d, st);
+    const RecArgs<T> r{(const T*)q, (const T*)dh, gb.bbar, gb.inv_den, gb.gbar, d.qk_scale, dc_last, nullptr,
+                       (float*)dc_states, nullptr, dc_initial, nullptr, d.S, d.L, d.NC, d.DHQK, d.DHHV};
+    if (dc_states == nullptr) return rec_final_t<T, true>(r, d, st);
+    PartArgs<T> a{};
+    int n = 0;
+    if (c_states != nullptr)   // the forward's states again
+      a.rec[n++] = RecArgs<T>{(const T*)k, (const T*)v, gb.abar, nullptr, gb.gbar, 1.f, c_initial, nullptr, (float*)c_states, nullptr, nullptr, nullptr,
+                              d.S, d.L, d.NC, d.DHQK, d.DHHV};
+    a.bwd[n] = true;
+    a.rec[n++] = r;
+    a.gate = score_gate(gb, d);
+    if (scores != nullptr) {
+      a.sc[0] = ScoreArgs<T>{(const T*)dh, (const T*)v, gb.inv_den, scores + simt_score_bytes(d, false) / sizeof(float), d.DHHV};
+      a.sc[1] = ScoreArgs<T>{(const T*)q, (const T*)k, nullptr, scores, d.DHQK};
+    }
+    return parts_t<T>(a, n, d, st);
   })
 }
 int simt_parallel_bw(int dtype, const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
-                     const void* c_states, const void* dc_states, void* dq, void* dk, void* dv, const ChunkwiseDims& d,
-                     cudaStream_t st) {
+                     const void* c_states, const void* dc_states, void* dq, void* dk, void* dv, const float* scores,
+                     const ChunkwiseDims& d, cudaStream_t st) {
   MLSTM_DISPATCH(dtype, {
     auto a = par_args<T>(q, k, v, gb, c_states, d);
     a.dh = (const T*)dh; a.dc_states = (const float*)dc_states;
     a.out_dq = (T*)dq; a.out_dk = (T*)dk; a.out_dv = (T*)dv;
+    if (scores != nullptr) { a.qk_blocks = scores; a.vh_blocks = scores + simt_score_bytes(d, false) / sizeof(float); }
     return par_t<T>(a, true, d, st);
   })
 }

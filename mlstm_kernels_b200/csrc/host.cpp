@@ -147,6 +147,8 @@ Forward run_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   if (!(for_backward && keep_states)) need += up256(p.states_bytes);
   const size_t ws_at = need;
   if (!for_backward) need += p.fw_bytes;
+  const size_t scores_bytes = mlstm::score_scratch_bytes(p.c, false), scores_at = up256(need);
+  if (scores_bytes > 0) need = scores_at + scores_bytes;
   const Tensor scratch = bytes(need, dev);
   char* sp = static_cast<char*>(scratch.mutable_data_ptr());
   if (for_backward) out.kept = bytes(p.fw_bytes + p.inv_den_bytes, dev);
@@ -160,7 +162,7 @@ Forward run_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
       reinterpret_cast<float*>(sp), reinterpret_cast<float*>(sp + up256(p.n_states_bytes)),
       fout(out.c_last), fout(out.n_last), fout(out.m_last),
       for_backward ? reinterpret_cast<float*>(kp + p.fw_bytes) : nullptr,
-      for_backward ? kp : sp + ws_at, p.fw_bytes, true};
+      for_backward ? kp : sp + ws_at, p.fw_bytes, true, scores_bytes > 0 ? sp + scores_at : nullptr};
   check(mlstm::run_chunkwise_fw(a, p.c), "mlstm_b200_chunkwise_fw");
   return out;
 }
@@ -205,7 +207,8 @@ class ChunkwiseFn : public torch::autograd::Function<ChunkwiseFn> {
     const Tensor di = empty(i.sizes(), i.scalar_type(), dev), df = empty(i.sizes(), i.scalar_type(), dev);
     const Tensor dc0 = cfg[3] >= 0 ? empty({c.B, c.NH, c.DHQK, c.DHHV}, at::kFloat, dev) : Tensor();
     const size_t ws_bytes = up256(mlstm_b200_chunkwise_workspace_bytes(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, c.variant, c.impl, 1));
-    const Tensor ws = bytes(ws_bytes + (states.defined() ? 0 : p.states_bytes), dev);
+    const size_t scores_bytes = mlstm::score_scratch_bytes(c, true), scores_at = up256(ws_bytes + (states.defined() ? 0 : p.states_bytes));
+    const Tensor ws = bytes(scores_at + scores_bytes, dev);
     char* wp = static_cast<char*>(ws.mutable_data_ptr());
     const char* kp = static_cast<const char*>(kept.const_data_ptr());
     const Tensor rc0 = f32c(c0);
@@ -214,7 +217,7 @@ class ChunkwiseFn : public torch::autograd::Function<ChunkwiseFn> {
         ptr(q), ptr(k), ptr(v), ptr(i), ptr(f), fptr(m0), ptr(states), states.defined() ? nullptr : wp + ws_bytes,
         fptr(rc0), nullptr, reinterpret_cast<const float*>(kp + p.fw_bytes), kp, p.fw_bytes, ptr(dh), fptr(dc_last),
         dq.mutable_data_ptr(), dk.mutable_data_ptr(), dv.mutable_data_ptr(), di.mutable_data_ptr(), df.mutable_data_ptr(),
-        c.gate_dtype, fout(dc0), wp, ws_bytes};
+        c.gate_dtype, fout(dc0), wp, ws_bytes, scores_bytes > 0 ? wp + scores_at : nullptr};
     check(mlstm::run_chunkwise_bw(a, p.c), "mlstm_b200_chunkwise_bw");
     if (g_check_status && mlstm_b200_device_status(1) != 0)
       TORCH_CHECK(false, "mlstm_kernels_b200: a bounded wait of the tcgen05 kernels ran out; results invalid");

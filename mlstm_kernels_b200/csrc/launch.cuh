@@ -24,17 +24,20 @@ int launch_state_dot(const void* c_states, const void* dc_states, float* anchors
                      const ChunkwiseDims& d, cudaStream_t st);
 
 // chunkwise_simt.cu : portable CUDA-core kernels, any shape, any element type
-int simt_recurrent_fw(int dtype, const void* k, const void* v, const GateBuffers& gb,
+// scores (nullable): scratch of simt_score_bytes(), filled by the recurrence's launch and read by the intra-chunk kernel
+size_t simt_score_bytes(const ChunkwiseDims& d, bool backward);
+int simt_recurrent_fw(int dtype, const void* q, const void* k, const void* v, const GateBuffers& gb,
                       const float* c_initial, const float* n_initial, void* c_states, float* n_states,
-                      float* c_last, float* n_last, const ChunkwiseDims& d, cudaStream_t st);
+                      float* c_last, float* n_last, float* scores, const ChunkwiseDims& d, cudaStream_t st);
 int simt_parallel_fw(int dtype, const void* q, const void* k, const void* v, const GateBuffers& gb,
-                     const void* c_states, const float* n_states, void* h, float* n_out, const ChunkwiseDims& d,
+                     const void* c_states, const float* n_states, void* h, float* n_out, const float* scores, const ChunkwiseDims& d,
                      cudaStream_t st);
-int simt_recurrent_bw(int dtype, const void* q, const void* dh, const GateBuffers& gb,
-                      const float* dc_last, void* dc_states, float* dc_initial, const ChunkwiseDims& d,
-                      cudaStream_t st);
+// c_states (nullable): where the forward's per-chunk states are written again, from c_initial
+int simt_recurrent_bw(int dtype, const void* q, const void* k, const void* v, const void* dh, const GateBuffers& gb,
+                      const float* dc_last, void* dc_states, float* dc_initial, const float* c_initial, void* c_states, float* scores,
+                      const ChunkwiseDims& d, cudaStream_t st);
 int simt_parallel_bw(int dtype, const void* q, const void* k, const void* v, const void* dh,
-                     const GateBuffers& gb, const void* c_states, const void* dc_states, void* dq, void* dk, void* dv,
+                     const GateBuffers& gb, const void* c_states, const void* dc_states, void* dq, void* dk, void* dv, const float* scores,
                      const ChunkwiseDims& d, cudaStream_t st);
 
 // chunkwise_sm100.cu : tcgen05 + TMA kernels (bf16 / fp16, L = 128, head dims multiples of 8)

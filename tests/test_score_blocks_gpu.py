@@ -1,0 +1,35 @@
+"""Portable kernels with the score blocks of a chunk computed once (what the PyTorch functions do where it pays) and with every
+output tile computing them anew (calls without that scratch): the same bits."""
+
+import pytest
+import torch
+
+from mlstm_kernels_b200 import _lib
+from mlstm_kernels_b200.chunkwise import (chunkwise_bw_raw, chunkwise_fw_raw, mlstm_chunkwise__b200_xl_chunk,
+                                          mlstm_siging_chunkwise__b200_xl_chunk)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("DHQK, DHHV", [(64, 64), (128, 256), (96, 128), (65, 190), (130, 100)])   # smallest, partial tiles, single elements
+@pytest.mark.parametrize("L", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("variant, recompute", [(_lib.EXP, True), (_lib.SIG, False), (_lib.SIG_NONORM, True)])
+def test_score_blocks_equal_scores_per_tile(DHQK, DHHV, L, dtype, variant, recompute):
+    B, NH, S = 2, 3, 3 * L
+    g = torch.Generator(device="cuda").manual_seed(DHQK + L)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k, v, dh = (rnd(B, NH, S, d).to(dtype) for d in (DHQK, DHQK, DHHV, DHHV))
+    i, f = rnd(B, NH, S), rnd(B, NH, S) + 3.0
+    kw = dict(chunk_size=L, impl="simt", eps=1e-6)
+    fw = chunkwise_fw_raw(q, k, v, i, f, variant=variant, **kw)
+    bw = chunkwise_bw_raw(q, k, v, i, f, None, fw["C_states"], fw["n_out"], dh, variant=variant, **kw)
+    x = [t.clone().requires_grad_(True) for t in (q, k, v, i, f)]
+    if variant == _lib.EXP:
+        h = mlstm_chunkwise__b200_xl_chunk(*x, recompute_states_in_bw=recompute, **kw)
+    else:
+        h = mlstm_siging_chunkwise__b200_xl_chunk(*x, normalize=variant == _lib.SIG, recompute_states_in_bw=recompute, **kw)
+    assert torch.equal(h, fw["H"])
+    grads = torch.autograd.grad(h, x, dh)
+    for a, b in zip(grads[:3], bw[:3]):
+        assert torch.equal(a, b)
