@@ -322,6 +322,8 @@ struct PartArgs {
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(NTHR) part_kernel(const __grid_constant__ PartArgs<T> p) {
   __shared__ __align__(16) float buf[4 * SLICE];
+  pdl_launch_dependents();
+  pdl_wait();
   const unsigned x = blockIdx.x;
   if (x < p.end[1]) {
     const int i = x >= p.end[0];
@@ -399,6 +401,8 @@ __device__ __forceinline__ void scan_tile(const ScanArgs& a, const float* gbar, 
 template <int V>
 __global__ void __launch_bounds__(128)
 rec_scan_kernel(const ScanArgs fw, const ScanArgs bw, const unsigned n_fw, const float* gbar, int NC, int DHQK, int DHHV) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (blockIdx.x < n_fw) scan_tile<V, false>(fw, gbar, NC, DHQK, DHHV, blockIdx.x);
   else scan_tile<V, true>(bw, gbar, NC, DHQK, DHHV, blockIdx.x - n_fw);
 }
@@ -453,7 +457,7 @@ __global__ void __launch_bounds__(NTHR) rec_final_kernel(RecArgs<T> p) {
 //   DV    K        Q        (c,r)   dHbar    abar            dC_{k+1}[a][o]
 //   DK    V        dHbar    (c,r)   Q        abar            dC_{k+1}[o][a]
 //   DQ    dHbar    V        (r,c)   K        qk_scale*bbar   C_k[o][a]
-// dHbar = deltaH / (den + eps).  grid (output tiles x B*NH*NC, ceil(L/64)); the backward's three modes share a launch
+// dHbar = deltaH / (den + eps).  1-D grid (output tiles x 64-row blocks of the chunk x B*NH*NC); the backward's three modes share a launch
 // (their CTAs fill each other's last wave and find a chunk's operands in L2).
 // The contraction runs on CUDA cores in exact f32: 64 x 64 tiles of the product above, at B=2 NH=4 S=512 128/256 a few
 // hundred CTAs of a few million multiply-adds each.
@@ -651,18 +655,22 @@ __device__ __forceinline__ void par_tile(const ParArgs<T>& p, const int mode, in
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(NTHR, 3) par_fw_kernel(ParArgs<T> p) {
   extern __shared__ __align__(16) float smem[];
-  const int n_ot = (p.DHHV + TILE - 1) / TILE;
-  par_tile<T, true, VEC>(p, PAR_H, blockIdx.x % n_ot, blockIdx.x / n_ot, blockIdx.y, smem);
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n_ot = (p.DHHV + TILE - 1) / TILE, n_rb = (p.L + TILE - 1) / TILE, y = blockIdx.x / n_ot;
+  par_tile<T, true, VEC>(p, PAR_H, blockIdx.x % n_ot, y / n_rb, y % n_rb, smem);
 }
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(NTHR, 3) par_bw_kernel(ParArgs<T> p) {
   extern __shared__ __align__(16) float smem[];
+  pdl_launch_dependents();
+  pdl_wait();
   const int n_v = (p.DHHV + TILE - 1) / TILE, n_k = (p.DHQK + TILE - 1) / TILE;
-  const int n = n_v + 2 * n_k, x = blockIdx.x % n, bc = blockIdx.x / n;
+  const int n = n_v + 2 * n_k, n_rb = (p.L + TILE - 1) / TILE, x = blockIdx.x % n, y = blockIdx.x / n;
   // the modes with the longer contraction first
   const int mode = x < n_k ? PAR_DK : x < 2 * n_k ? PAR_DQ : PAR_DV;
-  par_tile<T, false, VEC>(p, mode, x < n_k ? x : x < 2 * n_k ? x - n_k : x - 2 * n_k, bc, blockIdx.y, smem);
+  par_tile<T, false, VEC>(p, mode, x < n_k ? x : x < 2 * n_k ? x - n_k : x - 2 * n_k, y / n_rb, y % n_rb, smem);
 }
 
 static size_t par_smem_bytes(int L, int DHQK) {
@@ -682,9 +690,7 @@ static int parts_t(PartArgs<T> a, int n_rec, const ChunkwiseDims& d, cudaStream_
   a.end[1] = a.end[0] + (a.sc[1].out ? pairs : 0);
   a.end[2] = a.end[1] + tiles;
   a.end[3] = a.end[2] + (n_rec > 1 ? tiles : 0);
-  if (vec_dims(d)) part_kernel<T, true><<<a.end[3], NTHR, 0, st>>>(a);
-  else part_kernel<T, false><<<a.end[3], NTHR, 0, st>>>(a);
-  MLSTM_LAUNCH_CHECK();
+  if (int rc = launch_pdl(a.end[3] <= pdl_max_ctas(), vec_dims(d) ? part_kernel<T, true> : part_kernel<T, false>, a.end[3], NTHR, 0, st, a)) return rc;
   const size_t E = (size_t)d.DHQK * d.DHHV;
   const int V = E % 4 == 0 ? 4 : 1;
   ScanArgs scan[2] = {};   // forward, backward
@@ -696,10 +702,9 @@ static int parts_t(PartArgs<T> a, int n_rec, const ChunkwiseDims& d, cudaStream_
     scan[a.bwd[i]] = ScanArgs{r.c_states, r.c_init, r.c_final, r.n_states, r.n_init, r.n_final, nblk};
     n[a.bwd[i]] = (unsigned)nblk * (unsigned)(d.B * d.NH);
   }
-  if (V == 4) rec_scan_kernel<4><<<n[0] + n[1], 128, 0, st>>>(scan[0], scan[1], n[0], gbar, d.NC, d.DHQK, d.DHHV);
-  else rec_scan_kernel<1><<<n[0] + n[1], 128, 0, st>>>(scan[0], scan[1], n[0], gbar, d.NC, d.DHQK, d.DHHV);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  const unsigned grid = n[0] + n[1];
+  return launch_pdl(grid <= pdl_max_ctas(), V == 4 ? rec_scan_kernel<4> : rec_scan_kernel<1>, grid, 128, 0, st, scan[0], scan[1], n[0], gbar, d.NC,
+                    d.DHQK, d.DHHV);
 }
 
 template <typename T, bool BWD>
@@ -717,13 +722,11 @@ static int par_t(ParArgs<T>& a, bool backward, const ChunkwiseDims& d, cudaStrea
   PhaseScope ps(backward ? PH_PAR_BW : PH_PAR_FW, st);
   const size_t smem = par_smem_bytes(d.L, d.DHQK);
   const int n_v = ceil_div(d.DHHV, TILE), n_k = ceil_div(d.DHQK, TILE);
-  const dim3 grid((unsigned)(backward ? n_v + 2 * n_k : n_v) * (unsigned)(d.B * d.NH * d.NC), ceil_div(d.L, TILE));
+  const unsigned grid = (unsigned)(backward ? n_v + 2 * n_k : n_v) * (unsigned)(d.B * d.NH * d.NC) * (unsigned)ceil_div(d.L, TILE);
   auto kern = vec_dims(d) ? (backward ? par_bw_kernel<T, true> : par_fw_kernel<T, true>)
                           : (backward ? par_bw_kernel<T, false> : par_fw_kernel<T, false>);
   MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<grid, NTHR, smem, st>>>(a);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  return launch_pdl(grid <= pdl_max_ctas(), kern, grid, NTHR, smem, st, a);
 }
 
 template <typename T>

@@ -204,9 +204,10 @@ gates_kernel(const T* vecI, const T* vecF, const float* n_out, float* __restrict
 // mlstm_kernels/torch/chunkwise/triton_xl_chunk/chunkwise_gates.py:68-95. One warp per token.
 template <typename T>
 __global__ void __launch_bounds__(256)
-gate_grad_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ dq,
-                      const T* __restrict__ dk, float* __restrict__ acc, float* __restrict__ kdk,
+gate_grad_rows_kernel(const T* q, const T* k, const T* dq, const T* dk, float* __restrict__ acc, float* __restrict__ kdk,
                       size_t ntok, int DHQK) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t tok = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (tok >= ntok) return;
   const int lane = threadIdx.x & 31;
@@ -244,10 +245,11 @@ __device__ __forceinline__ void store_gate_grad(void* p, size_t idx, float x, in
 constexpr int kScanThreads = 1024;
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads)
-gate_grad_scan_kernel(const T* __restrict__ vecI, const T* __restrict__ vecF, const float* __restrict__ qdq,
-                      const float* __restrict__ kdk, void* __restrict__ dI, void* __restrict__ dF,
+gate_grad_scan_kernel(const T* vecI, const T* vecF, const float* qdq, const float* kdk, void* __restrict__ dI, void* __restrict__ dF,
                       int out_dtype, int S, int SP, int variant, int nparts, size_t part_stride) {
   __shared__ float s_part[kScanThreads];
+  pdl_launch_dependents();
+  pdl_wait();
   const int bh = blockIdx.x, t = threadIdx.x;
   const size_t base = (size_t)bh * S;      // gate logits and outputs: S tokens per (batch, head)
   const size_t pbase = (size_t)bh * SP;    // row sums: SP slots per (batch, head)
@@ -419,10 +421,9 @@ template <typename T>
 int launch_gate_grad_rows_t(const void* q, const void* k, const void* dq, const void* dk, float* acc, float* kdk,
                             const ChunkwiseDims& d, cudaStream_t st) {
   const size_t ntok = (size_t)d.B * d.NH * d.S;
-  gate_grad_rows_kernel<T><<<(unsigned)((ntok + 7) / 8), 256, 0, st>>>((const T*)q, (const T*)k, (const T*)dq,
-                                                                        (const T*)dk, acc, kdk, ntok, d.DHQK);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  const unsigned grid = (unsigned)((ntok + 7) / 8);
+  return launch_pdl(grid <= pdl_max_ctas(), gate_grad_rows_kernel<T>, grid, 256, 0, st, (const T*)q, (const T*)k, (const T*)dq, (const T*)dk,
+                    acc, kdk, ntok, d.DHQK);
 }
 
 
@@ -518,12 +519,10 @@ static int gate_grad_scan_t(const void* i, const void* f, const float* qdq, cons
     const unsigned grid = (unsigned)ceil_div(d.S, kAnchorThreads) * (unsigned)(d.B * d.NH);
     return launch_pdl(grid <= pdl_max_ctas(), gate_grad_anchored_kernel<T>, grid, kAnchorThreads, 0, st, (const T*)i, (const T*)f, qdq,
                       kdk, dI, dF, out_dtype, d.S, d.SP, d.variant, nparts, stride, anchors, n_anchors);
-  } else {
-    gate_grad_scan_kernel<T><<<d.B * d.NH, kScanThreads, 0, st>>>((const T*)i, (const T*)f, qdq, kdk, dI, dF, out_dtype, d.S, d.SP,
-                                                                  d.variant, nparts, stride);
   }
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  const unsigned grid = (unsigned)(d.B * d.NH);
+  return launch_pdl(grid <= pdl_max_ctas(), gate_grad_scan_kernel<T>, grid, kScanThreads, 0, st, (const T*)i, (const T*)f, qdq, kdk, dI, dF,
+                    out_dtype, d.S, d.SP, d.variant, nparts, stride);
 }
 
 int launch_gate_grad_scan(int dtype, const void* i, const void* f, const float* qdq, const float* kdk, int nparts,
