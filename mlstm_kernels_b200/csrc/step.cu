@@ -8,6 +8,7 @@
 // One CTA owns all DHQK rows of a TV-wide column slice of one (batch, head): the q.C' reduction is
 // local to the CTA; q.n' is recomputed per CTA (DHQK values, negligible).
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "launch.cuh"
 
 namespace mlstm {
@@ -169,20 +170,28 @@ step_kernel(const T* q, const T* k, const T* v, const void* gi, const void* gf, 
 // ROWS rows of four columns.  Tokens go through in blocks of SEQ_TB.  What a block needs besides C - gates and their
 // max-state recursion, scaled q and k, v, q.n' - is prepared for the whole block at once (one exposed load latency and
 // three barriers per block), the token loop itself runs on registers and broadcast shared-memory reads without a
-// barrier, and the partial h of the block's tokens are summed over the warps together.  Token by token with five
-// barriers and a load latency each it took 4.3 us per token (4 sequences x 13 tokens, 8 heads 256/512: 56.5 us, of which
-// the state traffic is 5.3); in blocks 24.1 us.  Bound by latency: a block's loads, preparation, token loop and reduction
-// follow one another (issue slots 42 % busy, the FMA pipe 26 %, memory less).
+// barrier, and the partial h of the block's tokens are summed over the warps together.  Bound by latency and the issue
+// slots: a block's loads, preparation, token loop and reduction follow one another.  What the parts gave, as time per call
+// (bf16, 8 heads 256/512 unless stated):
+//   token by token with five barriers and a load latency each: 56.5 us for 4 sequences x 13 tokens; in blocks 22.7, and
+//   39.1 for 1 x 64, 604 for 16 x 64 with 16 heads.
+//   All loads of a block before its first store to shared memory, packed multiply-adds (half the issue slots, the same
+//   roundings), the next launch started while this one drains: 20.0 / 41.1 / 558.
+//   No test of the row within the token loop where DHQK fills the rows (it kept a row's read of q and k behind the
+//   multiply-adds of the row before), two tokens unrolled: 1 x 64 41.1 -> 26.8.
+//   At most eight rows per thread up to DHQK = 256 and sixteen up to 512, by narrower slices (see the launch): 19.0 / 26.8 /
+//   490; 8 x 16 tokens, DHQK 512: 151 -> 83.
+// Two CTAs per SM hide a good part of the chain: left to itself the compiler takes more than 128 registers for the
+// sixteen-row form, and bounded by one CTA per SM for the eight-row form too (490 -> 775).
 constexpr int SEQ_TB = 8;
 
 template <typename T, int ROWS, int TV>
-__global__ void __launch_bounds__(STEP_THREADS)
-step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                     const void* __restrict__ gi, const void* __restrict__ gf, int gate_dtype, const float* __restrict__ c,
-                     const float* __restrict__ n, const float* __restrict__ m, T* __restrict__ h,
-                     float* __restrict__ c_new, float* __restrict__ n_new, float* __restrict__ m_new, int Tn, int DHQK,
-                     int DHHV, float eps) {
+__global__ void __launch_bounds__(STEP_THREADS, 2)
+step_sequence_kernel(const T* q, const T* k, const T* v, const void* gi, const void* gf, int gate_dtype, const float* c,
+                     const float* n, const float* m, T* __restrict__ h, float* __restrict__ c_new, float* __restrict__ n_new,
+                     float* __restrict__ m_new, int Tn, int DHQK, int DHHV, float eps) {
   constexpr int CG = TV / 4, RG = STEP_THREADS / CG, NW = STEP_THREADS / 32;
+  constexpr int NV = SEQ_TB * TV / STEP_THREADS;               // elements of v per thread and block
   constexpr int ND = ROWS * RG > STEP_THREADS ? 2 : 1;         // rows per thread of the q, k, n work
   extern __shared__ __align__(16) float sm[];
   float* s_v = sm;                                             // [SEQ_TB][TV]
@@ -198,12 +207,15 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
   const int e = e0 + cgi * 4;
   const float scale = rsqrtf((float)DHQK);
 
-  float4 C[ROWS];
+  pdl_launch_dependents();
+  pdl_wait();
+  uint64_t C[ROWS][2];   // four columns of a row, in pairs
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     const int d = rg + r * RG;
-    C[r] = (c && d < DHQK && e < DHHV) ? __ldcs(reinterpret_cast<const float4*>(c + ((size_t)bh * DHQK + d) * DHHV + e))
-                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 x = (c && d < DHQK && e < DHHV) ? ld_stream(reinterpret_cast<const float4*>(c + ((size_t)bh * DHQK + d) * DHHV + e))
+                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+    C[r][0] = f2(x.x, x.y); C[r][1] = f2(x.z, x.w);
   }
   float nv[ND];
 #pragma unroll
@@ -216,7 +228,7 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
   for (int t0 = 0; t0 < Tn; t0 += SEQ_TB) {
     const int nt = min(SEQ_TB, Tn - t0);
     const size_t tok0 = (size_t)bh * Tn + t0;
-    // raw operands of the block first: all loads of a thread in flight together
+    // raw operands of the block first, before anything is stored: all loads of a thread in flight together
     T qr[ND][SEQ_TB], kr[ND][SEQ_TB];
 #pragma unroll
     for (int u = 0; u < ND; ++u)
@@ -228,16 +240,21 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
           kr[u][t] = k[(tok0 + t) * DHQK + d];
         }
       }
-    for (int idx = tid; idx < nt * TV; idx += STEP_THREADS) {
-      const int t = idx / TV, col = e0 + idx % TV;
-      s_v[idx] = col < DHHV ? to_f32(v[(tok0 + t) * DHHV + col]) : 0.f;
+    float vr[NV];
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      const int t = (tid + u * STEP_THREADS) / TV, col = e0 + tid % TV;
+      vr[u] = (t < nt && col < DHHV) ? to_f32(v[(tok0 + t) * DHHV + col]) : 0.f;
     }
     // gates: lane t holds token t of the block (every warp for itself); the recursion hands m from lane to lane
     float lf = 0.f, iv = 0.f;
     if (lane < nt) {
-      lf = logsigmoid_f(load_gate(gf, tok0 + lane, gate_dtype));
+      lf = load_gate(gf, tok0 + lane, gate_dtype);
       iv = load_gate(gi, tok0 + lane, gate_dtype);
+      lf = logsigmoid_f(lf);
     }
+#pragma unroll
+    for (int u = 0; u < NV; ++u) s_v[tid + u * STEP_THREADS] = vr[u];
     float m_prev = 0.f, m_tok = 0.f;
     for (int t = 0; t < nt; ++t) {
       const float m_n = fmaxf(__shfl_sync(0xffffffffu, lf, t) + m_run, __shfl_sync(0xffffffffu, iv, t));
@@ -278,24 +295,26 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
     qn[0] += __shfl_xor_sync(0xffffffffu, qn[0], 1);
     if ((lane & 3) == 0) s_qn[lane >> 2][warp] = qn[0];   // bits 4, 3, 2 of the lane spell the token
     __syncthreads();
-#pragma unroll 1
-    for (int t = 0; t < nt; ++t) {
+    const auto token = [&](int t, auto full) {
       const float fbar = __shfl_sync(0xffffffffu, fbar_l, t);
-      const float4 vv = *reinterpret_cast<const float4*>(s_v + t * TV + cgi * 4);
-      float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
+      const ulonglong2 vv = *reinterpret_cast<const ulonglong2*>(s_v + t * TV + cgi * 4);
+      const uint64_t ff = f2(fbar, fbar);
+      uint64_t h2[2] = {0ull, 0ull};
       const float2* kq = s_kq + t * DHQK + rg;
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
-        if (rg + r * RG < DHQK) {
-          const float kk = kq[r * RG].x, qq = kq[r * RG].y;
-          C[r].x = fmaf(fbar, C[r].x, kk * vv.x);
-          C[r].y = fmaf(fbar, C[r].y, kk * vv.y);
-          C[r].z = fmaf(fbar, C[r].z, kk * vv.z);
-          C[r].w = fmaf(fbar, C[r].w, kk * vv.w);
-          hv.x = fmaf(qq, C[r].x, hv.x); hv.y = fmaf(qq, C[r].y, hv.y);
-          hv.z = fmaf(qq, C[r].z, hv.z); hv.w = fmaf(qq, C[r].w, hv.w);
+        if (decltype(full)::value || rg + r * RG < DHQK) {
+          const float2 x = kq[r * RG];
+          const uint64_t k2 = f2(x.x, x.x), q2 = f2(x.y, x.y);
+          C[r][0] = fma2(ff, C[r][0], mul2(k2, vv.x));
+          C[r][1] = fma2(ff, C[r][1], mul2(k2, vv.y));
+          h2[0] = fma2(q2, C[r][0], h2[0]);
+          h2[1] = fma2(q2, C[r][1], h2[1]);
         }
       }
+      float4 hv;
+      unf2(h2[0], hv.x, hv.y);
+      unf2(h2[1], hv.z, hv.w);
       // over the row groups of the warp (lanes CG apart)
 #pragma unroll
       for (int o = CG; o < 32; o <<= 1) {
@@ -305,6 +324,13 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
         hv.w += __shfl_xor_sync(0xffffffffu, hv.w, o);
       }
       if (lane < CG) *reinterpret_cast<float4*>(s_red + (t * NW + warp) * TV + cgi * 4) = hv;
+    };
+    if (ROWS * RG == DHQK) {
+#pragma unroll 2
+      for (int t = 0; t < nt; ++t) token(t, std::true_type());
+    } else {
+#pragma unroll 1
+      for (int t = 0; t < nt; ++t) token(t, std::false_type());
     }
     __syncthreads();
     for (int idx = tid; idx < nt * TV; idx += STEP_THREADS) {
@@ -321,7 +347,10 @@ step_sequence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     const int d = rg + r * RG;
-    if (d < DHQK && e < DHHV) __stcs(reinterpret_cast<float4*>(c_new + ((size_t)bh * DHQK + d) * DHHV + e), C[r]);
+    float4 x;
+    unf2(C[r][0], x.x, x.y);
+    unf2(C[r][1], x.z, x.w);
+    if (d < DHQK && e < DHHV) __stcs(reinterpret_cast<float4*>(c_new + ((size_t)bh * DHQK + d) * DHHV + e), x);
   }
   if (tile == 0) {
 #pragma unroll
@@ -382,26 +411,32 @@ int step_seq_t(const void* q, const void* k, const void* v, const void* i, const
                int DHQK, int DHHV, float eps, cudaStream_t st) {
   const unsigned grid = (unsigned)ceil_div(DHHV, TV) * (unsigned)(B * NH);
   const size_t smem = sizeof(float) * SEQ_TB * (TV + (STEP_THREADS / 32) * TV + 2 * (size_t)DHQK);
+  // Started while the launch before drains, CTAs go where there is room at that moment.  A grid that leaves SMs free ends up two
+  // to an SM, which a launch of many tokens pays for (1 x 64 tokens, 128 CTAs: 26.8 us, 36.3 overlapped; 1 x 24: 12.4, 15.1)
+  // and one of two blocks does not (1 x 13: 8.9 us, 7.6 overlapped).  Up to half the SMs both launches find SMs of their own,
+  // and a grid above their number shares them in any case.
+  const unsigned sms = (unsigned)sm_count();
+  const bool overlap = grid <= pdl_max_ctas() && (2 * grid <= sms || grid > sms || Tn <= 2 * SEQ_TB);
   auto kern = step_sequence_kernel<T, ROWS, TV>;
   if (smem > 48 * 1024) MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<grid, STEP_THREADS, smem, st>>>((const T*)q, (const T*)k, (const T*)v, i, f, gate_dtype, c, n, m,
-                                         (T*)h, c_new, n_new, m_new, Tn, DHQK, DHHV, eps);
-  MLSTM_LAUNCH_CHECK();
-  return MLSTM_OK;
+  return launch_pdl(overlap, kern, grid, STEP_THREADS, smem, st, (const T*)q, (const T*)k, (const T*)v, i, f, gate_dtype, c, n, m,
+                    (T*)h, c_new, n_new, m_new, Tn, DHQK, DHHV, eps);
 }
 
 template <typename T>
 int step_seq_rows(const void* q, const void* k, const void* v, const void* i, const void* f, int gate_dtype,
                   const float* c, const float* n, const float* m, void* h, float* c_new, float* n_new, float* m_new,
                   int B, int NH, int Tn, int DHQK, int DHHV, float eps, cudaStream_t st) {
-  // 32-column slices while 64-column ones would leave SMs without a CTA: half the multiply-adds per thread and token,
-  // for q, k and n prepared once more
-  const bool narrow = (long)ceil_div(DHHV, 64) * B * NH < sm_count();
+  // 32-column slices while 64-column ones would leave SMs without a CTA, and for DHQK above 128: half the rows per thread,
+  // for q, k and n prepared once more.  With sixteen rows in 64 columns instead of eight in 32 the registers run short (8 x 64
+  // tokens, 8 heads 256/512: 157 us, 125 in 32 columns); with eight in 64 they do not, and the second preparation costs more
+  // (16 x 8 tokens, 8 heads 128/256: 13.1 us, 18.6 in 32).
+  const bool narrow = DHQK > 128 || (long)ceil_div(DHHV, 64) * B * NH < sm_count();
 #define SEQ_CASE(R, TV) \
   if (ceil_div(DHQK, STEP_THREADS / (TV / 4)) <= R) \
     return step_seq_t<T, R, TV>(q, k, v, i, f, gate_dtype, c, n, m, h, c_new, n_new, m_new, B, NH, Tn, DHQK, DHHV, eps, st);
   if (narrow) { SEQ_CASE(4, 32) SEQ_CASE(8, 32) SEQ_CASE(16, 32) }
-  SEQ_CASE(4, 64) SEQ_CASE(8, 64) SEQ_CASE(16, 64) SEQ_CASE(32, 64)
+  SEQ_CASE(4, 64) SEQ_CASE(8, 64)
 #undef SEQ_CASE
   return MLSTM_ERR_SHAPE;
 }

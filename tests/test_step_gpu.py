@@ -152,6 +152,30 @@ def test_sequence_kernel_token_blocks(B, S, DHQK, DHHV):
         assert max_rel_err(npy(a), b) < 2e-5
 
 
+@pytest.mark.parametrize("S", [17, 20])
+@pytest.mark.parametrize("B,DHQK,DHHV", [(1, 128, 64), (1, 200, 64), (2, 300, 96), (19, 128, 128), (19, 104, 128), (37, 64, 60)])
+def test_sequence_kernel_full_and_partly_filled_rows(B, DHQK, DHHV, S):
+    """Register variants whose rows DHQK fills and does not fill, in both slice widths, over three blocks of tokens (an odd and
+    an even last block, the launches of a repeated call overlapping): every call against the oracle.  f32 throughout; the
+    tolerance is that of the test above."""
+    NH = 4
+    inp = make_step_inputs(dict(seed=7 + S + DHQK, B=B, NH=NH, DHQK=DHQK, DHHV=DHHV, steps=S))
+    q, k, v = (to_dev(np.moveaxis(inp[x], 0, 2), torch.float32) for x in "qkv")
+    i, f = (to_dev(np.moveaxis(inp[x][..., 0], 0, 2), torch.float32) for x in "if")
+    c, n, m = (to_dev(inp[x], torch.float32) for x in "cnm")
+    calls = [mk.mlstm_recurrent_sequence__b200(q, k, v, i, f, c, n, m, return_last_states=True) for _ in range(3)]
+    state = tuple(inp[x].astype(np.float64) for x in "cnm")
+    hs = []
+    for t in range(S):
+        ho, state = O.recurrent_step(*(inp[x][t].astype(np.float64) for x in "qkvif"), *state)
+        hs.append(ho)
+    for h, last in calls:
+        for t in range(S):
+            assert max_rel_err(npy(h[:, :, t]), hs[t]) < 2e-5, t
+        for a, b in zip(last, state):
+            assert max_rel_err(npy(a), b) < 2e-5
+
+
 def test_step_full_size_decay_property():
     """Size-independent check at the full decode geometry (B=64, NH=8, 256/512): with k = 0 the step
     must scale C by exp(logsigmoid(f) + m - m') exactly and leave it otherwise unchanged."""
