@@ -24,11 +24,11 @@
 //
 // What bounds it: the shared-memory port (128 bytes per cycle).  Every operand byte is written there by TMA and read by the
 // MMA, a 128 x 128 x 16 product of two shared operands by itself asks for the port's full rate, and E and the output pass
-// through it too: 1.15 MB per item at 256/256, 9200 of the 11400 cycles an item takes; HBM is at 0.8 of the copy rate
+// through it too: 1.15 MB per item at 256/256, 9200 of the 11000 cycles an item takes; HBM is at 0.8 of the copy rate
 // then.  (Before, one CTA per chunk and mode, two to an SM, each a chain of dependent steps: 8 x 8192 tokens, 16 heads
-// 256/256 1302 us, now 1130; 16 x 2048, 128/256 431, now 351; 4 x 1024, 4 heads 96/192 22.9, now 20.9.)
+// 256/256 1302 us, now 1089; 16 x 2048, 128/256 431, now 342; 4 x 1024, 4 heads 96/192 22.9, now 20.9.)
 // Measured and not taken: an accumulator of 256 columns (A read once for two tiles, 10 % less port traffic, but nothing left to
-// overlap the epilogue with: 1260 and 440 us); the modes of one chunk in one CTA (the 148 chunks in flight no longer fit
+// overlap the epilogue with: 1260 and 440 us where this form then took 1130 and 351); the modes of one chunk in one CTA (the 148 chunks in flight no longer fit
 // in L2: 1150 and 383); L2 prefetch of the next item's operands (1144-1230 and 396-408).
 #include <algorithm>
 
