@@ -147,7 +147,10 @@ par_bw_run_sm100(const __grid_constant__ BwMaps maps, const __grid_constant__ Bw
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = sh.tmem;
-  pdl_launch_dependents();
+  // No pdl_launch_dependents(): these CTAs take an SM each, registers and shared memory, for the whole launch, and CTAs of the next
+  // launch that are let in before they end go, all of them, to the few SMs that have none, and stay there (8 heads, 1024 tokens,
+  // forward and backward, with it at the start and without: 256/1024 263 and 141 us, 256/512 132 and 91; 3200 tokens 243 and 178;
+  // with it behind the last product, 128/256, 1152 tokens 68.9 and 64.8).
   pdl_wait();
 
   Items it(p);
