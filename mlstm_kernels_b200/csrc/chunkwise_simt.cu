@@ -305,6 +305,11 @@ __device__ __forceinline__ void score_tile(const ScoreArgs<T>& p, const ScoreGat
   }
 }
 
+// None of these kernels lets the next launch in before its CTAs end (there is no pdl_launch_dependents()): three of them fit an SM, more
+// in the scan, and the CTAs of a launch that does not fill the GPU, placed while another one still has most SMs, come to lie
+// three to an SM (2 x 4 x 512 tokens, 64/128, forward and backward in us, with it at the start and without: chunk 128 141 and 101,
+// chunk 64 87 and 69; 4 x 4 x 512, 104/104, chunk 256, raw calls 397 and 351; 1 x 4 x 64, 64/64 52.1 and 50.1).
+
 // The products that need nothing but inputs and gate vectors, in one launch: the score blocks (the longer ones, first) and the
 // chunks' contributions of one recurrence or two.  Alone each of them is a launch of one wave or less, bound by load and
 // barrier latency; the score blocks ran in every output tile of their chunk, a quarter of the forward's multiply-adds and 43 % of
@@ -322,7 +327,6 @@ struct PartArgs {
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(NTHR) part_kernel(const __grid_constant__ PartArgs<T> p) {
   __shared__ __align__(16) float buf[4 * SLICE];
-  pdl_launch_dependents();
   pdl_wait();
   const unsigned x = blockIdx.x;
   if (x < p.end[1]) {
@@ -401,7 +405,6 @@ __device__ __forceinline__ void scan_tile(const ScanArgs& a, const float* gbar, 
 template <int V>
 __global__ void __launch_bounds__(128)
 rec_scan_kernel(const ScanArgs fw, const ScanArgs bw, const unsigned n_fw, const float* gbar, int NC, int DHQK, int DHHV) {
-  pdl_launch_dependents();
   pdl_wait();
   if (blockIdx.x < n_fw) scan_tile<V, false>(fw, gbar, NC, DHQK, DHHV, blockIdx.x);
   else scan_tile<V, true>(bw, gbar, NC, DHQK, DHHV, blockIdx.x - n_fw);
@@ -655,7 +658,6 @@ __device__ __forceinline__ void par_tile(const ParArgs<T>& p, const int mode, in
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(NTHR, 3) par_fw_kernel(ParArgs<T> p) {
   extern __shared__ __align__(16) float smem[];
-  pdl_launch_dependents();
   pdl_wait();
   const int n_ot = (p.DHHV + TILE - 1) / TILE, n_rb = (p.L + TILE - 1) / TILE, y = blockIdx.x / n_ot;
   par_tile<T, true, VEC>(p, PAR_H, blockIdx.x % n_ot, y / n_rb, y % n_rb, smem);
@@ -664,7 +666,6 @@ __global__ void __launch_bounds__(NTHR, 3) par_fw_kernel(ParArgs<T> p) {
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(NTHR, 3) par_bw_kernel(ParArgs<T> p) {
   extern __shared__ __align__(16) float smem[];
-  pdl_launch_dependents();
   pdl_wait();
   const int n_v = (p.DHHV + TILE - 1) / TILE, n_k = (p.DHQK + TILE - 1) / TILE;
   const int n = n_v + 2 * n_k, n_rb = (p.L + TILE - 1) / TILE, x = blockIdx.x % n, y = blockIdx.x / n;
