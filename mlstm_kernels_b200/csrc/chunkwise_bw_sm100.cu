@@ -30,10 +30,10 @@
 // Measured and not taken: an accumulator of 256 columns (A read once for two tiles, 10 % less port traffic, but nothing left to
 // overlap the epilogue with: 1260 and 440 us where this form then took 1130 and 351); the modes of one chunk in one CTA (the 148 chunks in flight no longer fit
 // in L2: 1150 and 383); L2 prefetch of the next item's operands (1144-1230 and 396-408).
-#include <algorithm>
 
 #include "common.cuh"
 #include "launch.cuh"
+#include "par_bw_items.h"
 #include "sm100.cuh"
 #include "tensor_maps.cuh"
 
@@ -46,7 +46,6 @@ __device__ int g_par_bw_status = 0;  // first error code raised by a bounded wai
 namespace {
 
 constexpr int CL = 128;          // chunk length
-enum { PM_DV = 0, PM_DK = 1, PM_DQ = 2 };
 
 struct BwMaps {
   CUtensorMap q, k, v, dh;           // 128 tokens x 64 columns
@@ -54,24 +53,18 @@ struct BwMaps {
   CUtensorMap dq, dk, dv;            // outputs
 };
 
-struct BwParams {
+struct BwParams : BwItems {
   const float *vecB, *iota, *m_tok, *abar, *bbar, *inv_den;  // per token, f32
   float *rowdot_q, *rowdot_k;   // sum_d q dq (from DQ), sum_d k dk (from DK); one partial per output tile: [DHQK/128][tokens]
   size_t nslots;                // B * NH * SP
-  int S, SP, NC, DHQK, DHHV;    // SP = NC * 128: slots per (batch, head) of the per-token gate vectors
+  int S, SP;                    // SP = NC * 128: slots per (batch, head) of the per-token gate vectors
   float qk_scale;
-  int bh0;                      // first (batch, head) unit of this launch
-  int maxsub;                   // most output tiles (128 columns) of an item
-  int c_dv, c_dk;               // items of a chunk: deltaV's, and deltaK's and deltaQ's each
-  unsigned n_items, stride;     // work items of the launch; CTAs that go through a range of them side by side
-  int dx, dck, dbh;             // the stride as a step of (item of a chunk, chunk, unit)
 };
 
 constexpr int NST = 5;                   // operand ring depth
 constexpr int STAGE = 32768;
 constexpr int TILE = 32768;              // E tile and output staging, two of them
 constexpr int THREADS = 640;
-constexpr unsigned kRunItems = 24;       // work items of a CTA at most
 
 struct BwShared {
   uint64_t full[NST], empty[NST], sfull, sread, gready[2], afull[2], accfree[2], scaled[2], hfull[2], ready[2], staged[2];
@@ -85,35 +78,6 @@ struct BwShared {
 };
 constexpr int OFF_T = NST * STAGE, OFF_C = OFF_T + 2 * TILE, SMEM = OFF_C + 3072;
 static_assert(sizeof(BwShared) <= 3072 && SMEM <= 232448, "shared memory of one CTA");
-
-// The work items of a CTA: every `stride`-th in the order (chunk of a unit, mode and tile group), so that the CTAs of a wave go
-// through neighbouring items side by side and what one chunk's modes share is in L2 while they all run.
-struct Items {
-  int x, ck, bh, left;
-  __device__ __forceinline__ Items(const BwParams& p) {
-    const unsigned waves = gridDim.x / p.stride, w = blockIdx.x / p.stride;   // (the grid is a multiple of the stride)
-    const unsigned lo = (unsigned)((uint64_t)p.n_items * w / waves), hi = (unsigned)((uint64_t)p.n_items * (w + 1) / waves);
-    const unsigned first = lo + (blockIdx.x - w * p.stride);
-    left = first < hi ? (int)((hi - first + p.stride - 1) / p.stride) : 0;
-    const unsigned gx = p.c_dv + 2 * p.c_dk, r = first / gx;
-    x = (int)(first - r * gx); ck = (int)(r % (unsigned)p.NC); bh = p.bh0 + (int)(r / (unsigned)p.NC);
-  }
-  __device__ __forceinline__ void next(const BwParams& p) {
-    --left;
-    x += p.dx; ck += p.dck; bh += p.dbh;
-    if (x >= p.c_dv + 2 * p.c_dk) { x -= p.c_dv + 2 * p.c_dk; ++ck; }
-    if (ck >= p.NC) { ck -= p.NC; ++bh; }
-  }
-  __device__ __forceinline__ int mode(const BwParams& p) const { return x < p.c_dv ? PM_DV : (x < p.c_dv + p.c_dk ? PM_DK : PM_DQ); }
-  __device__ __forceinline__ int tile0(const BwParams& p) const {
-    return p.maxsub * (x < p.c_dv ? x : (x < p.c_dv + p.c_dk ? x - p.c_dv : x - p.c_dv - p.c_dk));
-  }
-  __device__ __forceinline__ int tiles(const BwParams& p) const {
-    return min(p.maxsub, ((mode(p) == PM_DV ? p.DHHV : p.DHQK) + 127) / 128 - tile0(p));
-  }
-  // slices of 64 columns in the contraction of the score and of the inter-chunk product
-  __device__ __forceinline__ int slices(const BwParams& p) const { return ((mode(p) == PM_DV ? p.DHQK : p.DHHV) + 63) / 64; }
-};
 
 // gate vectors of a token; scale: its abar or bbar
 struct RowGate { float b, iota, m, inv, scale; };
@@ -153,7 +117,7 @@ par_bw_run_sm100(const __grid_constant__ BwMaps maps, const __grid_constant__ Bw
   // with it behind the last product, 128/256, 1152 tokens 68.9 and 64.8).
   pdl_wait();
 
-  Items it(p);
+  BwRun it(p, blockIdx.x, gridDim.x);
   if (warp == 0) {
     // ---------------- TMA producer: same order as the MMA issuer ----------------
     if (elect_one()) {
@@ -292,7 +256,7 @@ par_bw_run_sm100(const __grid_constant__ BwMaps maps, const __grid_constant__ Bw
   } else if (warp == 2) {
     // ---------------- E tiles in, output tiles out ----------------
     if (elect_one()) {
-      Items ahead = it;                     // two tiles ahead of the tile that is stored
+      BwRun ahead = it;                     // two tiles ahead of the tile that is stored
       int asub = 0, loaded = 0;
       auto fill = [&]() {                   // make the buffer ready for the next tile, if there is one
         if (ahead.left <= 0) return;
@@ -400,7 +364,7 @@ par_bw_run_sm100(const __grid_constant__ BwMaps maps, const __grid_constant__ Bw
     const int r = quarter * 32 + lane;
     constexpr float kLog2e = 1.4426950408889634f;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    auto load_gate = [&](const Items& i) -> RowGate {
+    auto load_gate = [&](const BwRun& i) -> RowGate {
       const size_t tok = (size_t)i.bh * p.SP + i.ck * CL + r;
       return RowGate{p.vecB[tok], p.iota[tok], p.m_tok[tok], p.inv_den[tok], i.mode(p) == PM_DQ ? p.bbar[tok] : p.abar[tok]};
     };
@@ -535,23 +499,13 @@ int sm100_parallel_bw(const void* q, const void* k, const void* v, const void* d
       !state_map(&m.c_k, c_states, d, 128) || !state_map(&m.dc_mn, dc_states, d, 64) || !state_map(&m.dc_k, dc_states, d, 128) ||
       !tok_map(&m.dq, dq, d, d.DHQK) || !tok_map(&m.dk, dk, d, d.DHQK) || !tok_map(&m.dv, dv, d, d.DHHV))
     return MLSTM_ERR_CUDA;
-  BwParams p{gb.vecB, gb.iota, gb.m_tok, gb.abar, gb.bbar, gb.inv_den, qdq_parts, kdk_parts, (size_t)d.B * d.NH * d.SP,
-             d.S, d.SP, d.NC, d.DHQK, d.DHHV, d.qk_scale, ur.first};
-  const int T_dv = ceil_div(d.DHHV, 128), T_dk = ceil_div(d.DHQK, 128);
-  auto items = [&](int s) { return ((long)ceil_div(T_dv, s) + 2 * ceil_div(T_dk, s)) * d.NC * units; };
-  // The tiles of an item share its score tile; a launch of fewer items than SMs splits them instead, each computing the score
-  // for itself.
-  p.maxsub = std::min(4, std::max(T_dv, T_dk));
-  while (p.maxsub > 1 && items(p.maxsub) < sm_count()) p.maxsub = (p.maxsub + 1) / 2;
-  p.c_dv = ceil_div(T_dv, p.maxsub); p.c_dk = ceil_div(T_dk, p.maxsub);
-  p.n_items = (unsigned)items(p.maxsub);
-  p.stride = std::min(p.n_items, (unsigned)sm_count());
-  const int gx = p.c_dv + 2 * p.c_dk, chunks = (int)p.stride / gx;
-  p.dx = (int)p.stride % gx; p.dck = chunks % d.NC; p.dbh = chunks / d.NC;
+  const BwItems w = bw_plan(units, ur.first, d.NC, d.DHQK, d.DHHV, sm_count());
+  const BwParams p{w, gb.vecB, gb.iota, gb.m_tok, gb.abar, gb.bbar, gb.inv_den, qdq_parts, kdk_parts, (size_t)d.B * d.NH * d.SP,
+                   d.S, d.SP, d.qk_scale};
   // A CTA takes up to 24 items: its start (2 us) is then 1-2 % of its time, and a launch beside another chain's recurrence, which
   // frees the SMs one by one, still spreads over them (8 x 8192 tokens, 16 heads 256/256, alone: 3, 6, 12, 24, 96 items per CTA
   // 1271, 1246, 1210, 1219, 1217 us in the first form of the kernel; 16 x 2048, 128/256: 435, 413, 393, 389, 379).
-  const unsigned grid = p.stride * ((p.n_items + p.stride * kRunItems - 1) / (p.stride * kRunItems));
+  const unsigned grid = bw_grid(w);
   const bool f16 = d.dtype == MLSTM_F16;
   static bool attr_done[2][64] = {};
   if (int rc = f16 ? set_smem_once(par_bw_run_sm100<true>, SMEM, attr_done[1]) : set_smem_once(par_bw_run_sm100<false>, SMEM, attr_done[0])) return rc;

@@ -16,6 +16,9 @@ pytestmark = pytest.mark.gpu
     (3, 16, 500, 96, 320),       # one tile of two modes, three of the other, two of them partial
     (2, 11, 1030, 264, 136),     # nine chunks, the last of six tokens; a tile of eight columns
     (1, 4, 37900, 16, 16),       # more items than the CTAs of one wave take
+    (1, 16, 300, 128, 256),      # whole items in one round
+    (1, 8, 600, 256, 512),       # the same, with four tiles
+    (1, 8, 1000, 256, 512),      # split items in two rounds, with a stride of its own
 ])
 @pytest.mark.parametrize("dtype, tol", [(torch.bfloat16, 2e-2), (torch.float16, 2e-2)])
 @pytest.mark.parametrize("siging", [False, True])
