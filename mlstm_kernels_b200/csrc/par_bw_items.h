@@ -62,6 +62,9 @@ inline BwItems bw_items(int units, int bh0, int NC, int DHQK, int DHHV, int maxs
 }
 
 // One CTA per SM side by side, and up to four output tiles to an item: they share its score tile.
+// Where the SM count is a multiple of the items per chunk (four, with head dims of v above 512) every CTA would meet one kind of
+// item only, and kinds differ (256/1024: 24 ring stages for deltaV's, 50 for the others): a stride of one less goes through
+// the kinds in turn (8 heads, 14208 tokens: 256/1024 485 and 396 us, 128/1024 320 and 258).
 // A launch of less than two items per SM takes the split of its items and the stride (up to three less) that leave the busiest
 // CTA the fewest ring stages, if that is a tenth fewer: a split item's parts each compute the score for themselves.  (Splitting wherever
 // there are fewer items than SMs gave many of them a second round.  Kernel in us, 8 heads, so and now: 640 tokens 256/512 24.9 and
@@ -70,7 +73,8 @@ inline BwItems bw_items(int units, int bh0, int NC, int DHQK, int DHHV, int maxs
 inline BwItems bw_plan(int units, int bh0, int NC, int DHQK, int DHHV, int sms) {
   const int T = ((DHHV > DHQK ? DHHV : DHQK) + 127) / 128;
   const BwItems whole = bw_items(units, bh0, NC, DHQK, DHHV, T < 4 ? T : 4, sms);
-  if (whole.n_items >= 2u * (unsigned)sms) return whole;
+  if (whole.n_items >= 2u * (unsigned)sms)
+    return sms % whole.per_chunk() == 0 ? bw_items(units, bh0, NC, DHQK, DHHV, whole.maxsub, sms - 1) : whole;
   BwItems best = whole;
   int most = whole.busiest();
   for (int m = whole.maxsub;; m = (m + 1) / 2) {

@@ -70,7 +70,8 @@ def test_every_tile_once_and_bounded_runs(launches, size):
 
 @pytest.mark.parametrize("size", SIZES)
 def test_no_cta_has_more_to_do_than_whole_items_in_turn_would_give(launches, size):
-    """Splitting items never leaves the busiest CTA of a small launch more than the whole ones, dealt out one by one, would."""
+    """Splitting items never leaves the busiest CTA of a small launch more than the whole ones, dealt out one by one, would; in a
+    large one every CTA meets all kinds of items, so that none is further above the mean than two items."""
     units, _, NC, DHQK, DHHV = size
     stride, grid, items = launches[size]
     load = [0] * grid
@@ -81,3 +82,5 @@ def test_no_cta_has_more_to_do_than_whole_items_in_turn_would_give(launches, siz
              for t in range(0, T[mode], 4)]
     if len(whole) < 2 * SMS:
         assert max(load) <= max(sum(whole[b::SMS]) for b in range(SMS))
+    if grid == stride:
+        assert max(load) <= sum(load) / SMS + 2 * max(whole)

@@ -19,6 +19,7 @@ pytestmark = pytest.mark.gpu
     (1, 16, 300, 128, 256),      # whole items in one round
     (1, 8, 600, 256, 512),       # the same, with four tiles
     (1, 8, 1000, 256, 512),      # split items in two rounds, with a stride of its own
+    (2, 8, 1700, 256, 1024),     # two tile groups of one mode, every CTA in turn through all kinds of items
 ])
 @pytest.mark.parametrize("dtype, tol", [(torch.bfloat16, 2e-2), (torch.float16, 2e-2)])
 @pytest.mark.parametrize("siging", [False, True])
