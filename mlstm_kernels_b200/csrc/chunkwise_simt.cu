@@ -324,12 +324,14 @@ struct PartArgs {
   bool bwd[2];             // rec[i] is the state gradient's
 };
 
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(NTHR) part_kernel(const __grid_constant__ PartArgs<T> p) {
+// SCORES: there are score blocks.  Without them 64 registers do, and a fourth CTA to an SM (0: the compiler's choice, 80): 4 heads, 2048
+// tokens, 128/256, chunk 32, recurrence 52 us at 80, 41 at 64.
+template <typename T, bool VEC, bool SCORES>
+__global__ void __launch_bounds__(NTHR, SCORES ? 0 : 4) part_kernel(const __grid_constant__ PartArgs<T> p) {
   __shared__ __align__(16) float buf[4 * SLICE];
   pdl_wait();
   const unsigned x = blockIdx.x;
-  if (x < p.end[1]) {
+  if (SCORES && x < p.end[1]) {
     const int i = x >= p.end[0];
     score_tile<T, VEC>(p.sc[i], p.gate, i ? x - p.end[0] : x, buf);
   } else {
@@ -401,13 +403,14 @@ __device__ __forceinline__ void scan_tile(const ScanArgs& a, const float* gbar, 
                           a.n_final ? a.n_final + (size_t)bh * DHQK : nullptr, g, DHQK, t - (E + V - 1) / V, NC);
   }
 }
-// the first n_fw CTAs scan the forward's states, the others the gradient's
-template <int V>
+// the first n_fw CTAs scan the forward's states, the others the gradient's; FW, BW: whether there are any of them (one kind takes 40
+// registers, both in one kernel 56)
+template <int V, bool FW, bool BW>
 __global__ void __launch_bounds__(128)
 rec_scan_kernel(const ScanArgs fw, const ScanArgs bw, const unsigned n_fw, const float* gbar, int NC, int DHQK, int DHHV) {
   pdl_wait();
-  if (blockIdx.x < n_fw) scan_tile<V, false>(fw, gbar, NC, DHQK, DHHV, blockIdx.x);
-  else scan_tile<V, true>(bw, gbar, NC, DHQK, DHHV, blockIdx.x - n_fw);
+  if (FW && (!BW || blockIdx.x < n_fw)) scan_tile<V, false>(fw, gbar, NC, DHQK, DHHV, blockIdx.x);
+  else scan_tile<V, true>(bw, gbar, NC, DHQK, DHHV, FW ? blockIdx.x - n_fw : blockIdx.x);
 }
 
 // Final state only, one CTA per tile walking the chunks.
@@ -691,7 +694,9 @@ static int parts_t(PartArgs<T> a, int n_rec, const ChunkwiseDims& d, cudaStream_
   a.end[1] = a.end[0] + (a.sc[1].out ? pairs : 0);
   a.end[2] = a.end[1] + tiles;
   a.end[3] = a.end[2] + (n_rec > 1 ? tiles : 0);
-  if (int rc = launch_pdl(a.end[3] <= pdl_max_ctas(), vec_dims(d) ? part_kernel<T, true> : part_kernel<T, false>, a.end[3], NTHR, 0, st, a)) return rc;
+  const bool vec = vec_dims(d);
+  auto part = a.end[1] > 0 ? (vec ? part_kernel<T, true, true> : part_kernel<T, false, true>) : (vec ? part_kernel<T, true, false> : part_kernel<T, false, false>);
+  if (int rc = launch_pdl(a.end[3] <= pdl_max_ctas(), part, a.end[3], NTHR, 0, st, a)) return rc;
   const size_t E = (size_t)d.DHQK * d.DHHV;
   const int V = E % 4 == 0 ? 4 : 1;
   ScanArgs scan[2] = {};   // forward, backward
@@ -704,8 +709,10 @@ static int parts_t(PartArgs<T> a, int n_rec, const ChunkwiseDims& d, cudaStream_
     n[a.bwd[i]] = (unsigned)nblk * (unsigned)(d.B * d.NH);
   }
   const unsigned grid = n[0] + n[1];
-  return launch_pdl(grid <= pdl_max_ctas(), V == 4 ? rec_scan_kernel<4> : rec_scan_kernel<1>, grid, 128, 0, st, scan[0], scan[1], n[0], gbar, d.NC,
-                    d.DHQK, d.DHHV);
+  auto kern = n[1] == 0   ? (V == 4 ? rec_scan_kernel<4, true, false> : rec_scan_kernel<1, true, false>)
+              : n[0] == 0 ? (V == 4 ? rec_scan_kernel<4, false, true> : rec_scan_kernel<1, false, true>)
+                          : (V == 4 ? rec_scan_kernel<4, true, true> : rec_scan_kernel<1, true, true>);
+  return launch_pdl(grid <= pdl_max_ctas(), kern, grid, 128, 0, st, scan[0], scan[1], n[0], gbar, d.NC, d.DHQK, d.DHHV);
 }
 
 template <typename T, bool BWD>
