@@ -359,7 +359,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
     auto store_c = [&](const int n_out) {   // n_out: tiles written before this one
       if (p.c_states == nullptr) return;
       const int ob = n_out & 1;
-      const bool ok = n_out < 2 || mbar_wait(&bar_out_free[ob], ((n_out >> 1) - 1) & 1, &s_abort, &g_sm100_status, 107);
+      const bool ok = n_out < 2 || mbar_wait<true>(&bar_out_free[ob], ((n_out >> 1) - 1) & 1, &s_abort, &g_sm100_status, 107);
       // TN = 128: each group fills its own 64-column box; TN = 64: the groups share one box (four 16-byte pieces each)
       uint8_t* rowp = stage_base + ob * REC_OUT + (TN == 128 ? half * 16384 : 0) + row * 128;
       const int piece0 = (TN == 128) ? 0 : half * 4;
@@ -376,7 +376,7 @@ rec_body(const CUtensorMap& mapL, const CUtensorMap& mapR, const CUtensorMap& ma
     store_c(0);   // the state before the first step (slot 0 forward, slot NC backward)
     for (int s = 0; s < NS; ++s) {
       const int buf = s & 1;
-      const bool ok = mbar_wait(&bar_done[(2 * s + 1) & (REC_LBUF - 1)], ((2 * s + 1) / REC_LBUF) & 1, &s_abort, &g_sm100_status, 104);
+      const bool ok = mbar_wait<true>(&bar_done[(2 * s + 1) & (REC_LBUF - 1)], ((2 * s + 1) / REC_LBUF) & 1, &s_abort, &g_sm100_status, 104);
       tc_fence_after_sync();
       const float g = s_g[s & (G_RING - 1)];
       const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 128 + half * HC;

@@ -55,8 +55,8 @@ __device__ __forceinline__ bool aborted(uint32_t abort) {
 // and the flags at every wait the intra-chunk kernels, whose warps go through their code once or a few times, took 3 to 7 %
 // longer, waiting for instructions (8 heads, 4096 tokens 128/256: forward 19.6 -> 19.0 us, backward 41.3 -> 38.6).
 constexpr uint32_t kWaitLimit = 20u * 1000u * 1000u;
-static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, uint32_t abort, int* status, int code,
-                                                   uint32_t limit) {
+__device__ __forceinline__ bool mbar_poll_on(uint32_t bar, uint32_t parity, uint32_t abort, int* status, int code, uint32_t limit) {
+#pragma unroll 1
   for (uint32_t it = 0; it < limit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     __nanosleep(32);
@@ -66,13 +66,22 @@ static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity
   if (status != nullptr) atomicCAS(status, 0, code);
   return false;
 }
+static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, uint32_t abort, int* status, int code,
+                                                   uint32_t limit) {
+  return mbar_poll_on(bar, parity, abort, status, code, limit);
+}
+// IN_LINE: without the call, for a role that has its registers full (the call is never made in a run that goes well, but what
+// lives across it is kept where the call leaves it alone: with the call the state warps of the 128-column recurrences spilled 20 to
+// 56 bytes).
+template <bool IN_LINE = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* abort, int* status, int code,
                                           uint32_t limit = kWaitLimit) {
   const uint32_t b = smem_u32(bar);
 #pragma unroll 1
   for (int it = 0; it < 64; ++it)
     if (mbar_try_wait(b, parity)) return true;
-  return mbar_wait_long(b, parity, abort != nullptr ? smem_u32(abort) : 0u, status, code, limit);
+  const uint32_t a = abort != nullptr ? smem_u32(abort) : 0u;
+  return IN_LINE ? mbar_poll_on(b, parity, a, status, code, limit) : mbar_wait_long(b, parity, a, status, code, limit);
 }
 
 // Where a whole warp waits, every lane polls for itself, and a wait that runs out may do so in some lanes only: others still

@@ -26,6 +26,14 @@ def report(source):
     return {name: (int(regs), int(stores) + int(loads)) for name, stores, loads, regs in found}
 
 
+@pytest.mark.parametrize("source,least", [("chunkwise_sm100.cu", 16), ("chunkwise_bw_sm100.cu", 2)])
+def test_tcgen05_kernels_do_not_spill(source, least):
+    """(A local-memory access is a trip to L2 here: nearly all of L1 is shared memory.)"""
+    kernels = report(source)
+    assert len(kernels) >= least
+    assert {name: x for name, x in kernels.items() if x[1] > 0} == {}
+
+
 def test_portable_recurrence_without_score_blocks_keeps_its_resident_ctas():
     """Four CTAs of 256 threads, and twelve of 128 in the scan, to an SM of 65536 registers."""
     kernels = report("chunkwise_simt.cu")
