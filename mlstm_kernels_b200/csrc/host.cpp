@@ -68,6 +68,18 @@ void check(int rc, const char* what) {
 
 size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 Tensor bytes(size_t n, const at::Device& dev) { return empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, dev); }
+// `need` bytes, and behind them (from up256(need)) `extra` that only make the call faster: where memory is too short for both,
+// extra becomes 0 and the call does without.  (Asked for last: what a call allocates after it would have to fit beside the extra.)
+Tensor bytes_and(size_t need, size_t& extra, const at::Device& dev) {
+  if (extra > 0) {
+    try {
+      return bytes(up256(need) + extra, dev);
+    } catch (const c10::OutOfMemoryError&) {
+      extra = 0;
+    }
+  }
+  return bytes(need, dev);
+}
 
 // ---- chunkwise ------------------------------------------------------------------------------------------
 PyObject* g_select_chunk_size = nullptr;   // chunkwise.select_chunk_size: the rule of the portable kernels, and its errors
@@ -147,12 +159,12 @@ Forward run_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   if (!(for_backward && keep_states)) need += up256(p.states_bytes);
   const size_t ws_at = need;
   if (!for_backward) need += p.fw_bytes;
-  const size_t scores_bytes = mlstm::score_scratch_bytes(p.c, false), scores_at = up256(need);
-  if (scores_bytes > 0) need = scores_at + scores_bytes;
-  const Tensor scratch = bytes(need, dev);
-  char* sp = static_cast<char*>(scratch.mutable_data_ptr());
+  size_t scores_bytes = mlstm::score_scratch_bytes(p.c, false);
+  const size_t scores_at = up256(need);
   if (for_backward) out.kept = bytes(p.fw_bytes + p.inv_den_bytes, dev);
   if (for_backward && keep_states) out.states = bytes(p.states_bytes, dev);
+  const Tensor scratch = bytes_and(need, scores_bytes, dev);
+  char* sp = static_cast<char*>(scratch.mutable_data_ptr());
   char* kp = for_backward ? static_cast<char*>(out.kept.mutable_data_ptr()) : nullptr;
   p.c.stream = current_stream(dev);
   const mlstm::FwCall a{
@@ -207,11 +219,12 @@ class ChunkwiseFn : public torch::autograd::Function<ChunkwiseFn> {
     const Tensor di = empty(i.sizes(), i.scalar_type(), dev), df = empty(i.sizes(), i.scalar_type(), dev);
     const Tensor dc0 = cfg[3] >= 0 ? empty({c.B, c.NH, c.DHQK, c.DHHV}, at::kFloat, dev) : Tensor();
     const size_t ws_bytes = up256(mlstm_b200_chunkwise_workspace_bytes(c.B, c.NH, c.S, c.DHQK, c.DHHV, c.L, c.dtype, c.variant, c.impl, 1));
-    const size_t scores_bytes = mlstm::score_scratch_bytes(c, true), scores_at = up256(ws_bytes + (states.defined() ? 0 : p.states_bytes));
-    const Tensor ws = bytes(scores_at + scores_bytes, dev);
+    const Tensor rc0 = f32c(c0);
+    size_t scores_bytes = mlstm::score_scratch_bytes(c, true);
+    const size_t scores_at = up256(ws_bytes + (states.defined() ? 0 : p.states_bytes));
+    Tensor ws = bytes_and(scores_at, scores_bytes, dev);
     char* wp = static_cast<char*>(ws.mutable_data_ptr());
     const char* kp = static_cast<const char*>(kept.const_data_ptr());
-    const Tensor rc0 = f32c(c0);
     p.c.stream = current_stream(dev);
     const mlstm::BwCall a{
         ptr(q), ptr(k), ptr(v), ptr(i), ptr(f), fptr(m0), ptr(states), states.defined() ? nullptr : wp + ws_bytes,
@@ -221,6 +234,7 @@ class ChunkwiseFn : public torch::autograd::Function<ChunkwiseFn> {
     check(mlstm::run_chunkwise_bw(a, p.c), "mlstm_b200_chunkwise_bw");
     if (g_check_status && mlstm_b200_device_status(1) != 0)
       TORCH_CHECK(false, "mlstm_kernels_b200: a bounded wait of the tcgen05 kernels ran out; results invalid");
+    ws.reset();
     Tensor dc0_out, dn0, dm0;
     if (dc0.defined()) dc0_out = dc0.to((at::ScalarType)cfg[3]);
     if (cfg[4] >= 0) dn0 = at::zeros({c.B, c.NH, c.DHQK}, q.options().dtype((at::ScalarType)cfg[4]));

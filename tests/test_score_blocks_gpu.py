@@ -33,3 +33,34 @@ def test_score_blocks_equal_scores_per_tile(DHQK, DHHV, L, dtype, variant, recom
     grads = torch.autograd.grad(h, x, dh)
     for a, b in zip(grads[:3], bw[:3]):
         assert torch.equal(a, b)
+
+
+def test_a_call_that_memory_is_too_short_for_does_without_the_score_blocks():
+    """The allocator is kept (on the host) to less than the call takes with its score blocks, and to more than it needs."""
+    B, NH, S, DHQK, DHHV, L = 1, 8, 16384, 64, 64, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x = [rnd(B, NH, S, d).requires_grad_(True) for d in (DHQK, DHQK, DHHV)] + [rnd(B, NH, S).requires_grad_(True) for _ in "if"]
+    dh = rnd(B, NH, S, DHHV)
+
+    def call():
+        torch.cuda.empty_cache()
+        h = mlstm_chunkwise__b200_xl_chunk(*x, chunk_size=L, impl="simt")
+        torch.cuda.empty_cache()
+        return (h.detach(), *torch.autograd.grad(h, x, dh))
+
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    want = call()
+    most = torch.cuda.max_memory_reserved()
+    blocks = 2 * B * NH * S // L * 64 * 64 * 4     # of the backward, where the call takes most
+    want = [t.cpu() for t in want]
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((most - blocks // 2) / total)
+        got = call()
+        assert torch.cuda.max_memory_reserved() <= most
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for a, b in zip(got, want):
+        assert torch.equal(a.cpu(), b)
