@@ -178,15 +178,18 @@ step_kernel(const T* q, const T* k, const T* v, const void* gi, const void* gf, 
 //   All loads of a block before its first store to shared memory, packed multiply-adds (half the issue slots, the same
 //   roundings), the next launch started while this one drains: 20.0 / 41.1 / 558.
 //   No test of the row within the token loop where DHQK fills the rows (it kept a row's read of q and k behind the
-//   multiply-adds of the row before), two tokens unrolled: 1 x 64 41.1 -> 26.8.
+//   multiply-adds of the row before), two tokens unrolled: 1 x 64 41.1 -> 26.8.  For head dims of q and k above 128 that fill them in
+//   part, as many rows as there are, and a test of the last one or two only: 16 x 64, 16 heads 192/384 448 -> 350, 248/496 645 -> 527.
 //   At most eight rows per thread up to DHQK = 256 and sixteen up to 512, by narrower slices (see the launch): 19.0 / 26.8 /
 //   490; 8 x 16 tokens, DHQK 512: 151 -> 83.
-// Two CTAs per SM hide a good part of the chain: left to itself the compiler takes more than 128 registers for the
-// sixteen-row form, and bounded by one CTA per SM for the eight-row form too (490 -> 775).
+// Two CTAs per SM hide a good part of the chain: bounded by one, the compiler takes more than 128 registers for the eight-row form
+// too (490 -> 775).  Above DHQK = 256 the rows alone are up to 64 registers, and 128 leave 64 bytes of spills: a launch that has an
+// SM for every CTA takes all registers instead (2 x 48 tokens, 8 heads 264/256: 67.6 -> 34.8; 512/256 65.6 -> 36.9).
 constexpr int SEQ_TB = 8;
 
-template <typename T, int ROWS, int TV>
-__global__ void __launch_bounds__(STEP_THREADS, 2)
+// FULL: rows that every thread has (DHQK >= FULL * RG); CTAS: per SM
+template <typename T, int ROWS, int FULL, int TV, int CTAS>
+__global__ void __launch_bounds__(STEP_THREADS, CTAS)
 step_sequence_kernel(const T* q, const T* k, const T* v, const void* gi, const void* gf, int gate_dtype, const float* c,
                      const float* n, const float* m, T* __restrict__ h, float* __restrict__ c_new, float* __restrict__ n_new,
                      float* __restrict__ m_new, int Tn, int DHQK, int DHHV, float eps) {
@@ -303,7 +306,7 @@ step_sequence_kernel(const T* q, const T* k, const T* v, const void* gi, const v
       const float2* kq = s_kq + t * DHQK + rg;
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
-        if (decltype(full)::value || rg + r * RG < DHQK) {
+        if (r < FULL || decltype(full)::value || rg + r * RG < DHQK) {
           const float2 x = kq[r * RG];
           const uint64_t k2 = f2(x.x, x.x), q2 = f2(x.y, x.y);
           C[r][0] = fma2(ff, C[r][0], mul2(k2, vv.x));
@@ -325,7 +328,7 @@ step_sequence_kernel(const T* q, const T* k, const T* v, const void* gi, const v
       }
       if (lane < CG) *reinterpret_cast<float4*>(s_red + (t * NW + warp) * TV + cgi * 4) = hv;
     };
-    if (ROWS * RG == DHQK) {
+    if (FULL == ROWS || ROWS * RG == DHQK) {
 #pragma unroll 2
       for (int t = 0; t < nt; ++t) token(t, std::true_type());
     } else {
@@ -405,7 +408,7 @@ int launch_step(const void* q, const void* k, const void* v, const void* i, cons
   return MLSTM_ERR_DTYPE;
 }
 
-template <typename T, int ROWS, int TV>
+template <typename T, int ROWS, int FULL, int TV, int CTAS>
 int step_seq_t(const void* q, const void* k, const void* v, const void* i, const void* f, int gate_dtype, const float* c,
                const float* n, const float* m, void* h, float* c_new, float* n_new, float* m_new, int B, int NH, int Tn,
                int DHQK, int DHHV, float eps, cudaStream_t st) {
@@ -417,7 +420,7 @@ int step_seq_t(const void* q, const void* k, const void* v, const void* i, const
   // and a grid above their number shares them in any case.
   const unsigned sms = (unsigned)sm_count();
   const bool overlap = grid <= pdl_max_ctas() && (2 * grid <= sms || grid > sms || Tn <= 2 * SEQ_TB);
-  auto kern = step_sequence_kernel<T, ROWS, TV>;
+  auto kern = step_sequence_kernel<T, ROWS, FULL, TV, CTAS>;
   if (smem > 48 * 1024) MLSTM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   return launch_pdl(overlap, kern, grid, STEP_THREADS, smem, st, (const T*)q, (const T*)k, (const T*)v, i, f, gate_dtype, c, n, m,
                     (T*)h, c_new, n_new, m_new, Tn, DHQK, DHHV, eps);
@@ -432,11 +435,20 @@ int step_seq_rows(const void* q, const void* k, const void* v, const void* i, co
   // tokens, 8 heads 256/512: 157 us, 125 in 32 columns); with eight in 64 they do not, and the second preparation costs more
   // (16 x 8 tokens, 8 heads 128/256: 13.1 us, 18.6 in 32).
   const bool narrow = DHQK > 128 || (long)ceil_div(DHHV, 64) * B * NH < sm_count();
-#define SEQ_CASE(R, TV) \
+  // The form with the fewest rows that hold DHQK (up to 128 there is one for each width); at DHQK = 256 the eight-row form that also
+  // takes fewer is the faster one by 0.8 % (16 x 64 tokens, 16 heads: 499.5 and 503.5 us).
+#define SEQ_CASE(R, F, TV, CTAS) \
   if (ceil_div(DHQK, STEP_THREADS / (TV / 4)) <= R) \
-    return step_seq_t<T, R, TV>(q, k, v, i, f, gate_dtype, c, n, m, h, c_new, n_new, m_new, B, NH, Tn, DHQK, DHHV, eps, st);
-  if (narrow) { SEQ_CASE(4, 32) SEQ_CASE(8, 32) SEQ_CASE(16, 32) }
-  SEQ_CASE(4, 64) SEQ_CASE(8, 64)
+    return step_seq_t<T, R, F, TV, CTAS>(q, k, v, i, f, gate_dtype, c, n, m, h, c_new, n_new, m_new, B, NH, Tn, DHQK, DHHV, eps, st);
+  if (narrow) {
+    SEQ_CASE(4, 0, 32, 2) SEQ_CASE(5, 4, 32, 2) SEQ_CASE(6, 5, 32, 2) SEQ_CASE(7, 6, 32, 2)
+    if (DHQK == 256) { SEQ_CASE(8, 0, 32, 2) }
+    SEQ_CASE(8, 7, 32, 2)
+    if ((long)ceil_div(DHHV, 32) * B * NH <= sm_count()) { SEQ_CASE(12, 8, 32, 1) SEQ_CASE(14, 12, 32, 1) SEQ_CASE(16, 14, 32, 1) }
+    if (DHQK == 512) { SEQ_CASE(16, 16, 32, 2) }
+    SEQ_CASE(12, 8, 32, 2) SEQ_CASE(14, 12, 32, 2) SEQ_CASE(16, 14, 32, 2)
+  }
+  SEQ_CASE(4, 0, 64, 2) SEQ_CASE(8, 0, 64, 2)
 #undef SEQ_CASE
   return MLSTM_ERR_SHAPE;
 }

@@ -153,7 +153,12 @@ def test_sequence_kernel_token_blocks(B, S, DHQK, DHHV):
 
 
 @pytest.mark.parametrize("S", [17, 20])
-@pytest.mark.parametrize("B,DHQK,DHHV", [(1, 128, 64), (1, 200, 64), (2, 300, 96), (19, 128, 128), (19, 104, 128), (37, 64, 60)])
+@pytest.mark.parametrize("B,DHQK,DHHV", [(1, 128, 64), (1, 200, 64), (2, 300, 96), (19, 128, 128), (19, 104, 128), (37, 64, 60),
+                                         # the last row partly filled and filled, in the forms of five to eight rows
+                                         (2, 132, 64), (2, 160, 64), (2, 164, 40), (2, 192, 64), (2, 196, 32), (2, 224, 32), (2, 228, 32), (2, 256, 32),
+                                         # twelve to sixteen, with an SM for every CTA and without
+                                         (2, 260, 32), (2, 388, 32), (2, 452, 32), (2, 512, 32), (38, 260, 32), (38, 384, 32), (38, 388, 32),
+                                         (38, 448, 32), (38, 452, 32), (38, 512, 32)])
 def test_sequence_kernel_full_and_partly_filled_rows(B, DHQK, DHHV, S):
     """Register variants whose rows DHQK fills and does not fill, in both slice widths, over three blocks of tokens (an odd and
     an even last block, the launches of a repeated call overlapping): every call against the oracle.  f32 throughout; the
