@@ -1,15 +1,22 @@
 """Model of the recurrence kernel's protocol (csrc/chunkwise_sm100.cu, rec_body) with its two operand rings and the ring of
-gated tiles in tensor memory, run on the CPU under random interleavings: every parity wait against the true phase count,
-over-arrival, deadlock, tensor-memory tiles and accumulators overwritten under a reader, and races on the ring of chunk
-decays (vector clocks).  The depths are read from the source; the order of operations is kept next to the kernel by hand."""
+gated tiles in tensor memory, run on the CPU.
+
+Its roles hand work around rings whose barriers run on over the whole sequence (thousands of phases), every wait seeing only
+the phase PARITY: two TMA producers (the left and the right operand; one for both with 64-column tiles), two groups of four
+gating warps, the MMA thread, eight state warps, and the warp that stores the states and keeps n.  The order of waits,
+arrivals, copy issues and MMA commits of each is restated here and run under random interleavings - copies land in any order,
+commits fire in order - with every wait checked against the true phase count (a waiter two phases away from its barrier,
+early or late, is a hang or a corruption), every barrier against over-arrival, the run against deadlock, tensor-memory tiles
+and operand slots against being overwritten under a reader, and the ring of chunk decays against races: every thread
+carries a vector clock, handed on by arrivals and taken up by waits, and a read of a decay must be ordered after its write,
+the write that overwrites it after all its reads.  The depths are read from the source; the order of operations is kept next
+to the kernel by hand."""
 
 import os
 import random
 import re
 
 import pytest
-
-from test_rec_protocol_model import Bar, join
 
 SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlstm_kernels_b200", "csrc", "chunkwise_sm100.cu")
 
@@ -24,7 +31,40 @@ def depths():
     return [(int(pair[0][0]), int(pair[1][0]), *one, False), (int(pair[0][1]), int(pair[1][1]), *one, True)]
 
 
-def run(NC, do_n, store_states, seed, rings, slow=None):
+def join(into, other):
+    for a, t in other.items():
+        if into.get(a, 0) < t:
+            into[a] = t
+
+
+class Bar:
+    def __init__(self, name, count):
+        self.name, self.count, self.pending, self.phase = name, count, count, 0
+        self.clock, self.released = {}, {}    # of the arrivals of the current phase; per completed phase
+
+    def arrive(self, clock):
+        self.pending -= 1
+        assert self.pending >= 0, f"over-arrival on {self.name}"
+        join(self.clock, clock)
+        if self.pending == 0:
+            self.released = {self.phase: self.clock, self.phase - 1: self.released.get(self.phase - 1, {})}
+            self.phase += 1
+            self.pending = self.count
+            self.clock = {}
+
+    def test(self, want):
+        passes = (self.phase & 1) != (want & 1)      # what the hardware sees
+        truth = self.phase > want
+        if passes and not truth:
+            raise AssertionError(f"ALIAS early pass on {self.name}: want {want} at {self.phase}")
+        if truth and not passes:
+            raise AssertionError(f"ALIAS late wait on {self.name}: want {want} at {self.phase}")
+        return passes
+
+
+def run(NC, do_n, store_states, seed, rings, slow=None, decay_writer="left"):
+    """slow: a role that gets its turn late.  decay_writer: the lane that writes the decays, "left" being the one that arrives
+    on the stage's barrier."""
     left, right, lbuf, g_ring, joint = rings
     rnd = random.Random(seed)
     NH2 = 2 * NC
@@ -63,11 +103,11 @@ def run(NC, do_n, store_states, seed, rings, slow=None):
                 yield f"done{(h - left) % lbuf}", (h - left) // lbuf
             if h % 2 == 0:
                 for r, t in reads[s % g_ring]:
-                    assert clocks["left"].get(r, 0) >= t, f"decay of chunk {s - g_ring} overwritten before {r} is known to have read it"
+                    assert clocks[decay_writer].get(r, 0) >= t, f"decay of chunk {s - g_ring} overwritten before {r} is known to have read it"
                 if s >= g_ring:
                     assert len(reads[s % g_ring]) == 8 + do_n, "decay overwritten before it is read"
                 reads[s % g_ring].clear()
-                written[s % g_ring] = ("left", tick("left"), s)
+                written[s % g_ring] = (decay_writer, tick(decay_writer), s)
             tick("left")
             assert not joint or landed[h % right] == h - right
             loads.append((f"full{h % left}", dict(clocks["left"])))
@@ -134,12 +174,13 @@ def run(NC, do_n, store_states, seed, rings, slow=None):
     for w in range(8):
         agents[f"gate{w}"] = gating(f"gate{w}", w >> 2)
         agents[f"state{w}"] = state(f"state{w}")
-    clocks.update({a: {} for a in agents})
+    clocks.update({a: {} for a in [*agents, decay_writer]})
     blocked = {}
 
     def acquire(a, bar, phase):
         if phase >= 0:
-            join(clocks[a], B[bar].released.get(phase, {}))
+            for lane in {a, decay_writer} if a == "left" else (a,):
+                join(clocks[lane], B[bar].released.get(phase, {}))
 
     while agents:
         choices = list(agents) + (["land"] if loads else []) + (["commit"] if commits else [])
@@ -204,3 +245,19 @@ def test_a_shorter_ring_of_decays_would_race():
     with pytest.raises(AssertionError, match="decay"):
         for seed in range(50):
             run(40, False, True, seed, (left, right, lbuf, 8, joint), slow="state0")
+
+
+@pytest.mark.parametrize("left", [3, 5])
+def test_odd_left_ring_would_alias(left):
+    """With an odd number of stages a gating group returns to a stage two phases later, and its wait passes on the load before
+    the one it wants."""
+    _, right, lbuf, g_ring, _ = DEPTHS[0]
+    with pytest.raises(AssertionError, match="ALIAS early pass on full"):
+        for seed in range(400):
+            run(16, False, True, seed, (left, right, lbuf, g_ring, False), slow=("gate0", "gate5", None)[seed % 3])
+
+
+def test_decay_written_by_another_lane_than_the_arriving_one_would_race():
+    """Nothing orders another lane's write before the readers."""
+    with pytest.raises(AssertionError, match="unordered"):
+        run(4, True, True, 0, DEPTHS[0], decay_writer="another lane")
