@@ -83,34 +83,44 @@ def test_lanes_that_leave_alone_would_block_the_others():
             run(seed, "leave")
 
 
-# The waits of single threads, by their status code: the recurrence's producers and MMA thread, producer and MMA thread of the
-# intra-chunk forward, producer, MMA and E-tile thread of the intra-chunk backward, the expiry self-test; code 0 lets copies in
-# flight land on the error path.  Every other wait is a whole warp's.
-ONE_THREAD = {"101", "102", "103", "110", "111", "113", "201", "202", "203", "204", "212", "213", "215", "216", "217", "0", "code",
-              "301", "302", "303", "304", "305", "306", "307"}
+# The waits of single threads, by their status code: the MMA thread, the store thread, the intra-chunk producer, the
+# expiry self-test; code 0 lets copies in flight land on the error path.  Every other wait is a whole warp's.
+ONE_THREAD = {"102", "103", "108", "201", "202", "203", "204", "212", "213", "215", "216", "217", "0", "code"}
 
 
-def check_waits(calls):
+def test_no_lane_leaves_a_warp_alone():
+    with open(os.path.join(CSRC, "chunkwise_sm100.cu")) as f:
+        src = f.read()
+    calls = re.findall(r"^([^\n]*)\bmbar_wait\(&[^;\n]*?, (?:&g_sm100_status|nullptr), (\w+)(?:, limit)?\)([^\n]*)\n([^\n]*)",
+                       src, re.M)
+    assert len(calls) >= 25
     for before, code, after, next_line in calls:
         if code in ONE_THREAD:
             continue
         left = "break" in after or "return" in after or "break" in next_line or "return" in next_line
-        stands_by = "__syncwarp();" in next_line
+        stands_by = "stand_by(h, " in after or "__syncwarp();" in next_line
         assert stands_by or (not left and "if (!" not in before), f"wait with status code {code}"
-
-
-def test_no_lane_leaves_a_warp_alone():
-    src = ""
-    for name, status in (("chunkwise_bw_sm100.cu", "g_par_bw_status"), ("chunkwise_sm100.cu", "g_sm100_status")):
-        with open(os.path.join(CSRC, name)) as f:
-            src = f.read()
-        pattern = rf"\bmbar_wait(?:<true>)?\(&[^;\n]*?, (?:&{status}|nullptr), (\w+)(?:, limit)?\)"
-        calls = re.findall(rf"^([^\n]*){pattern}([^\n]*)\n([^\n]*)", src, re.M)
-        every = re.findall(r"\bmbar_wait(?:<true>)?\(", src)
-        assert len(re.findall(pattern, src)) == len(every) and len(calls) >= 11, name    # none is overlooked
-        check_waits(calls)
     # hand-overs to other roles depend on the wait before them
     for bar, flag in (("gated", "acc_ok"), ("accfree", r"!aborted\(smem_u32\(&sh\.abort\)\)"), (r"done\[sub & 1\]", r"!aborted\(smem_u32\(&sh\.abort\)\)")):
         assert re.findall(rf"(.*)mbar_arrive\(&sh\.bar_{bar}\)", src) == [re.search(rf" *if \({flag}\) (?=mbar_arrive\(&sh\.bar_{bar}\))", src).group(0)]
     for bar in ("out_full", "acc_free"):
         assert re.search(rf"warp_arrive\(&bar_{bar}\[\w+\], ok\)", src)
+
+
+# the same of the roles that the shipped recurrence and the intra-chunk backward have: the recurrence's producers, and producer,
+# MMA and E-tile thread of the backward
+ONE_THREAD_OF_RINGS = ONE_THREAD | {"101", "110", "111", "113", "301", "302", "303", "304", "305", "306", "307"}
+
+
+@pytest.mark.parametrize("name,status,least", [("chunkwise_sm100.cu", "g_sm100_status", 25), ("chunkwise_bw_sm100.cu", "g_par_bw_status", 11)])
+def test_no_lane_leaves_a_warp_alone_in_any_wait(name, status, least):
+    with open(os.path.join(CSRC, name)) as f:
+        src = f.read()
+    pattern = rf"\bmbar_wait(?:<true>)?\(&[^;\n]*?, (?:&{status}|nullptr), (\w+)(?:, limit)?\)"
+    calls = re.findall(rf"^([^\n]*){pattern}([^\n]*)\n([^\n]*)", src, re.M)
+    assert len(re.findall(pattern, src)) == len(re.findall(r"\bmbar_wait(?:<true>)?\(", src)) >= least    # none is overlooked
+    for before, code, after, next_line in calls:
+        if code in ONE_THREAD_OF_RINGS:
+            continue
+        left = "break" in after or "return" in after or "break" in next_line or "return" in next_line
+        assert "__syncwarp();" in next_line or (not left and "if (!" not in before), f"wait with status code {code}"

@@ -18,6 +18,8 @@ import re
 
 import pytest
 
+from test_rec_protocol_model import Bar, join
+
 SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlstm_kernels_b200", "csrc", "chunkwise_sm100.cu")
 
 
@@ -29,37 +31,6 @@ def depths():
     one = [int(re.search(rf"constexpr int {n} = (\d+);", src).group(1)) for n in ("REC_LBUF", "G_RING")]
     assert "constexpr bool JOINT = TN == 64;" in src
     return [(int(pair[0][0]), int(pair[1][0]), *one, False), (int(pair[0][1]), int(pair[1][1]), *one, True)]
-
-
-def join(into, other):
-    for a, t in other.items():
-        if into.get(a, 0) < t:
-            into[a] = t
-
-
-class Bar:
-    def __init__(self, name, count):
-        self.name, self.count, self.pending, self.phase = name, count, count, 0
-        self.clock, self.released = {}, {}    # of the arrivals of the current phase; per completed phase
-
-    def arrive(self, clock):
-        self.pending -= 1
-        assert self.pending >= 0, f"over-arrival on {self.name}"
-        join(self.clock, clock)
-        if self.pending == 0:
-            self.released = {self.phase: self.clock, self.phase - 1: self.released.get(self.phase - 1, {})}
-            self.phase += 1
-            self.pending = self.count
-            self.clock = {}
-
-    def test(self, want):
-        passes = (self.phase & 1) != (want & 1)      # what the hardware sees
-        truth = self.phase > want
-        if passes and not truth:
-            raise AssertionError(f"ALIAS early pass on {self.name}: want {want} at {self.phase}")
-        if truth and not passes:
-            raise AssertionError(f"ALIAS late wait on {self.name}: want {want} at {self.phase}")
-        return passes
 
 
 def run(NC, do_n, store_states, seed, rings, slow=None, decay_writer="left"):
