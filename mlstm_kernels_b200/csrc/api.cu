@@ -394,7 +394,7 @@ static int check_call(const CallDims& c) {
 // used to follow it.  Here the recurrence goes through the sequence in segments on a stream of the library, handing its
 // f32 state from one to the next, and the intra-chunk kernel of each finished segment runs on the caller's stream
 // beside it.  Same arithmetic in the same order, so the results are the same bits.
-// 8 heads 256/512, 131072 tokens: 2180 -> 1880 us; 65536 tokens: 1085 -> 970; 4 heads, 131072 tokens: 1573 -> 1341.
+// 8 heads 256/512, 131072 tokens: 2154 -> 1973 us; 65536 tokens: 1023 -> 935; 4 heads, 131072 tokens: 1398 -> 1140.
 static int forward_in_segments(const FwCall& a, const FwLayout& lay, const ChunkwiseDims& d, int n_seg, cudaStream_t st) {
   std::lock_guard<std::mutex> lk(g_side_mu);
   SideStream* s = side_stream_for_current_device();

@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "launch.cuh"
+#include "segments.h"
 #include "sm100.cuh"
 #include "tensor_maps.cuh"
 
@@ -992,22 +993,8 @@ static int launch_rec_tn(const CUtensorMap& mL, const CUtensorMap& mR, const CUt
   return launch_ex(ur.overlap && grid <= pdl_max_ctas(), ur.started, kern, grid, REC_THREADS, rec_smem_bytes(!BWD, TN), st, mL, mR, mS, rp);
 }
 
-// Segments of the sequence for a forward whose recurrence covers at most half of the SMs: the intra-chunk kernel of a
-// finished segment runs beside the recurrence of the next.  Estimate in microseconds, from measurements at 8 heads 256/512
-// (64 CTAs): the intra-chunk kernel alone takes 0.013 per chunk and 128 x 128 state tile; a chunk of the recurrence 1.15 with
-// 64-column tiles, 1.5 with the 128-column tiles that leave half of the SMs free; one more segment costs 15 (drain, launch,
-// refill).  What stays exposed is the last segment's intra-chunk work, which gives n = sqrt(P / 15).  Below a gain of 8 % the
-// extra launches are not worth their host time (8 heads, 32768 tokens: 522 us in one piece, 517 in four).  The score's share
-// of the intra-chunk cost does not grow with the state tiles, but the choice holds elsewhere too: 13 head geometries from
-// 64/64 to 512/1024, 1 to 32 units, 32768 to 262144 tokens, wherever it cuts the sequence: 1 to 25 % faster, none slower.
 int sm100_forward_segments(const ChunkwiseDims& d) {
-  const long c = sm100_recurrence_ctas(d);
-  if (2 * c > sm_count()) return 1;
-  const double P = 0.013 * (double)c * d.NC, slower = 4 * c <= sm_count() ? 0.0 : 0.35 * d.NC;
-  const int n = std::min(16, (int)std::lround(std::sqrt(P / 15.0)));
-  if (n < 2) return 1;
-  const double gain = P - P / n - 15.0 * (n - 1) - slower;
-  return gain > 0.08 * (P + 1.15 * d.NC) ? n : 1;
+  return forward_segments(sm100_recurrence_ctas(d), d.NC, d.B * d.NH, d.DHQK, d.DHHV, sm_count());
 }
 
 long sm100_recurrence_ctas(const ChunkwiseDims& d) {
