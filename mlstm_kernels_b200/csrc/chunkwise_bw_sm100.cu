@@ -22,10 +22,12 @@
 // so that an item is gated while its inter-chunk products run, a tile is scaled while the next product runs, and the epilogue
 // of a tile runs beside the next tile's products.
 //
-// What bounds it: the shared-memory port (128 bytes per cycle).  Every operand byte is written there by TMA and read by the
-// MMA, a 128 x 128 x 16 product of two shared operands by itself asks for the port's full rate, and E and the output pass
-// through it too: 1.15 MB per item at 256/256, 9200 of the 11000 cycles an item takes; HBM is at 0.8 of the copy rate
-// then.  (Before, one CTA per chunk and mode, two to an SM, each a chain of dependent steps: 8 x 8192 tokens, 16 heads
+// What bounds it: HBM and the shared memory together.  Every operand byte is written to shared memory by TMA and read by the
+// MMA, and E and the output pass through it too: 1.15 MB per item at 256/256, 9200 of the 11000 cycles that an item takes at 128 bytes
+// per cycle, the rate that a 128 x 128 x 16 product of two shared operands asks for by itself.  Counters (2 x 8192 tokens, 16 heads
+// 256/256, 260 us): 1.15 MB read and written per item (22 % of the banks' peak each way, which the counter puts at 256 bytes per
+// cycle), tensor pipe busy 43 % of the cycles, 1.46 GB from and to HBM, 0.86 of the copy rate.
+// (Before, one CTA per chunk and mode, two to an SM, each a chain of dependent steps: 8 x 8192 tokens, 16 heads
 // 256/256 1302 us, now 1089; 16 x 2048, 128/256 431, now 342; 4 x 1024, 4 heads 96/192 22.9, now 20.9.)
 // Measured and not taken: an accumulator of 256 columns (A read once for two tiles, 10 % less port traffic, but nothing left to
 // overlap the epilogue with: 1260 and 440 us where this form then took 1130 and 351); the modes of one chunk in one CTA (the 148 chunks in flight no longer fit

@@ -758,8 +758,9 @@ static ParArgs<T> par_args(const void* q, const void* k, const void* v, const Ga
   return MLSTM_ERR_DTYPE;
 
 // Scratch for the score blocks of a forward (one product) or a backward (two); 0 where they are not used.  A chunk of 64 or 128
-// tokens has one or three blocks of 16 KB, used by every output tile of it.  Shorter chunks would mostly store padding, longer
-// ones and small head dims would need more room than their states.
+// tokens has one or three blocks of 16 KB, used by every output tile of it.  Shorter chunks would mostly store padding.  Longer
+// ones and small head dims would need more room than what the call has for states anyway: one set of blocks beside the
+// forward's states, two beside the backward's states and state gradients.
 size_t simt_score_bytes(const ChunkwiseDims& d, bool backward) {
   if ((d.L != TILE && d.L != 2 * TILE) || d.DHQK * d.DHHV < score_pairs(d.L) * TILE * TILE) return 0;
   return (size_t)(backward ? 2 : 1) * d.B * d.NH * d.NC * score_pairs(d.L) * TILE * TILE * sizeof(float);

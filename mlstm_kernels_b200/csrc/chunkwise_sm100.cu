@@ -431,7 +431,7 @@ rec_pair_sm100(const __grid_constant__ CUtensorMap mL, const __grid_constant__ C
 //   G[r,c] = gate(r,c) * (Q[r,:] . K[c,:]),   gate = s * exp((b_r - b_c) + iota_c - m_r)
 // grid (ceil(DHHV / 128 / PAR_MAXSUB), NC, B*NH), two CTAs per SM; 320 threads: warp 0 TMA, warp 1 MMA, warps 2..9
 // element-wise (two warps per 32-row quarter of the tile, each owning two 32-column chunks).  One CTA produces up to
-// PAR_MAXSUB neighbouring output tiles of its chunk and mode, one after the other, from a single score tile.
+// PAR_MAXSUB neighbouring output tiles of its chunk, one after the other, from a single score tile.
 // Time line of a CTA's first tile (measured with time stamps at the benchmark size, two CTAs sharing an SM): first
 // slices land after ~1.8 us, score complete ~3.3 us, gating until ~5 us with the inter-chunk product arriving
 // underneath (~5.5 us), second product ~6.4 us, epilogue and stores until ~8.8 us; every further tile takes ~5.5 us.
@@ -529,7 +529,7 @@ par_body(const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* ma
   // Ring loads, in order: ND (A, B) slice pairs for the score product, ND (A, state) slice pairs for the inter-chunk
   // product (A comes from L2 the second time), the X tile.  The score is complete - and the element-wise
   // warps start gating - while the second group is still arriving.
-  // A CTA produces `nsub` (1 .. PAR_MAXSUB) neighbouring 128-column output tiles of the same chunk and mode.  The
+  // A CTA produces `nsub` (1 .. PAR_MAXSUB) neighbouring 128-column output tiles of the same chunk.  The
   // score tile and its gated form are the same for all of them, so every tile after the first only needs its own
   // state slices and X tile: the gated tile stays in tensor memory, the accumulator is reused once the previous
   // tile's epilogue has read it.
@@ -880,8 +880,8 @@ par_body(const CUtensorMap* mapA, const CUtensorMap* mapB, const CUtensorMap* ma
   tc_fence_before_sync();
   __syncthreads();
   const bool go_on = sh.abort == 0;   // (the next run sets it to the 0 that it is)
-  // Whichever role gave up: the copies in flight land before the CTA retires.  (Where the producer waits for them on every
-  // way out, as in the recurrence, its polling costs the backward 2 %.)
+  // Whichever role gave up: the copies in flight land before the CTA retires.  (On the abort flag alone: a producer that waited for
+  // them on every way out, as in the recurrence, would poll while the other roles still work.)
   if (tid == 0 && !go_on)
     for (int ld = max(0, sh.issued - PAR_NST); ld < sh.issued; ++ld)
       mbar_wait(&sh.bar_full[ld % PAR_NST], (ld / PAR_NST) & 1, nullptr, nullptr, 0);

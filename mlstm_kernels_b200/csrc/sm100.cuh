@@ -155,16 +155,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 //   K-major operand  : rows of 64 bf16 (128 B); 8-row groups 1024 B apart (SBO); LBO unused.
 //   MN-major operand : 64-element (128 B) runs along M/N; K rows 128 B apart inside an 8-row group,
 //                      groups SBO bytes apart; the next 64-wide M/N block LBO bytes away.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1 << 46;  // version
-  d |= (uint64_t)2 << 61;  // SWIZZLE_128B
-  return d;
-}
-// The same in two words, for issuing threads that go from operand to operand by adding (bytes >> 4) to the low one: a single
+// In two words, for issuing threads that go from operand to operand by adding (bytes >> 4) to the low one: a single
 // thread issues all products of a CTA, and putting a descriptor together anew for each costs it more than the issue.
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr & 0x3FFFFu) >> 4) | (lbo_bytes >> 4) << 16; }
 constexpr uint32_t umma_desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | 1u << 14 | 2u << 29; }
